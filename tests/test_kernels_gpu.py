@@ -1225,3 +1225,44 @@ def test_sampling_at_random_rows():
             between = p[lo:hi + 1].sum().item() - max(p[lo].item(), p[hi].item())
             assert between <= 1e-5, (
                 f"seed {seed}, {kind}, row {r}: kernel {got[r]}, plain {want[r]} with mass {between:.2e} between them")
+
+
+@pytest.mark.parametrize("V", [1, 3, 4095, 4097, 16388, 32769, 65537, 131075, 262144, 262180])
+def test_sampling_over_cluster_sizes(V):
+    """Vocabularies around every border of the sampling kernel's layout (one block, a cluster, the groups a thread holds, rows
+    read again beyond what a cluster holds), rows at odd strides, top-k and top-p on and off, masked (-inf) logits, greedy rows
+    among the others. The kernel sums in float32 (relative error below 1e-5 for these sizes), the plain sampler in float64: where
+    they differ, the plain draw's mass position must lie within 1e-5 of the border of the kernel's token."""
+    g = torch.Generator().manual_seed(V)
+    R = 5
+    wide = (3.0 * torch.randn(R, V + 3, generator=g)).float()
+    for off in (0, 3):                              # 3: the rows begin off a 16-byte border
+        logits = wide[:, off:off + V]
+        if V > 8:
+            logits[1, ::3] = -math.inf
+            logits[2, V // 2] = 60.0
+        dl = wide.to(DEV)[:, off:off + V]
+        seed = torch.arange(R, dtype=torch.int64, device=DEV) * 977 + 13
+        ctr = torch.arange(R, dtype=torch.int64, device=DEV)
+        for temps, k, p in (([0.7, 1.0, 0.6, 0.0, 1.5], 0, 0.9), ([1.0] * 5, 40, 0.95), ([0.8] * 5, 0, 1.0)):
+            out = torch.full((R,), -1, dtype=torch.int32, device=DEV)
+            ops().sample(dl, out, temperature=torch.tensor(temps, device=DEV), top_k=torch.full((R,), k, dtype=torch.int32, device=DEV),
+                         top_p=torch.full((R,), p, device=DEV), seed=seed, counter=ctr)
+            for r in range(R):
+                x, T, got = logits[r], temps[r], int(out[r])
+                if not T > 0:
+                    assert got == plain_llama.sample(x)
+                    continue
+                w = torch.exp((x - x.max()).double() / T)
+                order = torch.sort(x, descending=True).values
+                keep = x >= order[k - 1] if 0 < k < V else torch.ones(V, dtype=torch.bool)
+                if p < 1.0:
+                    ordered = torch.sort(torch.where(keep, x, torch.tensor(-math.inf)), descending=True).values
+                    mass = torch.cumsum(torch.exp((ordered - x.max()).double() / T), 0)
+                    at = min(int((mass < p * mass[-1]).sum()), V - 1)
+                    keep &= x >= ordered[at]
+                assert bool(keep[got]), (V, off, r)
+                c = torch.cumsum(torch.where(keep, w, torch.zeros_like(w)), 0)
+                u = plain_llama.uniform01(int(seed[r]), int(ctr[r])) * float(c[-1])
+                slack = 1e-5 * float(c[-1])
+                assert (float(c[got - 1]) if got else 0.0) - slack <= u < float(c[got]) + slack, (V, off, r, T, k, p)
