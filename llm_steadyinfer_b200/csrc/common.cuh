@@ -74,17 +74,22 @@ __device__ __forceinline__ void set_status(int* status, int code) {
   if (status) atomicMax(status, code);
 }
 
-// Programmatic dependent launch: a kernel that starts with pdl_prologue() lets the next kernel of
-// the stream begin launching while it still runs, and itself waits for the previous kernel's
-// results before touching any memory. Launched through si_launch() the kernel carries the
-// attribute that allows this overlap of launch latency; launched with <<<>>> both instructions
-// do nothing. SI_PDL=0 in the environment turns the attribute off.
-__device__ __forceinline__ void pdl_prologue() {
-#ifdef SI_PDL_EARLY_TRIGGER
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-#endif
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+// Programmatic dependent launch: a kernel launched through si_launch() carries the attribute that lets its launch overlap the end
+// of the kernel before it; it waits for that kernel's results (pdl_wait, or pdl_prologue at its start) before it touches what
+// others write. Launched with <<<>>> the instruction does nothing. SI_PDL=0 in the environment turns the attribute off.
+//
+// Loads through the read-only path (ld.global.nc, which the compiler also makes of const __restrict__ pointers) may be moved across
+// the wait by the assembler, since nothing in this kernel writes there: a product's rows were read so before the kernel before had
+// written them. Behind a branch on a value that comes with the wait they stay: a load is not made before it is known that it is to be.
+__device__ __forceinline__ void pdl_wait() {
+  unsigned sms;
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%nsmid;\n" : "=r"(sms) :: "memory");
+  if (sms == 0u) {                       // never
+    asm volatile("exit;\n");
+    __builtin_unreachable();
+  }
 }
+__device__ __forceinline__ void pdl_prologue() { pdl_wait(); }
 
 // A hint that [base, base + bytes) will be streamed soon: block `part` of `parts` asks the memory system
 // to bring its share into L2, one prefetch per 128-byte line. Kernels that wait on latency while HBM
@@ -99,13 +104,12 @@ __device__ __forceinline__ void l2_prefetch_share(const void* base, long long by
     asm volatile("prefetch.global.L2 [%0];\n" :: "l"(reinterpret_cast<const char*>(base) + c * LINE) : "memory");
 }
 
-// The two halves of pdl_prologue() for kernels that place them themselves. A small kernel (a norm, the
+// For kernels that let the next one launch early. A small kernel (a norm, the
 // position encoding) calls pdl_trigger() at its start: the kernel after it may then become resident and do
 // whatever does not depend on this one (set-up, the first loads of its weights) before its own pdl_wait().
 // Kernels of more than one wave do not trigger: blocks of the next kernel that sit waiting would take the
 // places of their own later blocks.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
 // SI_PDL_TRIGGER: 0 no kernel triggers; 1 the small kernels; 2 (default) also every kernel of one wave of
 // blocks, at its start; 3 also kernels of several waves, once their main loop is done.
