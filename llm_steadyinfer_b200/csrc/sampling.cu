@@ -399,6 +399,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
   cg::cluster_group cl = cg::this_cluster();
   const int blocks = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int r = blockIdx.x / blocks, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  cl.barrier_arrive();                   // waited for before the first store into another block's memory
   pdl_prologue();
   const float* x = logits + (size_t)r * row_stride;
   const int first = rank * per_block, end = min(vocab, first + per_block);     // this block's logits
@@ -439,6 +440,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
   least = -warp_max(-least);
   if (lane == 0) { sm.red[0][warp] = best; sm.red[1][warp] = __int_as_float(best_i); sm.red[2][warp] = least; }
   __syncthreads();
+  cl.barrier_wait();
   int turn = 0;
   if (warp == 0) {
     best = lane < SC_WARPS ? sm.red[0][lane] : -INFINITY;
