@@ -56,6 +56,9 @@ __device__ __forceinline__ void mma16816(float (&d)[4], unsigned a0, unsigned a1
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+struct true_type { static constexpr bool value = true; };
+struct false_type { static constexpr bool value = false; };
+
 template <typename TO> __device__ __forceinline__ void store_out(TO* p, float v);
 template <> __device__ __forceinline__ void store_out<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void store_out<bf16>(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
@@ -66,9 +69,9 @@ __device__ __forceinline__ uint4 ld_stream(const bf16* p) {      // weights: rea
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
-__device__ __forceinline__ uint4 ld_cached(const bf16* p) {      // x: small, shared by every block
+__device__ __forceinline__ uint4 ld_cached(const bf16* p) {      // x: small, shared by every block; written by the kernel before: not by the read-only path
   uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
 
@@ -96,79 +99,62 @@ gemm_skinny_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __rest
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
 
-  const int full = K >> 5;                      // whole 32-wide chunks
-  int c = warp;
+  const int full = K >> 5, nchunks = (K + 31) >> 5;      // whole 32-wide chunks; with the part of one (K is a multiple of 8)
   const bf16* xr[MT];
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) xr[mt] = x + (size_t)(mt * 8 + g < M ? mt * 8 + g : 0) * ldx + t * 8;
+  // UNROLL chunks of a warp with all their loads in flight. A round that is not whole (ALL false) loads only what is there: lanes
+  // past the end feed zeros, and every lane of the warp issues the same mma (mma.sync must not sit in a divergent branch).
+  // (A tail of single chunks instead, a round trip to memory each: two rows and K = 704, 1,408 and 2,816 took
+  // 3.5, 4.0 and 5.9 us, so 2.7, 3.3 and 5.3; K = 4,096, whole rounds, 6.0 either way)
   // The weights do not depend on the kernel before this one: the first round of their loads is in flight
   // before this kernel waits for that kernel's results (x).
+  auto round = [&](int c, bool first, auto all) {
+    constexpr bool ALL = decltype(all)::value;
+    constexpr int U = ALL || MT == 1 ? UNROLL : UNROLL / 2;      // (two row tiles and the tests: half the loads fit the registers)
+    uint4 a_lo[U], a_hi[U], xb[U][MT];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (c + u * WARPS) * 32;
+      if (!ALL) a_lo[u] = a_hi[u] = make_uint4(0, 0, 0, 0);
+      if (ALL || k + t * 8 < K) {
+        a_lo[u] = ld_stream(w0 + k);
+        a_hi[u] = ld_stream(w1 + k);
+      }
+    }
+    if (first) pdl_wait();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (c + u * WARPS) * 32;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        if (!ALL) xb[u][mt] = make_uint4(0, 0, 0, 0);
+        if (ALL || k + t * 8 < K) xb[u][mt] = ld_cached(xr[mt] + k);
+      }
+    }
+    if (!ALL) __syncwarp();
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (ALL || c + u * WARPS < nchunks) {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          mma16816(acc[mt], a_lo[u].x, a_hi[u].x, a_lo[u].y, a_hi[u].y, xb[u][mt].x, xb[u][mt].y);
+          mma16816(acc[mt], a_lo[u].z, a_hi[u].z, a_lo[u].w, a_hi[u].w, xb[u][mt].z, xb[u][mt].w);
+        }
+      }
+  };
+  constexpr int STEP = WARPS * (MT == 1 ? UNROLL : UNROLL / 2);
+  int c = warp;
   if (c + (UNROLL - 1) * WARPS < full) {
-    uint4 a_lo[UNROLL], a_hi[UNROLL], xb[UNROLL][MT];
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u) {
-      const int k = (c + u * WARPS) * 32;
-      a_lo[u] = ld_stream(w0 + k);
-      a_hi[u] = ld_stream(w1 + k);
-    }
-    pdl_wait();
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u) {
-      const int k = (c + u * WARPS) * 32;
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) xb[u][mt] = ld_cached(xr[mt] + k);
-    }
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u)
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        mma16816(acc[mt], a_lo[u].x, a_hi[u].x, a_lo[u].y, a_hi[u].y, xb[u][mt].x, xb[u][mt].y);
-        mma16816(acc[mt], a_lo[u].z, a_hi[u].z, a_lo[u].w, a_hi[u].w, xb[u][mt].z, xb[u][mt].w);
-      }
+    round(c, true, true_type());
     c += WARPS * UNROLL;
+    for (; c + (UNROLL - 1) * WARPS < full; c += WARPS * UNROLL) round(c, false, true_type());
   } else {
-    pdl_wait();
-  }
-  for (; c + (UNROLL - 1) * WARPS < full; c += WARPS * UNROLL) {
-    uint4 a_lo[UNROLL], a_hi[UNROLL], xb[UNROLL][MT];
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u) {
-      const int k = (c + u * WARPS) * 32;
-      a_lo[u] = ld_stream(w0 + k);
-      a_hi[u] = ld_stream(w1 + k);
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) xb[u][mt] = ld_cached(xr[mt] + k);
-    }
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u)
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        mma16816(acc[mt], a_lo[u].x, a_hi[u].x, a_lo[u].y, a_hi[u].y, xb[u][mt].x, xb[u][mt].y);
-        mma16816(acc[mt], a_lo[u].z, a_hi[u].z, a_lo[u].w, a_hi[u].w, xb[u][mt].z, xb[u][mt].w);
-      }
+    round(c, true, false_type());        // (also where a warp has no chunk at all: it waits like the others)
+    c += STEP;
   }
   if (trigger == 2) pdl_trigger();
-  // what is left: whole chunks one at a time, then the part of a chunk (K is a multiple of 8).
-  // Lanes past the end load nothing and feed zeros; every lane of the warp issues the same mma
-  // (mma.sync must not sit in a divergent branch).
-  const int nchunks = (K + 31) >> 5;
-  for (; c < nchunks; c += WARPS) {
-    const int k = c * 32;
-    const bool in = k + t * 8 < K;
-    uint4 lo = make_uint4(0, 0, 0, 0), hi = lo, xv[MT];
-    if (in) { lo = ld_stream(w0 + k); hi = ld_stream(w1 + k); }
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      xv[mt] = make_uint4(0, 0, 0, 0);
-      if (in) xv[mt] = ld_cached(xr[mt] + k);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      mma16816(acc[mt], lo.x, hi.x, lo.y, hi.y, xv[mt].x, xv[mt].y);
-      mma16816(acc[mt], lo.z, hi.z, lo.w, hi.w, xv[mt].z, xv[mt].w);
-    }
-  }
+  for (; c < nchunks; c += STEP) round(c, false, false_type());
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll

@@ -1266,3 +1266,13 @@ def test_sampling_over_cluster_sizes(V):
                 u = plain_llama.uniform01(int(seed[r]), int(ctr[r])) * float(c[-1])
                 slack = 1e-5 * float(c[-1])
                 assert (float(c[got - 1]) if got else 0.0) - slack <= u < float(c[got]) + slack, (V, off, r, T, k, p)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 48, 8), (3, 40, 264), (8, 96, 1408), (9, 64, 1416), (16, 128, 2816), (8, 64, 5632), (2, 5000, 768)])
+def test_few_row_product_at_ragged_k(M, N, K):
+    """The few-row product where k fills no whole round of a block's loads, against float64 (fp32 sums of K products)."""
+    g = torch.Generator().manual_seed(K + M)
+    x, w = torch.randn(M, K, generator=g).to(torch.bfloat16), (torch.randn(N, K, generator=g) / K ** 0.5).to(torch.bfloat16)
+    out = torch.full((M, N), 7.0, device=DEV)
+    ops().gemm_skinny(x.to(DEV), w.to(DEV), out)
+    assert (out.cpu().double() - x.double() @ w.double().t()).abs().max().item() <= 1e-5
