@@ -21,6 +21,7 @@ __global__ void rope_kv_write_kernel(T* __restrict__ qkv, long long row_stride,
                                      T* __restrict__ k_cache, T* __restrict__ v_cache,
                                      int num_pages, int page_size, int num_seqs, int H, int KV,
                                      int hs, int hpb, int* status) {
+  pdl_prologue();
   const int t = blockIdx.x;
   const int pos = positions[t];
   const int seq = row_seq[t];
@@ -205,12 +206,12 @@ SI_EXPORT int si_rope_kv_write(void* qkv, int dtype, long long row_stride, const
     return si_last_error();
   }
   if (dtype == SI_BF16)
-    rope_kv_write_kernel<__nv_bfloat16><<<grid, threads, 0, stream>>>(
+    si_launch(rope_kv_write_kernel<__nv_bfloat16>, grid, dim3(threads), 0, stream,
         (__nv_bfloat16*)qkv, row_stride, positions, row_seq, inv_freq, rot_dim, block_table,
         table_width, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, num_pages, page_size,
         num_seqs, H, KV, hs, hpb, status);
   else
-    rope_kv_write_kernel<float><<<grid, threads, 0, stream>>>(
+    si_launch(rope_kv_write_kernel<float>, grid, dim3(threads), 0, stream,
         (float*)qkv, row_stride, positions, row_seq, inv_freq, rot_dim, block_table, table_width,
         (float*)k_cache, (float*)v_cache, num_pages, page_size, num_seqs, H, KV, hs, hpb, status);
   return si_last_error();

@@ -44,6 +44,7 @@ __global__ void swiglu_vec_bf16_kernel(const __nv_bfloat16* __restrict__ gu, __n
 
 __global__ void swiglu_vec_f32_kernel(const float* __restrict__ gu, float* __restrict__ out, int F, int group,
                                       long long total_chunks) {
+  pdl_prologue();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total_chunks) return;
   const int cpr = F >> 2;
@@ -70,7 +71,7 @@ SI_EXPORT int si_swiglu(const void* gu, void* out, int dtype, int num_tokens, in
               (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, F, group, chunks);
   } else if (dtype == SI_F32 && aligned && group % 4 == 0) {
     const long long chunks = total / 4;
-    swiglu_vec_f32_kernel<<<(unsigned)((chunks + threads - 1) / threads), threads, 0, stream>>>(
+    si_launch(swiglu_vec_f32_kernel, dim3((unsigned)((chunks + threads - 1) / threads)), dim3(threads), 0, stream,
         (const float*)gu, (float*)out, F, group, chunks);
   } else {
     const unsigned blocks = (unsigned)((total + threads - 1) / threads);

@@ -1276,3 +1276,17 @@ def test_few_row_product_at_ragged_k(M, N, K):
     out = torch.full((M, N), 7.0, device=DEV)
     ops().gemm_skinny(x.to(DEV), w.to(DEV), out)
     assert (out.cpu().double() - x.double() @ w.double().t()).abs().max().item() <= 1e-5
+
+
+@pytest.mark.parametrize("M,N,K", [(700, 1000, 96), (641, 961, 68), (705, 1001, 33)])
+def test_gemm_f32_over_both_tiles(M, N, K):
+    """Enough tiles of 64 x 64 for every SM, rows of 16-byte words and not: against float64 (K fp32 sums of products of size one), and a
+    row by itself, which takes the smaller tiles, to the same bits."""
+    g = torch.Generator().manual_seed(K)
+    a, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    out, one = torch.empty(M, N, device=DEV), torch.empty(1, N, device=DEV)
+    ops().gemm_f32(a, w, out)
+    assert (out.double() - a.double() @ w.double().T).abs().max().item() <= 1e-6 * K * 4
+    for m in (0, 63, M - 1):
+        ops().gemm_f32(a[m:m + 1], w, one)
+        assert torch.equal(one[0], out[m])
