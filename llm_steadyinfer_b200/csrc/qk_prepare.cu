@@ -65,7 +65,7 @@ __device__ __forceinline__ void norm_rotate_vector(const T* __restrict__ src, T*
 }
 
 template <typename T, int ITEMS>
-__global__ void __launch_bounds__(256) qk_prepare_kernel(T* __restrict__ rows, long long row_stride, const float* __restrict__ q_w,
+__global__ void __launch_bounds__(1024) qk_prepare_kernel(T* __restrict__ rows, long long row_stride, const float* __restrict__ q_w,
     const float* __restrict__ k_w, float eps, const float* __restrict__ inv_freq, int rd, int interleaved,
     const int* __restrict__ positions, const int* __restrict__ row_seq, const int* __restrict__ block_table, int table_width,
     T* __restrict__ k_cache, T* __restrict__ v_cache, int num_pages, int page_size, int num_seqs, int NQ, int NK, int NV,
@@ -103,8 +103,14 @@ __global__ void __launch_bounds__(256) qk_prepare_kernel(T* __restrict__ rows, l
   float inv_q = -1.f, inv_k = -1.f;
   if (whole) {                                       // one norm over all of the row's q vectors, one over all its k vectors
     float sq = 0.f, sk = 0.f;
-    for (int i = threadIdx.x; i < NQ * dk; i += blockDim.x) { const float x = to_f32<T>(row[i]); sq = fmaf(x, x, sq); }
-    for (int i = threadIdx.x; i < NK * dk; i += blockDim.x) { const float x = to_f32<T>(row[(size_t)NQ * dk + i]); sk = fmaf(x, x, sk); }
+    // (256 threads whatever the block, so that a row's sums have one order)
+    const int n = min((int)blockDim.x, 256);
+    if (threadIdx.x < n) {
+#pragma unroll 8
+      for (int i = threadIdx.x; i < NQ * dk; i += n) { const float x = to_f32<T>(row[i]); sq = fmaf(x, x, sq); }
+#pragma unroll 4
+      for (int i = threadIdx.x; i < NK * dk; i += n) { const float x = to_f32<T>(row[(size_t)NQ * dk + i]); sk = fmaf(x, x, sk); }
+    }
     inv_q = q_w ? rsqrtf(block_sum(sq, red) / (float)(NQ * dk) + eps) : 1.f;
     inv_k = k_w ? rsqrtf(block_sum(sk, red) / (float)(NK * dk) + eps) : 1.f;
   }
@@ -142,8 +148,13 @@ SI_EXPORT int si_qk_prepare(void* rows, int dtype, long long row_stride, const f
   if (dk <= 0 || dk > 640 || rd < 0 || rd > dk || rd % 2 || (rd > 0 && !inv_freq)) return -2;
   if (maps < 1 || NK <= 0 || NQ % NK || NK % maps || (maps > 1 && q_out == rows)) return -2;
   const size_t smem = (size_t)(rd > 0 ? rd : 1) * sizeof(float);
-  // a warp a vector at a time; eight warps where there are vectors for them, so that a row's loads are in flight together
-  const dim3 grid(num_tokens), block(NQ + NK >= 8 ? 256 : 128);
+  // a warp a vector at a time; eight warps where there are vectors for them, so that a row's loads are in flight together; a warp
+  // for every vector, up to 32, while the rows are no more than the SMs: a vector is a chain of a load, a sum over the warp and a
+  // store, and a decode row waits for as many of them as its warps take in turn (four rows, 20
+  // vectors of 128: eight warps 13.6 us, a warp each 9.7)
+  int threads = NQ + NK >= 8 ? 256 : 128;
+  if (num_tokens <= si_sm_count() && NQ + NK > 8) threads = NQ + NK >= 32 ? 1024 : (NQ + NK + 7) / 8 * 256;
+  const dim3 grid(num_tokens), block(threads);
 #define QK_LAUNCH(T, ITEMS)                                                                                              \
   si_launch(qk_prepare_kernel<T, ITEMS>, grid, block, smem, stream, (T*)rows, row_stride, q_w, k_w, eps, inv_freq, rd,      \
             interleaved, positions, row_seq, block_table, table_width, (T*)k_cache, (T*)v_cache, num_pages, page_size,   \
