@@ -25,10 +25,20 @@
 // Keys and values narrower than a tile's columns (multiples of 8): the tensor maps end at their sizes, so the boxes' further
 // columns arrive as zeros; the queries are padded likewise and results beyond the value size are not stored.
 //
+// Instances: key size in NK halves of 64 columns (1 to 3), value size in NV (1 or 2); values beyond NV halves go to further blocks
+// (blockIdx.z), which make the scores again. With 192-wide keys the values have one stage, so that all fits shared memory. MODE
+// says what a score gets beside its scale: nothing, the extended form (slopes by distance, a query temperature, an output gate), a
+// bias by distance from a table, or a soft limit (see AttnExtras). All of it is fp32 arithmetic on the scores in registers, which
+// costs issue slots of the softmax threads: they, and their exponentials, bound the kernel, not the tensor cores.
+// Measured, a portion of 2,000 to 2,048 tokens, 16 query heads, in place of the mma.sync kernel: bias by distance 291 -> 62 us, 192-wide
+// latent keys 291 -> 51, a soft limit over 64-wide keys and 128-wide values 225 -> 46, four key heads a value head 264 -> 63. Keys of
+// one item cut over blocks (2,043 tokens at the end of 16,128, 24 query and 8 key heads, where 200 blocks were 1.4 waves of SMs): 564 ->
+// 457 us and 18 for the merge.
+//
 // The reference computes prompt attention row by row with its scalar split kernel
-// (src/source/op/kernels/cuda/paged_kernels.cu:96-206). Conditions here: key and value sizes up to 128, multiples of 8
-// (the extended instance: 64 or 128, both alike), page size
-// a power of two from 8 to 64, G <= 128; other layouts use the mma.sync kernel. Every mbarrier wait
+// (src/source/op/kernels/cuda/paged_kernels.cu:96-206). Conditions here: key sizes up to 192 and value sizes in multiples of 8
+// (the extended instance: 64 or 128, both alike), page size a power of two from 8 to 64 (or keys of one sequence in neighbouring
+// rows of a matrix, `dense`), G <= 128; other layouts use the mma.sync kernel. Every mbarrier wait
 // is bounded; when one runs out the block sets SI_WAIT_LIMIT and leaves without storing.
 #include "attention_common.cuh"
 #include "tma_common.cuh"
@@ -67,36 +77,72 @@ __device__ __forceinline__ bf16* half_ptr(bf16* base, int row, int chunk) {
   return base + (size_t)(chunk >> 3) * (NROWS * 64) + (size_t)row * 64 + (((chunk & 7) ^ (row & 7)) << 3);
 }
 
-// What the extended form (EXT) adds to a score and to the result, all fp32 arithmetic in the softmax threads:
-//   score(i, j) = scale * t(i) * q.k - slope[h] * (i - j),  t(i) = 1 + qt_coef * ln(floor((i + 1) / qt_every) + 1)  (qt_every 0: t = 1)
-//   result(i, h, d) *= sigmoid(gate[i, h * hs + d])   (gate null: none)
+// What a MODE adds to a score and to the result, all fp32 arithmetic in the softmax threads:
+//   EXT   score(i, j) = scale * t(i) * q.k - slope[h] * (i - j),  t(i) = 1 + qt_coef * ln(floor((i + 1) / qt_every) + 1)  (qt_every 0: t = 1)
+//         result(i, h, d) *= sigmoid(gate[i, h * hs + d])   (gate null: none)
+//   BIAS  score(i, j) = scale * q.k + bias[min(i - j, nd - 1), h]
+//   CAP   score(i, j) = cap * tanh(scale * q.k / cap)
+enum { MODE_PLAIN = 0, MODE_EXT = 1, MODE_BIAS = 2, MODE_CAP = 3 };
 struct AttnExtras {
   const float* slopes;                           // fp32 [H] or nullptr
   float qt_coef; int qt_every;
   const bf16* gate; long long gate_stride;       // rows 16-byte aligned
+  const float* bias; int nd;                     // fp32 [nd, H]
+  float cap_log2, scale_over_cap;                // cap * log2(e), scale / cap
+  int v_share;                                   // key heads that read one value head
+  int out_f32;                                   // p.out is fp32
+  int dense;                                     // keys and values [rows, KV * size]: a sequence's rows lie behind its table's first entry
+  // MODE_PLAIN, one block of values: an item's keys may be cut into shares, a block each. Entry (item, share, shares of the item, slot of
+  // its first share's partial results); a whole item has one share. Shares leave O, maximum and sum per row; a second kernel merges.
+  const int4* shares;
+  float* part_o;                                 // [slot][KV][256 rows][NV * 64]
+  float* part_ml;                                // [slot][KV][256 rows][2]
 };
 
-template <int NH, bool EXT>
+// Floats of a bias window in shared memory: the distances that a query tile's rows have to a key tile's keys, per head. The
+// pitch puts the lanes of a warp (G heads of neighbouring tokens) into different banks.
+__host__ __device__ __forceinline__ int bias_pitch(int G) { return (128 / G + 128 + 31) / 32 * 32 + (G < 32 ? 32 / G : 0); }
+
+// tanh for |z| <= 1/2: z + z^3 q(z^2), q a degree-3 polynomial fitted at Chebyshev points; absolute error 6e-8 in fp32 (the
+// quotient form below: 1.2e-7). Two at a time.
+__device__ __forceinline__ unsigned long long mul_f32x2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long tanh_small_f32x2(unsigned long long z) {
+  const unsigned long long c3 = pack_f32x2(0.017993388697504997f, 0.017993388697504997f), c2 = pack_f32x2(-0.053373366594314575f, -0.053373366594314575f),
+                           c1 = pack_f32x2(0.1333010345697403f, 0.1333010345697403f), c0 = pack_f32x2(-0.33333292603492737f, -0.33333292603492737f);
+  const unsigned long long u = mul_f32x2(z, z);
+  const unsigned long long q = fma_f32x2(fma_f32x2(fma_f32x2(c3, u, c2), u, c1), u, c0);
+  return fma_f32x2(z, mul_f32x2(u, q), z);
+}
+
+template <int NK, int NV, int MODE>
 __global__ void __launch_bounds__(320)
 attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap,
                          const __grid_constant__ CUtensorMap vmap, int log2_page, const AttnExtras x) {
-  constexpr int BM = 128, BN = 128, HS = NH * 64, STAGES = 2;
-  constexpr int TILE = NH * BN * 64;                 // elements of a K (or V) tile: NH halves of [128][64]
-  constexpr int TM_S = 0, TM_O = 2 * BN;             // tensor-memory columns: S of tile q at TM_S + q*BN, O at TM_O + q*HS
+  constexpr bool EXT = MODE == MODE_EXT;
+  constexpr int BM = 128, BN = 128, DK = NK * 64, DV = NV * 64, STAGES = 2, VST = NK > 2 ? 1 : 2;
+  constexpr int KTILE = NK * BN * 64, VTILE = NV * BN * 64;      // elements of a tile: halves of [128][64]
+  constexpr int TM_S = 0, TM_O = 2 * BN;             // tensor-memory columns: S of tile q at TM_S + q*BN, O at TM_O + q*DV
   constexpr int TM_COLS = 512;
   extern __shared__ unsigned char smem_dyn[];
-  __shared__ __align__(8) uint64_t k_full[STAGES], k_empty[STAGES], v_full[STAGES], v_empty[STAGES];
+  __shared__ __align__(8) uint64_t k_full[STAGES], k_empty[STAGES], v_full[VST], v_empty[VST];
   __shared__ __align__(8) uint64_t s_full[2], p_full[2], o_full[2];   // per query tile
   __shared__ unsigned tmem_slot;
   __shared__ int s_abort;
   unsigned char* smem_raw = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
-  bf16* Qs = reinterpret_cast<bf16*>(smem_raw);     // [2 tiles][NH][128][64]
-  bf16* Ks = Qs + 2 * BM * HS;                       // [STAGES][TILE]
-  bf16* Vs = Ks + STAGES * TILE;
+  bf16* Qs = reinterpret_cast<bf16*>(smem_raw);     // [2 tiles][NK][128][64]
+  bf16* Ks = Qs + 2 * BM * DK;                       // [STAGES][KTILE]
+  bf16* Vs = Ks + STAGES * KTILE;                    // [VST][VTILE]
+  float* Bs = reinterpret_cast<float*>(Vs + VST * VTILE);        // BIAS: [2 tiles][2 buffers][G][pitch]
 
   // Items of a prompt come in order of position, so the last ones have the most keys: start with those,
   // for all KV heads alike (blocks are handed out with x running fastest, and x is the KV head).
-  const AttnItem item = p.items[gridDim.y - 1 - blockIdx.y];
+  // (With shares the entries come longest first.)
+  const int4 share = (MODE == MODE_PLAIN && x.shares) ? x.shares[blockIdx.y] : make_int4(gridDim.y - 1 - blockIdx.y, 0, 1, 0);
+  const AttnItem item = p.items[share.x];
   if (item.ntok <= 0) return;
   const int g = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -107,18 +153,26 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
   const int* table = p.block_table + (size_t)item.seq * p.table_width;
   const int tile_tokens = BM / p.G;                  // tokens of one query tile
   const bool two = item.ntok > tile_tokens;          // the second query tile has rows
-  const int kv_end = item.pos0 + item.ntok;
+  int kv_end = item.pos0 + item.ntok;
   const int kv_lo = first_visible_key(item.pos0, p.window, p.chunk);
-  const int kv_begin = kv_lo / BN * BN;
-  const int ntiles = (kv_end - kv_begin + BN - 1) / BN;
-  const int page_rows = 1 << log2_page;
+  int kv_begin = kv_lo / BN * BN;
+  int ntiles = (kv_end - kv_begin + BN - 1) / BN;
+  if (MODE == MODE_PLAIN && share.z > 1) {           // this share's tiles
+    const int first = (int)((long long)ntiles * share.y / share.z), last = (int)((long long)ntiles * (share.y + 1) / share.z);
+    kv_begin += first * BN;
+    ntiles = last - first;
+    kv_end = min(kv_end, kv_begin + ntiles * BN);
+  }
+  const int page_rows = 1 << log2_page;              // dense: rows of a box
   const int pages_per_tile = BN >> log2_page;
+  const int v0 = blockIdx.z * DV;                    // first value column of this block
 
   pdl_trigger();
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
+      mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1);
+      if (s < VST) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
     }
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -132,13 +186,15 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
   if (warp == 9) tmem_alloc(&tmem_slot, TM_COLS);
   // rows that no copy fills must hold finite numbers (they meet zero probabilities): those behind the
   // last key in the last tile, and pages wholly before the window in the first
-  auto clear_stage = [&](int stage) {
-    uint4* kz = reinterpret_cast<uint4*>(Ks + (size_t)stage * TILE);
-    uint4* vz = reinterpret_cast<uint4*>(Vs + (size_t)stage * TILE);
-    for (int i = threadIdx.x; i < TILE / 8; i += blockDim.x) { kz[i] = make_uint4(0, 0, 0, 0); vz[i] = make_uint4(0, 0, 0, 0); }
+  // (dense rows are fetched whole: what lies behind a sequence is another's rows, or zeros behind the last)
+  auto clear_tile = [&](int t) {
+    uint4* kz = reinterpret_cast<uint4*>(Ks + (size_t)(t % STAGES) * KTILE);
+    uint4* vz = reinterpret_cast<uint4*>(Vs + (size_t)(t % VST) * VTILE);
+    for (int i = threadIdx.x; i < KTILE / 8; i += blockDim.x) kz[i] = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < VTILE / 8; i += blockDim.x) vz[i] = make_uint4(0, 0, 0, 0);
   };
-  if ((kv_end - kv_begin) % BN != 0) clear_stage((ntiles - 1) % STAGES);
-  if (kv_begin + page_rows <= kv_lo) clear_stage(0);
+  if (!x.dense && (kv_end - kv_begin) % BN != 0) clear_tile(ntiles - 1);
+  if (!x.dense && kv_begin + page_rows <= kv_lo) clear_tile(0);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   tc05_fence_before_sync();
   __syncthreads();                                   // barriers, tensor memory and the zeroed rows stand
@@ -150,14 +206,14 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
   if (warp != 8) {
     // Query rows, while the producer already fetches the first keys: row r of tile q is token
     // q * tile_tokens + r / G, head g*G + r % G. All loads of a thread are issued before its stores.
-    constexpr int NT = 288, PER = (2 * BM * (HS / 8) + NT - 1) / NT;
+    constexpr int NT = 288, PER = (2 * BM * (DK / 8) + NT - 1) / NT;
     const int tid = warp == 9 ? 256 + lane : threadIdx.x;
     const int rows = two ? 2 * BM : BM;              // the second tile is not read when it has no token
     uint4 v[PER];
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
       const int id = tid + i * NT;
-      const int row = id / (HS / 8), c = id % (HS / 8);
+      const int row = id / (DK / 8), c = id % (DK / 8);
       const int q = row / BM, r = row % BM;
       const int tl = r / p.G, hh = r - tl * p.G;
       const int tok = q * tile_tokens + tl;
@@ -168,8 +224,8 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
       const int id = tid + i * NT;
-      const int row = id / (HS / 8), c = id % (HS / 8);
-      if (row < rows) *reinterpret_cast<uint4*>(half_ptr<BM>(Qs + (size_t)(row / BM) * BM * HS, row % BM, c)) = v[i];
+      const int row = id / (DK / 8), c = id % (DK / 8);
+      if (row < rows) *reinterpret_cast<uint4*>(half_ptr<BM>(Qs + (size_t)(row / BM) * BM * DK, row % BM, c)) = v[i];
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("bar.sync 1, 288;\n" ::: "memory");   // warps 0-7 and 9
@@ -179,59 +235,49 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
     // ---- producer: box b = (page, half, K or V) of each tile, boxes spread over the lanes. K and V
     // have barriers of their own: a K stage is free as soon as both S have been computed from it, long
     // before the V stage of the same tile, so the next keys arrive under the softmax.
-    const int boxes = pages_per_tile * NH * 2;
-    for (int t = 0; t < ntiles; ++t) {
-      const int stage = t % STAGES;
-      const int j = kv_begin + t * BN;
-      int cnt = 0;                                   // boxes of K (the same number of V) this lane group fetches
-      int page_of[2] = {-1, -1};
+    const int gv = g / x.v_share, KVv = p.KV / x.v_share;
+    const int first_row = x.dense ? table[0] : 0;    // of the sequence's rows in the matrices
+    auto fetch = [&](int t, int j, bool keys) {
+      const int nh = keys ? NK : NV;
+      const int stage = t % (keys ? STAGES : VST), boxes = pages_per_tile * nh;
+      uint64_t* full = keys ? &k_full[stage] : &v_full[stage];
+      uint64_t* empty = keys ? &k_empty[stage] : &v_empty[stage];
+      bf16* tile = keys ? Ks + (size_t)stage * KTILE : Vs + (size_t)stage * VTILE;
+      int cnt = 0, row_of[2] = {-1, -1};             // this lane's boxes
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int b = lane + 32 * i;
-        const int pg = b / (2 * NH);
-        // pages past the last key, or wholly before the window, are not fetched
-        if (b < boxes && j + pg * page_rows < kv_end && j + (pg + 1) * page_rows > kv_lo) {
+        const int b = lane + 32 * i, pg = b / nh, j_pg = j + pg * page_rows;
+        if (b >= boxes) continue;
+        if (x.dense) {
+          row_of[i] = first_row + j_pg;
+        } else if (j_pg < kv_end && j_pg + page_rows > kv_lo) {    // pages past the last key, or wholly before the window, are not fetched
           const int slot = (j >> log2_page) + pg;
-          int page = slot < p.table_width ? table[slot] : -1;
-          if (page < 0 || page >= p.num_pages) { set_status(p.status, SI_BAD_PAGE); page = -1; }
-          page_of[i] = page;
-          cnt += (page >= 0) && !(b & 1);
+          const int page = slot < p.table_width ? table[slot] : -1;
+          if (page < 0 || page >= p.num_pages) set_status(p.status, SI_BAD_PAGE);
+          else row_of[i] = (page * (keys ? p.KV : KVv) + (keys ? g : gv)) << log2_page;
         }
+        cnt += row_of[i] >= 0;
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-      bool ok = true;
-      if (t >= STAGES) ok = mbar_wait_warp(&k_empty[stage], (unsigned)(((t / STAGES) - 1) & 1));
-      if (!ok) {
-        if (lane == 0) { set_status(p.status, SI_WAIT_LIMIT); s_abort = 1; }
-        break;
-      }
-      if (lane == 0) mbar_expect_tx(&k_full[stage], (unsigned)(cnt * page_rows * 128));
+      const int st = keys ? STAGES : VST;
+      if (t >= st && !mbar_wait_warp(empty, (unsigned)(((t / st) - 1) & 1))) return false;
+      if (lane == 0) mbar_expect_tx(full, (unsigned)(cnt * page_rows * 128));
       __syncwarp();
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int b = lane + 32 * i;
-        if (page_of[i] < 0 || (b & 1)) continue;
-        const int pg = b / (2 * NH), h = (b >> 1) % NH;
-        const int row = (page_of[i] * p.KV + g) << log2_page;
-        const size_t off = (size_t)stage * TILE + (size_t)h * (BN * 64) + (size_t)(pg * page_rows) * 64;
-        tma_load_2d(Ks + off, &kmap, &k_full[stage], h * 64, row);
+        const int b = lane + 32 * i, pg = b / nh, h = b % nh;
+        if (row_of[i] < 0) continue;
+        const int col = (x.dense ? (keys ? g * p.hs : gv * p.vs) : 0) + (keys ? 0 : v0) + h * 64;
+        tma_load_2d(tile + (size_t)h * (BN * 64) + (size_t)(pg * page_rows) * 64, keys ? &kmap : &vmap, full, col, row_of[i]);
       }
-      if (t >= STAGES) ok = mbar_wait_warp(&v_empty[stage], (unsigned)(((t / STAGES) - 1) & 1));
-      if (!ok) {
+      return true;
+    };
+    for (int t = 0; t < ntiles; ++t) {
+      const int j = kv_begin + t * BN;
+      if (!fetch(t, j, true) || !fetch(t, j, false)) {
         if (lane == 0) { set_status(p.status, SI_WAIT_LIMIT); s_abort = 1; }
         break;
-      }
-      if (lane == 0) mbar_expect_tx(&v_full[stage], (unsigned)(cnt * page_rows * 128));
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int b = lane + 32 * i;
-        if (page_of[i] < 0 || !(b & 1)) continue;
-        const int pg = b / (2 * NH), h = (b >> 1) % NH;
-        const int row = (page_of[i] * p.KV + g) << log2_page;
-        const size_t off = (size_t)stage * TILE + (size_t)h * (BN * 64) + (size_t)(pg * page_rows) * 64;
-        tma_load_2d(Vs + off, &vmap, &v_full[stage], h * 64, row);
       }
     }
   } else if (warp == 9) {
@@ -241,19 +287,19 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
     // fields (units of 16 bytes) advance. An instruction is accepted only as fast as the tensor cores
     // run, so whatever else this warp does between two of them leaves the tensor cores idle.
     constexpr unsigned idesc_s = umma_idesc_bf16(BM, BN, false);
-    constexpr unsigned idesc_o = umma_idesc_bf16(BM, HS, true);
-    constexpr unsigned U_TILE = TILE * 2 / 16, U_QTILE = BM * HS * 2 / 16, U_HALF = BN * 64 * 2 / 16;
+    constexpr unsigned idesc_o = umma_idesc_bf16(BM, DV, true);
+    constexpr unsigned U_KTILE = KTILE * 2 / 16, U_VTILE = VTILE * 2 / 16, U_QTILE = BM * DK * 2 / 16, U_HALF = BN * 64 * 2 / 16;
     const int nq = two ? 2 : 1;
     const unsigned long long qd0 = umma_desc_sw128(Qs, 16, 1024);
     const unsigned long long kd0 = umma_desc_sw128(Ks, 16, 1024);
     const unsigned long long vd0 = umma_desc_sw128(Vs, BN * 128, 1024);
-    auto issue_s = [&](int q, int t) {  // S_q[128, 128] = Q_q[128, HS] K_t[128 keys, HS]^T: 4 steps per 64-column half
+    auto issue_s = [&](int q, int t) {  // S_q[128, 128] = Q_q[128, DK] K_t[128 keys, DK]^T: 4 steps per 64-column half
       const unsigned long long qd = qd0 + (unsigned)q * U_QTILE;
-      const unsigned long long kd = kd0 + (unsigned)(t % STAGES) * U_TILE;
+      const unsigned long long kd = kd0 + (unsigned)(t % STAGES) * U_KTILE;
       const unsigned sd = tmem + TM_S + q * BN;
       if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < HS / 16; ++kk)
+        for (int kk = 0; kk < DK / 16; ++kk)
           tc05_mma_bf16(sd, qd + ((kk >> 2) * U_HALF + 2 * (kk & 3)), kd + ((kk >> 2) * U_HALF + 2 * (kk & 3)), idesc_s, kk != 0 ? 1u : 0u);
         tc05_commit(&s_full[q]);
         if (q == nq - 1) tc05_commit(&k_empty[t % STAGES]);      // the keys of this tile are not needed again
@@ -266,17 +312,17 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
       for (int q = 0; q < nq; ++q) issue_s(q, 0);
     }
     for (int t = 0; t < ntiles && ok; ++t) {
-      const int stage = t % STAGES;
+      const int stage = t % VST;
       const bool more = t + 1 < ntiles;
-      ok = mbar_wait_warp(&v_full[stage], (unsigned)((t / STAGES) & 1));
+      ok = mbar_wait_warp(&v_full[stage], (unsigned)((t / VST) & 1));
       for (int q = 0; q < nq && ok; ++q) {
         ok = mbar_wait_warp(&p_full[q], (unsigned)(t & 1));
         if (!ok) break;
         tc05_fence_after_sync();
-        // O_q[128, HS] (+)= P_q[128, 128 keys] V_t[128 keys, HS]: 8 steps of 16 keys; P lies packed in the first
+        // O_q[128, DV] (+)= P_q[128, 128 keys] V_t[128 keys, DV]: 8 steps of 16 keys; P lies packed in the first
         // 64 columns of S_q, V rows are keys (MN-major B)
-        const unsigned long long vd = vd0 + (unsigned)stage * U_TILE;
-        const unsigned sd = tmem + TM_S + q * BN, od = tmem + TM_O + q * HS;
+        const unsigned long long vd = vd0 + (unsigned)stage * U_VTILE;
+        const unsigned sd = tmem + TM_S + q * BN, od = tmem + TM_O + q * DV;
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < BN / 16; ++kk)
@@ -305,7 +351,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
     int lo = p.window > 0 ? pos - p.window + 1 : INT_MIN;           // visible keys: lo <= j <= pos
     if (p.chunk > 0) lo = max(lo, pos / p.chunk * p.chunk);
     const unsigned lane_base = (unsigned)((warp & 3) * 32) << 16;
-    const unsigned ts = tmem + lane_base + TM_S + q * BN, to = tmem + lane_base + TM_O + q * HS;
+    const unsigned ts = tmem + lane_base + TM_S + q * BN, to = tmem + lane_base + TM_O + q * DV;
     float m = -INFINITY, l = 0.f;                    // base of the exponentials (log2 domain), the row's sum
     bool alive = true;
     // EXT: the row's own scale (its query temperature) and its head's slope, base 2; the scores then carry scale and
@@ -315,16 +361,61 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
       if (x.qt_every > 0 && pos >= 0) row_scale *= 1.f + x.qt_coef * logf((float)((pos + 1) / x.qt_every + 1));
       if (x.slopes) sl2 = x.slopes[g * p.G + (hh < p.G ? hh : 0)] * 1.4426950408889634f;
     }
-    const float sc = EXT ? 1.f : p.scale_log2;
+    const float sc = MODE != MODE_PLAIN ? 1.f : p.scale_log2;
+    // BIAS: entry k of a head's window is the distance (last position of the query tile) - j0 - k; the tile's four warps
+    // copy the next key tile's window while this one's is read
+    const int pitch = MODE == MODE_BIAS ? bias_pitch(p.G) : 0, span = tile_tokens + BN - 1;
+    const int last_pos = item.pos0 + (q + 1) * tile_tokens - 1;
+    float* const window = Bs + (size_t)q * 2 * p.G * pitch;
+    auto stage_bias = [&](int t) {
+      float* dst = window + (size_t)(t & 1) * p.G * pitch;
+      const int d0 = last_pos - (kv_begin + t * BN);
+      for (int i = r; i < span * p.G; i += BM) {
+        const int k = i / p.G, h = i - k * p.G;
+        const int d = min(max(d0 - k, 0), x.nd - 1);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_u32(dst + h * pitch + k)), "l"(x.bias + (size_t)d * p.H + g * p.G + h));
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
+    };
+    if (MODE == MODE_BIAS && ntiles > 0) stage_bias(0);
     for (int t = 0; t < ntiles; ++t) {
       const int j0 = kv_begin + t * BN;
-      alive = mbar_wait_warp(&s_full[q], (unsigned)(t & 1));
-      if (!alive) break;
+      if (MODE == MODE_BIAS) {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        asm volatile("bar.sync %0, 128;\n" ::"r"(2 + q) : "memory");      // this window stands; nobody reads the one before any more
+        if (t + 1 < ntiles) stage_bias(t + 1);
+      }
+      alive = alive && mbar_wait_warp(&s_full[q], (unsigned)(t & 1));
+      if (!alive) {
+        if (MODE == MODE_BIAS) continue;             // the tile's other warps still count on this one at their barrier
+        break;
+      }
       tc05_fence_after_sync();
       float s[BN];
 #pragma unroll
       for (int c = 0; c < BN / 32; ++c) tmem_ld_32x32_issue(ts + 32 * c, s + 32 * c);
       tmem_ld_wait();
+      if (MODE == MODE_BIAS) {
+        const float* b = window + (size_t)(t & 1) * p.G * pitch + (hh < p.G ? hh : 0) * pitch + (tile_tokens - 1 - min(tl, tile_tokens - 1));
+#pragma unroll
+        for (int i = 0; i < BN; ++i) s[i] = fmaf(b[i], LOG2E, s[i] * p.scale_log2);
+      }
+      if (MODE == MODE_CAP) {
+        float top = 0.f;
+#pragma unroll
+        for (int i = 0; i < BN; i += 2) top = max3(top, fabsf(s[i]), fabsf(s[i + 1]));
+        if (__any_sync(0xffffffffu, !(top * x.scale_over_cap <= 0.5f))) {
+          // tanh(y) = 1 - 2 / (exp(2 y) + 1): absolute error of some 1e-7, which is what counts for a score
+          const float c2 = 2.f * LOG2E * x.scale_over_cap;
+#pragma unroll
+          for (int i = 0; i < BN; ++i) s[i] = x.cap_log2 * (1.f - __fdividef(2.f, exp2f(s[i] * c2) + 1.f));
+        } else {
+          const unsigned long long c2 = pack_f32x2(x.scale_over_cap, x.scale_over_cap), cap2 = pack_f32x2(x.cap_log2, x.cap_log2);
+#pragma unroll
+          for (int i = 0; i < BN; i += 2)
+            unpack_f32x2(mul_f32x2(tanh_small_f32x2(mul_f32x2(pack_f32x2(s[i], s[i + 1]), c2)), cap2), s[i], s[i + 1]);
+        }
+      }
       // most tiles lie wholly inside every row's visible range: then nothing is masked
       if (__any_sync(0xffffffffu, !(j0 >= lo && j0 + BN - 1 <= pos))) {
 #pragma unroll
@@ -361,7 +452,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
       if (raise) { factor = fast_exp2(m - mx); m = mx; }   // exp2(-inf) = 0 on the first keys
       if (t > 0 && __any_sync(0xffffffffu, raise)) {
 #pragma unroll 1
-        for (int c = 0; c < HS / 32; ++c) {
+        for (int c = 0; c < DV / 32; ++c) {
           float v[32];
           tmem_ld_32x32(to + c * 32, v);
 #pragma unroll
@@ -427,6 +518,26 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
     }
     if (alive && ntiles > 0) alive = mbar_wait_warp(&o_full[q], 0);
     if (!alive && lane == 0) { set_status(p.status, SI_WAIT_LIMIT); s_abort = 1; }
+    if (MODE == MODE_PLAIN && share.z > 1) {                 // a share's results as they are
+      const size_t row = (((size_t)(share.w + share.y) * p.KV + g) * 2 + q) * BM + r;
+      if (alive && valid) {
+        tc05_fence_after_sync();
+        x.part_ml[row * 2] = m;
+        x.part_ml[row * 2 + 1] = l;
+      }
+      if (alive)                                             // (the loads are the whole warp's)
+#pragma unroll 1
+        for (int c = 0; c < DV / 32; ++c) {
+          float v[32];
+          tc05_fence_after_sync();
+          tmem_ld_32x32(to + c * 32, v);
+          if (!valid) continue;
+          float4* dst = reinterpret_cast<float4*>(x.part_o + row * DV + c * 32);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+      alive = false;                                         // nothing is stored here
+    }
     if (alive) {
       tc05_fence_after_sync();
       float inv = l > 0.f ? 1.f / l : 0.f;
@@ -434,9 +545,10 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
         const float s2 = p.sink[g * p.G + (hh < p.G ? hh : 0)] * LOG2E, M = fmaxf(m, s2), f = fast_exp2(m - M);
         inv = f / (l * f + fast_exp2(s2 - M));
       }
-      bf16* dst = p.out + (size_t)(item.row0 + tok) * p.out_stride + (size_t)(g * p.G + hh) * p.vs;
+      const size_t at = (size_t)(item.row0 + tok) * p.out_stride + (size_t)(g * p.G + hh) * p.vs + v0;
+      bf16* dst = p.out + at;
 #pragma unroll
-      for (int c = 0; c < HS / 64; ++c) {
+      for (int c = 0; c < DV / 64; ++c) {
         float v[64];
         tmem_ld_32x32_issue(to + c * 64, v);
         tmem_ld_32x32_issue(to + c * 64 + 32, v + 32);
@@ -456,6 +568,14 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
               }
             }
           }
+          if (x.out_f32) {
+            float* f = reinterpret_cast<float*>(p.out) + at;
+#pragma unroll
+            for (int q8 = 0; q8 < 16; ++q8)
+              if (v0 + c * 64 + q8 * 4 < p.vs)
+                *reinterpret_cast<float4*>(f + c * 64 + q8 * 4) = make_float4(v[4 * q8] * inv, v[4 * q8 + 1] * inv, v[4 * q8 + 2] * inv, v[4 * q8 + 3] * inv);
+            continue;
+          }
 #pragma unroll
           for (int q8 = 0; q8 < 8; ++q8) {
             uint4 raw;
@@ -463,7 +583,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
             raw.y = pack_bf16(v[8 * q8 + 2] * inv, v[8 * q8 + 3] * inv);
             raw.z = pack_bf16(v[8 * q8 + 4] * inv, v[8 * q8 + 5] * inv);
             raw.w = pack_bf16(v[8 * q8 + 6] * inv, v[8 * q8 + 7] * inv);
-            if (c * 64 + q8 * 8 < p.vs) *reinterpret_cast<uint4*>(dst + c * 64 + q8 * 8) = raw;
+            if (v0 + c * 64 + q8 * 8 < p.vs) *reinterpret_cast<uint4*>(dst + c * 64 + q8 * 8) = raw;
           }
         }
       }
@@ -472,6 +592,44 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
   tc05_fence_before_sync();
   __syncthreads();
   if (warp == 9) tmem_dealloc(tmem, TM_COLS);
+}
+
+// Merge of the items whose keys were cut: entry (item, shares, slot of the first, -). A warp a row: the shares weighed by their maxima,
+// the sink in the denominator once.
+template <int NV>
+__global__ void __launch_bounds__(256) attn_portion_merge_kernel(const AttnParams p, const int4* __restrict__ cut, const float* __restrict__ part_o,
+                                                                 const float* __restrict__ part_ml) {
+  constexpr int DV = NV * 64, PER = DV / 32;
+  pdl_prologue();
+  const int4 e = cut[blockIdx.y];
+  const AttnItem item = p.items[e.x];
+  const int g = blockIdx.x, row = blockIdx.z * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int tile_tokens = 128 / p.G, q = row >> 7, r = row & 127, tl = r / p.G, hh = r - tl * p.G, tok = q * tile_tokens + tl;
+  if (tl >= tile_tokens || tok >= item.ntok) return;
+  const size_t first = ((size_t)e.z * p.KV + g) * 256 + row, step = (size_t)p.KV * 256;
+  const float m_own = lane < e.y ? part_ml[(first + lane * step) * 2] : -INFINITY, l_own = lane < e.y ? part_ml[(first + lane * step) * 2 + 1] : 0.f;
+  const int head = g * p.G + hh;
+  const float sk = p.sink ? p.sink[head] * LOG2E : -INFINITY;
+  const float M = fmaxf(warp_max(m_own), sk);
+  const float w_own = m_own == -INFINITY ? 0.f : fast_exp2(m_own - M);
+  const float L = warp_sum(l_own * w_own) + (p.sink ? fast_exp2(sk - M) : 0.f);
+  float acc[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) acc[i] = 0.f;
+  for (int s = 0; s < e.y; ++s) {
+    const float w = __shfl_sync(0xffffffffu, w_own, s);
+    const float* src = part_o + (first + s * step) * DV + lane * PER;
+#pragma unroll
+    for (int i = 0; i < PER; i += 2) {
+      const float2 v = *reinterpret_cast<const float2*>(src + i);
+      acc[i] = fmaf(v.x, w, acc[i]); acc[i + 1] = fmaf(v.y, w, acc[i + 1]);
+    }
+  }
+  const float inv = L > 0.f ? 1.f / L : 0.f;
+  bf16* dst = p.out + (size_t)(item.row0 + tok) * p.out_stride + (size_t)head * p.vs;
+#pragma unroll
+  for (int i = 0; i < PER; i += 2)
+    if (lane * PER + i < p.vs) *reinterpret_cast<__nv_bfloat162*>(dst + lane * PER + i) = __floats2bfloat162_rn(acc[i] * inv, acc[i + 1] * inv);
 }
 
 // ---- host side --------------------------------------------------------------------------------
@@ -486,20 +644,45 @@ SI_EXPORT int si_attn_portion_tc05_ok(int H, int KV, int hs, int vs, int page_si
 // Tokens of one item: two query tiles of floor(128 / G) each.
 SI_EXPORT int si_attn_portion_tc05_tokens(int H, int KV) { return 2 * (128 / (H / KV)); }
 
-template <int NH, bool EXT>
+template <int NK, int NV, int MODE>
 static int launch(const AttnParams& p, const CUtensorMap& km, const CUtensorMap& vm, int num_items, int log2_page,
                   cudaStream_t stream, const AttnExtras& x) {
-  constexpr int HS = NH * 64;
-  // Q of both query tiles, two stages of K and of V. The block takes all of tensor memory, so a second
+  constexpr int VST = NK > 2 ? 1 : 2;
+  // Q of both query tiles, the stages of K and of V, the biases. The block takes all of tensor memory, so a second
   // block on the same SM could only wait for it: ask for more than half of the shared memory.
-  size_t smem = (size_t)(2 * 128 * HS + 2 * 2 * NH * 128 * 64) * sizeof(bf16) + 1024;
+  size_t smem = (size_t)(2 * 128 * NK * 64 + 2 * NK * 128 * 64 + VST * NV * 128 * 64) * sizeof(bf16) + 1024;
+  if (MODE == MODE_BIAS) smem += (size_t)4 * p.G * bias_pitch(p.G) * sizeof(float);
   if (smem < 120 * 1024) smem = 120 * 1024;
-  auto k = attn_portion_tc05_kernel<NH, EXT>;
+  if (smem > 227 * 1024 - 256) return -2;
+  auto k = attn_portion_tc05_kernel<NK, NV, MODE>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  si_launch(k, dim3(p.KV, num_items), dim3(320), smem, stream, p, km, vm, log2_page, x);
+  si_launch(k, dim3(p.KV, num_items, (p.vs + NV * 64 - 1) / (NV * 64)), dim3(320), smem, stream, p, km, vm, log2_page, x);
   return si_last_error();
 }
+
+// Floats of partial results of `slots` shares.
+SI_EXPORT long long si_attn_portion_share_floats(int slots, int KV, int hs, int vs) {
+  return (long long)slots * KV * 256 * ((hs <= 64 && vs <= 64 ? 64 : 128) + 2);
+}
+
+static AttnParams make_params(const void* q, long long q_stride, const int* block_table, int table_width, const void* items, void* out,
+                              long long out_stride, int num_pages, int page_size, int num_seqs, int H, int KV, int hs, int vs,
+                              float scale, int window, int chunk, const float* sink, int* status) {
+  AttnParams p;
+  p.q = (const bf16*)q; p.q_stride = q_stride;
+  p.k_cache = nullptr; p.v_cache = nullptr;          // reached through the tensor maps
+  p.block_table = block_table; p.table_width = table_width;
+  p.items = (const AttnItem*)items;
+  p.out = (bf16*)out; p.out_stride = out_stride;
+  p.part_o = nullptr; p.part_ml = nullptr; p.counters = nullptr;
+  p.num_pages = num_pages; p.page_size = page_size; p.num_seqs = num_seqs;
+  p.H = H; p.KV = KV; p.G = H / KV; p.hs = hs; p.vs = vs;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.window = window; p.chunk = chunk; p.sink = sink; p.nsplit = 1; p.status = status;
+  return p;
+}
+static int log2_of(int n) { int l = 0; while ((1 << l) < n) ++l; return l; }
 
 // Same contract as si_attn_portion (attention_mma.cu) with the tensor maps of the layer's K and V cache
 // (made by si_attn_encode_cache_map of attention_tma.cu); items hold at most si_attn_portion_tc05_tokens().
@@ -510,32 +693,86 @@ SI_EXPORT int si_attn_portion_tc05(const void* q, long long q_stride, const void
                                    const void* items, int num_items, void* out, long long out_stride, int num_pages,
                                    int page_size, int num_seqs, int H, int KV, int hs, int vs, float scale, int window,
                                    const float* slopes, float qt_coef, int qt_every, const void* gate, long long gate_stride,
-                                   int chunk, const float* sink, int* status, cudaStream_t stream) {
+                                   int chunk, const float* sink, const int* shares, int num_shares, const int* cut, int num_cut,
+                                   int slots, float* scratch, int* status, cudaStream_t stream) {
   if (num_items <= 0) return 0;
   if (qt_every < 0 || chunk < 0 || (gate && (gate_stride % 8 || ((uintptr_t)gate % 16)))) return -2;
   // a temperature below zero would turn the order of the scores round: the plain kernels serve that
-  const AttnExtras x{slopes, qt_coef, qt_every, (const bf16*)gate, gate_stride};
+  AttnExtras x = {};
+  x.slopes = slopes; x.qt_coef = qt_coef; x.qt_every = qt_every; x.gate = (const bf16*)gate; x.gate_stride = gate_stride; x.v_share = 1;
   const bool ext = slopes || qt_every > 0 || gate;
   if (num_items > 65535) return -2;                  // the grid's second dimension
   if (!si_attn_portion_tc05_ok(H, KV, hs, vs, page_size) || !kmap || !vmap) return -2;
   if ((q_stride % 8) || (out_stride % 8) || ((uintptr_t)q % 16) || ((uintptr_t)out % 16)) return -2;
-  AttnParams p;
-  p.q = (const bf16*)q; p.q_stride = q_stride;
-  p.k_cache = (const bf16*)k_cache; p.v_cache = (const bf16*)v_cache;
-  p.block_table = block_table; p.table_width = table_width;
-  p.items = (const AttnItem*)items;
-  p.out = (bf16*)out; p.out_stride = out_stride;
-  p.part_o = nullptr; p.part_ml = nullptr; p.counters = nullptr;
-  p.num_pages = num_pages; p.page_size = page_size; p.num_seqs = num_seqs;
-  p.H = H; p.KV = KV; p.G = H / KV; p.hs = hs; p.vs = vs;
-  p.scale_log2 = scale * 1.4426950408889634f;
-  p.window = window; p.chunk = chunk; p.sink = sink; p.nsplit = 1; p.status = status;
-  int log2_page = 0;
-  while ((1 << log2_page) < page_size) ++log2_page;
+  const AttnParams p = make_params(q, q_stride, block_table, table_width, items, out, out_stride, num_pages, page_size, num_seqs, H, KV,
+                                   hs, vs, scale, window, chunk, sink, status);
+  const int log2_page = log2_of(page_size);
   const CUtensorMap& km = *(const CUtensorMap*)kmap;
   const CUtensorMap& vm = *(const CUtensorMap*)vmap;
   if (ext && (hs != vs || (hs != 64 && hs != 128))) return -2;
   const bool narrow = hs <= 64 && vs <= 64;
-  if (ext) return narrow ? launch<1, true>(p, km, vm, num_items, log2_page, stream, x) : launch<2, true>(p, km, vm, num_items, log2_page, stream, x);
-  return narrow ? launch<1, false>(p, km, vm, num_items, log2_page, stream, x) : launch<2, false>(p, km, vm, num_items, log2_page, stream, x);
+  if (shares) {                                      // see AttnExtras
+    if (ext || num_shares <= 0 || num_shares > 65535 || num_cut < 0 || num_cut > 65535 || (num_cut && (!cut || !scratch || slots <= 0))) return -2;
+    if (((uintptr_t)shares | (uintptr_t)cut | (uintptr_t)scratch) & 15) return -2;
+    const int dv = narrow ? 64 : 128;
+    x.shares = (const int4*)shares;
+    x.part_o = scratch;
+    x.part_ml = scratch + (long long)slots * KV * 256 * dv;
+    int rc = narrow ? launch<1, 1, MODE_PLAIN>(p, km, vm, num_shares, log2_page, stream, x) : launch<2, 2, MODE_PLAIN>(p, km, vm, num_shares, log2_page, stream, x);
+    if (rc || !num_cut) return rc;
+    const dim3 grid(KV, num_cut, 32);
+    if (narrow) si_launch(attn_portion_merge_kernel<1>, grid, dim3(256), 0, stream, p, (const int4*)cut, (const float*)x.part_o, (const float*)x.part_ml);
+    else si_launch(attn_portion_merge_kernel<2>, grid, dim3(256), 0, stream, p, (const int4*)cut, (const float*)x.part_o, (const float*)x.part_ml);
+    return si_last_error();
+  }
+  if (ext) return narrow ? launch<1, 1, MODE_EXT>(p, km, vm, num_items, log2_page, stream, x) : launch<2, 2, MODE_EXT>(p, km, vm, num_items, log2_page, stream, x);
+  return narrow ? launch<1, 1, MODE_PLAIN>(p, km, vm, num_items, log2_page, stream, x) : launch<2, 2, MODE_PLAIN>(p, km, vm, num_items, log2_page, stream, x);
+}
+
+// The general form: key size up to 192, values of any size (128 columns a block), key heads that share a value head, results in fp32,
+// and one of a bias by distance (fp32 [nd, H]) and a soft limit, over pages or (dense) over matrices of one row a token
+// [rows, KV * size] in which sequence s has the rows from block_table[s, 0] on. 1 when it takes the layout.
+#define DENSE_BOX 64
+SI_EXPORT int si_attn_portion_gen_ok(int H, int KV, int dk, int dv, int v_share, int page_size, int dense, int bias, int cap) {
+  if (KV <= 0 || H % KV || H / KV > 128 || v_share < 1 || KV % v_share) return 0;
+  if (dk <= 0 || dv <= 0 || dk > 192 || dk % 8 || dv % 8 || dv > 8192 || (bias && cap)) return 0;
+  if ((bias || cap) && dk > 128) return 0;
+  if (bias && H / KV > 16) return 0;                 // the windows beside the tiles in shared memory
+  if (!dense && page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64) return 0;
+  return si_encode_fn() != nullptr;
+}
+
+// `keys`, `values`: the caches' tensor maps, or (dense) the matrices themselves, of `num_pages` rows.
+SI_EXPORT int si_attn_portion_gen(const void* q, long long q_stride, const void* keys, const void* values, const int* block_table, int table_width,
+                                  const void* items, int num_items, void* out, int out_f32, long long out_stride, int num_pages, int page_size,
+                                  int dense, int num_seqs, int H, int KV, int dk, int dv, int v_share, float scale, int window, int chunk,
+                                  const float* sink, const float* bias, int nd, float softcap, int* status, cudaStream_t stream) {
+  if (num_items <= 0) return 0;
+  if (num_items > 65535 || chunk < 0 || softcap < 0.f || !keys || !values || (bias && nd <= 0) || table_width <= 0) return -2;
+  if (!si_attn_portion_gen_ok(H, KV, dk, dv, v_share, page_size, dense, bias != nullptr, softcap > 0.f)) return -2;
+  if ((q_stride % 8) || (out_stride % 8) || ((uintptr_t)q % 16) || ((uintptr_t)out % 16)) return -2;
+  AttnExtras x = {};
+  x.v_share = v_share; x.out_f32 = out_f32; x.dense = dense; x.bias = bias; x.nd = nd;
+  if (softcap > 0.f) { x.cap_log2 = softcap * 1.4426950408889634f; x.scale_over_cap = scale / softcap; }
+  const AttnParams p = make_params(q, q_stride, block_table, table_width, items, out, out_stride, num_pages, page_size, num_seqs, H, KV,
+                                   dk, dv, scale, window, chunk, sink, status);
+  const int log2_page = log2_of(dense ? DENSE_BOX : page_size), nk = (dk + 63) / 64;
+  alignas(64) CUtensorMap km, vm;
+  if (dense) {
+    if (num_pages <= 0 || ((uintptr_t)keys % 16) || ((uintptr_t)values % 16)) return -2;
+    const unsigned long long kc = (unsigned long long)KV * dk, vc = (unsigned long long)(KV / v_share) * dv;
+    int rc = si_encode_bf16_2d(&km, keys, (unsigned long long)num_pages, kc, kc, DENSE_BOX);
+    if (!rc) rc = si_encode_bf16_2d(&vm, values, (unsigned long long)num_pages, vc, vc, DENSE_BOX);
+    if (rc) return rc;
+  } else {
+    km = *(const CUtensorMap*)keys;
+    vm = *(const CUtensorMap*)values;
+  }
+#define GEN_LAUNCH(NK, MODE) return launch<NK, 2, MODE>(p, km, vm, num_items, log2_page, stream, x)
+  if (bias) { if (nk == 1) GEN_LAUNCH(1, MODE_BIAS); GEN_LAUNCH(2, MODE_BIAS); }
+  if (softcap > 0.f) { if (nk == 1) GEN_LAUNCH(1, MODE_CAP); GEN_LAUNCH(2, MODE_CAP); }
+  if (nk == 1) GEN_LAUNCH(1, MODE_PLAIN);
+  if (nk == 2) GEN_LAUNCH(2, MODE_PLAIN);
+  GEN_LAUNCH(3, MODE_PLAIN);
+#undef GEN_LAUNCH
 }

@@ -5,6 +5,7 @@ Nothing here computes on the CPU or through a library: a missing build fails lou
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -118,6 +119,10 @@ def _fn(libname: str, symbol: str, argtypes):
         f.restype = _c_int
         _fn_cache[key] = f
     return f
+
+
+# What a kernel takes, and the sizes of its work items and scratch, follow from whole numbers alone; every layer asks in every step.
+_of_sizes = functools.lru_cache(maxsize=1024)
 
 
 def _i32(t: Optional[torch.Tensor], name: str) -> None:
@@ -981,11 +986,13 @@ def attn_portion_tc05_tokens(H: int, KV: int) -> int:
 
 def attn_portion_tc05(q, k_cache, v_cache, block_table, items, out, page_size: int, num_seqs: int, H: int,
                       KV: int, hs: int, scale: float, window: int = 0, status=None, slopes=None, q_temp=None, gate=None,
-                      chunk: int = 0, sink=None, vs: Optional[int] = None) -> None:
+                      chunk: int = 0, sink=None, vs: Optional[int] = None, shares=None) -> None:
     """``attn_portion`` on the tcgen05 tensor cores (TMA-fed K/V tiles, S and P V in tensor memory);
     head_dim 64 or 128, page sizes 8 to 64, items of at most ``attn_portion_tc05_tokens`` tokens. ``v_cache`` None: the
     values are the keys. ``slopes``, ``q_temp`` (a coefficient that is not negative), ``gate``, ``chunk`` and ``sink`` as in
-    ``attention_general`` (the gate's rows 16-byte aligned). ``vs``: size of the values where it is not the keys'."""
+    ``attention_general`` (the gate's rows 16-byte aligned). ``vs``: size of the values where it is not the keys'. ``shares``
+    ``(entries, cut, slots, scratch)``: items whose keys are cut over several blocks (``cut_portions`` makes the lists; ``scratch``:
+    ``attn_portion_share_floats(slots, ...)`` floats); not with slopes, a temperature or a gate."""
     if v_cache is None:
         v_cache = k_cache
     vs = hs if vs is None else vs
@@ -999,12 +1006,111 @@ def attn_portion_tc05(q, k_cache, v_cache, block_table, items, out, page_size: i
                            and gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0), "attn_portion_tc05: gate must be bf16 [T, H*hs], rows 16-byte aligned")
     f = _fn("attention_tc05", "si_attn_portion_tc05",
             [_c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_p, _c_int, _c_p, _c_ll, _c_int, _c_int, _c_int,
-             _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_p, _c_f, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_p, _c_p])
+             _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_p, _c_f, _c_int, _c_p, _c_ll, _c_int, _c_p, _c_p, _c_int, _c_p, _c_int,
+             _c_int, _c_p, _c_p, _c_p])
+    entries, cut, slots, scratch = shares if shares is not None else (None, None, 0, None)
+    if shares is not None:
+        _cuda(entries, cut, scratch)
+        _i32(entries, "shares"); _i32(cut, "cut")
+        _need(entries.shape[1] == 4 and cut.shape[1] == 4 and scratch.dtype == torch.float32
+              and scratch.numel() >= attn_portion_share_floats(slots, KV, hs, vs), "attn_portion_tc05: shares")
     _check(f(_ptr(q), q.stride(0), _ptr(k_cache), _ptr(v_cache), _cache_map(k_cache), _cache_map(v_cache),
              _ptr(block_table), block_table.shape[1], _ptr(items), items.shape[0], _ptr(out), out.stride(0),
              k_cache.shape[0], page_size, num_seqs, H, KV, hs, vs, float(scale), int(window or 0), _ptr(slopes), qt_coef, qt_every,
-             _ptr(gate), gate.stride(0) if gate is not None else 0, int(chunk or 0), _ptr(sink), _ptr(status),
-             _stream()), f"attn_portion_tc05(heads={H}, kv_heads={KV}, head_dim={hs}, page_size={page_size})")
+             _ptr(gate), gate.stride(0) if gate is not None else 0, int(chunk or 0), _ptr(sink), _ptr(entries),
+             entries.shape[0] if entries is not None else 0, _ptr(cut), cut.shape[0] if cut is not None else 0, int(slots), _ptr(scratch),
+             _ptr(status), _stream()), f"attn_portion_tc05(heads={H}, kv_heads={KV}, head_dim={hs}, page_size={page_size})", kernels=2 if cut is not None and cut.shape[0] else 1)
+
+
+@_of_sizes
+def attn_portion_share_floats(slots: int, KV: int, hs: int, vs: int) -> int:
+    lib = build.load("attention_tc05")
+    lib.si_attn_portion_share_floats.restype = _c_llr
+    return lib.si_attn_portion_share_floats(_c_int(slots), _c_int(KV), _c_int(hs), _c_int(vs))
+
+
+def cut_portions(tiles, copies: int, blocks: int, least: int = 16):
+    """Cut work items (``tiles[i]`` key tiles each, every item run for ``copies`` key/value heads) so that ``blocks`` blocks that run at
+    once end together: a long prompt's portion is a few items more than the blocks, and the last ones would run alone. Tries longest
+    shares from the longest item down and takes the shortest schedule (longest share first to the block that is free first; a share
+    costs its tiles and about two for its start, a cut item's share three more for handing over). No share is below ``least`` tiles.
+    Returns (entries int32 [n, 4] of (item, share, shares, first slot), longest first, cut int32 [m, 4] of (item, shares, first slot, 0),
+    slots), or None where whole items are within a twentieth of the best."""
+    import heapq
+    import numpy as np
+
+    def schedule(limit):
+        cost = sorted((sh + 2 + (3 if n > 1 else 0) for t in tiles for n in (-(-t // limit),) for sh in [-(-t // n)] * n), reverse=True)
+        heap = [0] * blocks
+        for c in cost:
+            for _ in range(copies):
+                heapq.heapreplace(heap, heap[0] + c)
+        return max(heap)
+
+    longest = max(tiles)
+    total = sum(tiles) * copies
+    if longest < 2 * least or len(tiles) * copies > 8 * blocks:
+        return None
+    whole = schedule(longest)
+    if whole * 0.95 <= total / blocks:
+        return None
+    limits = sorted({max(least, -(-longest // n)) for n in (2, 3, 4, 6, 9, 13, 18) if n <= 6 or len(tiles) * copies * n <= 4 * blocks})
+    best, limit = min((schedule(l), l) for l in limits if l < longest)
+    if best > 0.95 * whole:
+        return None
+    entries, cut, slots = [], [], 0
+    for i, t in enumerate(tiles):
+        n = min(32, -(-t // limit))
+        entries += [(-(-t // n), i, s, n, slots if n > 1 else 0) for s in range(n)]
+        if n > 1:
+            cut.append((i, n, slots, 0))
+            slots += n
+    entries.sort(key=lambda e: -e[0])
+    return np.asarray([e[1:] for e in entries], dtype=np.int32), np.asarray(cut, dtype=np.int32).reshape(-1, 4), slots
+
+
+@_of_sizes
+def attn_portion_gen_ok(H: int, KV: int, dk: int, dv: int, v_share: int = 1, page_size: int = 0, bias: bool = False, cap: bool = False) -> bool:
+    """True when ``attn_portion_gen`` takes the layout (``page_size`` 0: the dense form)."""
+    lib = build.load("attention_tc05")
+    lib.si_attn_portion_gen_ok.restype = _c_int
+    return bool(lib.si_attn_portion_gen_ok(_c_int(H), _c_int(KV), _c_int(dk), _c_int(dv), _c_int(v_share), _c_int(page_size),
+                                           _c_int(0 if page_size else 1), _c_int(1 if bias else 0), _c_int(1 if cap else 0)))
+
+
+def attn_portion_gen(q, k, v, block_table, items, out, page_size: int, num_seqs: int, H: int, KV: int, dk: int, dv: int, scale: float,
+                     window: int = 0, dist_bias=None, sink=None, status=None, softcap: float = 0.0, v_share: int = 1, chunk: int = 0) -> None:
+    """``attn_flex``'s prompt portions on the tcgen05 tensor cores: key sizes up to 192, values of any size, one of a bias by distance and a
+    soft limit; items (in order of position) of at most ``attn_portion_tc05_tokens`` tokens; ``out`` bf16 or fp32. ``page_size`` 0, the dense
+    form: ``k`` [rows, KV * dk] and ``v`` [rows, KV / v_share * dv] hold a row a token, and sequence s of an item has the rows from
+    ``block_table[s, 0]`` on (``block_table``: any int32 [seqs, width] view with contiguous rows)."""
+    _cuda(q, k, v, block_table, items, out, dist_bias, sink, status)
+    _i32(items, "items")
+    _need(block_table.dtype == torch.int32 and block_table.dim() == 2 and block_table.stride(1) == 1, "attn_portion_gen: block_table")
+    _need(q.dtype == k.dtype == v.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32) and k.is_contiguous() and v.is_contiguous(),
+          "attn_portion_gen: bfloat16 tensors only")
+    _need(q.stride(1) == 1 and out.stride(1) == 1 and q.shape[1] == H * dk and out.shape[1] == H * dv and v_share >= 1 and KV % v_share == 0,
+          "attn_portion_gen: q must be [T, H*dk], out [T, H*dv]")
+    if page_size:
+        _need(tuple(k.shape[1:]) == (KV, page_size, dk) and tuple(v.shape) == (k.shape[0], KV // v_share, page_size, dv),
+              "attn_portion_gen: keys must be [pages, KV, page_size, dk], values [pages, KV / v_share, page_size, dv]")
+    else:
+        _need(k.dim() == 2 and k.shape[1] == KV * dk and tuple(v.shape) == (k.shape[0], KV // v_share * dv), "attn_portion_gen: dense keys and values")
+    _need(items.dim() == 2 and items.shape[1] == 4, "attn_portion_gen: items must be int32 [n, 4]")
+    nd = 0
+    if dist_bias is not None:
+        _need(dist_bias.dim() == 2 and dist_bias.shape[1] == H, "attn_portion_gen: dist_bias must be [nd, H]")
+        _f32v(dist_bias, "dist_bias")
+        nd = dist_bias.shape[0]
+    _f32v(sink, "sink", H)
+    f = _fn("attention_tc05", "si_attn_portion_gen",
+            [_c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_p, _c_int, _c_p, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
+             _c_int, _c_int, _c_f, _c_int, _c_int, _c_p, _c_p, _c_int, _c_f, _c_p, _c_p])
+    _check(f(_ptr(q), q.stride(0), _cache_map(k) if page_size else _ptr(k), _cache_map(v) if page_size else _ptr(v), _ptr(block_table),
+             block_table.stride(0), _ptr(items), items.shape[0], _ptr(out), 1 if out.dtype == torch.float32 else 0, out.stride(0), k.shape[0],
+             page_size, 0 if page_size else 1, num_seqs, H, KV, dk, dv, int(v_share), float(scale), int(window or 0), int(chunk or 0), _ptr(sink),
+             _ptr(dist_bias), nd, float(softcap or 0.0), _ptr(status), _stream()),
+           f"attn_portion_gen(heads={H}, kv_heads={KV}, dk={dk}, dv={dv}, page_size={page_size})")
 
 
 # ---- general attention, stores, latent form -------------------------------------------------------

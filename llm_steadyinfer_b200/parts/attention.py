@@ -255,7 +255,7 @@ class Attention(Mixer):
             names.append("attention_flex")
             if self.hs % 8 or self.vs % 8:                                             # sizes that kernel does not take
                 names.append("attention_general")
-            if self.general_tc05_ok(page_size):
+            if self.general_tc05_ok(page_size) or self.gen_ok(page_size):
                 names += ["attention_tma", "attention_tc05"]
             return tuple(names)
         names = ["rope_kv"] + (["gemm_f32"] if self.dtype == torch.float32 else ["gemm_skinny", "gemm_rows", "gemm_tc05"])
@@ -305,6 +305,11 @@ class Attention(Mixer):
         """The general form's long portions on the tcgen05 prompt kernel: its layouts, and nothing it does not know."""
         return (USE_TC05 and self.bias_spec is None and self.vs == self.hs and (self.q_temp is None or self.q_temp[0] >= 0)
                 and ops.attn_portion_tc05_ok(self.H, self.KV, self.hs, page_size))
+
+    def gen_ok(self, page_size: int) -> bool:
+        """Long portions that kernel's extended form does not take (a bias by distance, a value size of its own), on its general form."""
+        return (USE_TC05 and self.own_v and not self.general_tc05_ok(page_size) and self.slopes is None and self.q_temp is None
+                and self.gate_name is None and flex_plan.gen_ok(self.H, self.KV, self.hs, self.vs, page_size, bias=self.bias_spec is not None))
 
     def _plan_general_tc05(self, ctx, page_size: int) -> dict:
         """Which sequences of the step go to the tcgen05 prompt kernel (those that bring at least one full item of rows),
@@ -374,7 +379,7 @@ class Attention(Mixer):
             big = self._plan_general_tc05(ctx, cache.page_size)
             if not big["all"]:
                 flex_plan.attend(flex_plan.plan(ctx, self.device, H, KV, hs, vs, self.own_v, self.window, skip=big["skip"],
-                                                chunk=self.chunk),
+                                                chunk=self.chunk, gen=self.gen_ok(cache.page_size)),
                                  q, cache.k, v_cache, cache.block_table, attn, cache.page_size, ctx.seq_slots, H, KV,
                                  hs, vs, self.scale, self.window, dist_bias=self.dist_bias, sink=self.sink, status=ctx.status,
                                  slopes=self.slopes, q_temp=self.q_temp, gate=gate, chunk=self.chunk)
@@ -425,7 +430,7 @@ class Attention(Mixer):
                 big = self._plan_general_tc05(ctx, cache.page_size)
                 if not big["all"]:
                     flex_plan.plan(ctx, self.device, self.H, self.KV, self.hs, self.vs, self.own_v, self.window, skip=big["skip"],
-                                   chunk=self.chunk)
+                                   chunk=self.chunk, gen=self.gen_ok(cache.page_size))
             return
         if not self.general and not self.uses_tensor_cores():
             return
@@ -492,8 +497,19 @@ class Attention(Mixer):
                 n = ops.attn_decode_scratch_floats(len(dec), self.H, self.KV, self.hs, nsplit)
                 plan["scratch"] = ctx.buf("attn_split", (n,), torch.float32)
         if por:
-            plan["por"] = ctx.upload_ints(f"attn_por_{self._tag()}",
-                                          np.asarray(por, dtype=np.int32)).view(-1, 4)
+            shares = None
+            if tc05:
+                tiles = [-(-(pos0 + n - first_visible_key(pos0, self.window, self.chunk) // 128 * 128) // 128) for _, _, n, pos0 in por]
+                shares = ops.cut_portions(tiles, self.KV, ops.sm_count(self.device))
+            if shares is None:
+                plan["por"] = ctx.upload_ints(f"attn_por_{self._tag()}", np.asarray(por, dtype=np.int32)).view(-1, 4)
+            else:
+                entries, cut, slots = shares
+                ints = ctx.upload_ints(f"attn_por_{self._tag()}", np.concatenate([np.asarray(por, dtype=np.int32), entries, cut])).view(-1, 4)
+                a, b = len(por), len(por) + len(entries)
+                plan["por"] = ints[:a]
+                plan["shares"] = (ints[a:b], ints[b:], slots,
+                                  ctx.buf("attn_shares", (ops.attn_portion_share_floats(slots, self.KV, self.hs, self.vs),), torch.float32))
         ctx.plans[key] = plan
 
     def attend(self, q, cache, ctx, out):
@@ -515,6 +531,8 @@ class Attention(Mixer):
                                 nsplit=plan["nsplit"], scratch=plan["scratch"], status=ctx.status)
         if plan["por"] is not None:
             portion = ops.attn_portion_tc05 if plan["tc05"] else ops.attn_portion
+            if plan.get("shares") is not None:
+                extra = dict(extra, shares=plan["shares"])
             portion(q, cache.k, cache.v, cache.block_table, plan["por"], out, *args, status=ctx.status, **extra)
 
 

@@ -102,7 +102,11 @@ class DiffAttention(Mixer):
     def kernel_files(self, page_size):
         if self.dtype == torch.float32:
             return ("qk_prepare", "attention_general", "gemm_f32")
-        return ("qk_prepare", "attention_flex" if self.uses_flex() else "attention_general", "gemm_skinny", "gemm_rows", "gemm_tc05")
+        return ("qk_prepare", "gemm_skinny", "gemm_rows", "gemm_tc05") + (
+            ("attention_flex", "attention_tma", "attention_tc05") if self.uses_flex() else ("attention_general",))
+
+    def gen_ok(self, page_size) -> bool:
+        return flex_plan.gen_ok(self.H * MAPS, self.G * MAPS, self.dk, self.dv, page_size, v_share=MAPS, cap=self.softcap > 0)
 
     def uses_flex(self) -> bool:
         """The maps on the tensor cores: bfloat16 and sizes in multiples of 8."""
@@ -111,7 +115,7 @@ class DiffAttention(Mixer):
 
     def prepare(self, ctx, cache):
         if self.uses_flex() and cache.k is not None:
-            flex_plan.plan(ctx, self.device, self.H * MAPS, self.G * MAPS, self.dk, self.dv, True, self.window)
+            flex_plan.plan(ctx, self.device, self.H * MAPS, self.G * MAPS, self.dk, self.dv, True, self.window, gen=self.gen_ok(cache.page_size))
 
     def forward(self, x, ctx, cache):
         T = x.shape[0]
@@ -139,7 +143,7 @@ class DiffAttention(Mixer):
         """Both maps of every head as 2 H query heads over 2 G key heads; neighbouring key heads share a value head."""
         if self.uses_flex():
             H, G = self.H * MAPS, self.G * MAPS
-            flex_plan.attend(flex_plan.plan(ctx, self.device, H, G, self.dk, self.dv, True, self.window), q, cache.k, cache.v,
+            flex_plan.attend(flex_plan.plan(ctx, self.device, H, G, self.dk, self.dv, True, self.window, gen=self.gen_ok(cache.page_size)), q, cache.k, cache.v,
                              cache.block_table, maps, cache.page_size, ctx.seq_slots, H, G, self.dk, self.dv, self.scale,
                              self.window, status=ctx.status, softcap=self.softcap, v_share=MAPS)
             return

@@ -2,7 +2,8 @@
 
 A sequence's rows of the step become work items of at most ``ops.attn_flex_tokens`` tokens. Sequences that bring
 few rows (decode rows, short ends of prompts: one item) form one launch whose items have their keys cut into
-shares, as many as fill the device; longer portions form another without shares. A plan is kept under a key of
+shares, as many as fill the device; longer portions form another without shares, or, where the caller's form is one that
+the tcgen05 prompt kernel takes (``gen_ok``) and they fill a tile of its rows, go there. A plan is kept under a key of
 the step's context, so layers with the same head layout make it once.
 """
 from __future__ import annotations
@@ -16,23 +17,33 @@ from .base import first_visible_key
 MAX_SPLITS = 32
 MIN_KEYS_PER_SPLIT = 256
 BLOCKS_PER_SM = 2
+GEN_MIN_ROWS = 128        # rows (tokens x query heads of a key head) of a sequence from which on the tcgen05 prompt kernel serves it
 
 
-def plan(ctx, device, H: int, KV: int, dk: int, dv: int, own_v: bool, window, skip=frozenset(), chunk=None) -> dict:
-    """``skip``: sequences of the step that get no items (another path serves them). ``window``, ``chunk``: what a row sees."""
-    key = ("flex", H, KV, dk, dv, own_v, window, chunk, tuple(sorted(skip)))
+def gen_ok(H: int, KV: int, dk: int, dv: int, page_size: int, v_share: int = 1, bias: bool = False, cap: bool = False) -> bool:
+    """True when portions of this form (values of their own; no slopes, temperature or gate) go to the tcgen05 prompt kernel."""
+    return ops.attn_portion_gen_ok(H, KV, dk, dv, v_share, page_size, bias, cap)
+
+
+def plan(ctx, device, H: int, KV: int, dk: int, dv: int, own_v: bool, window, skip=frozenset(), chunk=None, gen: bool = False) -> dict:
+    """``skip``: sequences of the step that get no items (another path serves them). ``window``, ``chunk``: what a row sees. ``gen``: what
+    ``gen_ok`` says of the form."""
+    key = ("flex", H, KV, dk, dv, own_v, window, chunk, gen, tuple(sorted(skip)))
     got = ctx.plans.get(key)
     if got is not None:
         return got
     per_item = ops.attn_flex_tokens(H, KV)
-    dec, por = [], []
+    gen_item = ops.attn_portion_tc05_tokens(H, KV) if gen else 0
+    dec, por, big = [], [], []
     qs, cl = ctx.h_q_start, ctx.h_ctx_len
     for s in range(ctx.num_seqs):
         if s in skip:
             continue
         row0, n = int(qs[s]), int(qs[s + 1] - qs[s])
         pos0 = int(cl[s]) - n
-        if n <= per_item:
+        if gen and n * (H // KV) >= GEN_MIN_ROWS:
+            big += [(s, row0 + b, min(gen_item, n - b), pos0 + b) for b in range(0, n, gen_item)]
+        elif n <= per_item:
             dec.append((s, row0, n, pos0))
         else:
             for b in range(0, n, per_item):
@@ -40,7 +51,7 @@ def plan(ctx, device, H: int, KV: int, dk: int, dv: int, own_v: bool, window, sk
     fixed = ctx.seq_cap is not None
     if fixed:                                         # fixed shapes: pad with empty items, shares by the shape alone
         dec += [(0, 0, 0, 0)] * (ctx.seq_cap - len(dec))
-    out = {"dec": None, "por": None, "nsplit": 1, "scratch": None, "dec_rows": 0}
+    out = {"dec": None, "por": None, "gen": None, "nsplit": 1, "scratch": None, "dec_rows": 0}
     tag = f"{H}_{KV}_{dk}_{dv}_{int(own_v)}_{window}" + (f"_c{chunk}" if chunk else "") + ("_rest" if skip else "")
     if dec:
         # blocks one item gets without shares: kv heads x parts of the query heads x slices of the value columns
@@ -64,6 +75,9 @@ def plan(ctx, device, H: int, KV: int, dk: int, dv: int, own_v: bool, window, sk
     if por:
         por.sort(key=lambda it: -(it[3] + it[2]))     # the items with most keys first: the last blocks to start are short
         out["por"] = ctx.upload_ints("flex_por_" + tag, np.asarray(por, dtype=np.int32)).view(-1, 4)
+    if big:
+        big.sort(key=lambda it: it[3] + it[2])        # this kernel starts with the last ones
+        out["gen"] = ctx.upload_ints("flex_gen_" + tag, np.asarray(big, dtype=np.int32)).view(-1, 4)
     ctx.plans[key] = out
     return out
 
@@ -79,3 +93,6 @@ def attend(pl: dict, q, k_cache, v_cache, block_table, out, page_size, seq_slots
     if pl["por"] is not None:
         ops.attn_flex(q, k_cache, v_cache, block_table, pl["por"], out, *args, dist_bias=dist_bias, sink=sink, status=status,
                       softcap=softcap, v_share=v_share, slopes=slopes, q_temp=q_temp, gate=gate, chunk=chunk or 0)
+    if pl["gen"] is not None:
+        ops.attn_portion_gen(q, k_cache, v_cache, block_table, pl["gen"], out, *args, dist_bias=dist_bias, sink=sink, status=status,
+                             softcap=softcap, v_share=v_share, chunk=chunk or 0)

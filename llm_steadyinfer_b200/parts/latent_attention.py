@@ -122,7 +122,7 @@ class LatentAttention(Mixer):
 
     def kernel_files(self, page_size):
         names = ("attention_general", "norm")
-        return names + (("gemm_f32",) if self.dtype == torch.float32 else ("attention_flex", "gemm_heads", "gemm_skinny", "gemm_rows", "gemm_tc05"))
+        return names + (("gemm_f32",) if self.dtype == torch.float32 else ("attention_flex", "attention_tc05", "gemm_heads", "gemm_skinny", "gemm_rows", "gemm_tc05"))
 
     def uses_flex(self) -> bool:
         """Attention on the tensor cores: bfloat16 and sizes in multiples of 8."""
@@ -131,6 +131,9 @@ class LatentAttention(Mixer):
     def expands(self) -> bool:
         return (self.uses_flex() and EXPAND_MIN_ROWS > 0
                 and ops.attn_flex_ok(self.H, self.H, self.dq + self.dr, self.dv, True))
+
+    def expands_on_tc05(self) -> bool:
+        return flex_plan.gen_ok(self.H, self.H, self.dq + self.dr, self.dv, 0)
 
     def prepare(self, ctx, cache):
         if not self.uses_flex() or cache.k is None:
@@ -151,7 +154,8 @@ class LatentAttention(Mixer):
         chosen = [s for s in range(ctx.num_seqs) if int(qs[s + 1] - qs[s]) >= EXPAND_MIN_ROWS]
         if not chosen:
             return none
-        per_item = ops.attn_flex_tokens(self.H, self.H)
+        gen = self.expands_on_tc05()
+        per_item = ops.attn_portion_tc05_tokens(self.H, self.H) if gen else ops.attn_flex_tokens(self.H, self.H)
         seqs, items, total = [], [], 0
         for e, s in enumerate(chosen):
             row0, n, end = int(qs[s]), int(qs[s + 1] - qs[s]), int(cl[s])
@@ -162,17 +166,19 @@ class LatentAttention(Mixer):
             for b in range(0, n, per_item):
                 items.append((e, row0 + b, min(per_item, n - b), keys - n + b))
             total += keys
-        items.sort(key=lambda it: -(it[3] + it[2]))
+        items.sort(key=lambda it: (it[3] + it[2]) * (1 if gen else -1))      # either kernel starts with the longest
         width = max(k for _, _, k, _ in seqs)
         tag = f"latent_exp_{self.H}_{self.dq}_{self.dr}_{self.dv}_{self.rk}"
         both = ctx.upload_ints(tag, np.concatenate([np.asarray(seqs, dtype=np.int32).reshape(-1),
                                                     np.asarray(items, dtype=np.int32).reshape(-1)]))
         seqs_d, items_d = both[:4 * len(seqs)].view(-1, 4), both[4 * len(seqs):].view(-1, 4)
-        # the expanded rows are "pages" of one key: row j of sequence e is page first_row(e) + j
-        table = ctx.buf(tag + "_table", (len(seqs), width), torch.int32)
-        torch.add(seqs_d[:, 1:2], torch.arange(width, dtype=torch.int32, device=self.device).view(1, -1), out=table)
+        if gen:                                              # the first of a sequence's rows is all that kernel asks for
+            table = seqs_d[:, 1:2]
+        else:                                                # the expanded rows are "pages" of one key: row j of sequence e is page first_row(e) + j
+            table = ctx.buf(tag + "_table", (len(seqs), width), torch.int32)
+            torch.add(seqs_d[:, 1:2], torch.arange(width, dtype=torch.int32, device=self.device).view(1, -1), out=table)
         return {"skip": frozenset(chosen), "all": len(chosen) == ctx.num_seqs, "total": total, "seqs": seqs_d,
-                "items": items_d, "table": table, "width": width}
+                "items": items_d, "table": table, "width": width, "gen": gen}
 
     def forward(self, x, ctx, cache):
         T = x.shape[0]
@@ -225,6 +231,10 @@ class LatentAttention(Mixer):
         linear(dense[:, :rk], self.uv.view(H * dv, rk), values, ctx.status)
         keys = ctx.buf("lat_keys", (n, H * (dq + dr)), self.dtype)
         ops.latent_expand_keys(plain, dense, keys, H, dq, dr, rk)
+        if ex["gen"]:
+            ops.attn_portion_gen(q_exp, keys, values, ex["table"], ex["items"], attn, 0, ex["table"].shape[0], H, H, dq + dr, dv, self.scale,
+                                 self.window or 0, sink=self.sink, status=ctx.status)
+            return
         ops.attn_flex(q_exp, keys.view(n, H, 1, dq + dr), values.view(n, H, 1, dv), ex["table"], ex["items"], attn, 1,
                       ex["table"].shape[0], H, H, dq + dr, dv, self.scale, self.window or 0, sink=self.sink, status=ctx.status)
 

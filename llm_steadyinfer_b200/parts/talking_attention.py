@@ -105,7 +105,11 @@ class TalkingAttention(Mixer):
     def kernel_files(self, page_size):
         if self.dtype == torch.float32:
             return ("qk_prepare", "attention_general", "gemm_f32")
-        return ("qk_prepare", "attention_flex" if self.uses_flex() else "attention_general", "gemm_skinny", "gemm_rows", "gemm_tc05")
+        return ("qk_prepare", "gemm_skinny", "gemm_rows", "gemm_tc05") + (
+            ("attention_flex", "attention_tma", "attention_tc05") if self.uses_flex() else ("attention_general",))
+
+    def gen_ok(self, page_size) -> bool:
+        return flex_plan.gen_ok(self.H, self.G, self.dk, self.wide, page_size, v_share=self.G)
 
     def uses_flex(self) -> bool:
         """On the tensor cores: bfloat16 and sizes in multiples of 8."""
@@ -114,7 +118,7 @@ class TalkingAttention(Mixer):
 
     def prepare(self, ctx, cache):
         if self.uses_flex() and cache.k is not None:
-            flex_plan.plan(ctx, self.device, self.H, self.G, self.dk, self.wide, True, self.window)
+            flex_plan.plan(ctx, self.device, self.H, self.G, self.dk, self.wide, True, self.window, gen=self.gen_ok(cache.page_size))
 
     def forward_heads(self, x, ctx, cache, out, scale: float = 1.0):
         """The gated heads, times ``scale``, into ``out`` [T, H * dv] (a view with a row stride): everything but W_o."""
@@ -129,7 +133,7 @@ class TalkingAttention(Mixer):
         a = ctx.buf("tattn_all", (T, H * self.wide), torch.float32)
         q = u[:, :self.nq]
         if self.uses_flex():
-            flex_plan.attend(flex_plan.plan(ctx, self.device, H, G, dk, self.wide, True, self.window), q, cache.k, cache.v,
+            flex_plan.attend(flex_plan.plan(ctx, self.device, H, G, dk, self.wide, True, self.window, gen=self.gen_ok(cache.page_size)), q, cache.k, cache.v,
                              cache.block_table, a, cache.page_size, ctx.seq_slots, H, G, dk, self.wide, self.scale, self.window,
                              sink=self.sink, status=ctx.status, v_share=G)
         else:

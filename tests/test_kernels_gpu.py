@@ -1278,6 +1278,129 @@ def test_few_row_product_at_ragged_k(M, N, K):
     assert (out.cpu().double() - x.double() @ w.double().t()).abs().max().item() <= 1e-5
 
 
+@pytest.mark.parametrize("H,KV,dk,dv,share,page,bias,cap,window,chunk,sink,n,pos0", [
+    (8, 2, 128, 128, 1, 16, 40, 0.0, 0, 0, True, 150, 0),          # a bias by distance, its table shorter than the context
+    (8, 2, 128, 128, 1, 8, 300, 0.0, 0, 0, False, 64, 203),        # a whole item behind a context
+    (6, 2, 72, 40, 1, 16, 7, 0.0, 50, 0, True, 131, 77),           # heads that do not fill a tile, sizes below a half
+    (3, 3, 64, 128, 1, 32, 33, 0.0, 0, 64, False, 300, 1),         # one head a key head, chunks
+    (16, 8, 64, 128, 2, 16, 0, 30.0, 100, 0, False, 190, 30),      # a soft limit, key heads that share values, a window
+    (8, 4, 128, 64, 4, 64, 0, 2.0, 0, 0, False, 129, 0),           # a limit that cuts (the quotient form)
+    (8, 2, 128, 256, 2, 16, 0, 0.0, 0, 0, True, 140, 12),          # values in two blocks
+    (4, 1, 40, 520, 1, 16, 0, 0.0, 33, 0, True, 70, 100),          # values in five, the last one narrow
+    (4, 4, 192, 128, 1, 0, 0, 0.0, 0, 0, True, 300, 17),           # rows of matrices, keys of three halves
+    (3, 3, 136, 72, 1, 0, 0, 0.0, 90, 0, False, 257, 40),          # the same at sizes that are no halves: boxes reach into the next head
+    (4, 2, 192, 128, 1, 16, 0, 0.0, 0, 0, False, 70, 129),         # wide keys in pages
+])
+@pytest.mark.parametrize("f32", [False, True])
+def test_portions_in_the_general_form_on_tcgen05(H, KV, dk, dv, share, page, bias, cap, window, chunk, sink, n, pos0, f32):
+    """The tcgen05 prompt kernel's general form against float64 on the same bf16 inputs, two sequences a launch, pages scattered over
+    a pool whose other pages hold numbers that would show. Probabilities meet the values as bf16 (2^-9 relative each) and results
+    are stored in bf16 or fp32: 2^-7 of the largest value is allowed, the plain kernels' bound."""
+    o = ops()
+    if not o.attn_portion_gen_ok(H, KV, dk, dv, share, page, bias > 0, cap > 0):
+        pytest.skip("no tensor-map encoder")
+    g = torch.Generator().manual_seed(H * 1000 + dk + n)
+    KVv, scale, ends = KV // share, 2.0 * dk ** -0.5, [pos0 + n, pos0 + n + 35]
+    starts = [pos0, pos0 + 35]
+    ks = [torch.randn(e, KV, dk, generator=g).to(torch.bfloat16) for e in ends]
+    vs = [torch.randn(e, KVv, dv, generator=g).to(torch.bfloat16) for e in ends]
+    q = torch.randn(2 * n + 3, H * dk, generator=g).to(torch.bfloat16)
+    rel = torch.randn(bias, H, generator=g) * 2 if bias else None
+    sk = torch.randn(H, generator=g) * 2 if sink else None
+    if page:
+        need = [-(-e // page) for e in ends]
+        pool = sum(need) + 3
+        order = torch.randperm(pool, generator=g).tolist()
+        kc = torch.full((pool, KV, page, dk), 50.0, dtype=torch.bfloat16)
+        vc = torch.full((pool, KVv, page, dv), 50.0, dtype=torch.bfloat16)
+        table = torch.full((2, max(need) + 2), -1, dtype=torch.int32)
+        for s in range(2):
+            first = max(0, starts[s] - window + 1) if window else (starts[s] // chunk * chunk if chunk else 0)
+            for b in range(need[s]):
+                pg = order.pop()
+                a, e = b * page, min(ends[s], (b + 1) * page)
+                kc[pg, :, :e - a], vc[pg, :, :e - a] = ks[s][a:e].transpose(0, 1), vs[s][a:e].transpose(0, 1)
+                table[s, b] = -1 if e <= first else pg               # pages before every row's window have been given back
+        k_in, v_in = kc.to(DEV), vc.to(DEV)
+    else:
+        k_in, v_in = torch.cat(ks).reshape(-1, KV * dk).to(DEV), torch.cat(vs).reshape(-1, KVv * dv).to(DEV)
+        table = torch.tensor([[0], [ends[0]]], dtype=torch.int32)
+    per, items = o.attn_portion_tc05_tokens(H, KV), []
+    for s, row0 in ((0, 1), (1, n + 2)):
+        items += [(s, row0 + b, min(per, n - b), starts[s] + b) for b in range(0, n, per)]
+    items.sort(key=lambda it: it[2] + it[3])
+    out = torch.full((2 * n + 3, H * dv), 7.0, dtype=torch.float32 if f32 else torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    o.attn_portion_gen(q.to(DEV), k_in, v_in, table.to(DEV), torch.tensor(items, dtype=torch.int32, device=DEV), out, page, 2, H, KV, dk, dv, scale,
+                       window, dist_bias=None if rel is None else rel.to(DEV), sink=None if sk is None else sk.to(DEV), status=status, softcap=cap,
+                       v_share=share, chunk=chunk)
+    assert status.item() == 0
+    got = out.cpu().double()
+    for s, row0 in ((0, 1), (1, n + 2)):
+        i, j = torch.arange(starts[s], ends[s])[:, None], torch.arange(ends[s])[None, :]
+        seen = j <= i
+        if window:
+            seen &= i - j < window
+        if chunk:
+            seen &= i // chunk == j // chunk
+        for h in range(H):
+            kh = h * KV // H
+            z = q[row0:row0 + n, h * dk:(h + 1) * dk].double() @ ks[s][:, kh].double().t() * scale
+            if cap:
+                z = cap * torch.tanh(z / cap)
+            if rel is not None:
+                z = z + rel[:, h].double()[(i - j).clamp(0, bias - 1)]
+            z = z.masked_fill(~seen, -math.inf)
+            m = z.amax(-1, keepdim=True)
+            den = torch.exp(z - m).sum(-1, keepdim=True) + (torch.exp(sk[h].double() - m) if sk is not None else 0.0)
+            want = torch.exp(z - m) / den @ vs[s][:, kh // share].double()
+            diff = (got[row0:row0 + n, h * dv:(h + 1) * dv] - want).abs().max().item()
+            assert diff <= 2 ** -7 * vs[s].abs().max().item(), (s, h, diff)
+    for r in (0, n + 1, 2 * n + 2):
+        assert bool((got[r] == 7.0).all()), "rows of no item stay as they are"
+
+
+@pytest.mark.parametrize("H,KV,hs,n,pos0,window,sink,blocks", [(6, 2, 128, 200, 5000, 0, True, 9), (8, 8, 64, 300, 4444, 0, False, 24), (4, 1, 96, 70, 6000, 4300, True, 9)])
+def test_portions_whose_keys_are_cut_over_blocks(H, KV, hs, n, pos0, window, sink, blocks):
+    """A long prompt's portion on the tcgen05 kernel with its items' keys cut into shares, against float64 (sampled rows) and against
+    whole items: probabilities and results are bf16, so 2^-7 of the largest value either way. Rows whose window lies behind a share's
+    keys get nothing from it."""
+    o = ops()
+    g = torch.Generator().manual_seed(n)
+    end, page, G = pos0 + n, 16, H // KV
+    need = -(-end // page)
+    table = torch.randperm(need + 2, generator=g)[:need].int().view(1, -1)
+    kc, vc = (torch.randn(need + 2, KV, page, hs, generator=g).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(n, H * hs, generator=g).to(torch.bfloat16)
+    sk = torch.randn(H, generator=g).to(DEV) if sink else None
+    per = o.attn_portion_tc05_tokens(H, KV)
+    items = [(0, b, min(per, n - b), pos0 + b) for b in range(0, n, per)]
+    first = lambda p: max(0, p - window + 1) // 128 * 128 if window else 0          # noqa: E731
+    tiles = [-(-(p0 + m - first(p0)) // 128) for _, _, m, p0 in items]
+    entries, cut, slots = o.cut_portions(tiles, KV, blocks)
+    assert len(cut) and (entries[:, 2] > 1).any() and len({(e[0], e[1]) for e in entries.tolist()}) == len(entries)
+    assert sorted(e[0] for e in entries.tolist() if e[1] == 0) == list(range(len(items))), "every item once"
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = []
+    for shares in (None, (torch.tensor(entries, device=DEV), torch.tensor(cut, device=DEV), slots,
+                          torch.full((o.attn_portion_share_floats(slots, KV, hs, hs),), float("nan"), device=DEV))):
+        out = torch.full((n, H * hs), 7.0, dtype=torch.bfloat16, device=DEV)
+        o.attn_portion_tc05(q.to(DEV), kc.to(DEV), vc.to(DEV), table.to(DEV), torch.tensor(items, dtype=torch.int32, device=DEV), out, page, 1, H, KV, hs,
+                            1.5 * hs ** -0.5, window, status=status, sink=sk, vs=hs, shares=shares)
+        outs.append(out.cpu().double())
+    assert status.item() == 0
+    k, v = (c[table[0].long()].transpose(0, 1).reshape(KV, -1, hs)[:, :end].double() for c in (kc, vc))
+    bound = 2 ** -7 * v.abs().max().item()
+    assert (outs[1] - outs[0]).abs().max().item() <= bound
+    for r in (0, 1, n // 2, n - 1):
+        lo = max(0, pos0 + r - window + 1) if window else 0
+        for h in range(H):
+            z = k[h // G, lo:pos0 + r + 1] @ q[r, h * hs:(h + 1) * hs].double() * 1.5 * hs ** -0.5
+            e = torch.exp(z - z.max())
+            den = e.sum() + (torch.exp(sk[h].cpu().double() - z.max()) if sink else 0.0)
+            assert (outs[1][r, h * hs:(h + 1) * hs] - e @ v[h // G, lo:pos0 + r + 1] / den).abs().max().item() <= bound
+
+
 @pytest.mark.parametrize("M,N,K", [(700, 1000, 96), (641, 961, 68), (705, 1001, 33)])
 def test_gemm_f32_over_both_tiles(M, N, K):
     """Enough tiles of 64 x 64 for every SM, rows of 16-byte words and not: against float64 (K fp32 sums of products of size one), and a
