@@ -12,7 +12,8 @@
 //                never depends on timing.
 //   moe_gemm     C[place] = act(A[row of place] W_e^T) for every place of expert e: a grouped product whose row tiles are
 //                found from the offsets by every block itself (blocks beyond the last tile leave). bf16 on mma.sync
-//                m16n8k16 with fp32 sums, tiles of 64 or 16 rows x 64 columns, three cp.async stages; fp32 on FFMA.
+//                m16n8k16 with fp32 sums: few places an expert stream its weights (moe_stream_kernel), more go by tiles of 64
+//                rows x 64 columns, three cp.async stages; fp32 on FFMA.
 //                act "glu_limited": W_e holds gate and up rows in turn (row 2i the gate of entry i, row 2i + 1 its up), and
 //                C[place, i] = g sigmoid(alpha g) (u + shift) with g = min(gate sum, limit), u = clamp(up sum, -limit, limit)
 //                (no limit, alpha 1 and shift 0: silu(gate) * up).
@@ -28,44 +29,96 @@ typedef __nv_bfloat16 bf16;
 
 // ---- router -------------------------------------------------------------------------------------------------------------
 // x [T, d]; w [E + extra, d] (router rows, then `extra` gate rows) in the compute dtype; ids int32 [T, top]; wts fp32
-// [T, top]; gates fp32 [T, extra]. mode 0: sigmoid scores; 1: softmax over the experts. One block a row.
-template <typename T>
-__global__ void __launch_bounds__(256) moe_route_kernel(const T* __restrict__ x, long long x_stride, const T* __restrict__ w,
-    int E, int extra, int d, int top, float scale, int mode, int renorm, float renorm_eps, int groups, int keep,
+// [T, top]; gates fp32 [T, extra]. mode 0: sigmoid scores; 1: softmax over the experts. A block takes RB rows, a warp a weight
+// row at a time for all of them. Few rows: one a block, as many warps as weight rows, and a warp's first 256 x ROUTE_AHEAD
+// weights, which do not depend on the kernel before, are in flight before the block waits for x. Many rows: four a block, so that
+// the weight rows are read from L2 a quarter as often. A row's sums run over k in the same order either way. Both are bound by
+// latency (a round trip for the weights, one for the row, the choice by one warp): measured
+// for four rows of 32 to 64 experts, d = 1,536 to 2,048: 5.8 to 6.7 us, where eight warps that read the weights after the wait took 15 to 18.
+#define ROUTE_AHEAD 4
+template <typename T, int RB>
+__global__ void __launch_bounds__(RB == 1 ? 1024 : 256) moe_route_kernel(const T* __restrict__ x, long long x_stride, const T* __restrict__ w,
+    int E, int extra, int d, int top, float scale, int mode, int renorm, float renorm_eps, int groups, int keep, int rows,
     const float* __restrict__ choice_bias, int* __restrict__ ids, float* __restrict__ wts, float* __restrict__ gates) {
-  extern __shared__ float rsm[];                       // the row [d], scores [E + extra], used [E], choice keys [E]
-  pdl_prologue();
-  float* xr = rsm;
-  float* sc = rsm + d;
-  float* used = sc + E + extra;
-  float* key = used + E;
-  const long long t = blockIdx.x;
+  extern __shared__ float rsm[];                       // rows [RB, d]; a row's scores [E + extra], used [E], choice keys [E] (and groups' scores)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int i = threadIdx.x; i < d; i += blockDim.x) xr[i] = to_f32<T>(x[t * x_stride + i]);
-  for (int e = threadIdx.x; e < E; e += blockDim.x) used[e] = 0.f;
+  const long long t0 = (long long)blockIdx.x * RB;
+  const int per = 3 * E + extra + (groups > 1 ? groups : 0);
+  float* const scores = rsm + (size_t)RB * d;
+  const bool wide = sizeof(T) == 2 && d % 8 == 0 && ((uintptr_t)w & 15) == 0;      // rows of 16-byte pieces: eight entries a load
+  uint4 ahead[ROUTE_AHEAD];
+  if (RB == 1 && wide && warp < E + extra) {
+#pragma unroll
+    for (int u = 0; u < ROUTE_AHEAD; ++u)
+      if (lane * 8 + u * 256 < d) ahead[u] = *reinterpret_cast<const uint4*>(w + (size_t)warp * d + lane * 8 + u * 256);
+  }
+  pdl_wait();
+  if (wide && x_stride % 8 == 0 && ((uintptr_t)x & 15) == 0) {
+    for (int i = threadIdx.x; i < RB * (d / 8); i += blockDim.x) {
+      const int r = i / (d / 8), at = (i - r * (d / 8)) * 8;
+      uint4 raw = make_uint4(0, 0, 0, 0);
+      if (t0 + r < rows) raw = *reinterpret_cast<const uint4*>(x + (t0 + r) * x_stride + at);
+      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) reinterpret_cast<float2*>(rsm + (size_t)r * d + at)[j] = __bfloat1622float2(h2[j]);
+    }
+  } else {
+    for (int i = threadIdx.x; i < RB * d; i += blockDim.x) {
+      const int r = i / d;
+      rsm[i] = t0 + r < rows ? to_f32<T>(x[(t0 + r) * x_stride + (i - r * d)]) : 0.f;
+    }
+  }
+  for (int i = threadIdx.x; i < RB * E; i += blockDim.x) scores[(i / E) * per + E + extra + i % E] = 0.f;
   __syncthreads();
   for (int e = warp; e < E + extra; e += nwarps) {
     const T* we = w + (size_t)e * d;
-    float acc = 0.f;
-    if (sizeof(T) == 2 && d % 8 == 0 && ((uintptr_t)w & 15) == 0) {      // rows of 16-byte pieces: eight entries a load
-      for (int i = lane * 8; i < d; i += 256) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(we + i);
-        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    float acc[RB];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = __bfloat1622float2(h2[j]);
-          acc = fmaf(f.x, xr[i + 2 * j], acc);
-          acc = fmaf(f.y, xr[i + 2 * j + 1], acc);
+    for (int r = 0; r < RB; ++r) acc[r] = 0.f;
+    auto piece = [&](const uint4& raw, int i) {
+      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+      for (int j = 0; j < 4; j += 2) {
+        const float2 f = __bfloat1622float2(h2[j]), h = __bfloat1622float2(h2[j + 1]);
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+          const float4 xv = *reinterpret_cast<const float4*>(rsm + (size_t)r * d + i + 2 * j);
+          acc[r] = fmaf(f.x, xv.x, acc[r]);
+          acc[r] = fmaf(f.y, xv.y, acc[r]);
+          acc[r] = fmaf(h.x, xv.z, acc[r]);
+          acc[r] = fmaf(h.y, xv.w, acc[r]);
         }
       }
+    };
+    if (wide) {
+      int from = 0;
+      if (RB == 1 && e == warp) {
+#pragma unroll
+        for (int u = 0; u < ROUTE_AHEAD; ++u)
+          if (lane * 8 + u * 256 < d) piece(ahead[u], lane * 8 + u * 256);
+        from = ROUTE_AHEAD * 256;
+      }
+#pragma unroll 4
+      for (int i = from + lane * 8; i < d; i += 256) piece(*reinterpret_cast<const uint4*>(we + i), i);
     } else {
-      for (int i = lane; i < d; i += 32) acc = fmaf(to_f32<T>(we[i]), xr[i], acc);
+      for (int i = lane; i < d; i += 32) {
+        const float f = to_f32<T>(we[i]);
+#pragma unroll
+        for (int r = 0; r < RB; ++r) acc[r] = fmaf(f, rsm[(size_t)r * d + i], acc[r]);
+      }
     }
-    acc = warp_sum(acc);
-    if (lane == 0) sc[e] = acc;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+      const float s = warp_sum(acc[r]);
+      if (lane == 0) scores[r * per + e] = s;
+    }
   }
   __syncthreads();
-  if (warp != 0) return;
+  if (warp >= RB || t0 + warp >= rows) return;           // a warp chooses for a row
+  const long long t = t0 + warp;
+  float* sc = scores + warp * per;
+  float* used = sc + E + extra;
+  float* key = used + E;
   for (int e = lane; e < extra; e += 32) gates[t * extra + e] = 1.f / (1.f + expf(-sc[E + e]));
   float zmax = -INFINITY, zsum = 0.f;
   if (mode == 1) {
@@ -103,9 +156,20 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const T* __restrict__ x,
   }
   float total = 0.f, mine = 0.f;
   int my_id = 0;
+  // up to 32 experts: a lane an expert, the largest of order-preserving whole numbers in one instruction
+  unsigned held = 0u;
+  if (E <= 32 && lane < E && used[lane] == 0.f) {
+    unsigned u = __float_as_uint(key[lane] + 0.f);       // (-0 becomes 0: equal keys tie)
+    held = max((u & 0x80000000u) ? ~u : (u | 0x80000000u), 1u);
+  }
   for (int c = 0; c < top; ++c) {
     float best = -INFINITY;
     int idx = -1;
+    if (E <= 32) {
+      const unsigned most = __reduce_max_sync(0xffffffffu, held);
+      if (most) idx = __ffs(__ballot_sync(0xffffffffu, held == most)) - 1;
+      if (lane == idx) held = 0u;
+    } else {
     for (int e = lane; e < E; e += 32)
       if (used[e] == 0.f && (idx < 0 || key[e] > best)) { best = key[e]; idx = e; }
 #pragma unroll
@@ -113,6 +177,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const T* __restrict__ x,
       const float ob = __shfl_xor_sync(0xffffffffu, best, o);
       const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
       if (oi >= 0 && (idx < 0 || ob > best || (ob == best && oi < idx))) { best = ob; idx = oi; }
+    }
     }
     if (idx < 0) idx = 0;                              // fewer experts than choices: never with a checked configuration
     const float z = sc[idx];
@@ -135,18 +200,22 @@ SI_EXPORT int si_moe_route(const void* x, int dtype, long long x_stride, const v
   if (E <= 0 || top <= 0 || top > E || top > 32 || extra < 0 || d <= 0 || mode < 0 || mode > 1) return -2;
   if (groups > 1 && (E % groups || keep < 1 || keep > groups || !choice_bias)) return -2;      // groups go by choice scores
   if (groups > 1 && (long long)keep * (E / groups) < top) return -2;
-  const size_t smem = (size_t)(d + 3 * E + extra + (groups > 1 ? groups : 0)) * sizeof(float);
+  // Four rows a block from the rows on that give every SM a block of four, where they fit (a fp32 copy of a row each).
+  const size_t per_row = (size_t)(d + 3 * E + extra + (groups > 1 ? groups : 0)) * sizeof(float);
+  const int rb = rows >= 4 * si_sm_count() && 4 * per_row <= 48 * 1024 ? 4 : 1;
+  const size_t smem = rb * per_row;
   if (smem > 160 * 1024) return -2;
-  const dim3 grid(rows), block(E + extra >= 8 ? 256 : 128);
+  const int warps = E + extra < 32 ? E + extra : 32;
+  const dim3 grid((rows + rb - 1) / rb), block(rb == 4 ? 256 : 32 * (rows <= si_sm_count() ? warps : (warps < 8 ? warps : 8)));
 #define ROUTE_LAUNCH(T)                                                                                                \
   {                                                                                                                  \
     static size_t configured = 0;                                                                                    \
     if (smem > 48 * 1024 && smem > configured) {                                                                     \
-      if (cudaFuncSetAttribute(moe_route_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -2; \
+      if (cudaFuncSetAttribute(moe_route_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -2; \
       configured = smem;                                                                                             \
     }                                                                                                                \
-    si_launch(moe_route_kernel<T>, grid, block, smem, stream, (const T*)x, x_stride, (const T*)w, E, extra, d, top, scale, \
-              mode, renorm, renorm_eps, groups, keep, choice_bias, ids, wts, gates);                                                           \
+    si_launch(rb == 4 ? moe_route_kernel<T, 4> : moe_route_kernel<T, 1>, grid, block, smem, stream, (const T*)x, x_stride, (const T*)w, E, extra, d, top, scale, \
+              mode, renorm, renorm_eps, groups, keep, rows, choice_bias, ids, wts, gates);                                             \
   }
   if (dtype == SI_BF16) ROUTE_LAUNCH(bf16) else ROUTE_LAUNCH(float)
 #undef ROUTE_LAUNCH
@@ -297,9 +366,7 @@ __device__ __forceinline__ bool moe_find_tile(const int* __restrict__ offsets, i
 }
 
 #define MOE_BN 64
-// A tile row in shared memory holds BK + 8 bf16 entries (fragment loads without bank conflicts). Tiles of 16 places stream
-// an expert's weights for a handful of rows: 64 entries of k a stage and four stages keep enough bytes in flight; tiles of
-// 64 places take 32 and three (static shared memory).
+// A tile row in shared memory holds BK + 8 bf16 entries (fragment loads without bank conflicts).
 
 __device__ __forceinline__ void moe_cp16(void* dst, const void* src, int bytes) {       // bytes < 16: the rest is zeros
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes));
@@ -323,8 +390,8 @@ __global__ void __launch_bounds__(128) moe_gemm_bf16_kernel(const bf16* __restri
   __syncthreads();
   const bf16* We = W + (size_t)e * N * K;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
-  constexpr int NT = BM == 64 ? BN / 8 : BN / 32;    // n-tiles of 8 columns a warp: warps over the rows, or over the columns
-  const int wr0 = BM == 64 ? warp * 16 : 0, wn0 = BM == 64 ? 0 : warp * (BN / 4);
+  constexpr int NT = BN / 8;                         // n-tiles of 8 columns a warp; warps over the rows
+  const int wr0 = warp * 16, wn0 = 0;
   float acc[NT][4];
 #pragma unroll
   for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
@@ -416,6 +483,166 @@ __global__ void __launch_bounds__(128) moe_gemm_bf16_kernel(const bf16* __restri
   }
 }
 
+// Few places an expert (decode rows, short portions): a stream of the chosen experts' weights, as gemm_skinny.cu streams a
+// matrix. A block takes 16 columns of one expert for up to 16 of its places; its eight warps take the 32-wide chunks of k in turn,
+// with a warp's loads of four chunks (both operands, 16 bytes a lane) in flight at once, straight into the fragments of
+// mma.sync m16n8k16 (the weights are its 16 rows, the places its 8 columns), and their sums are added in warp order. The places come
+// from the plan (offsets and rows), or, where a step has at most 32 (row, choice) pairs, straight from the ids: a pair is then a
+// place of its own, every block finds its expert's pairs by one warp instruction, and no plan is made.
+// Measured, an average of the two products of 2,048 columns and experts of 1,408: one row of two experts 22.3 -> 6.2 us, three rows
+// 24.2 -> 11.3, two rows of four experts 29.1 -> 15.7 (before: tiles of 16 places, a chain of K steps a block).
+__device__ __forceinline__ void moe_mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint4 moe_ld(const bf16* p, bool stream) {
+  uint4 v;
+  if (stream) asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  else asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+#define STREAM_WARPS 8
+template <int MT>
+__device__ __forceinline__ void moe_stream_tile(const bf16* __restrict__ A, long long a_stride, const int* src_row, const bf16* __restrict__ We,
+                                                int n0, int N, int K, float (*red)[2][32][4]) {
+  constexpr int U = MT == 1 ? 4 : 2;     // three blocks an SM: one's start and end under the others' loads
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const bf16* w0 = We + (size_t)min(n0 + g, N - 1) * K + t * 8;          // rows beyond N stand for the last one: never stored
+  const bf16* w1 = We + (size_t)min(n0 + 8 + g, N - 1) * K + t * 8;
+  const bf16* xr[MT];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) xr[mt] = A + (size_t)src_row[mt * 8 + g] * a_stride + t * 8;
+  float acc[MT][4];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
+  const int nchunks = (K + 31) >> 5;
+  for (int c = warp; c < nchunks; c += STREAM_WARPS * U) {
+    uint4 lo[U], hi[U], xb[U][MT];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (c + u * STREAM_WARPS) * 32;
+      lo[u] = hi[u] = make_uint4(0, 0, 0, 0);
+      if (k + t * 8 < K) { lo[u] = moe_ld(w0 + k, true); hi[u] = moe_ld(w1 + k, true); }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (c + u * STREAM_WARPS) * 32;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        xb[u][mt] = make_uint4(0, 0, 0, 0);
+        if (k + t * 8 < K) xb[u][mt] = moe_ld(xr[mt] + k, false);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c + u * STREAM_WARPS < nchunks) {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          moe_mma(acc[mt], lo[u].x, hi[u].x, lo[u].y, hi[u].y, xb[u][mt].x, xb[u][mt].y);
+          moe_mma(acc[mt], lo[u].z, hi[u].z, lo[u].w, hi[u].w, xb[u][mt].z, xb[u][mt].w);
+        }
+      }
+  }
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) red[warp][mt][lane][i] = acc[mt][i];
+}
+
+// ids given: at most 32 pairs of at most 16 rows, `choices` a row, a pair's row of A is pair / a_div; else offsets and a_rows.
+__global__ void __launch_bounds__(STREAM_WARPS * 32, 3) moe_stream_kernel(const bf16* __restrict__ A, long long a_stride,
+    const int* __restrict__ a_rows, const int* __restrict__ ids, int a_div, const bf16* __restrict__ W, void* __restrict__ C,
+    long long c_stride, int c_f32, const int* __restrict__ offsets, int P, int E, int N, int K, int act, float limit, float alpha,
+    float shift) {
+  __shared__ float red[STREAM_WARPS][2][32][4];
+  __shared__ int place[16], src_row[16], info[2];
+  pdl_prologue();
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    int e = -1, rows = 0, mine = -1;                     // lane l < 16: the tile's place l
+    if (ids) {
+      int id = lane < P ? ids[lane] : -1;
+      if (id < 0 || id >= E) id = -1;                    // (identity experts and none: no product)
+      const unsigned same = __match_any_sync(0xffffffffu, id);
+      const unsigned leaders = __ballot_sync(0xffffffffu, id >= 0 && __ffs(same) - 1 == lane);
+      if ((int)blockIdx.y < __popc(leaders)) {
+        const int lead = __fns(leaders, 0, blockIdx.y + 1);
+        e = __shfl_sync(0xffffffffu, id, lead);
+        const unsigned members = __shfl_sync(0xffffffffu, same, lead);
+        rows = min(__popc(members), 16);
+        if (lane < rows) mine = (int)__fns(members, 0, lane + 1);
+      }
+    } else {
+      int before = 0, first = 0;
+      for (int base = 0; base < E && e < 0; base += 32) {
+        const int x = base + lane;
+        const int a = x < E ? offsets[x] : 0, n = x < E ? offsets[x + 1] - a : 0;
+        const int tiles = (n + 15) / 16;
+        int upto = tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += v;
+        }
+        upto += before;
+        const unsigned past = __ballot_sync(0xffffffffu, (int)blockIdx.y < upto);
+        if (past) {
+          const int at = __ffs(past) - 1;
+          const int skip = ((int)blockIdx.y - (upto - tiles)) * 16;      // of lane `at`: places of the expert before this tile
+          first = __shfl_sync(0xffffffffu, a + skip, at);
+          rows = __shfl_sync(0xffffffffu, min(n - skip, 16), at);
+          e = base + at;
+        }
+        before = __shfl_sync(0xffffffffu, upto, 31);
+      }
+      if (e >= 0 && lane < rows) mine = first + lane;
+    }
+    const int head = __shfl_sync(0xffffffffu, mine, 0);
+    if (lane < 16) {                                     // places that are not there stand for the first one: never stored
+      const int p = mine >= 0 ? mine : head;
+      place[lane] = mine;
+      src_row[lane] = p < 0 ? 0 : ids ? p / a_div : a_rows ? a_rows[p] : p;
+    }
+    if (lane == 0) { info[0] = e; info[1] = rows; }
+  }
+  __syncthreads();
+  const int e = info[0], rows = info[1], n0 = blockIdx.x * 16;
+  if (e < 0) return;
+  const bf16* We = W + (size_t)e * N * K;
+  if (rows <= 8) moe_stream_tile<1>(A, a_stride, src_row, We, n0, N, K, red);
+  else moe_stream_tile<2>(A, a_stride, src_row, We, n0, N, K, red);
+  __syncthreads();
+  const bool pair = act == MOE_ACT_GLU_LIMITED;
+  // a thread adds the warps' sums of one column (or of a gate and its up, neighbours) of one place
+  const int per_place = pair ? 8 : 16;
+  for (int i = threadIdx.x; i < rows * per_place; i += STREAM_WARPS * 32) {
+    const int r = i / per_place, q = i % per_place, mt = r >> 3;
+    auto sum = [&](int col) {                            // column of the 16: fragment (lane (col % 8, r % 8 / 2), element)
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < STREAM_WARPS; ++w) v += red[w][mt][(col & 7) * 4 + ((r & 7) >> 1)][(col >> 3) * 2 + (r & 1)];
+      return v;
+    };
+    const size_t at = (size_t)place[r] * c_stride;
+    float v;
+    int n;
+    if (pair) {
+      n = n0 + 2 * q;
+      if (n + 1 >= N) continue;
+      v = moe_glu_limited(sum(2 * q), sum(2 * q + 1), limit, alpha, shift);
+      n >>= 1;
+    } else {
+      n = n0 + q;
+      if (n >= N) continue;
+      v = moe_act(sum(q), act);
+    }
+    if (c_f32) reinterpret_cast<float*>(C)[at + n] = v;
+    else reinterpret_cast<bf16*>(C)[at + n] = __float2bfloat16_rn(v);
+  }
+}
+
 // True 32-bit: tiles of 32 places x 64 columns, 16 entries of k at a time, a thread 2 x 4 results.
 __global__ void __launch_bounds__(256) moe_gemm_f32_kernel(const float* __restrict__ A, long long a_stride,
     const int* __restrict__ a_rows, const float* __restrict__ W, float* __restrict__ C, long long c_stride,
@@ -495,16 +722,30 @@ SI_EXPORT int si_moe_gemm(const void* A, int dtype, long long a_stride, const in
     return si_last_error();
   }
   const int wide = (K % 8 == 0 && a_stride % 8 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0) ? 1 : 0;
-  if (P < 32LL * E) {                                 // few rows an expert: tiles of 16 places
-    // (32 columns a block, twice the blocks, measured no faster: 0.61 against 0.58 ms for the 16 launches of a decode step)
-    const dim3 grid((P + 15) / 16 + E, ny), block(128);
-    si_launch(moe_gemm_bf16_kernel<16, 64, 64, 4>, grid, block, 0, stream, (const bf16*)A, a_stride, a_rows, (const bf16*)W, C, c_stride,
-              c_dtype == SI_F32 ? 1 : 0, offsets, E, N, K, act, wide, limit, alpha, shift);
+  if ((P < 32LL * E || P < 128) && wide) {              // few rows an expert, or few at all
+    const long long tiles = P < (P + 15) / 16 + E ? P : (P + 15) / 16 + E;       // no more can there be
+    if (tiles > 65535) return -2;
+    si_launch(moe_stream_kernel, dim3((N + 15) / 16, (unsigned)tiles), dim3(STREAM_WARPS * 32), 0, stream, (const bf16*)A, a_stride, a_rows,
+              nullptr, 1, (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, offsets, P, E, N, K, act, limit, alpha, shift);
   } else {
     const dim3 grid((P + 63) / 64 + E, ny), block(128);
     si_launch(moe_gemm_bf16_kernel<64, 64, 32, 3>, grid, block, 0, stream, (const bf16*)A, a_stride, a_rows, (const bf16*)W, C, c_stride,
               c_dtype == SI_F32 ? 1 : 0, offsets, E, N, K, act, wide, limit, alpha, shift);
   }
+  return si_last_error();
+}
+
+// The grouped product without a plan: P = rows x choices pairs, at most 32 of at most 16 rows; pair p of expert ids[p] reads row
+// p / a_div of A and writes row p of C. Pairs whose id is not below E are left alone. bf16; returns -2 for what it does not take.
+SI_EXPORT int si_moe_gemm_pairs(const void* A, long long a_stride, int a_div, const int* ids, const void* W, void* C, int c_dtype,
+                                long long c_stride, int P, int choices, int E, int N, int K, int act, float limit, float alpha,
+                                float shift, cudaStream_t stream) {
+  if (P <= 0) return 0;
+  if (E <= 0 || N <= 0 || K <= 0 || act < 0 || act > MOE_ACT_GLU_LIMITED || choices <= 0 || P % choices || P > 32 || P / choices > 16 || a_div <= 0) return -2;
+  if (act == MOE_ACT_GLU_LIMITED && (N % 2 || !(limit > 0.f))) return -2;
+  if (K % 8 || a_stride % 8 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return -2;
+  si_launch(moe_stream_kernel, dim3((N + 15) / 16, P < E ? P : E), dim3(STREAM_WARPS * 32), 0, stream, (const bf16*)A, a_stride, nullptr, ids, a_div,
+            (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, nullptr, P, E, N, K, act, limit, alpha, shift);
   return si_last_error();
 }
 
@@ -544,7 +785,8 @@ SI_EXPORT int si_moe_gather(const void* a, int dtype, long long a_stride, const 
 
 // ---- combine --------------------------------------------------------------------------------------------------------------
 // out[t, :] = sum_c wts[t, c] * Y[place_of[t, c], :] + gate[t] * shared[t, :]   (gate absent: 1; shared absent: none)
-// Y fp32 or the compute dtype; shared and out in the compute dtype. Sums in fp32, the choices in their own order.
+// Y fp32 or the compute dtype; shared and out in the compute dtype. Sums in fp32, the choices in their own order. No place_of: a
+// pair is its own place.
 template <typename TY, typename T>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const TY* __restrict__ Y, long long y_stride, const int* __restrict__ place_of,
     const float* __restrict__ wts, int top, const T* __restrict__ shared, long long shared_stride, const float* __restrict__ gate,
@@ -556,7 +798,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const TY* __restrict__
     float acc = 0.f;
     for (int c = 0; c < top; ++c) {
       const bool same = ids && ids[t * top + c] >= real;           // an identity expert: the row itself
-      const float y = same ? to_f32<T>(x[t * x_stride + i]) : to_f32<TY>(Y[(size_t)place_of[t * top + c] * y_stride + i]);
+      const float y = same ? to_f32<T>(x[t * x_stride + i]) : to_f32<TY>(Y[(size_t)(place_of ? place_of[t * top + c] : t * top + c) * y_stride + i]);
       acc = fmaf(wts[t * top + c], y, acc);
     }
     if (shared) acc = fmaf(gate ? gate[t * gate_stride] : 1.f, to_f32<T>(shared[t * shared_stride + i]), acc);

@@ -2004,21 +2004,50 @@ def moe_gemm(a, a_rows, w, out, offsets, act: str = "none", gathered=None, statu
         moe_gemm_tiles(a, a_rows, w, out, offsets, act, limit, alpha, shift)
 
 
+def moe_pairs_ok(x, w_up, w_down, T: int, top: int) -> bool:
+    """True when a step's (row, choice) pairs are few enough for ``moe_gemm_pairs``: bf16, at most 32 pairs of at most 16 rows,
+    sizes and rows in 16-byte pieces."""
+    return (x.dtype == torch.bfloat16 and T <= 16 and T * top <= 32 and w_up.shape[2] % 8 == 0 and w_down.shape[2] % 8 == 0
+            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
+
+
+def moe_gemm_pairs(a, ids, w, out, by_row: bool, act: str = "none", limit: float = 0.0, alpha: float = 1.702, shift: float = 1.0) -> None:
+    """The grouped product without a plan, for few pairs: out[p, :] = act(a[row, :] @ w[e]^T) for the pair p of ``ids`` int32
+    [T, top] that chose expert e, row = p / top (``by_row``: ``a`` [T, K]) or p (``a`` [T * top, K]). Pairs whose id is not below
+    E are left alone. ``out`` and ``act`` as for ``moe_gemm``."""
+    _cuda(a, ids, w, out)
+    _i32(ids, "ids")
+    _need(act in MOE_ACTS, f"moe_gemm_pairs: act {act!r} is not one of {sorted(MOE_ACTS)}")
+    E, N, K = w.shape
+    T, top = ids.shape
+    P = T * top
+    pair = act == "glu_limited"
+    _need(not pair or (N % 2 == 0 and limit > 0), "moe_gemm_pairs: glu_limited needs an even N and a positive limit")
+    _need(a.dtype == torch.bfloat16 and a.shape == (T if by_row else P, K) and a.stride(1) == 1 and w.is_contiguous() and w.dtype == a.dtype
+          and ids.is_contiguous(), "moe_gemm_pairs: a [rows, K], w [E, N, K]")
+    _need(out.shape == (P, N // 2 if pair else N) and out.stride(1) == 1 and out.dtype in (a.dtype, torch.float32), "moe_gemm_pairs: out must be [P, N]")
+    f = _fn("moe", "si_moe_gemm_pairs", [_c_p, _c_ll, _c_int, _c_p, _c_p, _c_p, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int,
+                                         _c_int, _c_f, _c_f, _c_f, _c_p])
+    _check(f(_ptr(a), a.stride(0), top if by_row else 1, _ptr(ids), _ptr(w), _ptr(out), _dt(out), out.stride(0), P, top, E, N, K,
+             MOE_ACTS[act], float(limit), float(alpha), float(shift), _stream()), f"moe_gemm_pairs(experts={E}, N={N}, K={K})")
+
+
 def moe_combine(y, place_of, wts, out, shared=None, gate=None, ids=None, real: int = 0, x=None) -> None:
     """out[t, :] = sum_c wts[t, c] * y[place_of[t, c], :] (+ gate[t] * shared[t, :]): ``y`` [P, d] (fp32 or out's dtype),
-    ``place_of`` int32 [T, top], ``wts`` fp32 [T, top], ``shared`` [T, d] in out's dtype or None, ``gate`` fp32 [T] (a strided
+    ``place_of`` int32 [T, top] (None: a pair is its own place), ``wts`` fp32 [T, top], ``shared`` [T, d] in out's dtype or None, ``gate`` fp32 [T] (a strided
     view; None: 1), ``out`` [T, d]. With ``ids`` (int32 [T, top]) a choice whose id is ``real`` or above is an identity expert:
     its result is the row ``x[t]`` itself (``x`` [T, d] in out's dtype) and ``y`` is not read there."""
     _cuda(y, place_of, wts, out, shared, gate, ids, x)
     if ids is not None:
         _i32(ids, "ids")
-        _need(ids.shape == tuple(place_of.shape) and ids.is_contiguous() and x is not None and x.shape == tuple(out.shape)
+        _need(ids.shape == tuple(wts.shape) and ids.is_contiguous() and x is not None and x.shape == tuple(out.shape)
               and x.stride(1) == 1 and x.dtype == out.dtype, "moe_combine: ids [T, top] with x [T, d]")
     _i32(place_of, "place_of")
     T, d = out.shape
     top = wts.shape[1]
     _need(y.shape[1] == d and y.stride(1) == 1 and out.stride(1) == 1 and y.dtype in (out.dtype, torch.float32), "moe_combine: y [P, d]")
-    _need(place_of.shape == (T, top) and wts.shape == (T, top) and wts.dtype == torch.float32 and wts.is_contiguous(), "moe_combine: wts, place_of")
+    _need(y.shape[0] >= T * top, "moe_combine: y [P, d]")
+    _need((place_of is None or place_of.shape == (T, top)) and wts.shape == (T, top) and wts.dtype == torch.float32 and wts.is_contiguous(), "moe_combine: wts, place_of")
     if shared is not None:
         _need(shared.shape == (T, d) and shared.stride(1) == 1 and shared.dtype == out.dtype, "moe_combine: shared must be [T, d]")
     if gate is not None:

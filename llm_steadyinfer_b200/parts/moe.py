@@ -137,18 +137,23 @@ class RoutedMLP(FeedForward):
         R = self.routes                                           # experts with weights, then the identity experts
         ops.moe_route(x, self.w_route, R, top, self.scale, ids, wts, gates, scores=self.scores, renorm=self.renorm,
                       choice_bias=self.choice_bias, renorm_eps=self.renorm_eps, groups=self.groups)
-        scratch = ctx.buf("moe_plan", (ops.moe_plan_ints(P, R),), torch.int32)
-        offsets = ctx.buf("moe_offsets", (R + 1,), torch.int32)
-        row_of = ctx.buf("moe_row_of", (P,), torch.int32)
-        place_of = ctx.buf("moe_place_of", (T, top), torch.int32)
-        ops.moe_plan(ids, R, scratch, offsets, row_of, place_of)
-        # the places of the identity experts lie behind offsets[E]: the grouped products never reach them
         act = ctx.buf("moe_act", (P, self.inter), self.dtype)
-        gathered = ctx.buf("moe_x", (P, self.hidden), self.dtype) if ops.moe_gemm_grouped_ok(x, self.w_up, act, P, self.act) else None
-        ops.moe_gemm(x, row_of, self.w_up, act, offsets, act=self.act, gathered=gathered, status=ctx.status,
-                     limit=self.limit, alpha=self.alpha, shift=self.shift)
         y = ctx.buf("moe_y", (P, self.hidden), torch.float32)
-        ops.moe_gemm(act, None, self.w_down, y, offsets, status=ctx.status)
+        place_of = None
+        if ops.moe_pairs_ok(x, self.w_up, self.w_down, T, top):  # few pairs: each its own place, no plan
+            ops.moe_gemm_pairs(x, ids, self.w_up, act, True, act=self.act, limit=self.limit, alpha=self.alpha, shift=self.shift)
+            ops.moe_gemm_pairs(act, ids, self.w_down, y, False)
+        else:
+            scratch = ctx.buf("moe_plan", (ops.moe_plan_ints(P, R),), torch.int32)
+            offsets = ctx.buf("moe_offsets", (R + 1,), torch.int32)
+            row_of = ctx.buf("moe_row_of", (P,), torch.int32)
+            place_of = ctx.buf("moe_place_of", (T, top), torch.int32)
+            ops.moe_plan(ids, R, scratch, offsets, row_of, place_of)
+            # the places of the identity experts lie behind offsets[E]: the grouped products never reach them
+            gathered = ctx.buf("moe_x", (P, self.hidden), self.dtype) if ops.moe_gemm_grouped_ok(x, self.w_up, act, P, self.act) else None
+            ops.moe_gemm(x, row_of, self.w_up, act, offsets, act=self.act, gathered=gathered, status=ctx.status,
+                         limit=self.limit, alpha=self.alpha, shift=self.shift)
+            ops.moe_gemm(act, None, self.w_down, y, offsets, status=ctx.status)
         shared = self.shared.forward(x, ctx) if self.shared is not None else None
         out = ctx.buf("moe_out", (T, self.hidden), self.dtype)
         ops.moe_combine(y, place_of, wts, out, shared=shared, gate=gates[:, 0] if gates is not None else None,

@@ -1268,6 +1268,44 @@ def test_sampling_over_cluster_sizes(V):
                 assert (float(c[got - 1]) if got else 0.0) - slack <= u < float(c[got]) + slack, (V, off, r, T, k, p)
 
 
+@pytest.mark.parametrize("act", ["none", "relu2", "glu_limited"])
+@pytest.mark.parametrize("T,top,E,N,K", [(1, 1, 3, 16, 8), (1, 2, 5, 40, 264), (5, 4, 4, 18, 1408), (8, 4, 9, 50, 2056), (16, 2, 40, 34, 520), (16, 2, 2, 64, 4096)])
+def test_experts_weights_streamed_for_few_places(T, top, E, N, K, act):
+    """The streaming grouped product at the edges of its tiles (columns and chunks of k that fill none, one to sixteen places an
+    expert, experts without any, ids of identity experts): pairs without a plan against float64, and with a plan to the same
+    bits. Sums of K products of bf16 numbers of size one in fp32: 1e-6 sqrt(K) of the sum, before the activation."""
+    g = torch.Generator().manual_seed(T * 100 + E)
+    a = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    w = (torch.randn(E, N, K, generator=g) / K ** 0.5).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(E + 1, generator=g)[:top] for _ in range(T)]).int()      # id E: an identity expert
+    o, P, pair = ops(), T * top, act == "glu_limited"
+    kw = {"limit": 0.7, "alpha": 1.5, "shift": 1.0} if pair else {}
+    out = torch.full((P, N // 2 if pair else N), 7.0, device=DEV)
+    assert o.moe_pairs_ok(a.to(DEV), w.to(DEV), w.to(DEV), T, top)
+    o.moe_gemm_pairs(a.to(DEV), ids.to(DEV), w.to(DEV), out, True, act, **kw)
+    own = torch.full_like(out, 7.0)                                # rows by pair instead of by row
+    o.moe_gemm_pairs(a.repeat_interleave(top, 0).to(DEV), ids.to(DEV), w.to(DEV), own, False, act, **kw)
+    assert torch.equal(own, out)
+    planned = torch.full_like(out, 7.0)
+    scratch = torch.zeros(o.moe_plan_ints(P, E + 1), dtype=torch.int32, device=DEV)
+    offsets, row_of = torch.zeros(E + 2, dtype=torch.int32, device=DEV), torch.zeros(P, dtype=torch.int32, device=DEV)
+    place_of = torch.zeros(T, top, dtype=torch.int32, device=DEV)
+    o.moe_plan(ids.to(DEV), E + 1, scratch, offsets, row_of, place_of)
+    o.moe_gemm_tiles(a.to(DEV), row_of, w.to(DEV), planned, offsets, act, **kw)
+    for p, e in enumerate(ids.flatten().tolist()):
+        if e == E:
+            assert bool((out[p] == 7.0).all())
+            continue
+        z = a[p // top].double() @ w[e].double().t()
+        if pair:
+            gv, uv = z[0::2].clamp(max=0.7), z[1::2].clamp(-0.7, 0.7)
+            z = gv * torch.sigmoid(1.5 * gv) * (uv + 1.0)
+        elif act == "relu2":
+            z = z.clamp(min=0) ** 2
+        assert (out[p].cpu().double() - z).abs().max().item() <= 2e-6 * K ** 0.5 * max(1.0, z.abs().max().item())
+        assert torch.equal(planned[place_of.view(-1)[p]], out[p])
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 48, 8), (3, 40, 264), (8, 96, 1408), (9, 64, 1416), (16, 128, 2816), (8, 64, 5632), (2, 5000, 768)])
 def test_few_row_product_at_ragged_k(M, N, K):
     """The few-row product where k fills no whole round of a block's loads, against float64 (fp32 sums of K products)."""
