@@ -62,7 +62,8 @@ def plan(ctx, device, H: int, KV: int, dk: int, dv: int, own_v: bool, window, sk
         if not own_v and slices > 1 and out["dec_rows"] <= 16:
             slices = -(-slices // 4)                  # a block's four warps take a slice each
         per = KV * ((H // KV) // gb) * slices
-        nsplit = max(1, min(MAX_SPLITS, BLOCKS_PER_SM * ops.sm_count(device) // (len(dec) * per)))
+        # keys that are their own values are wide (a latent): a tile is 32 of them, so a share may be half as many keys
+        nsplit = max(1, min(MAX_SPLITS if own_v else 2 * MAX_SPLITS, BLOCKS_PER_SM * ops.sm_count(device) // (len(dec) * per)))
         if not fixed:
             longest = max(d[3] + d[2] - first_visible_key(d[3], window, chunk) for d in dec)
             nsplit = min(nsplit, max(1, longest // MIN_KEYS_PER_SPLIT))
