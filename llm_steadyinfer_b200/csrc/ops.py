@@ -1748,11 +1748,13 @@ def channel_delta_groups_ok(dk: int, dv: int) -> bool:
     return ok
 
 
-def channel_delta_groups(xc, ba, b_off: int, dec, a_log, dt_bias, rec, sc, row_seq, q_start, num_seqs: int, G: int, H: int, dk: int) -> None:
+def channel_delta_groups(xc, ba, b_off: int, dec, a_log, dt_bias, rec, sc, row_seq, q_start, num_seqs: int, G: int, H: int, dk: int,
+                         a_off: int = -1) -> None:
     """``channel_delta_prepare`` for the recurrence in groups of four tokens (counted from each sequence's first row of the step). ``rec``
     fp32 [T, H, 3, dk] receives, with c the product of the group's decays up to the token and s that of those behind it, c k, c q and s k;
     ``sc`` fp32 [T, H, 8] beta and the token's inner products with the group's earlier tokens (k with k: 3, q with k, its own included: 4);
-    ``dec`` fp32 [T, H*dk] holds the raw decay values and, in the rows that start a group, receives the product of all its decays."""
+    ``dec`` fp32 [T, H*dk] holds the raw decay values and, in the rows that start a group, receives the product of all its decays.
+    ``a_off`` >= 0: one decay a head, whose raw values stand at ``ba[:, a_off:a_off + H]`` (``dt_bias`` [H]; ``dec`` is only written)."""
     _cuda(xc, ba, dec, a_log, dt_bias, rec, sc, row_seq, q_start)
     _i32(row_seq, "row_seq"); _i32(q_start, "q_start")
     T = xc.shape[0]
@@ -1760,11 +1762,12 @@ def channel_delta_groups(xc, ba, b_off: int, dec, a_log, dt_bias, rec, sc, row_s
     _need(ba.shape[0] == T and ba.stride(1) == 1 and ba.shape[1] >= b_off + H, "channel_delta_groups: ba rows")
     _need(dec.dtype == torch.float32 and dec.shape == (T, H * dk) and dec.stride(1) == 1, "channel_delta_groups: dec must be fp32 [T, H*dk]")
     _f32v(rec, "rec", T * H * 3 * dk); _f32v(sc, "sc", T * H * GROUP_SCALARS)
-    _f32v(a_log, "a_log", H); _f32v(dt_bias, "dt_bias", H * dk)
+    _f32v(a_log, "a_log", H); _f32v(dt_bias, "dt_bias", H * dk if a_off < 0 else H)
+    _need(a_off < 0 or ba.shape[1] >= a_off + H, "channel_delta_groups: ba rows")
     f = _fn("delta_rule", "si_channel_delta_groups",
-            [_c_p, _c_ll, _c_p, _c_int, _c_ll, _c_int, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
+            [_c_p, _c_ll, _c_p, _c_int, _c_ll, _c_int, _c_int, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int,
              _c_int, _c_p])
-    _check(f(_ptr(xc), xc.stride(0), _ptr(ba), _dt(ba), ba.stride(0), int(b_off), _ptr(dec), dec.stride(0), _ptr(a_log), _ptr(dt_bias),
+    _check(f(_ptr(xc), xc.stride(0), _ptr(ba), _dt(ba), ba.stride(0), int(b_off), int(a_off), _ptr(dec), dec.stride(0), _ptr(a_log), _ptr(dt_bias),
              _ptr(rec), _ptr(sc), _ptr(row_seq), _ptr(q_start), T, int(num_seqs), G, H, dk, _stream()), f"channel_delta_groups(heads={H}, dk={dk})")
 
 

@@ -110,7 +110,16 @@ class GatedDeltaRule(Mixer):
         bg = ctx.buf("delta_bg", (T, 2 * H + G), torch.float32)
         ops.delta_prepare(xc, u, self.b_off, self.a_off, self.a_log, self.dt_bias, bg, G, H, dk, dk ** -0.5)
         y = ctx.buf("delta_y", (T, self.nv), torch.float32)
-        ops.delta_scan(xc, bg, state, y, ctx.q_start, ctx.ctx_len, ctx.slots, ctx.seq_slots, G, H, dk, dv)
+        if row_kinds(ctx) & 2 and USE_GROUPS and ops.channel_delta_groups_ok(dk, dv):
+            # portions: the recurrence with a decay per channel, all channels of a head alike, four tokens at a time
+            dec = ctx.buf("delta_decay", (T, H * dk), torch.float32)
+            rec = ctx.buf("delta_groups", (T, H, 3, dk), torch.float32)
+            sc = ctx.buf("delta_scalars", (T, H, ops.GROUP_SCALARS), torch.float32)
+            ops.channel_delta_groups(xc, u, self.b_off, dec, self.a_log, self.dt_bias, rec, sc, ctx.row_seq, ctx.q_start, ctx.seq_slots,
+                                     G, H, dk, a_off=self.a_off)
+            ops.channel_delta_group_scan(rec, sc, dec, xc, state, y, ctx.q_start, ctx.ctx_len, ctx.slots, ctx.seq_slots, G, H, dk, dv)
+        else:
+            ops.delta_scan(xc, bg, state, y, ctx.q_start, ctx.ctx_len, ctx.slots, ctx.seq_slots, G, H, dk, dv)
         gated = ctx.buf("delta_gated", (T, self.nv), self.dtype)
         ops.head_norm_gate(y, u[:, self.g_off:self.g_off + self.nv], self.norm_w, gated, H, dv, self.eps)
         out = ctx.buf("delta", (T, self.hidden), self.dtype)

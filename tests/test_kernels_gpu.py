@@ -1439,6 +1439,43 @@ def test_portions_whose_keys_are_cut_over_blocks(H, KV, hs, n, pos0, window, sin
             assert (outs[1][r, h * hs:(h + 1) * hs] - e @ v[h // G, lo:pos0 + r + 1] / den).abs().max().item() <= bound
 
 
+@pytest.mark.parametrize("G,H,dk,dv", [(1, 2, 128, 128), (2, 2, 64, 40), (1, 3, 100, 12)])
+def test_gated_delta_portions_in_groups_of_four(G, H, dk, dv):
+    """The gated delta rule (one decay a head) by groups of four tokens against the token-by-token scan, both fp32: portions of 1 to 9
+    rows beside each other, from position 0 and going on from a slot. Unit keys and decays below one keep the state of the values'
+    size, so the two orders of the sums differ by some 1e-6 a token: 2e-5 of the largest value is allowed."""
+    o = ops()
+    if not o.channel_delta_groups_ok(dk, dv):
+        pytest.skip("sizes that go token by token")
+    g = torch.Generator().manual_seed(dk)
+    lens, starts = [9, 1, 4, 7, 2], [0, 5, 0, 3, 11]
+    T, S, C = sum(lens), len(lens), 2 * G * dk + H * dv
+    xc = torch.randn(T, C, generator=g).to(DEV)
+    u = torch.randn(T, 2 * H + 3, generator=g).to(DEV)
+    a_log, dt_bias = torch.rand(H, generator=g).to(DEV), (torch.rand(H, generator=g) * 4 - 5).to(DEV)
+    q_start = torch.tensor([sum(lens[:i]) for i in range(S + 1)], dtype=torch.int32, device=DEV)
+    ctx_len = torch.tensor([n + p for n, p in zip(lens, starts)], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([4, 0, 2, 1, 3], dtype=torch.int32, device=DEV)
+    row_seq = torch.repeat_interleave(torch.arange(S), torch.tensor(lens)).int().to(DEV)
+    bg = torch.empty(T, 2 * H + G, device=DEV)
+    o.delta_prepare(xc, u, 0, H, a_log, dt_bias, bg, G, H, dk, dk ** -0.5)
+    one = torch.zeros(S, H * o.delta_state_floats(dk, dv) + 8, device=DEV)
+    seen, was = torch.randn(sum(starts), C, generator=g).to(DEV), torch.randn(sum(starts), 2 * H + 3, generator=g).to(DEV)
+    before = torch.tensor([sum(starts[:i]) for i in range(S + 1)], dtype=torch.int32, device=DEV)
+    bg0 = torch.empty(sum(starts), 2 * H + G, device=DEV)
+    o.delta_prepare(seen, was, 0, H, a_log, dt_bias, bg0, G, H, dk, dk ** -0.5)
+    o.delta_scan(seen, bg0, one, torch.empty(sum(starts), H * dv, device=DEV), before, torch.tensor(starts, dtype=torch.int32, device=DEV), slots, S,
+                 G, H, dk, dv)                                     # what the slots hold
+    four = one.clone()
+    y1, y4 = torch.empty(T, H * dv, device=DEV), torch.full((T, H * dv), 7.0, device=DEV)
+    o.delta_scan(xc, bg, one, y1, q_start, ctx_len, slots, S, G, H, dk, dv)
+    dec, rec, sc = torch.empty(T, H * dk, device=DEV), torch.empty(T, H, 3, dk, device=DEV), torch.empty(T, H, o.GROUP_SCALARS, device=DEV)
+    o.channel_delta_groups(xc, u, 0, dec, a_log, dt_bias, rec, sc, row_seq, q_start, S, G, H, dk, a_off=H)
+    o.channel_delta_group_scan(rec, sc, dec, xc, four, y4, q_start, ctx_len, slots, S, G, H, dk, dv)
+    for a, b in ((y1, y4), (one, four)):
+        assert bool(torch.isfinite(b).all()) and (a - b).abs().max().item() <= 2e-5 * a.abs().max().item()
+
+
 @pytest.mark.parametrize("M,N,K", [(700, 1000, 96), (641, 961, 68), (705, 1001, 33)])
 def test_gemm_f32_over_both_tiles(M, N, K):
     """Enough tiles of 64 x 64 for every SM, rows of 16-byte words and not: against float64 (K fp32 sums of products of size one), and a
