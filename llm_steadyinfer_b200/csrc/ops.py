@@ -1633,6 +1633,33 @@ def decay_scan(xs, u, state, y, q_start, ctx_len, slots, num_seqs: int, H: int, 
     _check(f(_ptr(xs), xs.stride(0), _ptr(u), _ptr(state), state.stride(0), _ptr(y), y.stride(0), _ptr(q_start), _ptr(ctx_len),
              _ptr(slots), int(num_seqs), H, n, _stream()), f"decay_scan(heads={H}, n={n})")
 
+@_of_sizes
+def decay_groups_ok(n: int) -> bool:
+    """True when the recurrence by groups of four tokens takes heads of ``n`` rows."""
+    lib = build.load("time_mix")
+    lib.si_decay_groups_ok.restype = _c_int
+    return bool(lib.si_decay_groups_ok(_c_int(n)))
+
+
+def decay_group_scan(xs, u, sc, state, y, row_seq, q_start, ctx_len, slots, num_seqs: int, H: int, n: int) -> None:
+    """``decay_scan`` four tokens at a time (portions of several rows): the same state, the same result up to the order of its sums.
+    ``xs`` is used up; ``sc`` fp32 [T, H, 4] is scratch; ``row_seq`` int32 [T]."""
+    _cuda(xs, u, sc, state, y, row_seq, q_start, ctx_len, slots)
+    for t, nm in ((row_seq, "row_seq"), (q_start, "q_start"), (ctx_len, "ctx_len"), (slots, "slots")):
+        _i32(t, nm)
+    T, C = y.shape
+    _need(C == H * n and xs.dtype == torch.float32 and xs.shape == (T, 4 * C) and xs.stride(1) == 1 and row_seq.numel() >= T,
+          "decay_group_scan: xs must be fp32 [T, 4*H*n]")
+    _need(y.dtype == torch.float32 and y.stride(1) == 1 and state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
+          and state.shape[1] >= H * decay_state_floats(n), "decay_group_scan: y, state")
+    _f32v(u, "u", H * n); _f32v(sc, "sc", T * H * 4)
+    f = _fn("time_mix", "si_decay_groups", [_c_p, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p])
+    _check(f(_ptr(xs), xs.stride(0), _ptr(u), _ptr(sc), _ptr(row_seq), _ptr(q_start), T, int(num_seqs), H, n, _stream()), f"decay_groups(heads={H}, n={n})")
+    f = _fn("time_mix", "si_decay_group_scan", [_c_p, _c_ll, _c_p, _c_p, _c_ll, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p])
+    _check(f(_ptr(xs), xs.stride(0), _ptr(sc), _ptr(state), state.stride(0), _ptr(y), y.stride(0), _ptr(q_start), _ptr(ctx_len), _ptr(slots),
+             int(num_seqs), H, n, _stream()), f"decay_group_scan(heads={H}, n={n})")
+
+
 
 # ---- gated delta rule ------------------------------------------------------------------------------------------------
 

@@ -460,3 +460,268 @@ SI_EXPORT int si_decay_scan(const float* xs, long long xs_stride, const float* u
 #undef DECAY_LAUNCH
   return si_last_error();
 }
+
+// ---- the recurrence, four tokens at a time ---------------------------------------------------------------------------------
+// For portions of several rows. With c_i the product of a group's decays before token i, s_i that of those behind it, C that of all
+// four and S the state before the group (groups counted from the portion's start, the last one may be shorter):
+//   o_i = (c_i r_i) . S + sum_(j<i) (r_i . diag(w_(j+1) .. w_(i-1)) k_j) v_j + (r_i . diag(u) k_i) v_i;   S <- C S + sum_i (s_i k_i) v_i^T
+// which is the token-by-token recurrence written out, in fp32 and with products of decays alone. The reads of the state and the sums over
+// the lanes of four tokens and two columns go together, and what is a chain is one update of the state in four tokens.
+// Measured, three portions of up to 1,200 rows, 32 heads of 64: 240 us by the token, 157 so and 10 for the preparation.
+// Heads of 36 to 64 rows, where a thread's rows are four of one column as in decay_scan_kernel (the slot's layout is the same).
+#define DECAY_GROUP 4
+#define DECAY_GROUP_AHEAD 4
+
+// xs fp32 [T, 4C] = [r | k | v | decay] becomes [c r | s k | v | C in the rows that start a group]; sc fp32 [T, H, 4]: a token's factors
+// on the group's values. A warp takes a (group, head), a lane two rows.
+__global__ void __launch_bounds__(256) decay_groups_kernel(float* __restrict__ xs, long long xs_stride, const float* __restrict__ u,
+    float* __restrict__ sc, const int* __restrict__ row_seq, const int* __restrict__ q_start, int num_seqs, int H, int n) {
+  pdl_prologue();
+  const int t = blockIdx.x, h = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int seq = row_seq[t];
+  if (seq < 0 || seq >= num_seqs || h >= H) return;
+  if ((t - q_start[seq]) % DECAY_GROUP) return;
+  const int m = min(DECAY_GROUP, q_start[seq + 1] - t), C = H * n, i0 = 2 * lane;
+  const bool in = i0 < n;
+  float* base = xs + (size_t)t * xs_stride + (size_t)h * n + i0;
+  float2 r[4], k[4], w[4], uu = make_float2(0.f, 0.f);
+  if (in) uu = *reinterpret_cast<const float2*>(u + (size_t)h * n + i0);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    r[i] = k[i] = make_float2(0.f, 0.f);
+    w[i] = make_float2(1.f, 1.f);
+    if (in && i < m) {
+      const float* row = base + (size_t)i * xs_stride;
+      r[i] = *reinterpret_cast<const float2*>(row);
+      k[i] = *reinterpret_cast<const float2*>(row + C);
+      w[i] = *reinterpret_cast<const float2*>(row + 3 * (size_t)C);
+    }
+  }
+  float dots[16];                                          // (i, j <= i) at i (i + 1) / 2 + j
+#pragma unroll
+  for (int v = 0; v < 16; ++v) dots[v] = 0.f;
+  float2 c = make_float2(1.f, 1.f);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    dots[i * (i + 1) / 2 + i] = fmaf(r[i].x * uu.x, k[i].x, r[i].y * uu.y * k[i].y);
+    float2 b = k[i];                                       // k_i as the tokens behind it see it
+#pragma unroll
+    for (int l = i + 1; l < 4; ++l) {
+      dots[l * (l + 1) / 2 + i] = fmaf(r[l].x, b.x, r[l].y * b.y);
+      b.x *= w[l].x; b.y *= w[l].y;
+    }
+    if (in && i < m) {
+      float* row = base + (size_t)i * xs_stride;
+      *reinterpret_cast<float2*>(row) = make_float2(c.x * r[i].x, c.y * r[i].y);
+      *reinterpret_cast<float2*>(row + C) = b;
+    }
+    c.x *= w[i].x; c.y *= w[i].y;
+  }
+  if (in) *reinterpret_cast<float2*>(base + 3 * (size_t)C) = c;
+  // the sums over the warp by exchanging halves: lanes 2v and 2v + 1 end with sum v
+#pragma unroll
+  for (int half = 8, bit = 16; half > 0; half >>= 1, bit >>= 1) {
+    const bool up = lane & bit;
+#pragma unroll
+    for (int v = 0; v < half; ++v) {
+      const float keep = up ? dots[v + half] : dots[v], send = up ? dots[v] : dots[v + half];
+      dots[v] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+    }
+  }
+  const float dot = dots[0] + __shfl_xor_sync(0xffffffffu, dots[0], 1);
+  const int v = lane >> 1;
+  int i = 4, j = 0;
+  if (!(lane & 1)) { if (v < 10) { i = v < 1 ? 0 : v < 3 ? 1 : v < 6 ? 2 : 3; j = v - i * (i + 1) / 2; } }
+  else if (v < 6) { i = v < 3 ? 0 : v < 5 ? 1 : 2; j = v < 3 ? 1 + v : v < 5 ? v - 1 : 3; }      // j > i: zeros
+  if (i < m) sc[((size_t)(t + i) * H + h) * 4 + j] = (lane & 1) ? 0.f : dot;
+}
+
+// A thread keeps four rows of two neighbouring columns of S; the sixteen parts of a column pair are neighbouring lanes. Shared memory:
+// two buffers of DECAY_GROUP_AHEAD groups of 4 x [c r: 64 | s k: 64 | v: cols | factors: 4] and C: 64.
+template <int SLOTS>
+__global__ void __launch_bounds__(256, 2) decay_group_scan_kernel(const float* __restrict__ xs, long long xs_stride,
+    const float* __restrict__ sc, float* __restrict__ state, long long state_stride, float* __restrict__ y, long long y_stride,
+    const int* __restrict__ q_start, const int* __restrict__ ctx_len, const int* __restrict__ slots, int H, int n, int cols) {
+  extern __shared__ __align__(16) float sm[];
+  pdl_prologue();
+  constexpr int NP = 16, M = DECAY_GROUP, DKP = 64;
+  const int s = blockIdx.x, h = blockIdx.y, j0 = blockIdx.z * cols;
+  const int row0 = q_start[s], cnt = q_start[s + 1] - row0;
+  if (cnt <= 0) return;
+  const int pos0 = ctx_len[s] - cnt, groups = (cnt + M - 1) / M, C = H * n;
+  const int p = threadIdx.x % NP, jc = threadIdx.x / NP * 2, j = j0 + jc;
+  const int TOK = 2 * DKP + cols + 4, GROUP = M * TOK + DKP;
+  float* S = state + (size_t)slots[s] * state_stride + (size_t)h * DKP * n + p;
+  const size_t s_step = (size_t)n * NP;
+  float2 st[2][2];
+  bool ok[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    ok[c] = j + c < n;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const float* src = S + (size_t)(2 * r) * s_step + (size_t)(j + c) * NP;
+      st[c][r].x = (ok[c] && pos0 > 0) ? src[0] : 0.f;
+      st[c][r].y = (ok[c] && pos0 > 0) ? src[s_step] : 0.f;
+    }
+  }
+  for (int idx = threadIdx.x; idx < 2 * DECAY_GROUP_AHEAD * GROUP; idx += blockDim.x) sm[idx] = 0.f;      // rows beyond n stay zero
+  __syncthreads();
+  const int pr = 2 * n / 4, pv = cols / 4, per = pr + pv + 1, pieces = M * per + n / 4;
+  const float* src[SLOTS];
+  int dst[SLOTS], tok[SLOTS];                             // place in a group; token of the group (-1: no piece)
+  unsigned step[SLOTS];                                   // entries from group to group
+#pragma unroll
+  for (int q = 0; q < SLOTS; ++q) {
+    const int idx = threadIdx.x + q * blockDim.x;
+    src[q] = xs; dst[q] = 0; tok[q] = -1; step[q] = (unsigned)(M * xs_stride);
+    if (idx < M * per) {
+      const int i = idx / per, e = idx - i * per;
+      const float* row = xs + (size_t)(row0 + i) * xs_stride;
+      tok[q] = i;
+      if (e < pr) {
+        const int part = e / (n / 4), at = (e - part * (n / 4)) * 4;
+        src[q] = row + (size_t)part * C + (size_t)h * n + at;
+        dst[q] = i * TOK + part * DKP + at;
+      } else if (e < pr + pv) {
+        const int at = (e - pr) * 4;
+        if (j0 + at >= n) tok[q] = -1;                    // columns beyond the head's
+        src[q] = row + (size_t)2 * C + (size_t)h * n + j0 + at;
+        dst[q] = i * TOK + 2 * DKP + at;
+      } else {
+        src[q] = sc + ((size_t)(row0 + i) * H + h) * 4;
+        dst[q] = i * TOK + 2 * DKP + cols;
+        step[q] = (unsigned)(M * H * 4);
+      }
+    } else if (idx < pieces) {
+      const int at = (idx - M * per) * 4;
+      tok[q] = 0;
+      src[q] = xs + (size_t)row0 * xs_stride + (size_t)3 * C + (size_t)h * n + at;
+      dst[q] = M * TOK + at;
+    }
+  }
+  auto fetch = [&](int g0, int buf) {                     // groups in order: the sources move on
+    for (int a = 0; a < DECAY_GROUP_AHEAD; ++a) {
+      if (g0 + a >= groups) break;
+      float* base = sm + (size_t)(buf * DECAY_GROUP_AHEAD + a) * GROUP;
+      const int left = cnt - (g0 + a) * M;                // tokens of the portion from this group on
+#pragma unroll
+      for (int q = 0; q < SLOTS; ++q) {
+        if (tok[q] >= 0) {
+          const int bytes = tok[q] < left ? 16 : 0;       // tokens behind the portion are zeros
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(base + dst[q])),
+                       "l"(bytes ? src[q] : xs), "r"(bytes));
+          src[q] += step[q];
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  fetch(0, 0);
+  const int my_i = (p >> 1) & 3, my_c = p & 1;
+  float* yp = y + (size_t)(row0 + my_i) * y_stride + (size_t)h * n + j + my_c;
+  const bool writes = p < 8 && j + my_c < n;
+  int buf = 0;
+  for (int g0 = 0; g0 < groups; g0 += DECAY_GROUP_AHEAD, buf ^= 1) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();                                      // these groups have arrived, and everyone is done with the other buffer
+    if (g0 + DECAY_GROUP_AHEAD < groups) fetch(g0 + DECAY_GROUP_AHEAD, buf ^ 1);
+    const int ga = min(DECAY_GROUP_AHEAD, groups - g0);
+    for (int a = 0; a < ga; ++a) {
+      const float* base = sm + (size_t)(buf * DECAY_GROUP_AHEAD + a) * GROUP;
+      float val[8];                                       // [token | column]
+      float2 vv[M];
+#pragma unroll
+      for (int i = 0; i < M; ++i) {
+        const float4 rv = reinterpret_cast<const float4*>(base + i * TOK)[p];
+        vv[i] = *reinterpret_cast<const float2*>(base + i * TOK + 2 * DKP + jc);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const float2 x = __ffma2_rn(make_float2(rv.z, rv.w), st[c][1], __fmul2_rn(make_float2(rv.x, rv.y), st[c][0]));
+          val[2 * i + c] = x.x + x.y;
+        }
+      }
+#pragma unroll
+      for (int half = 4; half > 0; half >>= 1) {
+        const bool up = p & half;
+#pragma unroll
+        for (int v = 0; v < half; ++v) {
+          const float keep = up ? val[v + half] : val[v], send = up ? val[v] : val[v + half];
+          val[v] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+        }
+      }
+      float o = val[0] + __shfl_xor_sync(0xffffffffu, val[0], 8);
+      const float4 f = *reinterpret_cast<const float4*>(base + my_i * TOK + 2 * DKP + cols);      // zeros behind token my_i
+      o = fmaf(f.x, my_c ? vv[0].y : vv[0].x, o);
+      o = fmaf(f.y, my_c ? vv[1].y : vv[1].x, o);
+      o = fmaf(f.z, my_c ? vv[2].y : vv[2].x, o);
+      o = fmaf(f.w, my_c ? vv[3].y : vv[3].x, o);
+      if (writes && (g0 + a) * M + my_i < cnt) *yp = o;
+      yp += M * y_stride;
+      const float4 cv = reinterpret_cast<const float4*>(base + M * TOK)[p];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        st[c][0] = __fmul2_rn(make_float2(cv.x, cv.y), st[c][0]);
+        st[c][1] = __fmul2_rn(make_float2(cv.z, cv.w), st[c][1]);
+      }
+#pragma unroll
+      for (int i = 0; i < M; ++i) {
+        const float4 kv = reinterpret_cast<const float4*>(base + i * TOK + DKP)[p];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const float2 u2 = c ? make_float2(vv[i].y, vv[i].y) : make_float2(vv[i].x, vv[i].x);
+          st[c][0] = __ffma2_rn(make_float2(kv.x, kv.y), u2, st[c][0]);
+          st[c][1] = __ffma2_rn(make_float2(kv.z, kv.w), u2, st[c][1]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+    if (ok[c]) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        float* d = S + (size_t)(2 * r) * s_step + (size_t)(j + c) * NP;
+        d[0] = st[c][r].x;
+        d[s_step] = st[c][r].y;
+      }
+    }
+}
+
+// 1 when the form by groups takes heads of n rows: four rows a thread in sixteen parts.
+SI_EXPORT int si_decay_groups_ok(int n) {
+  if (n <= 0 || n > 64 || n % 4) return 0;
+  const DecayShape s = decay_shape(n);
+  return s.rpt == 4 && s.np == 16;
+}
+
+SI_EXPORT int si_decay_groups(float* xs, long long xs_stride, const float* u, float* sc, const int* row_seq, const int* q_start, int num_tokens,
+                              int num_seqs, int H, int n, cudaStream_t stream) {
+  if (num_tokens <= 0) return 0;
+  if (H <= 0 || !si_decay_groups_ok(n) || xs_stride % 4 || (((uintptr_t)xs | (uintptr_t)sc) & 15) || ((uintptr_t)u & 7)) return -2;
+  si_launch(decay_groups_kernel, dim3(num_tokens, (H + 7) / 8), dim3(H >= 8 ? 256 : 32 * H), 0, stream, xs, xs_stride, u, sc, row_seq, q_start,
+            num_seqs, H, n);
+  return si_last_error();
+}
+
+SI_EXPORT int si_decay_group_scan(const float* xs, long long xs_stride, const float* sc, float* state, long long state_stride, float* y,
+                                  long long y_stride, const int* q_start, const int* ctx_len, const int* slots, int num_seqs, int H, int n,
+                                  cudaStream_t stream) {
+  if (num_seqs <= 0) return 0;
+  if (H <= 0 || H > 65535 || !si_decay_groups_ok(n) || state_stride < (long long)H * 64 * n || xs_stride % 4 || 4 * xs_stride >= (1LL << 31)) return -2;
+  if (((uintptr_t)xs | (uintptr_t)sc) & 15) return -2;
+  // columns a block: 32, 16 while the blocks do not fill the device
+  const int cols = (long long)num_seqs * H * ((n + 31) / 32) < si_sm_count() ? 16 : 32;
+  const size_t smem = (size_t)2 * DECAY_GROUP_AHEAD * (DECAY_GROUP * (128 + cols + 4) + 64) * sizeof(float);
+  const int pieces = DECAY_GROUP * (2 * n / 4 + cols / 4 + 1) + n / 4, threads = cols * 8;
+  const dim3 grid(num_seqs, H, (n + cols - 1) / cols);
+  if (pieces <= threads)
+    si_launch(decay_group_scan_kernel<1>, grid, dim3(threads), smem, stream, xs, xs_stride, sc, state, state_stride, y, y_stride, q_start, ctx_len,
+              slots, H, n, cols);
+  else if (pieces <= 2 * threads)
+    si_launch(decay_group_scan_kernel<2>, grid, dim3(threads), smem, stream, xs, xs_stride, sc, state, state_stride, y, y_stride, q_start, ctx_len,
+              slots, H, n, cols);
+  else
+    return -2;
+  return si_last_error();
+}

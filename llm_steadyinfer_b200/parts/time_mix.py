@@ -20,6 +20,7 @@ import torch
 from ..csrc import ops
 from .base import Mixer, StateNeed, register_mixer
 from .linear import linear, linear_batched
+from .step_rows import row_kinds
 
 MIXES = ("r", "k", "v", "g", "w")
 
@@ -96,7 +97,11 @@ class TimeMix(Mixer):
         xs = ctx.buf("tmix_xs", (T, 4 * C), torch.float32)
         ops.time_mix_prepare(proj[0], proj[1], proj[2], z[:, :self.L], self.w2t, self.w0, xs)
         y = ctx.buf("tmix_y", (T, C), torch.float32)
-        ops.decay_scan(xs, self.u, state, y, ctx.q_start, ctx.ctx_len, ctx.slots, ctx.seq_slots, H, n)
+        if row_kinds(ctx) & 2 and ops.decay_groups_ok(n):       # portions: four tokens at a time
+            sc = ctx.buf("tmix_factors", (T, H, 4), torch.float32)
+            ops.decay_group_scan(xs, self.u, sc, state, y, ctx.row_seq, ctx.q_start, ctx.ctx_len, ctx.slots, ctx.seq_slots, H, n)
+        else:
+            ops.decay_scan(xs, self.u, state, y, ctx.q_start, ctx.ctx_len, ctx.slots, ctx.seq_slots, H, n)
         ops.head_norm_gate(y, proj[3], self.norm_w, out, H, n, self.eps, post=scale)
 
     def forward(self, x, ctx, cache):

@@ -1476,6 +1476,38 @@ def test_gated_delta_portions_in_groups_of_four(G, H, dk, dv):
         assert bool(torch.isfinite(b).all()) and (a - b).abs().max().item() <= 2e-5 * a.abs().max().item()
 
 
+@pytest.mark.parametrize("H,n", [(2, 64), (9, 36), (1, 44)])
+def test_decaying_state_in_groups_of_four(H, n):
+    """Time mixing's recurrence by groups of four tokens against the token-by-token scan, both fp32: portions of 1 to 9 rows beside each
+    other, from position 0 and going on from a slot. Sums of n products in another order: 2e-5 of the largest value is allowed."""
+    o = ops()
+    assert o.decay_groups_ok(n)
+    g = torch.Generator().manual_seed(n)
+    lens, starts = [9, 1, 4, 7, 2], [0, 5, 0, 3, 11]
+    T, S, C = sum(lens), len(lens), H * n
+    xs = torch.randn(T, 4 * C, generator=g)
+    xs[:, 3 * C:] = 1.0 - 0.3 * torch.rand(T, C, generator=g)
+    xs = xs.to(DEV)
+    u = torch.randn(H, n, generator=g).to(DEV)
+    q_start = torch.tensor([sum(lens[:i]) for i in range(S + 1)], dtype=torch.int32, device=DEV)
+    ctx_len = torch.tensor([m + p for m, p in zip(lens, starts)], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([4, 0, 2, 1, 3], dtype=torch.int32, device=DEV)
+    row_seq = torch.repeat_interleave(torch.arange(S), torch.tensor(lens)).int().to(DEV)
+    width = H * o.decay_state_floats(n) + 8
+    one = torch.zeros(S, width, device=DEV)
+    seen = torch.randn(sum(starts), 4 * C, generator=g)
+    seen[:, 3 * C:] = 0.9
+    before = torch.tensor([sum(starts[:i]) for i in range(S + 1)], dtype=torch.int32, device=DEV)
+    y0 = torch.empty(sum(starts), C, device=DEV)
+    o.decay_scan(seen.to(DEV), u, one, y0, before, torch.tensor(starts, dtype=torch.int32, device=DEV), slots, S, H, n)      # what the slots hold
+    four = one.clone()
+    y1, y4 = torch.empty(T, C, device=DEV), torch.full((T, C), 7.0, device=DEV)
+    o.decay_scan(xs, u, one, y1, q_start, ctx_len, slots, S, H, n)
+    o.decay_group_scan(xs.clone(), u, torch.empty(T, H, 4, device=DEV), four, y4, row_seq, q_start, ctx_len, slots, S, H, n)
+    for a, b in ((y1, y4), (one, four)):
+        assert bool(torch.isfinite(b).all()) and (a - b).abs().max().item() <= 2e-5 * a.abs().max().item()
+
+
 @pytest.mark.parametrize("M,N,K", [(700, 1000, 96), (641, 961, 68), (705, 1001, 33)])
 def test_gemm_f32_over_both_tiles(M, N, K):
     """Enough tiles of 64 x 64 for every SM, rows of 16-byte words and not: against float64 (K fp32 sums of products of size one), and a
