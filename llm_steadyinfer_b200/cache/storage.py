@@ -10,6 +10,7 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import List, Optional
 
+import numpy as np
 import torch
 
 from .manager import CacheLayout, CacheManager
@@ -42,6 +43,11 @@ class CacheStorage:
             # a group without values of their own (value_dim 0) has no second tensor
             vshape = (len(grp.layers), grp.pool.num_pages, grp.need.v_heads, ps, grp.need.v_dim)
             self.values.append(torch.zeros(vshape, dtype=dtype, device=self.device) if grp.need.v_dim else None)
+        # every place's view of its group's tensors, made once: a step asks for all of them
+        self._pages = []
+        for i in range(len(layout.needs)):
+            g, j = layout.layer_group[i], layout.layer_index_in_group[i]
+            self._pages.append(None if g is None else (g, self.keys[g][j], None if self.values[g] is None else self.values[g][j]))
         self.states: List[Optional[torch.Tensor]] = []
         for s in layout.states:
             self.states.append(None if s is None else torch.zeros(
@@ -51,11 +57,16 @@ class CacheStorage:
         n = sum(t.numel() * t.element_size() for t in self.keys + self.values if t is not None)
         return n + sum(t.numel() * t.element_size() for t in self.states if t is not None)
 
-    def zero_new_slots(self) -> None:
-        """State of requests admitted (or reset) since the last call starts at zero."""
+    def zero_new_slots(self, upload=None) -> None:
+        """State of requests admitted (or reset) since the last call starts at zero. ``upload(key, values, capacity)``: a device copy of
+        a small int32 array that the host does not wait for (None: a copy that it waits for)."""
         slots = self.manager.new_slots
         if slots and any(t is not None for t in self.states):
-            idx = torch.tensor(sorted(set(slots)), dtype=torch.long, device=self.device)
+            fresh = sorted(set(slots))
+            if upload is None:
+                idx = torch.tensor(fresh, dtype=torch.long, device=self.device)
+            else:
+                idx = upload("new_slots", np.asarray(fresh, dtype=np.int32), self.manager.slots.num_slots).to(torch.long)
             for t in self.states:
                 if t is not None:
                     t.index_fill_(0, idx, 0)
@@ -65,12 +76,10 @@ class CacheStorage:
         """``tables[g]``: this step's device block table of group g."""
         views = []
         ps = self.manager.page_size
-        for i in range(len(self.layout.needs)):
-            g = self.layout.layer_group[i]
-            if g is None:
+        for i, pages in enumerate(self._pages):
+            if pages is None:
                 views.append(LayerCache(None, None, None, ps, False, self.states[i], None))
-                continue
-            j = self.layout.layer_index_in_group[i]
-            views.append(LayerCache(self.keys[g][j], None if self.values[g] is None else self.values[g][j], tables[g], ps,
-                                    self.layout.cache_from[i] is None, self.states[i], g))
+            else:
+                g, k, v = pages
+                views.append(LayerCache(k, v, tables[g], ps, self.layout.cache_from[i] is None, self.states[i], g))
         return views

@@ -410,6 +410,7 @@ def selftest_wait_runs_out(status, limit: int = 4096, gave_up=None) -> None:
 _c_llr = ctypes.c_longlong
 
 
+@_of_sizes
 def attn_portion_tokens(H: int, KV: int, hs: int) -> int:
     """Most tokens of one item of the portion kernel (0: this head layout is not supported)."""
     lib = build.load("attention_mma")
@@ -417,6 +418,7 @@ def attn_portion_tokens(H: int, KV: int, hs: int) -> int:
     return lib.si_attn_portion_tokens(_c_int(H), _c_int(KV), _c_int(hs))
 
 
+@_of_sizes
 def attn_decode_rows(H: int, KV: int, hs: int) -> int:
     """Rows (tokens * heads per kv head) one item of the decode kernel may have; 0: none."""
     lib = build.load("attention_mma")
@@ -424,6 +426,7 @@ def attn_decode_rows(H: int, KV: int, hs: int) -> int:
     return lib.si_attn_decode_rows(_c_int(H), _c_int(KV), _c_int(hs))
 
 
+@_of_sizes
 def attn_decode_scratch_floats(num_items: int, H: int, KV: int, hs: int, nsplit: int) -> int:
     lib = build.load("attention_mma")
     lib.si_attn_decode_scratch_floats.restype = _c_llr
@@ -497,6 +500,7 @@ def _keep_map(table: dict, key, ent) -> None:
 _tensor_maps = {}
 
 
+@_of_sizes
 def attn_decode_tma_ok(H: int, KV: int, hs: int, page_size: int, vs: Optional[int] = None) -> bool:
     """True when the TMA decode kernel takes this head layout and page size: heads of 64 or 128, or, for callers that name
     the value size ``vs``, key and value sizes of any multiple of 8 up to 128 (padded inside the kernel)."""
@@ -507,12 +511,14 @@ def attn_decode_tma_ok(H: int, KV: int, hs: int, page_size: int, vs: Optional[in
     return bool(lib.si_attn_decode_tma_ok(_c_int(H), _c_int(KV), _c_int(hs), _c_int(hs if vs is None else vs), _c_int(page_size)))
 
 
+@_of_sizes
 def attn_decode_tma_rows(H: int, KV: int) -> int:
     lib = build.load("attention_tma")
     lib.si_attn_decode_tma_rows.restype = _c_int
     return lib.si_attn_decode_tma_rows(_c_int(H), _c_int(KV))
 
 
+@_of_sizes
 def attn_decode_tma_scratch_floats(num_items: int, H: int, KV: int, hs: int, nsplit: int) -> int:
     lib = build.load("attention_tma")
     lib.si_attn_decode_tma_scratch_floats.restype = _c_llr
@@ -615,17 +621,11 @@ def _split_work(np, tiles, budget, entries, max_splits, min_tiles):
     return out
 
 
-_work_floats_memo: dict = {}
-
-
+@_of_sizes
 def attn_decode_tma_work_floats(slots: int, H: int, KV: int, hs: int) -> int:
-    key = (slots, H, KV, hs)
-    n = _work_floats_memo.get(key)
-    if n is None:
-        lib = build.load("attention_tma")
-        lib.si_attn_decode_tma_work_floats.restype = _c_llr
-        n = _work_floats_memo[key] = lib.si_attn_decode_tma_work_floats(_c_int(slots), _c_int(H), _c_int(KV), _c_int(hs))
-    return n
+    lib = build.load("attention_tma")
+    lib.si_attn_decode_tma_work_floats.restype = _c_llr
+    return lib.si_attn_decode_tma_work_floats(_c_int(slots), _c_int(H), _c_int(KV), _c_int(hs))
 
 
 def attn_decode_tma(q, k_cache, v_cache, block_table, items, out, page_size: int, num_seqs: int, H: int, KV: int,
@@ -968,6 +968,7 @@ def gemm_rows_swiglu(a, w, out, status=None) -> None:
 
 # ---- prompt-portion attention on tcgen05 ---------------------------------------------------------
 
+@_of_sizes
 def attn_portion_tc05_ok(H: int, KV: int, hs: int, page_size: int, vs: Optional[int] = None) -> bool:
     """As ``attn_decode_tma_ok``, for the tcgen05 prompt kernel."""
     if vs is None and hs not in (64, 128):
@@ -977,6 +978,7 @@ def attn_portion_tc05_ok(H: int, KV: int, hs: int, page_size: int, vs: Optional[
     return bool(lib.si_attn_portion_tc05_ok(_c_int(H), _c_int(KV), _c_int(hs), _c_int(hs if vs is None else vs), _c_int(page_size)))
 
 
+@_of_sizes
 def attn_portion_tc05_tokens(H: int, KV: int) -> int:
     """Most tokens of one work item of ``attn_portion_tc05``."""
     lib = build.load("attention_tc05")
@@ -1360,12 +1362,14 @@ def gated_part_norm(y, z, weight, out, parts: int, eps: float) -> None:
 
 # ---- general attention on the tensor cores (bf16) ---------------------------------------------------------
 
+@_of_sizes
 def attn_flex_ok(H: int, KV: int, dk: int, dv: int, own_v: bool) -> bool:
     lib = build.load("attention_flex")
     lib.si_attn_flex_ok.restype = _c_int
     return bool(lib.si_attn_flex_ok(_c_int(H), _c_int(KV), _c_int(dk), _c_int(dv), _c_int(1 if own_v else 0)))
 
 
+@_of_sizes
 def attn_flex_tokens(H: int, KV: int) -> int:
     """Most tokens of one work item of ``attn_flex``."""
     lib = build.load("attention_flex")
@@ -1373,6 +1377,7 @@ def attn_flex_tokens(H: int, KV: int) -> int:
     return lib.si_attn_flex_tokens(_c_int(H), _c_int(KV))
 
 
+@_of_sizes
 def attn_flex_scratch_floats(num_items: int, H: int, KV: int, dv: int, nsplit: int) -> int:
     lib = build.load("attention_flex")
     lib.si_attn_flex_scratch_floats.restype = _c_llr

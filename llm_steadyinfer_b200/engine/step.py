@@ -88,7 +88,8 @@ class _PinnedRing:
     def __init__(self, cap: int, device):
         self.cap = cap
         self.hosts = [torch.empty(cap, dtype=torch.int32, pin_memory=True) for _ in range(4)]
-        self.events: List[Optional[torch.cuda.Event]] = [None] * 4
+        self.events: List[Optional[torch.cuda.Event]] = [None] * 4      # one a buffer, recorded anew behind every copy
+        self.arrays = [h.numpy() for h in self.hosts]
         self.dev = torch.zeros(cap, dtype=torch.int32, device=device)
         self.turn = 0
 
@@ -97,14 +98,15 @@ class _PinnedRing:
         ev = self.events[self.turn]
         if ev is not None:
             ev.synchronize()
-        return self.hosts[self.turn].numpy()
+        return self.arrays[self.turn]
 
     def send(self, n: int) -> None:
         if n:
             self.dev[:n].copy_(self.hosts[self.turn][:n], non_blocking=True)
-            ev = torch.cuda.Event()
+            ev = self.events[self.turn]
+            if ev is None:
+                ev = self.events[self.turn] = torch.cuda.Event()
             ev.record()
-            self.events[self.turn] = ev
 
 
 class ModelRunner:
@@ -150,6 +152,7 @@ class ModelRunner:
         self._stage = _PinnedRing(4 * (T + 4) + 3 * (S + 4) + 8 + G * S * W, self.device)
         self._table_arrays: Dict[Tuple[int, Hashable], Tuple[int, np.ndarray]] = {}
         self._graphs: Dict[Tuple[int, int], dict] = {}
+        self._stage_views: Dict[Tuple[int, int], tuple] = {}      # of fixed-shape steps: their inputs lie in the same places
         # Shapes whose recording failed: they run directly from then on, as the reference marks a batch size
         # capture_failed and keeps to its direct path (src/source/model/model.cpp:189-227, 251).
         self.capture_failed: Dict[Tuple[int, int], str] = {}
@@ -215,7 +218,7 @@ class ModelRunner:
             ctx = self._prepare(entries)
             if feed is not None:
                 self._feed_tokens(ctx, feed)
-            self.storage.zero_new_slots()
+            self.storage.zero_new_slots(self.upload_ints)
             caches = self.storage.layer_views(self._tables)
             before = ops.launch_count()
             self.model.prepare(ctx, caches)
@@ -261,7 +264,7 @@ class ModelRunner:
         ctx = self._prepare(entries, seq_cap=cap, width_cap=self.max_width)
         if feed is not None:
             self._feed_tokens(ctx, feed)
-        self.storage.zero_new_slots()
+        self.storage.zero_new_slots(self.upload_ints)
         caches = self.storage.layer_views(self._tables)
         self.model.prepare(ctx, caches)
         key = (cap, self.max_width)
@@ -422,19 +425,18 @@ class ModelRunner:
         ctx.seq_cap = seq_cap
         ctx.num_tokens, ctx.num_seqs, ctx.num_logit_rows = T_cap, S, R_cap
         ctx.seq_slots = S_cap
-        ctx.tokens = dev[b_tok:b_tok + T_cap]
-        ctx.positions = dev[b_pos:b_pos + T_cap]
-        ctx.row_seq = dev[b_seq:b_seq + T_cap]
-        ctx.logit_rows = dev[b_lr:b_lr + R_cap]
-        ctx.q_start = dev[b_qs:b_qs + S_cap + 1]
-        ctx.ctx_len = dev[b_cl:b_cl + S_cap]
-        ctx.slots = dev[b_sl:b_sl + S_cap]
+        views = self._stage_views.get((S_cap, W_cap)) if fixed else None
+        if views is None:
+            dtabs = dev[table_off:table_off + G * S_cap * W_cap].view(G, S_cap, W_cap)
+            views = (dev[b_tok:b_tok + T_cap], dev[b_pos:b_pos + T_cap], dev[b_seq:b_seq + T_cap], dev[b_lr:b_lr + R_cap],
+                     dev[b_qs:b_qs + S_cap + 1], dev[b_cl:b_cl + S_cap], dev[b_sl:b_sl + S_cap], [dtabs[g] for g in range(G)])
+            if fixed:
+                self._stage_views[(S_cap, W_cap)] = views
+        (ctx.tokens, ctx.positions, ctx.row_seq, ctx.logit_rows, ctx.q_start, ctx.ctx_len, ctx.slots, self._tables) = views
         ctx.h_positions = h[b_pos:b_pos + T].copy()
         ctx.h_q_start = h[b_qs:b_qs + S + 1].copy()
         ctx.h_ctx_len = h[b_cl:b_cl + S].copy()
         ctx.h_slots = h[b_sl:b_sl + S].copy()
-        dtabs = dev[table_off:table_off + G * S_cap * W_cap].view(G, S_cap, W_cap)
-        self._tables = [dtabs[g] for g in range(G)]
         return ctx
 
     def _check_pages_written(self, entries: Sequence[StepEntry]) -> None:

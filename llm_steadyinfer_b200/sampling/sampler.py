@@ -19,7 +19,9 @@ class Sampler:
         # per row: temperature f32, top_p f32, top_k i32, pad, seed i64, counter i64 -> 8 int32 words
         # (four pinned copies in turn: with a step in flight the host already writes the next one's)
         self._hosts = [torch.empty(max_rows * 8, dtype=torch.int32, pin_memory=True) for _ in range(4)]
-        self._host_events = [None] * 4
+        self._arrays = [h.numpy() for h in self._hosts]
+        self._host_events = [None] * 4     # one a copy, recorded anew every time
+        self._device_views = {}            # per number of rows: what the kernel is given of the device copy
         self._host_turn = 0
         self._dev = torch.empty(max_rows * 8, dtype=torch.int32, device=self.device)
         self._out = torch.empty(max_rows, dtype=torch.int32, device=self.device)
@@ -35,29 +37,31 @@ class Sampler:
         if R != len(rows) or R > self.max_rows:
             raise ValueError(f"sampler got {R} logits rows for {len(rows)} requests (limit {self.max_rows})")
         out = self._out[:R]
-        if all(p.greedy for p, _, _ in rows):
+        params = [r[0] for r in rows]
+        temperature = [p.temperature for p in params]
+        if not any(t > 0 for t in temperature):
             ops.argmax(logits, out, self._argmax_scratch)
             return out
-        self._host_turn = (self._host_turn + 1) % 4
-        if self._host_events[self._host_turn] is not None:
-            self._host_events[self._host_turn].synchronize()
-        host = self._hosts[self._host_turn]
-        h = host.numpy()
+        turn = self._host_turn = (self._host_turn + 1) % 4
+        if self._host_events[turn] is not None:
+            self._host_events[turn].synchronize()
+        h = self._arrays[turn]
         n = self.max_rows
-        h[0:R].view(np.float32)[:] = [p.temperature for p, _, _ in rows]
-        h[n:n + R].view(np.float32)[:] = [p.top_p for p, _, _ in rows]
-        h[2 * n:2 * n + R] = [p.top_k for p, _, _ in rows]
-        h[4 * n:4 * n + 2 * R].view(np.uint64)[:] = [s & 0xFFFFFFFFFFFFFFFF for _, s, _ in rows]
-        h[6 * n:6 * n + 2 * R].view(np.int64)[:] = [c for _, _, c in rows]
-        self._dev.copy_(host, non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record()
-        self._host_events[self._host_turn] = ev
+        h[0:R].view(np.float32)[:] = temperature
+        h[n:n + R].view(np.float32)[:] = [p.top_p for p in params]
+        h[2 * n:2 * n + R] = [p.top_k for p in params]
+        h[4 * n:4 * n + 2 * R].view(np.uint64)[:] = [r[1] & 0xFFFFFFFFFFFFFFFF for r in rows]
+        h[6 * n:6 * n + 2 * R].view(np.int64)[:] = [r[2] for r in rows]
         d = self._dev
-        ops.sample(logits, out,
-                   temperature=d[0:R].view(torch.float32), top_p=d[n:n + R].view(torch.float32),
-                   top_k=d[2 * n:2 * n + R], seed=d[4 * n:4 * n + 2 * R].view(torch.int64),
-                   counter=d[6 * n:6 * n + 2 * R].view(torch.int64))
+        d.copy_(self._hosts[turn], non_blocking=True)
+        if self._host_events[turn] is None:
+            self._host_events[turn] = torch.cuda.Event()
+        self._host_events[turn].record()
+        v = self._device_views.get(R)
+        if v is None:
+            v = self._device_views[R] = (d[0:R].view(torch.float32), d[n:n + R].view(torch.float32), d[2 * n:2 * n + R],
+                                         d[4 * n:4 * n + 2 * R].view(torch.int64), d[6 * n:6 * n + 2 * R].view(torch.int64))
+        ops.sample(logits, out, temperature=v[0], top_p=v[1], top_k=v[2], seed=v[3], counter=v[4])
         return out
 
     def last_ids(self) -> torch.Tensor:
