@@ -44,9 +44,9 @@ __device__ __forceinline__ unsigned movmatrix_trans(unsigned v) {
 // this way a tile costs half the instructions, and the consumer warps, one per scheduler, are bound
 // by their instruction stream.
 template <int NH, int MT, int STAGES, bool SWAP>
-__global__ void __launch_bounds__(160)
+__global__ void __launch_bounds__(160, SWAP ? (NH == 1 ? 4 : 2) : 1)
 attn_decode_tma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap,
-                       const __grid_constant__ CUtensorMap vmap, int log2_page, const int4* __restrict__ work, int trigger) {
+                       const __grid_constant__ CUtensorMap vmap, int log2_page, const int4* __restrict__ work) {
   constexpr int NWARPS = 4, THREADS = 128, BLOCK_N = 64, ROWS = 16 * MT, HS_PAD = NH * 64;   // consumer warps/threads
   constexpr int KT = HS_PAD / 16, DT = HS_PAD / 8;
   constexpr int TILE = NH * BLOCK_N * 64;             // elements of one K (or V) tile
@@ -60,7 +60,6 @@ attn_decode_tma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k
   bf16* Vs = Ks + STAGES * TILE;
   bf16* Qs = Vs + STAGES * TILE;                     // [NH][ROWS][64]
 
-  if (trigger) pdl_trigger();
   // Until its pdl_wait() below no thread reads what the kernel before this one writes (the queries and the
   // newest keys and values): the work list, the items and the block table were copied in before it began.
   // Which share of which item: with a work list, entry blockIdx.x = (item, split, splits of the item, first
@@ -93,6 +92,22 @@ attn_decode_tma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k
   const int kv_end = min(kv_end_all, kv_begin_all + t_end * BLOCK_N);
   const int page_rows = 1 << log2_page;
   const int pages_per_tile = BLOCK_N >> log2_page;
+
+  // ---- producer warp: lane l fetches box (page l / (2 NH), half (l / 2) % NH, K or V) of each tile. The page numbers are read
+  // three tiles ahead: a lookup in the loop would put the latency of a load from global memory into every tile's turn. The first
+  // ones are on their way while the block sets up.
+  const int boxes = pages_per_tile * NH * 2;
+  const int pg = lane / (2 * NH), h = (lane >> 1) % NH, is_v = lane & 1;
+  constexpr int NOT_NEEDED = -2;
+  auto lookup = [&](int t) {
+    const int j = kv_begin + t * BLOCK_N;
+    // pages past the last key, or wholly before the window, are not fetched
+    if (t >= ntiles || lane >= boxes || j + pg * page_rows >= kv_end || j + (pg + 1) * page_rows <= kv_lo) return NOT_NEEDED;
+    const int slot = (j >> log2_page) + pg;
+    return slot < p.table_width ? __ldg(table + slot) : -1;
+  };
+  int ahead0 = NOT_NEEDED, ahead1 = NOT_NEEDED, ahead2 = NOT_NEEDED;
+  if (warp == NWARPS) { ahead0 = lookup(0); ahead1 = lookup(1); ahead2 = lookup(2); }
 
   if (threadIdx.x == 0) {
 #pragma unroll
@@ -127,20 +142,6 @@ attn_decode_tma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k
   }
 
   if (warp == NWARPS) {
-    // ---- producer warp: lane l fetches box (page l / (2 NH), half (l / 2) % NH, K or V) of each tile
-    const int boxes = pages_per_tile * NH * 2;
-    const int pg = lane / (2 * NH), h = (lane >> 1) % NH, is_v = lane & 1;
-    // The page numbers are read three tiles ahead: a lookup in the loop would put the latency of a load
-    // from global memory into every tile's turn.
-    constexpr int NOT_NEEDED = -2;
-    auto lookup = [&](int t) {
-      const int j = kv_begin + t * BLOCK_N;
-      // pages past the last key, or wholly before the window, are not fetched
-      if (t >= ntiles || lane >= boxes || j + pg * page_rows >= kv_end || j + (pg + 1) * page_rows <= kv_lo) return NOT_NEEDED;
-      const int slot = (j >> log2_page) + pg;
-      return slot < p.table_width ? __ldg(table + slot) : -1;
-    };
-    int ahead0 = lookup(0), ahead1 = lookup(1), ahead2 = lookup(2);
     // Tiles that end before the item's first position hold nothing that the kernel before this one writes
     // (it stores the keys and values of the step's own tokens): their copies start before this kernel waits.
     bool waited = false;
@@ -434,49 +435,53 @@ attn_decode_tma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k
   asm volatile("bar.sync 1, 128;\n" ::: "memory");
   if (!s_last) return;
   __threadfence();
-  // The merge reads nsplit partial results per output. Loads that follow one another in a loop would each
-  // cost a trip to L2, so (1) the maxima and sums of all splits come into shared memory in one pass,
-  // (2) one thread per row turns them into the weights of the splits and the row's sum, and (3) the
-  // outputs are summed over the splits eight loads at a time. (The warps' merge buffers are free by now.)
+  // The merge reads nsplit partial results per output, four outputs a thread. The first sixteen splits of a thread's first outputs (a
+  // decode step's only ones) are on their way before anything else; the maxima and sums of all splits come into shared memory in one
+  // pass, and a warp a row turns them into the weights of the splits and the row's sum: one round trip to L2 for up to sixteen splits.
+  // (The warps' merge buffers are free by now.)
   float* w_s = reinterpret_cast<float*>(smem_raw);              // [rows_used][nsplit] maxima, then weights
   float* l_s = w_s + rows_used * nsplit;                        // [rows_used][nsplit] sums
   float* L_s = l_s + rows_used * nsplit;                        // [rows_used]
+  const int vs4 = p.vs >> 2;
+  const size_t step = slab_step * p.vs;                         // from one split of an output to the next
+  float4 v[16];
+  auto fetch = [&](int idx, int sp) {
+    const int r = idx / vs4, d = (idx - r * vs4) << 2;
+    const float* src = p.part_o + (slab0 + r) * p.vs + d + (size_t)sp * step;
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+      v[u] = sp + u < nsplit ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)u * step)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  if (threadIdx.x < rows_used * vs4) fetch(threadIdx.x, 0);
   for (int i = threadIdx.x; i < rows_used * nsplit; i += THREADS) {
     const int r = i / nsplit, sp = i - r * nsplit;
-    const size_t slab = slab0 + (size_t)sp * slab_step + r;
-    w_s[i] = __ldcg(p.part_ml + slab * 2);
-    l_s[i] = __ldcg(p.part_ml + slab * 2 + 1);
+    const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (slab0 + (size_t)sp * slab_step + r) * 2));
+    w_s[i] = ml.x;
+    l_s[i] = ml.y;
   }
   asm volatile("bar.sync 1, 128;\n" ::: "memory");
-  for (int r = threadIdx.x; r < rows_used; r += THREADS) {
+  for (int r = warp; r < rows_used; r += NWARPS) {
     const float s2 = p.sink ? p.sink[g * p.G + r % p.G] * LOG2E : -INFINITY;
     float M = s2;
-    for (int sp = 0; sp < nsplit; ++sp) M = fmaxf(M, w_s[r * nsplit + sp]);
-    float L = p.sink ? exp2f(s2 - M) : 0.f;
-    for (int sp = 0; sp < nsplit; ++sp) {
+    for (int sp = lane; sp < nsplit; sp += 32) M = fmaxf(M, w_s[r * nsplit + sp]);
+    M = warp_max(M);
+    float L = 0.f;
+    for (int sp = lane; sp < nsplit; sp += 32) {
       const float ms = w_s[r * nsplit + sp];
       const float wgt = ms == -INFINITY ? 0.f : exp2f(ms - M);
       L += l_s[r * nsplit + sp] * wgt;
       w_s[r * nsplit + sp] = wgt;
     }
-    L_s[r] = L;
+    L = warp_sum(L);
+    if (lane == 0) L_s[r] = p.sink ? L + exp2f(s2 - M) : L;
   }
   asm volatile("bar.sync 1, 128;\n" ::: "memory");
-  // four outputs a thread, sixteen 16-byte loads in flight: with a few rows (a decode step) every thread has
-  // one turn, and the splits cost two round trips to L2 instead of one for every eight scalar loads
-  const int vs4 = p.vs >> 2;
   for (int idx = threadIdx.x; idx < rows_used * vs4; idx += THREADS) {
     const int r = idx / vs4, d = (idx - r * vs4) << 2;
-    const float* src = p.part_o + (slab0 + r) * p.vs + d;       // split sp lies sp * slab_step * vs further
-    const size_t step = slab_step * p.vs;
     const float* wr = w_s + r * nsplit;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int sp = 0; sp < nsplit; sp += 16) {
-      float4 v[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u)
-        v[u] = sp + u < nsplit ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)(sp + u) * step))
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (sp || idx != threadIdx.x) fetch(idx, sp);
 #pragma unroll
       for (int u = 0; u < 16; ++u)
         if (sp + u < nsplit) {                                   // in the order of the splits
@@ -548,8 +553,9 @@ static int launch(const AttnParams& p, const CUtensorMap& km, const CUtensorMap&
     if (e != cudaSuccess) return (int)e;
   }
   const dim3 grid = work ? dim3(num_work, p.KV, 1) : dim3(num_items, p.KV, p.nsplit);
-  si_launch(k, grid, dim3(160), smem, stream, p, km, vm, log2_page, work,
-            si_pdl_trigger_mode((long long)grid.x * grid.y * grid.z, 2 * si_sm_count()) == 1 ? 1 : 0);
+  // (No early trigger: with one, the kernels behind it are resident beside it and a step of 8 sequences and 32 layers took 4.9 ms
+  // instead of 3.3.)
+  si_launch(k, grid, dim3(160), smem, stream, p, km, vm, log2_page, work);
   return si_last_error();
 }
 

@@ -471,10 +471,17 @@ class Attention(Mixer):
             for (_, _, n, pos0) in dec:
                 first = first_visible_key(pos0, self.window, self.chunk) // 64 * 64
                 tiles.append(-(-(pos0 + n - first) // 64) if n > 0 else 0)
-            # Entries: every item whole, the shares that run at once, and room for finer cuts when items outnumber
-            # those (entries without work are blocks that start and leave, so not more room than pays)
+            # Entries: the shares that run at once while there are as many as items (the cut never takes more); else every item
+            # whole and room for finer cuts. Entries without work are blocks that start and leave, and those that wait
+            # for a place to start delay the end (8 sequences of 1,024 to 2,032 keys, 32 heads of 128: 16.2 us with 69 entries
+            # for 37 shares at once, 13.9 without the empty ones; 8 of up to 1,000 keys, 16 heads: 10.4 and 8.4).
             budget = max(1, self.target_blocks() // self.KV)
-            entries = budget + len(dec) + min(3 * len(dec), 2 * budget)
+            # Tiles of 64 columns and items of up to eight rows leave room for four blocks on a multiprocessor: taken where all items
+            # start at once only so (32 heads of 64: 61 sequences of 32 to 2,016 keys 23.5 us with two, 19.9 with four; but 8 sequences
+            # 11.2 and 11.6, 100 31.9 and 31.6, 250 55.7 and 57.5).
+            if max(self.hs, self.vs) <= 64 and plan["dec_rows"] <= 8 and budget < len(dec) <= 2 * self.target_blocks() // self.KV:
+                budget = 2 * self.target_blocks() // self.KV
+            entries = budget if len(dec) <= budget else budget + len(dec) + min(3 * len(dec), 2 * budget)
             work = ops.split_work(tiles, budget, entries, MAX_SPLITS, MIN_TILES_PER_SPLIT)
             if ctx.seq_cap is None:                    # shapes are free: only the entries with work
                 work = work[:max(1, int((work[:, 0] >= 0).sum()))]

@@ -68,3 +68,13 @@ def test_more_items_than_slots():
     # with no room for finer cuts the items stay whole
     sp, _ = _shares(split_work([128] * 40, 37, 37 + 40, 32, 2))
     assert set(sp.values()) == {1}
+
+
+def test_shares_that_run_at_once_need_no_more_entries():
+    """With no more items than the budget, as many entries as the budget hold every cut (a fixed shape's plan has no others)."""
+    rng = random.Random(3)
+    for _ in range(200):
+        budget = rng.randint(1, 80)
+        tiles = [rng.choice([0, 1, rng.randint(1, 40), rng.randint(1, 2000)]) for _ in range(rng.randint(1, budget))]
+        sp, live = _shares(split_work(tiles, budget, budget, 32, 2))
+        assert len(live) <= budget and all((sp.get(i, 0) >= 1) == (t > 0) for i, t in enumerate(tiles))
