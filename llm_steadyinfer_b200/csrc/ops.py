@@ -1341,10 +1341,10 @@ def ssm_scan(xbc, dt_raw, dt_bias, a_log, d_skip, state, y, q_start, ctx_len, sl
     _f32v(dt_bias, "dt_bias", heads); _f32v(a_log, "a_log", heads); _f32v(d_skip, "d_skip", heads)
     f = _fn("ssm", "si_ssm_scan",
             [_c_p, _c_ll, _c_p, _c_int, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_p, _c_ll, _c_p, _c_p, _c_p, _c_int,
-             _c_int, _c_int, _c_int, _c_int, _c_p])
+             _c_int, _c_int, _c_int, _c_int, _c_int, _c_p])
     _check(f(_ptr(xbc), xbc.stride(0), _ptr(dt_raw), _dt(dt_raw), dt_raw.stride(0), _ptr(dt_bias), _ptr(a_log),
              _ptr(d_skip), _ptr(state), state.stride(0), _ptr(y), y.stride(0), _ptr(q_start), _ptr(ctx_len), _ptr(slots),
-             int(num_seqs), heads, groups, N, P, _stream()), f"ssm_scan(heads={heads}, state={N}, head_dim={P})")
+             T, int(num_seqs), heads, groups, N, P, _stream()), f"ssm_scan(heads={heads}, state={N}, head_dim={P})")
 
 
 def gated_part_norm(y, z, weight, out, parts: int, eps: float) -> None:

@@ -121,7 +121,12 @@ SI_EXPORT int si_causal_conv(const void* u, int dtype, long long u_stride, const
 // the NS threads of one p (neighbouring lanes) read B and C from shared memory as consecutive 16-byte words, without
 // bank conflicts; they add their parts of y_t with shuffles. Tokens are walked in order, SCAN_CHUNK at a time; the
 // chunk after the one being computed is on its way into the other half of shared memory meanwhile (cp.async for B,
-// C and x; step size and decay by the first threads).
+// C and x; step size and decay by the first threads, whose raw step sizes are loaded a chunk before that).
+// A portion is bound by shared memory: a column's lanes read all of B and C for every token. COLS 2 (steps of portions, eight lanes
+// a column): a thread keeps the same entries of two columns, so a read serves both, with packed fp32 arithmetic (two entries an
+// instruction, the same roundings). A decode row is bound by the latency of its state's loads, which more threads serve better.
+// Measured, 64 heads of 64 columns, state 128, one column and two: a portion of 2,048 rows 438 and 334 us, two of 1,024 370 and 248, 2,000
+// and 100 719 and 478, 61 of 32 385 and 307.
 #define SCAN_CHUNK 32
 #ifndef SCAN_UNROLL
 #define SCAN_UNROLL 8        // tokens whose loads the compiler may issue ahead of the sums of the token before
@@ -135,14 +140,38 @@ __device__ __forceinline__ void scan_cp4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
 
-template <typename T, int NPT>
-__global__ void ssm_scan_kernel(const float* __restrict__ xbc, long long xbc_stride,     // conv output: [x | B | C]
-                                const T* __restrict__ dt_raw, long long dt_stride,
-                                const float* __restrict__ dt_bias, const float* __restrict__ a_log,
-                                const float* __restrict__ Dskip, float* __restrict__ state, long long state_stride,
-                                float* __restrict__ y, long long y_stride, const int* __restrict__ q_start,
-                                const int* __restrict__ ctx_len, const int* __restrict__ slots, int heads,
-                                int groups, int N, int P, int NS, int Pb) {
+struct ssm_true { static constexpr bool value = true; };
+struct ssm_false { static constexpr bool value = false; };
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+#define SCAN_PARAMS const float* __restrict__ xbc, long long xbc_stride, \
+                                const T* __restrict__ dt_raw, long long dt_stride, \
+                                const float* __restrict__ dt_bias, const float* __restrict__ a_log, \
+                                const float* __restrict__ Dskip, float* __restrict__ state, long long state_stride, \
+                                float* __restrict__ y, long long y_stride, const int* __restrict__ q_start, \
+                                const int* __restrict__ ctx_len, const int* __restrict__ slots, int heads, \
+                                int groups, int N, int P, int NS, int Pb
+template <typename T, int NPT, int COLS>
+__device__ __forceinline__ void ssm_scan(SCAN_PARAMS) {
   extern __shared__ __align__(16) float sm[];
   pdl_prologue();
   const int s = blockIdx.x, h = blockIdx.y;
@@ -159,15 +188,18 @@ __global__ void ssm_scan_kernel(const float* __restrict__ xbc, long long xbc_str
   // the block's columns of the state: [p0, p0 + Pb) (blockIdx.z cuts P where that gives the device more blocks)
   const int p0 = blockIdx.z * Pb;
   const int ns = tid % NS;
-  const bool live = tid / NS < Pb && p0 + tid / NS < P;      // threads beyond the columns follow idly
+  const int Pt = Pb / COLS;                                  // columns p and, with COLS 2, p + Pt
+  const bool live = tid / NS < Pt && p0 + tid / NS < P;      // threads beyond the columns follow idly
   const int p = live ? p0 + tid / NS : p0;
   const int gtid = p * NS + ns;            // the thread's place in the head's state, whatever the cut
   // the head's state in the order of the threads: entry i of thread gtid at i * (P * NS) + gtid
   float* st = state + (size_t)slots[s] * state_stride + (size_t)h * Npad * P;
   const int held = P * NS;
-  float S[NPT];
+  float S[COLS][NPT];
 #pragma unroll
-  for (int i = 0; i < NPT; ++i) S[i] = (live && pos0 > 0) ? st[(size_t)i * held + gtid] : 0.f;
+  for (int j = 0; j < COLS; ++j)
+#pragma unroll
+    for (int i = 0; i < NPT; ++i) S[j][i] = (live && pos0 > 0) ? st[(size_t)i * held + gtid + j * Pt * NS] : 0.f;
   const float rate = expf(a_log[h]);
   const float bias = dt_bias[h];
   const float dskip = Dskip[h];
@@ -178,6 +210,11 @@ __global__ void ssm_scan_kernel(const float* __restrict__ xbc, long long xbc_str
                    && ((size_t)xbc % 16 == 0);
   const int pcols = min(Pb, P - p0);
 
+  // the raw step size of row tid of a chunk: loaded before the chunk is staged, by the first threads
+  float raw = 0.f;
+  auto fetch_raw = [&](int c0) {
+    if (tid < min(SCAN_CHUNK, n_rows - c0)) raw = to_f32<T>(dt_raw[(size_t)(row0 + c0 + tid) * dt_stride + h]);
+  };
   auto stage = [&](int c0, int buf) {
     const int cn = min(SCAN_CHUNK, n_rows - c0);
     float* hB = sm + (size_t)buf * half_floats;
@@ -210,13 +247,15 @@ __global__ void ssm_scan_kernel(const float* __restrict__ xbc, long long xbc_str
       }
     }
     asm volatile("cp.async.commit_group;\n" ::);
-    for (int idx = tid; idx < cn; idx += blockDim.x) {
-      const float dt = softplus_f(to_f32<T>(dt_raw[(size_t)(row0 + c0 + idx) * dt_stride + h]) + bias);
-      hDec[idx] = expf(-rate * dt);
-      hDec[SCAN_CHUNK + idx] = dt;
+    if (tid < cn) {                                          // (a block has at least a warp of threads)
+      const float dt = softplus_f(raw + bias);
+      hDec[tid] = expf(-rate * dt);
+      hDec[SCAN_CHUNK + tid] = dt;
     }
+    fetch_raw(c0 + SCAN_CHUNK);
   };
 
+  fetch_raw(0);
   stage(0, 0);
   int buf = 0;
   for (int c0 = 0; c0 < n_rows; c0 += SCAN_CHUNK, buf ^= 1) {
@@ -232,7 +271,57 @@ __global__ void ssm_scan_kernel(const float* __restrict__ xbc, long long xbc_str
     const float* hC = hB + SCAN_CHUNK * Npad;
     const float* hX = hC + SCAN_CHUNK * Npad;
     const float* hDec = hX + SCAN_CHUNK * Pbp;
-    if (NS == 8) {
+    if constexpr (COLS == 2) {
+      // Eight lanes a column: the sums over the lanes as below, for both columns
+      unsigned long long* S0 = reinterpret_cast<unsigned long long*>(S[0]);
+      unsigned long long* S1 = reinterpret_cast<unsigned long long*>(S[1]);
+      const bool b4 = ns & 4, b2 = ns & 2, b1 = ns & 1;
+      auto eight = [&](int r0, auto whole) {
+        constexpr bool WHOLE = decltype(whole)::value;
+        float acc[2][8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          acc[0][u] = acc[1][u] = 0.f;
+          if (WHOLE || r0 + u < cn) {
+            const int r = r0 + u;
+            const float dec = hDec[r], dt = hDec[SCAN_CHUNK + r];
+            const float x0 = hX[r * Pbp + p - p0] * dt, x1 = hX[r * Pbp + p - p0 + Pt] * dt;
+            const unsigned long long dec2 = pack2(dec, dec), dx0 = pack2(x0, x0), dx1 = pack2(x1, x1);
+            const ulonglong2* Br = reinterpret_cast<const ulonglong2*>(hB + r * Npad) + ns;
+            const ulonglong2* Cr = reinterpret_cast<const ulonglong2*>(hC + r * Npad) + ns;
+            unsigned long long a0 = 0ull, a1 = 0ull;
+#pragma unroll
+            for (int i4 = 0; i4 < NPT / 4; ++i4) {
+              const ulonglong2 b = Br[i4 * 8], c = Cr[i4 * 8];
+              S0[2 * i4] = fma2(dec2, S0[2 * i4], mul2(dx0, b.x)); a0 = fma2(S0[2 * i4], c.x, a0);
+              S1[2 * i4] = fma2(dec2, S1[2 * i4], mul2(dx1, b.x)); a1 = fma2(S1[2 * i4], c.x, a1);
+              S0[2 * i4 + 1] = fma2(dec2, S0[2 * i4 + 1], mul2(dx0, b.y)); a0 = fma2(S0[2 * i4 + 1], c.y, a0);
+              S1[2 * i4 + 1] = fma2(dec2, S1[2 * i4 + 1], mul2(dx1, b.y)); a1 = fma2(S1[2 * i4 + 1], c.y, a1);
+            }
+            const float2 f0 = unpack2(a0), f1 = unpack2(a1);
+            acc[0][u] = f0.x + f0.y;
+            acc[1][u] = f1.x + f1.y;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float h4[4], h2[2];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            h4[u] = (b4 ? acc[j][4 + u] : acc[j][u]) + __shfl_xor_sync(0xffffffffu, b4 ? acc[j][u] : acc[j][4 + u], 4);
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            h2[u] = (b2 ? h4[2 + u] : h4[u]) + __shfl_xor_sync(0xffffffffu, b2 ? h4[u] : h4[2 + u], 2);
+          const float v = (b1 ? h2[1] : h2[0]) + __shfl_xor_sync(0xffffffffu, b1 ? h2[0] : h2[1], 1);
+          const int r = r0 + ns;
+          if ((WHOLE || r < cn) && live)
+            y[(size_t)(row0 + c0 + r) * y_stride + (size_t)h * P + p + j * Pt] = v + dskip * hX[r * Pbp + p - p0 + j * Pt];
+        }
+      };
+      int r0 = 0;
+      for (; r0 + 8 <= cn; r0 += 8) eight(r0, ssm_true());
+      if (r0 < cn) eight(r0, ssm_false());
+    } else if (NS == 8) {
       // Eight lanes a column: the lanes' partial sums of eight tokens are added up together by exchanging halves
       // (4 + 2 + 1 shuffles for eight tokens, and off the per-token chain), lane ns ending with token ns of the eight.
       for (int r0 = 0; r0 < cn; r0 += 8) {
@@ -250,10 +339,10 @@ __global__ void ssm_scan_kernel(const float* __restrict__ xbc, long long xbc_str
 #pragma unroll
             for (int i4 = 0; i4 < NPT / 4; ++i4) {
               const float4 b = Br[i4 * 8], c = Cr[i4 * 8];
-              S[4 * i4 + 0] = fmaf(dec, S[4 * i4 + 0], dx * b.x); a0 = fmaf(S[4 * i4 + 0], c.x, a0);
-              S[4 * i4 + 1] = fmaf(dec, S[4 * i4 + 1], dx * b.y); a1 = fmaf(S[4 * i4 + 1], c.y, a1);
-              S[4 * i4 + 2] = fmaf(dec, S[4 * i4 + 2], dx * b.z); a0 = fmaf(S[4 * i4 + 2], c.z, a0);
-              S[4 * i4 + 3] = fmaf(dec, S[4 * i4 + 3], dx * b.w); a1 = fmaf(S[4 * i4 + 3], c.w, a1);
+              S[0][4 * i4 + 0] = fmaf(dec, S[0][4 * i4 + 0], dx * b.x); a0 = fmaf(S[0][4 * i4 + 0], c.x, a0);
+              S[0][4 * i4 + 1] = fmaf(dec, S[0][4 * i4 + 1], dx * b.y); a1 = fmaf(S[0][4 * i4 + 1], c.y, a1);
+              S[0][4 * i4 + 2] = fmaf(dec, S[0][4 * i4 + 2], dx * b.z); a0 = fmaf(S[0][4 * i4 + 2], c.z, a0);
+              S[0][4 * i4 + 3] = fmaf(dec, S[0][4 * i4 + 3], dx * b.w); a1 = fmaf(S[0][4 * i4 + 3], c.w, a1);
             }
             acc[u] = a0 + a1;
           }
@@ -282,10 +371,10 @@ __global__ void ssm_scan_kernel(const float* __restrict__ xbc, long long xbc_str
 #pragma unroll
       for (int i4 = 0; i4 < NPT / 4; ++i4) {
         const float4 b = Br[i4 * NS], c = Cr[i4 * NS];
-        S[4 * i4 + 0] = fmaf(dec, S[4 * i4 + 0], dx * b.x); acc0 = fmaf(S[4 * i4 + 0], c.x, acc0);
-        S[4 * i4 + 1] = fmaf(dec, S[4 * i4 + 1], dx * b.y); acc1 = fmaf(S[4 * i4 + 1], c.y, acc1);
-        S[4 * i4 + 2] = fmaf(dec, S[4 * i4 + 2], dx * b.z); acc0 = fmaf(S[4 * i4 + 2], c.z, acc0);
-        S[4 * i4 + 3] = fmaf(dec, S[4 * i4 + 3], dx * b.w); acc1 = fmaf(S[4 * i4 + 3], c.w, acc1);
+        S[0][4 * i4 + 0] = fmaf(dec, S[0][4 * i4 + 0], dx * b.x); acc0 = fmaf(S[0][4 * i4 + 0], c.x, acc0);
+        S[0][4 * i4 + 1] = fmaf(dec, S[0][4 * i4 + 1], dx * b.y); acc1 = fmaf(S[0][4 * i4 + 1], c.y, acc1);
+        S[0][4 * i4 + 2] = fmaf(dec, S[0][4 * i4 + 2], dx * b.z); acc0 = fmaf(S[0][4 * i4 + 2], c.z, acc0);
+        S[0][4 * i4 + 3] = fmaf(dec, S[0][4 * i4 + 3], dx * b.w); acc1 = fmaf(S[0][4 * i4 + 3], c.w, acc1);
       }
       float acc = acc0 + acc1;
       for (int o = NS >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, NS);
@@ -296,15 +385,26 @@ __global__ void ssm_scan_kernel(const float* __restrict__ xbc, long long xbc_str
   }
   if (live) {
 #pragma unroll
-    for (int i = 0; i < NPT; ++i) st[(size_t)i * held + gtid] = S[i];
+    for (int j = 0; j < COLS; ++j)
+#pragma unroll
+      for (int i = 0; i < NPT; ++i) st[(size_t)i * held + gtid + j * Pt * NS] = S[j][i];
   }
+}
+
+template <typename T, int NPT>
+__global__ void ssm_scan_kernel(SCAN_PARAMS) {
+  ssm_scan<T, NPT, 1>(xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, Dskip, state, state_stride, y, y_stride, q_start, ctx_len, slots, heads, groups, N, P, NS, Pb);
+}
+template <typename T, int NPT>
+__global__ void __launch_bounds__(256) ssm_scan_wide_kernel(SCAN_PARAMS) {
+  ssm_scan<T, NPT, 2>(xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, Dskip, state, state_stride, y, y_stride, q_start, ctx_len, slots, heads, groups, N, P, NS, Pb);
 }
 
 template <typename T, int NPT>
 static int scan_launch(const float* xbc, long long xbc_stride, const void* dt_raw, long long dt_stride,
                        const float* dt_bias, const float* a_log, const float* Dskip, float* state,
                        long long state_stride, float* y, long long y_stride, const int* q_start, const int* ctx_len,
-                       const int* slots, int num_seqs, int heads, int groups, int N, int P, int NS, cudaStream_t stream) {
+                       const int* slots, int num_tokens, int num_seqs, int heads, int groups, int N, int P, int NS, cudaStream_t stream) {
   // Cut the columns over more blocks while the blocks still find a multiprocessor each, down to 8 columns a block:
   // a block's time goes to reading B and C from shared memory once per column, so columns on idle multiprocessors
   // are time saved; beyond one block each, the cut only repeats the staging of B and C (measured at 64 heads, one
@@ -312,14 +412,15 @@ static int scan_launch(const float* xbc, long long xbc_stride, const void* dt_ra
   // layout does not depend on the cut.
   int Pb = P;
   while (Pb % 2 == 0 && Pb / 2 >= 8 && 2LL * num_seqs * heads * (P / Pb) <= si_sm_count()) Pb /= 2;
-  int threads = (Pb * NS + 31) / 32 * 32;
+  // portions, and a state of up to 128 rows: two columns a thread
+  constexpr int WIDE = NPT == 8 || NPT == 16 ? NPT : 8;
+  const bool two = WIDE == NPT && NS == 8 && Pb % 2 == 0 && Pb <= 64 && num_tokens >= 4LL * num_seqs;
+  const int threads = (Pb / (two ? 2 : 1) * NS + 31) / 32 * 32;
   const size_t smem = (size_t)2 * (2 * SCAN_CHUNK * NS * NPT + SCAN_CHUNK * ((Pb + 3) / 4 * 4) + 2 * SCAN_CHUNK) * sizeof(float);
   if (smem > 200 * 1024) return -2;
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(ssm_scan_kernel<T, NPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return -2;
-  }
-  si_launch(ssm_scan_kernel<T, NPT>, dim3(num_seqs, heads, P / Pb), dim3(threads), smem, stream, xbc, xbc_stride,
+  auto k = two ? ssm_scan_wide_kernel<T, WIDE> : ssm_scan_kernel<T, NPT>;
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -2;
+  si_launch(k, dim3(num_seqs, heads, P / Pb), dim3(threads), smem, stream, xbc, xbc_stride,
             (const T*)dt_raw, dt_stride, dt_bias, a_log, Dskip, state, state_stride, y, y_stride, q_start, ctx_len,
             slots, heads, groups, N, P, NS, Pb);
   return si_last_error();
@@ -347,7 +448,7 @@ SI_EXPORT int si_ssm_padded_state(int N, int P) {
 SI_EXPORT int si_ssm_scan(const float* xbc, long long xbc_stride, const void* dt_raw, int dtype, long long dt_stride,
                           const float* dt_bias, const float* a_log, const float* Dskip, float* state,
                           long long state_stride, float* y, long long y_stride, const int* q_start,
-                          const int* ctx_len, const int* slots, int num_seqs, int heads, int groups, int N, int P,
+                          const int* ctx_len, const int* slots, int num_tokens, int num_seqs, int heads, int groups, int N, int P,
                           cudaStream_t stream) {
   if (num_seqs <= 0) return 0;
   if (heads <= 0 || groups <= 0 || heads % groups || N <= 0 || P <= 0 || P > 1024 || heads > 65535) return -2;
@@ -355,7 +456,7 @@ SI_EXPORT int si_ssm_scan(const float* xbc, long long xbc_stride, const void* dt
   const int NS = scan_shape(N, P, &per);
   if (NS == 0) return -2;
 #define SCAN_GO(TT, NPT) scan_launch<TT, NPT>(xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, Dskip, state, \
-                                              state_stride, y, y_stride, q_start, ctx_len, slots, num_seqs, heads, \
+                                              state_stride, y, y_stride, q_start, ctx_len, slots, num_tokens, num_seqs, heads, \
                                               groups, N, P, NS, stream)
   if (dtype == SI_BF16) {
     if (per <= 4) return SCAN_GO(__nv_bfloat16, 4);

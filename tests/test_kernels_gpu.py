@@ -1520,3 +1520,30 @@ def test_gemm_f32_over_both_tiles(M, N, K):
     for m in (0, 63, M - 1):
         ops().gemm_f32(a[m:m + 1], w, one)
         assert torch.equal(one[0], out[m])
+
+
+@pytest.mark.parametrize("heads,groups,N,P", [(4, 2, 128, 64), (3, 1, 64, 64), (2, 2, 100, 60), (64, 8, 128, 64)])
+def test_state_space_portions_two_columns_a_thread(heads, groups, N, P):
+    """A portion in one call (two columns a thread) and in pieces of three rows (one column): the same sums in the same order, so the
+    same bits, in the results and in the slots; rows that fill no whole group of eight or chunk of 32, one sequence that continues."""
+    o = ops()
+    g = torch.Generator().manual_seed(N)
+    lens = [37, 64, 1, 5, 0, 90]
+    S, T, W = len(lens), sum(lens), heads * P + 2 * groups * N
+    xbc, dt = torch.randn(T, W, generator=g).to(DEV), torch.randn(T, heads, generator=g).to(torch.bfloat16).to(DEV)
+    dt_bias, a_log, skip = (torch.randn(heads, generator=g).to(DEV) for _ in range(3))
+    start = torch.tensor([sum(lens[:i]) for i in range(S + 1)], dtype=torch.int32, device=DEV)
+    before = torch.tensor([0, 0, 7, 0, 0, 12], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([3, 0, 5, 1, 2, 4], dtype=torch.int32, device=DEV)
+    whole = torch.randn(S, heads * o.ssm_padded_state(N, P) * P + 4, generator=g).to(DEV)
+    parts = whole.clone()
+    y, yp = torch.full((T, heads * P), 7.0, device=DEV), torch.full((T, heads * P), 7.0, device=DEV)
+    ctx = before + torch.tensor(lens, dtype=torch.int32, device=DEV)
+    o.ssm_scan(xbc, dt, dt_bias, a_log, skip, whole, y, start, ctx, slots, S, heads, groups, N, P)
+    for s in range(S):
+        for a in range(0, lens[s], 3):
+            b = min(a + 3, lens[s])
+            i0 = int(start[s])
+            o.ssm_scan(xbc[i0 + a:i0 + b], dt[i0 + a:i0 + b], dt_bias, a_log, skip, parts, yp[i0 + a:i0 + b],
+                       torch.tensor([0, b - a], dtype=torch.int32, device=DEV), before[s:s + 1] + b, slots[s:s + 1], 1, heads, groups, N, P)
+    assert torch.isfinite(y).all() and torch.equal(y, yp) and torch.equal(whole, parts)
