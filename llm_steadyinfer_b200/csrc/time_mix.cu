@@ -170,39 +170,58 @@ SI_EXPORT int si_shift_mix(const void* x, int dtype, long long x_stride, const f
 // r, k, v: rows of C values each in the compute dtype; z [T, L] likewise; w2t fp32 [L, C] (the second low-rank matrix,
 // transposed); w0 fp32 [C]; xs fp32 [T, 4C] = [r | k | v | decay]. A block takes ROWS rows and 256 channels (blockIdx.y),
 // a thread one channel: it walks the L rows of w2t once for all its rows, in the order l = 0, 1, ... whatever ROWS is, so a
-// row's decay does not depend on how many rows the step has.
+// row's decay does not depend on how many rows the step has. A single row is a chain of loads: the first PREP_AHEAD rows of w2t, which
+// do not depend on the kernel before, are on their way before the wait for it, then the row's r, k and v while its low-rank values
+// come in: three rows, C = 2,048, L = 64, 9.0 us before and 3.9 so.
+#define PREP_AHEAD 64
 template <typename T, int ROWS>
 __global__ void __launch_bounds__(256) time_mix_prepare_kernel(const T* __restrict__ r, long long r_stride, const T* __restrict__ k,
     long long k_stride, const T* __restrict__ v, long long v_stride, const T* __restrict__ z, long long z_stride,
     const float* __restrict__ w2t, const float* __restrict__ w0, float* __restrict__ xs, int rows, int C, int L) {
   extern __shared__ float th[];                      // [L][ROWS]: tanh of the rows' low-rank values
-  pdl_prologue();
   const int t0 = blockIdx.x * ROWS;
+  const int c = blockIdx.y * blockDim.x + threadIdx.x;
+  constexpr int AHEAD = ROWS == 1 ? PREP_AHEAD : 1;
+  float ahead[AHEAD], rkv[3];
+  if (ROWS == 1 && c < C) {
+#pragma unroll
+    for (int l = 0; l < AHEAD; ++l) ahead[l] = l < L ? w2t[(size_t)l * C + c] : 0.f;
+  }
+  const float b = c < C ? w0[c] : 0.f;
+  pdl_wait();
+  if (ROWS == 1 && c < C) {
+    rkv[0] = to_f32<T>(r[(size_t)t0 * r_stride + c]);
+    rkv[1] = to_f32<T>(k[(size_t)t0 * k_stride + c]);
+    rkv[2] = to_f32<T>(v[(size_t)t0 * v_stride + c]);
+  }
   for (int idx = threadIdx.x; idx < ROWS * L; idx += blockDim.x) {
     const int rr = idx / L, l = idx - rr * L;
     th[l * ROWS + rr] = t0 + rr < rows ? tanhf(to_f32<T>(z[(size_t)(t0 + rr) * z_stride + l])) : 0.f;
   }
   __syncthreads();
-  const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= C) return;
   float acc[ROWS];
 #pragma unroll
   for (int rr = 0; rr < ROWS; ++rr) acc[rr] = 0.f;
-#pragma unroll(ROWS == 1 ? 16 : 4)             // a single row's walk is a chain of loads: many of them in flight
-  for (int l = 0; l < L; ++l) {
+  if (ROWS == 1) {
+#pragma unroll
+    for (int l = 0; l < AHEAD; ++l)
+      if (l < L) acc[0] = fmaf(ahead[l], th[l], acc[0]);
+  }
+#pragma unroll(ROWS == 1 ? 16 : 4)
+  for (int l = ROWS == 1 ? AHEAD : 0; l < L; ++l) {
     const float w = w2t[(size_t)l * C + c];
 #pragma unroll
     for (int rr = 0; rr < ROWS; ++rr) acc[rr] = fmaf(w, th[l * ROWS + rr], acc[rr]);
   }
-  const float b = w0[c];
 #pragma unroll
   for (int rr = 0; rr < ROWS; ++rr) {
     const int t = t0 + rr;
     if (t >= rows) break;
     float* o = xs + (size_t)t * 4 * C;
-    o[c] = to_f32<T>(r[(size_t)t * r_stride + c]);
-    o[C + c] = to_f32<T>(k[(size_t)t * k_stride + c]);
-    o[2 * C + c] = to_f32<T>(v[(size_t)t * v_stride + c]);
+    o[c] = ROWS == 1 ? rkv[0] : to_f32<T>(r[(size_t)t * r_stride + c]);
+    o[C + c] = ROWS == 1 ? rkv[1] : to_f32<T>(k[(size_t)t * k_stride + c]);
+    o[2 * C + c] = ROWS == 1 ? rkv[2] : to_f32<T>(v[(size_t)t * v_stride + c]);
     o[3 * C + c] = expf(-expf(acc[rr] + b));
   }
 }
