@@ -1279,7 +1279,8 @@ def causal_conv(u, weight, bias, state, conv_off: int, out, positions, row_seq, 
                 num_seqs: int, status=None) -> None:
     """out[t, c] (fp32) = silu(bias[c] + sum_k weight[c, k] * u[t - (K-1) + k, c]) per sequence, zeros before its
     start; inputs of earlier steps come from ``state[slot, conv_off:]`` ([K-1, C], fp32), which is renewed with
-    this step's last K - 1 inputs afterwards (two launches)."""
+    this step's last K - 1 inputs afterwards (two launches; one where no more rows than sequences come in and rows, channels and
+    state lie in fours of entries)."""
     _cuda(u, weight, bias, state, out, positions, row_seq, q_start, ctx_len, slots, status)
     for t, nm in ((positions, "positions"), (row_seq, "row_seq"), (q_start, "q_start"), (ctx_len, "ctx_len"), (slots, "slots")):
         _i32(t, nm)
@@ -1290,12 +1291,14 @@ def causal_conv(u, weight, bias, state, conv_off: int, out, positions, row_seq, 
     _need(out.dtype == torch.float32 and out.is_contiguous() and out.shape == (T, C), "causal_conv: out must be fp32 [T, C]")
     _need(state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
           and state.shape[1] >= conv_off + (K - 1) * C, "causal_conv: state must be fp32 [slots, >= conv_off + (K-1)*C]")
+    one = (T <= num_seqs and K <= 4 and (C | u.stride(0) | state.stride(0) | int(conv_off)) % 4 == 0
+           and u.data_ptr() % (4 * u.element_size()) == 0 and (state.data_ptr() | out.data_ptr()) % 16 == 0)
     f = _fn("ssm", "si_causal_conv",
             [_c_p, _c_int, _c_ll, _c_p, _c_p, _c_p, _c_ll, _c_ll, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int,
-             _c_int, _c_int, _c_p, _c_p])
+             _c_int, _c_int, _c_int, _c_p, _c_p])
     _check(f(_ptr(u), _dt(u), u.stride(0), _ptr(weight), _ptr(bias), _ptr(state), state.stride(0), int(conv_off), _ptr(out),
              _ptr(positions), _ptr(row_seq), _ptr(q_start), _ptr(ctx_len), _ptr(slots), T, int(num_seqs), C, K,
-             _ptr(status), _stream()), f"causal_conv(channels={C}, taps={K})", kernels=2 if K > 1 else 1)
+             int(one), _ptr(status), _stream()), f"causal_conv(channels={C}, taps={K})", kernels=2 if K > 1 and not one else 1)
 
 
 def ssm_padded_state(N: int, P: int) -> int:

@@ -1547,3 +1547,47 @@ def test_state_space_portions_two_columns_a_thread(heads, groups, N, P):
             o.ssm_scan(xbc[i0 + a:i0 + b], dt[i0 + a:i0 + b], dt_bias, a_log, skip, parts, yp[i0 + a:i0 + b],
                        torch.tensor([0, b - a], dtype=torch.int32, device=DEV), before[s:s + 1] + b, slots[s:s + 1], 1, heads, groups, N, P)
     assert torch.isfinite(y).all() and torch.equal(y, yp) and torch.equal(whole, parts)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("C,K", [(12, 4), (2048, 4), (516, 1), (516, 3), (10, 4), (64, 7)])
+def test_causal_convolution_of_portions_and_single_rows(C, K, dtype):
+    """Portions, then single rows beside a padding row, then a step of two rows of one sequence and none of another: results and
+    slots against float64 over the whole sequences (K fp32 products of size one; the channels that fill no fours and the longer taps
+    take the plain kernel)."""
+    o = ops()
+    g = torch.Generator().manual_seed(C + K)
+    S, off = 4, 8
+    slots = [2, 0, 3, 1]
+    w, b = torch.randn(C, K, generator=g), torch.randn(C, generator=g)
+    seqs = [torch.randn(80, C, generator=g).to(dtype) for _ in range(S)]
+    want = [torch.nn.functional.silu(torch.nn.functional.conv1d(torch.nn.functional.pad(q.double().t()[None], (K - 1, 0)), w.double()[:, None],
+                                                                b.double(), groups=C))[0].t() for q in seqs]
+    state = torch.full((S, off + (K - 1) * C + 4), float("nan"), device=DEV)         # what stale slots hold must not be read
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    done = [0] * S
+    for lens, pad in (([1, 2, 17, 33], 0), ([30, 1, 1, 9], 0), ([1, 1, 1, 1], 0), ([1, 1, 1, 0], 1), ([2, 0, 1, 1], 0), ([20, 1, 1, 1], 0)):
+        T = sum(lens) + pad
+        rows = torch.full((T, C + 4), 3.0).to(dtype)
+        seq, pos, at = [-1] * T, [0] * T, 0
+        for s, n in enumerate(lens):
+            rows[at:at + n, 4:] = seqs[s][done[s]:done[s] + n]
+            seq[at:at + n], pos[at:at + n] = [s] * n, list(range(done[s], done[s] + n))
+            at += n
+        out = torch.full((T, C), 7.0, device=DEV)
+        o.causal_conv(rows.to(DEV)[:, 4:], w.to(DEV), b.to(DEV), state, off, out, i32(pos), i32(seq), i32([sum(lens[:s]) for s in range(S + 1)]),
+                      i32([done[s] + lens[s] for s in range(S)]), i32(slots), S, status=status)
+        at = 0
+        for s, n in enumerate(lens):
+            if n:
+                assert (out[at:at + n].double().cpu() - want[s][done[s]:done[s] + n]).abs().max().item() <= 1e-6 * K * 16
+            at += n
+            done[s] += n
+            if lens[s]:
+                kept = state[slots[s], off:off + (K - 1) * C].view(K - 1, C).cpu()
+                past = torch.cat([torch.zeros(K - 1, C), seqs[s][:done[s]].float()])[len(seqs[s][:done[s]]):]
+                assert torch.equal(kept, past[-(K - 1):] if K > 1 else past[:0])
+        if pad:
+            assert (out[-pad:] == 0).all()
+    assert status.item() == 0
