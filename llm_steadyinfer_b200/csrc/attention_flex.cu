@@ -380,7 +380,7 @@ attn_flex_kernel(const FlexParams p) {
 
 // Merge of the shares of split items: a block per (item, gy, row and 128 value columns); the first warp weighs the shares while all
 // threads have the first 32 shares' sums of their column in flight, then every thread adds up its column's. Bound by latency: two
-// round trips. Measured at four rows of 16 heads: 3.1 us (value size 128) and 4.1 (512), where a block a row, a share at a time, took 5.2 and 8.7.
+// round trips. Measured at four rows of 16 heads: 3.1 us (value size 128) and 4.1 (512; 5.6 over 64 shares instead of 32), where a block a row, a share at a time, took 5.2 and 8.7.
 __global__ void __launch_bounds__(128) attn_flex_merge_kernel(const FlexParams p, int col_blocks) {
   __shared__ float w[64];
   __shared__ float s_inv;
