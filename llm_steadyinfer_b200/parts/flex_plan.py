@@ -34,6 +34,7 @@ def plan(ctx, device, H: int, KV: int, dk: int, dv: int, own_v: bool, window, sk
         return got
     per_item = ops.attn_flex_tokens(H, KV)
     gen_item = ops.attn_portion_tc05_tokens(H, KV) if gen else 0
+    fixed = ctx.seq_cap is not None
     dec, por, big = [], [], []
     qs, cl = ctx.h_q_start, ctx.h_ctx_len
     for s in range(ctx.num_seqs):
@@ -41,14 +42,15 @@ def plan(ctx, device, H: int, KV: int, dk: int, dv: int, own_v: bool, window, sk
             continue
         row0, n = int(qs[s]), int(qs[s + 1] - qs[s])
         pos0 = int(cl[s]) - n
-        if gen and n * (H // KV) >= GEN_MIN_ROWS:
+        # (never in a fixed shape, whose lists must not depend on the number of sequences, nor for what is one item of the other
+        # kernel, which cuts its keys)
+        if gen and not fixed and n > per_item and n * (H // KV) >= GEN_MIN_ROWS:
             big += [(s, row0 + b, min(gen_item, n - b), pos0 + b) for b in range(0, n, gen_item)]
         elif n <= per_item:
             dec.append((s, row0, n, pos0))
         else:
             for b in range(0, n, per_item):
                 por.append((s, row0 + b, min(per_item, n - b), pos0 + b))
-    fixed = ctx.seq_cap is not None
     if fixed:                                         # fixed shapes: pad with empty items, shares by the shape alone
         dec += [(0, 0, 0, 0)] * (ctx.seq_cap - len(dec))
     out = {"dec": None, "por": None, "gen": None, "nsplit": 1, "scratch": None, "dec_rows": 0}

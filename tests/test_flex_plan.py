@@ -1,0 +1,70 @@
+"""The work lists of the general tensor-core attention (host side only; the kernels' own answers are stood in for)."""
+import numpy as np
+import pytest
+
+from llm_steadyinfer_b200.parts import flex_plan
+
+
+class Upload:
+    """An uploaded list: the buffer's contents are whatever was uploaded under its name last."""
+
+    def __init__(self, store, key, n):
+        self.store, self.key, self.n = store, key, n
+
+    def view(self, *shape):
+        return self
+
+    def items(self):
+        return [tuple(r) for r in self.store[self.key][:self.n].reshape(-1, 4).tolist()]
+
+
+class Ctx:
+    """What a plan asks of a step: its sequences (rows they bring, keys they end with) and places to keep things."""
+
+    def __init__(self, seqs, seq_cap=None):
+        self.num_seqs, self.seq_cap, self.plans, self.uploads = len(seqs), seq_cap, {}, {}
+        self.h_q_start = np.cumsum([0] + [n for n, _ in seqs])
+        self.h_ctx_len = np.array([end for _, end in seqs])
+
+    def upload_ints(self, key, values, capacity=None):
+        self.uploads[key] = np.ascontiguousarray(values).reshape(-1)
+        return Upload(self.uploads, key, values.size)
+
+    def buf(self, key, shape, dtype):
+        return (key, tuple(shape))
+
+
+@pytest.fixture(autouse=True)
+def kernels(monkeypatch):
+    """What the kernels say of their items: 64 rows in parts of a divisor of the heads, two tiles of 128 rows."""
+    def flex_tokens(H, KV):
+        return 64 // max(g for g in range(1, min(H // KV, 64) + 1) if (H // KV) % g == 0)
+    monkeypatch.setattr(flex_plan.ops, "attn_flex_tokens", flex_tokens)
+    monkeypatch.setattr(flex_plan.ops, "attn_portion_tc05_tokens", lambda H, KV: 2 * (128 // (H // KV)))
+    monkeypatch.setattr(flex_plan.ops, "attn_flex_scratch_floats", lambda items, H, KV, dv, nsplit: items * H * dv * nsplit)
+    monkeypatch.setattr(flex_plan.ops, "sm_count", lambda device=None: 148)
+
+
+def plan(ctx, H, KV, gen=True, dk=128, dv=128):
+    return flex_plan.plan(ctx, None, H, KV, dk, dv, True, None, gen=gen)
+
+
+@pytest.mark.parametrize("G", [1, 16, 128])
+def test_a_fixed_shape_has_the_same_lists_for_every_number_of_sequences(G):
+    """A recorded step is replayed with more or fewer sequences than it was recorded with: its lists keep their lengths."""
+    shapes = set()
+    for live in (1, 3, 4):
+        p = plan(Ctx([(1, 700 + s) for s in range(live)], seq_cap=4), G, 1)
+        assert p["gen"] is None and p["por"] is None
+        items = p["dec"].items()
+        assert [it[0] for it in items if it[2]] == list(range(live)), "every sequence has its item"
+        shapes.add((len(items), p["nsplit"], p["scratch"], p["dec_rows"]))
+    assert len(shapes) == 1
+
+
+def test_single_rows_keep_their_shares_of_keys():
+    """A row of 128 query heads a key head fills the prompt kernel's tile, but it is a decode row: its keys are cut over blocks."""
+    p = plan(Ctx([(1, 9000)]), 128, 1)
+    assert p["gen"] is None and p["nsplit"] > 1 and p["dec"].items() == [(0, 0, 1, 8999)]
+    p = plan(Ctx([(2, 9000)]), 128, 1)
+    assert p["dec"] is None and p["gen"].items() == [(0, 0, 2, 8998)]
