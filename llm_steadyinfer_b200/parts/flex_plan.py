@@ -54,7 +54,7 @@ def plan(ctx, device, H: int, KV: int, dk: int, dv: int, own_v: bool, window, sk
     if fixed:                                         # fixed shapes: pad with empty items, shares by the shape alone
         dec += [(0, 0, 0, 0)] * (ctx.seq_cap - len(dec))
     out = {"dec": None, "por": None, "gen": None, "nsplit": 1, "scratch": None, "dec_rows": 0}
-    tag = f"{H}_{KV}_{dk}_{dv}_{int(own_v)}_{window}" + (f"_c{chunk}" if chunk else "") + ("_rest" if skip else "")
+    tag = f"{H}_{KV}_{dk}_{dv}_{int(own_v)}_{window}" + (f"_c{chunk}" if chunk else "") + ("_rest" if skip else "") + ("_gen" if gen else "")
     if dec:
         # blocks one item gets without shares: kv heads x parts of the query heads x slices of the value columns
         gb = max(g for g in range(1, min(H // KV, 64) + 1) if (H // KV) % g == 0)

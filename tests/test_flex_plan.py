@@ -68,3 +68,17 @@ def test_single_rows_keep_their_shares_of_keys():
     assert p["gen"] is None and p["nsplit"] > 1 and p["dec"].items() == [(0, 0, 1, 8999)]
     p = plan(Ctx([(2, 9000)]), 128, 1)
     assert p["dec"] is None and p["gen"].items() == [(0, 0, 2, 8998)]
+
+
+def test_layers_that_differ_in_the_prompt_kernel_keep_lists_of_their_own():
+    """Two layers of one head layout, one whose form the prompt kernel takes and one whose it does not, in one step: both plans are made
+    before either is used, so neither upload may take the other's place."""
+    seqs = [(100, 100), (300, 300)]                   # one key head a query head: 100 rows stay with the general kernel, 300 do not
+    ctx = Ctx(seqs)
+    with_gen, without = plan(ctx, 4, 4, gen=True), plan(ctx, 4, 4, gen=False)
+    for p, want in ((with_gen, {0: 100}), (without, {0: 100, 1: 300})):
+        rows = {}
+        for seq, _, n, _ in p["por"].items():
+            rows[seq] = rows.get(seq, 0) + n
+        assert rows == want
+    assert sum(n for _, _, n, _ in with_gen["gen"].items()) == 300
