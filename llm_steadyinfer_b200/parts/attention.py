@@ -314,12 +314,13 @@ class Attention(Mixer):
     def _plan_general_tc05(self, ctx, page_size: int) -> dict:
         """Which sequences of the step go to the tcgen05 prompt kernel (those that bring at least one full item of rows),
         and their work items; the others are the general tensor-core kernel's."""
-        key = ("attention_general_tc05", self.H, self.KV, self.hs, self.window, self.chunk)
+        ok = ctx.seq_cap is None and self.general_tc05_ok(page_size)
+        key = ("attention_general_tc05", self.H, self.KV, self.hs, self.window, self.chunk, ok)
         got = ctx.plans.get(key)
         if got is not None:
             return got
         out = {"skip": frozenset(), "all": False, "items": None}
-        if ctx.seq_cap is None and self.general_tc05_ok(page_size):
+        if ok:
             per = ops.attn_portion_tc05_tokens(self.H, self.KV)
             qs, cl = ctx.h_q_start, ctx.h_ctx_len
             chosen, items = [], []

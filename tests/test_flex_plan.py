@@ -1,8 +1,11 @@
 """The work lists of the general tensor-core attention (host side only; the kernels' own answers are stood in for)."""
+from types import SimpleNamespace
+
 import numpy as np
 import pytest
 
 from llm_steadyinfer_b200.parts import flex_plan
+from llm_steadyinfer_b200.parts.attention import Attention
 
 
 class Upload:
@@ -82,3 +85,14 @@ def test_layers_that_differ_in_the_prompt_kernel_keep_lists_of_their_own():
             rows[seq] = rows.get(seq, 0) + n
         assert rows == want
     assert sum(n for _, _, n, _ in with_gen["gen"].items()) == 300
+
+
+@pytest.mark.parametrize("first", [True, False])
+def test_a_layer_whose_scores_the_extended_form_does_not_know_gets_no_items_there(first):
+    """Layers of one head layout in one step, one with a gate (the extended form takes it), one with a bias by distance (it does not)."""
+    ctx = Ctx([(400, 400)])
+    layers = {ok: SimpleNamespace(H=4, KV=4, hs=128, window=None, chunk=None, _tag=lambda: "4_4_128_None", general_tc05_ok=lambda page, ok=ok: ok)
+              for ok in (True, False)}
+    got = {ok: Attention._plan_general_tc05(layers[ok], ctx, 16) for ok in (first, not first)}
+    assert got[False] == {"skip": frozenset(), "all": False, "items": None}
+    assert got[True]["all"] and sum(n for _, _, n, _ in got[True]["items"].items()) == 400
