@@ -644,16 +644,20 @@ SI_EXPORT int si_attn_portion_tc05_ok(int H, int KV, int hs, int vs, int page_si
 // Tokens of one item: two query tiles of floor(128 / G) each.
 SI_EXPORT int si_attn_portion_tc05_tokens(int H, int KV) { return 2 * (128 / (H / KV)); }
 
+// Bytes of shared memory of a block: Q of both query tiles, the stages of K and of V, the biases. The block takes all of tensor
+// memory, so a second block on the same SM could only wait for it: ask for more than half of the shared memory.
+#define PORTION_SMEM_LIMIT (227 * 1024 - 256)            // beside the barriers
+static size_t portion_smem(int nk, int nv, bool bias, int G) {
+  size_t smem = (size_t)(2 * 128 * nk * 64 + 2 * nk * 128 * 64 + (nk > 2 ? 1 : 2) * nv * 128 * 64) * sizeof(bf16) + 1024;
+  if (bias) smem += (size_t)4 * G * bias_pitch(G) * sizeof(float);
+  return smem < 120 * 1024 ? 120 * 1024 : smem;
+}
+
 template <int NK, int NV, int MODE>
 static int launch(const AttnParams& p, const CUtensorMap& km, const CUtensorMap& vm, int num_items, int log2_page,
                   cudaStream_t stream, const AttnExtras& x) {
-  constexpr int VST = NK > 2 ? 1 : 2;
-  // Q of both query tiles, the stages of K and of V, the biases. The block takes all of tensor memory, so a second
-  // block on the same SM could only wait for it: ask for more than half of the shared memory.
-  size_t smem = (size_t)(2 * 128 * NK * 64 + 2 * NK * 128 * 64 + VST * NV * 128 * 64) * sizeof(bf16) + 1024;
-  if (MODE == MODE_BIAS) smem += (size_t)4 * p.G * bias_pitch(p.G) * sizeof(float);
-  if (smem < 120 * 1024) smem = 120 * 1024;
-  if (smem > 227 * 1024 - 256) return -2;
+  const size_t smem = portion_smem(NK, NV, MODE == MODE_BIAS, p.G);
+  if (smem > PORTION_SMEM_LIMIT) return -2;
   auto k = attn_portion_tc05_kernel<NK, NV, MODE>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
@@ -737,7 +741,8 @@ SI_EXPORT int si_attn_portion_gen_ok(int H, int KV, int dk, int dv, int v_share,
   if (KV <= 0 || H % KV || H / KV > 128 || v_share < 1 || KV % v_share) return 0;
   if (dk <= 0 || dv <= 0 || dk > 192 || dk % 8 || dv % 8 || dv > 8192 || (bias && cap)) return 0;
   if ((bias || cap) && dk > 128) return 0;
-  if (bias && H / KV > 16) return 0;                 // the windows beside the tiles in shared memory
+  // a bias's windows stand beside the tiles in shared memory: up to 13 heads a key head with two halves of key columns
+  if (bias && (H / KV > 16 || portion_smem((dk + 63) / 64, 2, true, H / KV) > PORTION_SMEM_LIMIT)) return 0;
   if (!dense && page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64) return 0;
   return si_encode_fn() != nullptr;
 }

@@ -77,6 +77,21 @@ def test_each_mechanism_alone(folders, plains, name, dtype):
         check(rp, steps, reqs, plains[name], dtype, f"{name}/{mode}")
 
 
+@pytest.mark.parametrize("dim,heads", [(64, 13), (64, 14), (64, 16), (128, 13), (128, 14), (128, 16), (128, 32)])
+def test_biased_prompts_with_many_heads_a_key_head(tmp_path, dim, heads):
+    """One layer whose query heads share a key head, prompts whole and in portions: heads whose bias windows fit the prompt kernel's
+    shared memory and heads whose do not (14 and more at a key size of 128), which the general kernel serves."""
+    cfg = mc._model(200, 64, 1e-5, None, [mc._layer("attention", mc._attn(heads, 1, dim, 64, 40.0, 12), ff=None)])
+    folder = mc.write_folder(str(tmp_path / "m"), cfg, seed=dim + heads)
+    reqs = {f"q{i}": ru.random_tokens(cfg["vocab"], n, i) for i, n in enumerate([3, 9, 150])}
+    from llm_steadyinfer_b200.csrc import ops
+    from llm_steadyinfer_b200.engine.replay import Replayer
+    assert ops.attn_portion_gen_ok(heads, 1, dim, 64, 1, 16, bias=True) == (heads <= 13 or (heads <= 16 and dim <= 64))
+    for what, steps in (("whole", ru.trace_whole(reqs)), ("tail", ru.trace_tail(reqs, tail=20))):
+        rp = Replayer(folder, torch.bfloat16, 160, page_size=16, max_requests=4)
+        check(rp, steps, reqs, ru.PlainLogits(folder, pm), torch.bfloat16, what)
+
+
 @pytest.mark.parametrize("name", ["mixed_a", "mixed_b"])
 def test_layers_one_by_one_in_32_bit(folders, name):
     """The residual stream after every layer run against the plain one (shared-weight runs counted each time)."""
