@@ -82,7 +82,11 @@ __device__ __forceinline__ bf16* half_ptr(bf16* base, int row, int chunk) {
 //         result(i, h, d) *= sigmoid(gate[i, h * hs + d])   (gate null: none)
 //   BIAS  score(i, j) = scale * q.k + bias[min(i - j, nd - 1), h]
 //   CAP   score(i, j) = cap * tanh(scale * q.k / cap)
-enum { MODE_PLAIN = 0, MODE_EXT = 1, MODE_BIAS = 2, MODE_CAP = 3 };
+//   GEN   score(i, j) = scale * q.k
+// BIAS, CAP and GEN are the general form: key heads that share values, fp32 results, values in several blocks, dense rows. What its
+// tiles hold behind an item's last key (a page's earlier owner's rows, another sequence's) is zeroed before it meets the probabilities:
+// those are zeros there, but zero times a number that is not finite is none.
+enum { MODE_PLAIN = 0, MODE_EXT = 1, MODE_BIAS = 2, MODE_CAP = 3, MODE_GEN = 4 };
 struct AttnExtras {
   const float* slopes;                           // fp32 [H] or nullptr
   float qt_coef; int qt_every;
@@ -122,7 +126,7 @@ template <int NK, int NV, int MODE>
 __global__ void __launch_bounds__(320)
 attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap,
                          const __grid_constant__ CUtensorMap vmap, int log2_page, const AttnExtras x) {
-  constexpr bool EXT = MODE == MODE_EXT;
+  constexpr bool EXT = MODE == MODE_EXT, GENERAL = MODE >= MODE_BIAS;
   constexpr int BM = 128, BN = 128, DK = NK * 64, DV = NV * 64, STAGES = 2, VST = NK > 2 ? 1 : 2;
   constexpr int KTILE = NK * BN * 64, VTILE = NV * BN * 64;      // elements of a tile: halves of [128][64]
   constexpr int TM_S = 0, TM_O = 2 * BN;             // tensor-memory columns: S of tile q at TM_S + q*BN, O at TM_O + q*DV
@@ -186,7 +190,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
   if (warp == 9) tmem_alloc(&tmem_slot, TM_COLS);
   // rows that no copy fills must hold finite numbers (they meet zero probabilities): those behind the
   // last key in the last tile, and pages wholly before the window in the first
-  // (dense rows are fetched whole: what lies behind a sequence is another's rows, or zeros behind the last)
+  // (dense tiles are fetched whole: what lies behind a sequence is another's rows, or zeros behind the last)
   auto clear_tile = [&](int t) {
     uint4* kz = reinterpret_cast<uint4*>(Ks + (size_t)(t % STAGES) * KTILE);
     uint4* vz = reinterpret_cast<uint4*>(Vs + (size_t)(t % VST) * VTILE);
@@ -268,8 +272,10 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
       for (int i = 0; i < 2; ++i) {
         const int b = lane + 32 * i, pg = b / nh, h = b % nh;
         if (row_of[i] < 0) continue;
-        const int col = (x.dense ? (keys ? g * p.hs : gv * p.vs) : 0) + (keys ? 0 : v0) + h * 64;
-        tma_load_2d(tile + (size_t)h * (BN * 64) + (size_t)(pg * page_rows) * 64, keys ? &kmap : &vmap, full, col, row_of[i]);
+        const int col = (keys ? 0 : v0) + h * 64;
+        bf16* to = tile + (size_t)h * (BN * 64) + (size_t)(pg * page_rows) * 64;
+        if (GENERAL && x.dense) tma_load_3d(to, keys ? &kmap : &vmap, full, col, keys ? g : gv, row_of[i]);
+        else tma_load_2d(to, keys ? &kmap : &vmap, full, col, row_of[i]);
       }
       return true;
     };
@@ -315,6 +321,15 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
       const int stage = t % VST;
       const bool more = t + 1 < ntiles;
       ok = mbar_wait_warp(&v_full[stage], (unsigned)((t / VST) & 1));
+      if (GENERAL && ok && !more && (kv_end - kv_begin) % BN != 0) {      // a row is 128 bytes of each half, whatever the swizzle
+        const int first = (kv_end - kv_begin) % BN;
+        for (int i = lane; i < (BN - first) * NV * 8; i += 32) {
+          const int half = i / ((BN - first) * 8), at = i - half * (BN - first) * 8;
+          reinterpret_cast<uint4*>(Vs + (size_t)stage * VTILE + (size_t)half * (BN * 64) + (size_t)first * 64)[at] = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncwarp();
+      }
       for (int q = 0; q < nq && ok; ++q) {
         ok = mbar_wait_warp(&p_full[q], (unsigned)(t & 1));
         if (!ok) break;
@@ -361,7 +376,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
       if (x.qt_every > 0 && pos >= 0) row_scale *= 1.f + x.qt_coef * logf((float)((pos + 1) / x.qt_every + 1));
       if (x.slopes) sl2 = x.slopes[g * p.G + (hh < p.G ? hh : 0)] * 1.4426950408889634f;
     }
-    const float sc = MODE != MODE_PLAIN ? 1.f : p.scale_log2;
+    const float sc = MODE != MODE_PLAIN && MODE != MODE_GEN ? 1.f : p.scale_log2;
     // BIAS: entry k of a head's window is the distance (last position of the query tile) - j0 - k; the tile's four warps
     // copy the next key tile's window while this one's is read
     const int pitch = MODE == MODE_BIAS ? bias_pitch(p.G) : 0, span = tile_tokens + BN - 1;
@@ -765,9 +780,8 @@ SI_EXPORT int si_attn_portion_gen(const void* q, long long q_stride, const void*
   alignas(64) CUtensorMap km, vm;
   if (dense) {
     if (num_pages <= 0 || ((uintptr_t)keys % 16) || ((uintptr_t)values % 16)) return -2;
-    const unsigned long long kc = (unsigned long long)KV * dk, vc = (unsigned long long)(KV / v_share) * dv;
-    int rc = si_encode_bf16_2d(&km, keys, (unsigned long long)num_pages, kc, kc, DENSE_BOX);
-    if (!rc) rc = si_encode_bf16_2d(&vm, values, (unsigned long long)num_pages, vc, vc, DENSE_BOX);
+    int rc = si_encode_bf16_heads(&km, keys, (unsigned long long)num_pages, KV, dk, DENSE_BOX);
+    if (!rc) rc = si_encode_bf16_heads(&vm, values, (unsigned long long)num_pages, KV / v_share, dv, DENSE_BOX);
     if (rc) return rc;
   } else {
     km = *(const CUtensorMap*)keys;
@@ -776,8 +790,8 @@ SI_EXPORT int si_attn_portion_gen(const void* q, long long q_stride, const void*
 #define GEN_LAUNCH(NK, MODE) return launch<NK, 2, MODE>(p, km, vm, num_items, log2_page, stream, x)
   if (bias) { if (nk == 1) GEN_LAUNCH(1, MODE_BIAS); GEN_LAUNCH(2, MODE_BIAS); }
   if (softcap > 0.f) { if (nk == 1) GEN_LAUNCH(1, MODE_CAP); GEN_LAUNCH(2, MODE_CAP); }
-  if (nk == 1) GEN_LAUNCH(1, MODE_PLAIN);
-  if (nk == 2) GEN_LAUNCH(2, MODE_PLAIN);
-  GEN_LAUNCH(3, MODE_PLAIN);
+  if (nk == 1) GEN_LAUNCH(1, MODE_GEN);
+  if (nk == 2) GEN_LAUNCH(2, MODE_GEN);
+  GEN_LAUNCH(3, MODE_GEN);
 #undef GEN_LAUNCH
 }

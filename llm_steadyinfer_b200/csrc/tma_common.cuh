@@ -46,6 +46,10 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
                ::"r"(tma_smem_u32(dst)), "l"(map), "r"(tma_smem_u32(bar)), "r"(x), "r"(y) : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
+               ::"r"(tma_smem_u32(dst)), "l"(map), "r"(tma_smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
+}
 
 // ---- tcgen05 (5th generation tensor cores, accumulators in tensor memory) ------------------------
 // Allocate `ncols` (power of two >= 32) columns of tensor memory; executed by one whole warp.
@@ -244,6 +248,22 @@ static inline int si_encode_bf16_2d(CUtensorMap* map, const void* base, unsigned
   const cuuint32_t box[2] = {64, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : 1000 + (int)r;
+}
+
+// bf16 matrix of rows of `heads` heads of `cols` columns each, boxes of [box_rows, one head, 64 columns] that end at their head: what
+// a box has beyond `cols` arrives as zeros, not as the next head's columns. Coordinates (column, head, row).
+static inline int si_encode_bf16_heads(CUtensorMap* map, const void* base, unsigned long long rows, int heads, int cols,
+                                       unsigned box_rows) {
+  SiEncodeTiledFn fn = si_encode_fn();
+  if (!fn) return -3;
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)heads, rows};
+  const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)heads * cols * 2};
+  const cuuint32_t box[3] = {64, 1, box_rows};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : 1000 + (int)r;

@@ -1591,3 +1591,43 @@ def test_causal_convolution_of_portions_and_single_rows(C, K, dtype):
         if pad:
             assert (out[-pad:] == 0).all()
     assert status.item() == 0
+
+
+@pytest.mark.parametrize("H,KV,dk,dv,share,page,bias,cap", [
+    (2, 2, 192, 128, 1, 0, 0, 0.0),          # rows of matrices: the next sequence's rows stand behind the last
+    (2, 2, 136, 72, 1, 0, 0, 0.0),           # boxes wider than a head
+    (4, 2, 64, 264, 2, 16, 0, 0.0),          # pages: what an earlier owner left in them, values in three blocks
+    (4, 2, 128, 128, 1, 64, 9, 0.0),
+    (4, 2, 64, 64, 1, 8, 0, 20.0),
+])
+@pytest.mark.parametrize("end", [1, 63, 130, 255, 300])
+def test_portions_in_the_general_form_beside_numbers_that_are_not_finite(H, KV, dk, dv, share, page, bias, cap, end):
+    """What lies behind a sequence's last key, in its last page or in the next sequence's rows, and what other key heads hold, reaches no
+    result: the same bits with zeros and with NaN and infinities there."""
+    o = ops()
+    assert o.attn_portion_gen_ok(H, KV, dk, dv, share, page, bias > 0, cap > 0)
+    g = torch.Generator().manual_seed(dk + end)
+    KVv = KV // share
+    rows = end + 200 if not page else -(-end // page) * page
+    q = torch.randn(end, H * dk, generator=g).to(torch.bfloat16).to(DEV)
+    k, v = torch.randn(rows, KV, dk, generator=g).to(torch.bfloat16), torch.randn(rows, KVv, dv, generator=g).to(torch.bfloat16)
+    rel = torch.randn(bias, H, generator=g).to(DEV) if bias else None
+    per = o.attn_portion_tc05_tokens(H, KV)
+    items = torch.tensor([(0, b, min(per, end - b), b) for b in range(0, end, per)], dtype=torch.int32, device=DEV)
+    G, got = H // KV, []
+    for behind in (0.0, math.nan, math.inf):
+        k[end:], v[end:] = behind, behind
+        k[:, 1:] = behind                       # (queries of the first key head only are looked at; values stay where heads share them)
+        if KVv > 1:
+            v[:, 1:] = behind
+        if page:
+            def paged(t):
+                return t.view(-1, page, *t.shape[1:]).transpose(1, 2).contiguous().to(DEV)
+            k_in, v_in, table = paged(k), paged(v), torch.arange(rows // page, dtype=torch.int32, device=DEV).view(1, -1)
+        else:
+            k_in, v_in, table = k.reshape(rows, -1).to(DEV), v.reshape(rows, -1).to(DEV), torch.zeros(1, 1, dtype=torch.int32, device=DEV)
+        out = torch.zeros(end, H * dv, device=DEV)
+        o.attn_portion_gen(q, k_in, v_in, table, items, out, page, 1, H, KV, dk, dv, dk ** -0.5, dist_bias=rel, softcap=cap, v_share=share)
+        got.append(out[:, :G * dv].clone())
+    assert bool(torch.isfinite(got[0]).all()) and bool(got[0].abs().amax() > 0)
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
