@@ -86,7 +86,10 @@ __device__ __forceinline__ bf16* half_ptr(bf16* base, int row, int chunk) {
 // BIAS, CAP and GEN are the general form: key heads that share values, fp32 results, values in several blocks, dense rows. What its
 // tiles hold behind an item's last key (a page's earlier owner's rows, another sequence's) is zeroed before it meets the probabilities:
 // those are zeros there, but zero times a number that is not finite is none.
-enum { MODE_PLAIN = 0, MODE_EXT = 1, MODE_BIAS = 2, MODE_CAP = 3, MODE_GEN = 4 };
+// CUT is PLAIN with items whose keys are cut over blocks (AttnExtras::shares). What only some forms have is decided when their instance is
+// compiled: 2,048 tokens of 32 query and 8 key heads of 128 took 51.7 us where the plain form asked for shares, dense rows and the rest as
+// it ran, and 50.0 so.
+enum { MODE_PLAIN = 0, MODE_CUT = 1, MODE_EXT = 2, MODE_BIAS = 3, MODE_CAP = 4, MODE_GEN = 5 };
 struct AttnExtras {
   const float* slopes;                           // fp32 [H] or nullptr
   float qt_coef; int qt_every;
@@ -96,7 +99,7 @@ struct AttnExtras {
   int v_share;                                   // key heads that read one value head
   int out_f32;                                   // p.out is fp32
   int dense;                                     // keys and values [rows, KV * size]: a sequence's rows lie behind its table's first entry
-  // MODE_PLAIN, one block of values: an item's keys may be cut into shares, a block each. Entry (item, share, shares of the item, slot of
+  // MODE_CUT, one block of values: an item's keys may be cut into shares, a block each. Entry (item, share, shares of the item, slot of
   // its first share's partial results); a whole item has one share. Shares leave O, maximum and sum per row; a second kernel merges.
   const int4* shares;
   float* part_o;                                 // [slot][KV][256 rows][NV * 64]
@@ -126,7 +129,8 @@ template <int NK, int NV, int MODE>
 __global__ void __launch_bounds__(320)
 attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap,
                          const __grid_constant__ CUtensorMap vmap, int log2_page, const AttnExtras x) {
-  constexpr bool EXT = MODE == MODE_EXT, GENERAL = MODE >= MODE_BIAS;
+  constexpr bool CUT = MODE == MODE_CUT, EXT = MODE == MODE_EXT, GENERAL = MODE >= MODE_BIAS;
+  const bool dense = GENERAL && x.dense;
   constexpr int BM = 128, BN = 128, DK = NK * 64, DV = NV * 64, STAGES = 2, VST = NK > 2 ? 1 : 2;
   constexpr int KTILE = NK * BN * 64, VTILE = NV * BN * 64;      // elements of a tile: halves of [128][64]
   constexpr int TM_S = 0, TM_O = 2 * BN;             // tensor-memory columns: S of tile q at TM_S + q*BN, O at TM_O + q*DV
@@ -145,7 +149,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
   // Items of a prompt come in order of position, so the last ones have the most keys: start with those,
   // for all KV heads alike (blocks are handed out with x running fastest, and x is the KV head).
   // (With shares the entries come longest first.)
-  const int4 share = (MODE == MODE_PLAIN && x.shares) ? x.shares[blockIdx.y] : make_int4(gridDim.y - 1 - blockIdx.y, 0, 1, 0);
+  const int4 share = CUT ? x.shares[blockIdx.y] : make_int4(gridDim.y - 1 - blockIdx.y, 0, 1, 0);
   const AttnItem item = p.items[share.x];
   if (item.ntok <= 0) return;
   const int g = blockIdx.x;
@@ -161,7 +165,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
   const int kv_lo = first_visible_key(item.pos0, p.window, p.chunk);
   int kv_begin = kv_lo / BN * BN;
   int ntiles = (kv_end - kv_begin + BN - 1) / BN;
-  if (MODE == MODE_PLAIN && share.z > 1) {           // this share's tiles
+  if (CUT && share.z > 1) {           // this share's tiles
     const int first = (int)((long long)ntiles * share.y / share.z), last = (int)((long long)ntiles * (share.y + 1) / share.z);
     kv_begin += first * BN;
     ntiles = last - first;
@@ -169,7 +173,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
   }
   const int page_rows = 1 << log2_page;              // dense: rows of a box
   const int pages_per_tile = BN >> log2_page;
-  const int v0 = blockIdx.z * DV;                    // first value column of this block
+  const int v0 = GENERAL ? blockIdx.z * DV : 0;                    // first value column of this block
 
   pdl_trigger();
   if (threadIdx.x == 0) {
@@ -197,8 +201,8 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
     for (int i = threadIdx.x; i < KTILE / 8; i += blockDim.x) kz[i] = make_uint4(0, 0, 0, 0);
     for (int i = threadIdx.x; i < VTILE / 8; i += blockDim.x) vz[i] = make_uint4(0, 0, 0, 0);
   };
-  if (!x.dense && (kv_end - kv_begin) % BN != 0) clear_tile(ntiles - 1);
-  if (!x.dense && kv_begin + page_rows <= kv_lo) clear_tile(0);
+  if (!dense && (kv_end - kv_begin) % BN != 0) clear_tile(ntiles - 1);
+  if (!dense && kv_begin + page_rows <= kv_lo) clear_tile(0);
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   tc05_fence_before_sync();
   __syncthreads();                                   // barriers, tensor memory and the zeroed rows stand
@@ -239,49 +243,39 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
     // ---- producer: box b = (page, half, K or V) of each tile, boxes spread over the lanes. K and V
     // have barriers of their own: a K stage is free as soon as both S have been computed from it, long
     // before the V stage of the same tile, so the next keys arrive under the softmax.
-    const int gv = g / x.v_share, KVv = p.KV / x.v_share;
-    const int first_row = x.dense ? table[0] : 0;    // of the sequence's rows in the matrices
-    auto fetch = [&](int t, int j, bool keys) {
-      const int nh = keys ? NK : NV;
-      const int stage = t % (keys ? STAGES : VST), boxes = pages_per_tile * nh;
-      uint64_t* full = keys ? &k_full[stage] : &v_full[stage];
-      uint64_t* empty = keys ? &k_empty[stage] : &v_empty[stage];
-      bf16* tile = keys ? Ks + (size_t)stage * KTILE : Vs + (size_t)stage * VTILE;
-      int cnt = 0, row_of[2] = {-1, -1};             // this lane's boxes
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int b = lane + 32 * i, pg = b / nh, j_pg = j + pg * page_rows;
-        if (b >= boxes) continue;
-        if (x.dense) {
-          row_of[i] = first_row + j_pg;
-        } else if (j_pg < kv_end && j_pg + page_rows > kv_lo) {    // pages past the last key, or wholly before the window, are not fetched
-          const int slot = (j >> log2_page) + pg;
-          const int page = slot < p.table_width ? table[slot] : -1;
-          if (page < 0 || page >= p.num_pages) set_status(p.status, SI_BAD_PAGE);
-          else row_of[i] = (page * (keys ? p.KV : KVv) + (keys ? g : gv)) << log2_page;
-        }
-        cnt += row_of[i] >= 0;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-      const int st = keys ? STAGES : VST;
-      if (t >= st && !mbar_wait_warp(empty, (unsigned)(((t / st) - 1) & 1))) return false;
-      if (lane == 0) mbar_expect_tx(full, (unsigned)(cnt * page_rows * 128));
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int b = lane + 32 * i, pg = b / nh, h = b % nh;
-        if (row_of[i] < 0) continue;
-        const int col = (keys ? 0 : v0) + h * 64;
-        bf16* to = tile + (size_t)h * (BN * 64) + (size_t)(pg * page_rows) * 64;
-        if (GENERAL && x.dense) tma_load_3d(to, keys ? &kmap : &vmap, full, col, keys ? g : gv, row_of[i]);
-        else tma_load_2d(to, keys ? &kmap : &vmap, full, col, row_of[i]);
-      }
-      return true;
-    };
+    const int gv = GENERAL ? g / x.v_share : g, KVv = GENERAL ? p.KV / x.v_share : p.KV;
+    const int first_row = dense ? table[0] : 0;    // of the sequence's rows in the matrices
     for (int t = 0; t < ntiles; ++t) {
       const int j = kv_begin + t * BN;
-      if (!fetch(t, j, true) || !fetch(t, j, false)) {
+      int page = -1;                                 // lane l: the page of the tile's keys from l * page_rows on
+      // pages past the last key, or wholly before the window, are not fetched
+      if (!dense && lane < pages_per_tile && j + lane * page_rows < kv_end && j + (lane + 1) * page_rows > kv_lo) {
+        const int slot = (j >> log2_page) + lane;
+        page = slot < p.table_width ? table[slot] : -1;
+        if (page < 0 || page >= p.num_pages) { set_status(p.status, SI_BAD_PAGE); page = -1; }
+      }
+      const int pages = dense ? pages_per_tile : __popc(__ballot_sync(0xffffffffu, page >= 0));
+      auto fetch = [&](bool keys) {
+        const int nh = keys ? NK : NV, st = keys ? STAGES : VST, stage = t % st;
+        uint64_t* full = keys ? &k_full[stage] : &v_full[stage];
+        uint64_t* empty = keys ? &k_empty[stage] : &v_empty[stage];
+        bf16* tile = keys ? Ks + (size_t)stage * KTILE : Vs + (size_t)stage * VTILE;
+        if (t >= st && !mbar_wait_warp(empty, (unsigned)(((t / st) - 1) & 1))) return false;
+        if (lane == 0) mbar_expect_tx(full, (unsigned)(pages * nh * page_rows * 128));
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int b = lane + 32 * i, pg = b / nh, h = b % nh;
+          const int of = __shfl_sync(0xffffffffu, page, pg & 31);
+          if (pg >= pages_per_tile || (!dense && of < 0)) continue;
+          bf16* to = tile + (size_t)h * (BN * 64) + (size_t)(pg * page_rows) * 64;
+          const int col = (keys ? 0 : v0) + h * 64;
+          if (dense) tma_load_3d(to, keys ? &kmap : &vmap, full, col, keys ? g : gv, first_row + j + pg * page_rows);
+          else tma_load_2d(to, keys ? &kmap : &vmap, full, col, (of * (keys ? p.KV : KVv) + (keys ? g : gv)) << log2_page);
+        }
+        return true;
+      };
+      if (!fetch(true) || !fetch(false)) {
         if (lane == 0) { set_status(p.status, SI_WAIT_LIMIT); s_abort = 1; }
         break;
       }
@@ -376,7 +370,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
       if (x.qt_every > 0 && pos >= 0) row_scale *= 1.f + x.qt_coef * logf((float)((pos + 1) / x.qt_every + 1));
       if (x.slopes) sl2 = x.slopes[g * p.G + (hh < p.G ? hh : 0)] * 1.4426950408889634f;
     }
-    const float sc = MODE != MODE_PLAIN && MODE != MODE_GEN ? 1.f : p.scale_log2;
+    const float sc = EXT || MODE == MODE_BIAS || MODE == MODE_CAP ? 1.f : p.scale_log2;
     // BIAS: entry k of a head's window is the distance (last position of the query tile) - j0 - k; the tile's four warps
     // copy the next key tile's window while this one's is read
     const int pitch = MODE == MODE_BIAS ? bias_pitch(p.G) : 0, span = tile_tokens + BN - 1;
@@ -533,7 +527,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
     }
     if (alive && ntiles > 0) alive = mbar_wait_warp(&o_full[q], 0);
     if (!alive && lane == 0) { set_status(p.status, SI_WAIT_LIMIT); s_abort = 1; }
-    if (MODE == MODE_PLAIN && share.z > 1) {                 // a share's results as they are
+    if (CUT && share.z > 1) {                 // a share's results as they are
       const size_t row = (((size_t)(share.w + share.y) * p.KV + g) * 2 + q) * BM + r;
       if (alive && valid) {
         tc05_fence_after_sync();
@@ -583,7 +577,7 @@ attn_portion_tc05_kernel(const AttnParams p, const __grid_constant__ CUtensorMap
               }
             }
           }
-          if (x.out_f32) {
+          if (GENERAL && x.out_f32) {
             float* f = reinterpret_cast<float*>(p.out) + at;
 #pragma unroll
             for (int q8 = 0; q8 < 16; ++q8)
@@ -737,7 +731,7 @@ SI_EXPORT int si_attn_portion_tc05(const void* q, long long q_stride, const void
     x.shares = (const int4*)shares;
     x.part_o = scratch;
     x.part_ml = scratch + (long long)slots * KV * 256 * dv;
-    int rc = narrow ? launch<1, 1, MODE_PLAIN>(p, km, vm, num_shares, log2_page, stream, x) : launch<2, 2, MODE_PLAIN>(p, km, vm, num_shares, log2_page, stream, x);
+    int rc = narrow ? launch<1, 1, MODE_CUT>(p, km, vm, num_shares, log2_page, stream, x) : launch<2, 2, MODE_CUT>(p, km, vm, num_shares, log2_page, stream, x);
     if (rc || !num_cut) return rc;
     const dim3 grid(KV, num_cut, 32);
     if (narrow) si_launch(attn_portion_merge_kernel<1>, grid, dim3(256), 0, stream, p, (const int4*)cut, (const float*)x.part_o, (const float*)x.part_ml);
