@@ -812,6 +812,7 @@ __global__ void __launch_bounds__(256, RPT <= 8 && SLOTS <= 4 ? 2 : 1) channel_d
   fetch(0, 0);
   const bool has_q = p & 8;
   const int my_i = (p >> 1) & 3, my_c = p & 1;
+  const unsigned up_to[3] = {my_i > 0 ? ~0u : 0u, my_i > 1 ? ~0u : 0u, my_i > 2 ? ~0u : 0u};
   float* yp = y + (size_t)(row0 + my_i) * y_stride + (size_t)h * dv + j + my_c;
   const bool writes = has_q && j + my_c < dv;
   int buf = 0;
@@ -873,11 +874,12 @@ __global__ void __launch_bounds__(256, RPT <= 8 && SLOTS <= 4 ? 2 : 1) channel_d
         }
       }
       {
-        const float4 qk = *reinterpret_cast<const float4*>(base + my_i * TOK + 3 * DKP + cols + 4);      // zeros behind token my_i
+        // (zeros behind token my_i, on both sides: what stands there need not be finite)
+        const float4 qk = *reinterpret_cast<const float4*>(base + my_i * TOK + 3 * DKP + cols + 4);
         float o = fmaf(qk.x, my_c ? u[0][1] : u[0][0], mine);
-        o = fmaf(qk.y, my_c ? u[1][1] : u[1][0], o);
-        o = fmaf(qk.z, my_c ? u[2][1] : u[2][0], o);
-        o = fmaf(qk.w, my_c ? u[3][1] : u[3][0], o);
+        o = fmaf(qk.y, __uint_as_float(__float_as_uint(my_c ? u[1][1] : u[1][0]) & up_to[0]), o);
+        o = fmaf(qk.z, __uint_as_float(__float_as_uint(my_c ? u[2][1] : u[2][0]) & up_to[1]), o);
+        o = fmaf(qk.w, __uint_as_float(__float_as_uint(my_c ? u[3][1] : u[3][0]) & up_to[2]), o);
         if (writes && (g0 + a) * M + my_i < n) *yp = o;
         yp += M * y_stride;
       }

@@ -638,6 +638,7 @@ __global__ void __launch_bounds__(256, 2) decay_group_scan_kernel(const float* _
   };
   fetch(0, 0);
   const int my_i = (p >> 1) & 3, my_c = p & 1;
+  const unsigned up_to[3] = {my_i > 0 ? ~0u : 0u, my_i > 1 ? ~0u : 0u, my_i > 2 ? ~0u : 0u};
   float* yp = y + (size_t)(row0 + my_i) * y_stride + (size_t)h * n + j + my_c;
   const bool writes = p < 8 && j + my_c < n;
   int buf = 0;
@@ -670,11 +671,12 @@ __global__ void __launch_bounds__(256, 2) decay_group_scan_kernel(const float* _
         }
       }
       float o = val[0] + __shfl_xor_sync(0xffffffffu, val[0], 8);
-      const float4 f = *reinterpret_cast<const float4*>(base + my_i * TOK + 2 * DKP + cols);      // zeros behind token my_i
+      // (zeros behind token my_i, on both sides: what stands there need not be finite)
+      const float4 f = *reinterpret_cast<const float4*>(base + my_i * TOK + 2 * DKP + cols);
       o = fmaf(f.x, my_c ? vv[0].y : vv[0].x, o);
-      o = fmaf(f.y, my_c ? vv[1].y : vv[1].x, o);
-      o = fmaf(f.z, my_c ? vv[2].y : vv[2].x, o);
-      o = fmaf(f.w, my_c ? vv[3].y : vv[3].x, o);
+      o = fmaf(f.y, __uint_as_float(__float_as_uint(my_c ? vv[1].y : vv[1].x) & up_to[0]), o);
+      o = fmaf(f.z, __uint_as_float(__float_as_uint(my_c ? vv[2].y : vv[2].x) & up_to[1]), o);
+      o = fmaf(f.w, __uint_as_float(__float_as_uint(my_c ? vv[3].y : vv[3].x) & up_to[2]), o);
       if (writes && (g0 + a) * M + my_i < cnt) *yp = o;
       yp += M * y_stride;
       const float4 cv = reinterpret_cast<const float4*>(base + M * TOK)[p];

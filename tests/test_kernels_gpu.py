@@ -1631,3 +1631,40 @@ def test_portions_in_the_general_form_beside_numbers_that_are_not_finite(H, KV, 
         got.append(out[:, :G * dv].clone())
     assert bool(torch.isfinite(got[0]).all()) and bool(got[0].abs().amax() > 0)
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("kind", ["delta", "decay"])
+@pytest.mark.parametrize("at", [1, 2, 3, 6, 8])
+def test_groups_of_four_keep_the_order_of_tokens(kind, at):
+    """A token whose value is not finite leaves every earlier token's result as it is, also those of its own group of four: the same
+    bits as with another number there."""
+    o = ops()
+    g = torch.Generator().manual_seed(at)
+    H, n, T = 2, 64, 9
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    q_start, ctx, slot, row_seq = i32([0, T]), i32([T]), i32([0]), i32([0] * T)
+    outs = []
+    if kind == "delta":
+        xc, u = torch.randn(T, 2 * n + H * n, generator=g), torch.randn(T, 2 * H, generator=g).to(DEV)
+        a_log, dt_bias = torch.rand(H, generator=g).to(DEV), torch.rand(H, generator=g).to(DEV)
+    else:
+        xs, u = torch.randn(T, 4 * H * n, generator=g), torch.randn(H, n, generator=g).to(DEV)
+        xs[:, 3 * H * n:] = 0.9
+    for odd in (1.0, math.nan, math.inf):
+        y = torch.zeros(T, H * n, device=DEV)
+        if kind == "delta":
+            x = xc.clone()
+            x[at, 2 * n:] = odd
+            x = x.to(DEV)
+            state, bg = torch.zeros(1, H * o.delta_state_floats(n, n), device=DEV), torch.empty(T, 2 * H + 1, device=DEV)
+            o.delta_prepare(x, u, 0, H, a_log, dt_bias, bg, 1, H, n, n ** -0.5)
+            dec, rec, sc = torch.empty(T, H * n, device=DEV), torch.empty(T, H, 3, n, device=DEV), torch.empty(T, H, o.GROUP_SCALARS, device=DEV)
+            o.channel_delta_groups(x, u, 0, dec, a_log, dt_bias, rec, sc, row_seq, q_start, 1, 1, H, n, a_off=H)
+            o.channel_delta_group_scan(rec, sc, dec, x, state, y, q_start, ctx, slot, 1, 1, H, n, n)
+        else:
+            x = xs.clone()
+            x[at, 2 * H * n:3 * H * n] = odd
+            state = torch.zeros(1, H * o.decay_state_floats(n), device=DEV)
+            o.decay_group_scan(x.to(DEV), u, torch.empty(T, H, 4, device=DEV), state, y, row_seq, q_start, ctx, slot, 1, H, n)
+        outs.append(y[:at].cpu())
+    assert bool(torch.isfinite(outs[0]).all()) and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
