@@ -917,14 +917,27 @@ __global__ void __launch_bounds__(256, RPT <= 8 && SLOTS <= 4 ? 2 : 1) channel_d
     }
 }
 
-// 1 when the form by groups takes a state of dk x dv: sixteen parts a column, sizes in multiples of 4.
+#define GROUP_COLS 32                                     // most columns a block (16, 64: no faster)
+#define GROUP_SLOTS 8                                     // most pieces of a group a thread copies
+static int group_cols(int dv) {
+  int cols = GROUP_COLS;
+  while (cols > 8 && cols / 2 >= dv) cols /= 2;
+  return cols;
+}
+static int group_slots(int dk, int cols) {                // eight threads a column
+  const int pieces = GROUP_TOKENS * (3 * dk / 4 + cols / 4 + 2) + dk / 4, threads = cols * 8;
+  return (pieces + threads - 1) / threads;
+}
+
+// 1 when the form by groups takes a state of dk x dv: sixteen parts a column, sizes in multiples of 4, and enough columns that their
+// threads copy a group's pieces (a block has 16 columns at least where there are as many).
 SI_EXPORT int si_channel_delta_groups_ok(int dk, int dv) {
   if (dk <= 0 || dv <= 0 || dk % 4 || dv % 4 || dk > 256) return 0;
   const DeltaShape sh = delta_shape(dk);
-  return sh.np == 16 && sh.rpt <= 16;
+  const int cols = group_cols(dv);
+  return sh.np == 16 && sh.rpt <= 16 && group_slots(dk, cols > 16 ? 16 : cols) <= GROUP_SLOTS;
 }
 
-#define GROUP_COLS 32                                     // most columns a block (16, 64: no faster)
 SI_EXPORT int si_channel_delta_group_scan(const float* rec, const float* sc, const float* dec, long long dec_stride, const float* xc,
                                           long long xc_stride, float* state, long long state_stride, float* y, long long y_stride,
                                           const int* q_start, const int* ctx_len, const int* slots, int num_seqs, int G, int H, int dk,
@@ -936,14 +949,13 @@ SI_EXPORT int si_channel_delta_group_scan(const float* rec, const float* sc, con
   const DeltaShape sh = delta_shape(dk);
   if (state_stride < (long long)H * sh.rpt * sh.np * dv) return -2;
   // columns a block, a multiple of 4: fewer while the blocks do not fill the device, so that every scheduler has a warp
-  int cols = GROUP_COLS;
-  while (cols > 8 && cols / 2 >= dv) cols /= 2;
+  int cols = group_cols(dv);
   const long long per = (long long)num_seqs * H;
   while (cols > 16 && per * ((dv + cols - 1) / cols) < si_sm_count()) cols /= 2;
   const int zb = (dv + cols - 1) / cols, threads = cols * 8;
-  const int pieces = GROUP_TOKENS * (3 * dk / 4 + cols / 4 + 2) + dk / 4, need = (pieces + threads - 1) / threads;
+  const int need = group_slots(dk, cols);
   const size_t smem = (size_t)2 * GROUP_AHEAD * (GROUP_TOKENS * (3 * sh.rpt * 16 + cols + GROUP_SCALARS) + sh.rpt * 16) * sizeof(float);
-  if (zb > 65535 || need > 8 || smem > 220 * 1024) return -2;
+  if (zb > 65535 || need > GROUP_SLOTS || smem > 220 * 1024) return -2;
   const dim3 grid(num_seqs, H, zb), block(threads);
 #define GROUP_LAUNCH(R, Q)                                                                                           \
   {                                                                                                                  \

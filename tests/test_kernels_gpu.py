@@ -1668,3 +1668,19 @@ def test_groups_of_four_keep_the_order_of_tokens(kind, at):
             o.decay_group_scan(x.to(DEV), u, torch.empty(T, H, 4, device=DEV), state, y, row_seq, q_start, ctx, slot, 1, H, n)
         outs.append(y[:at].cpu())
     assert bool(torch.isfinite(outs[0]).all()) and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("dk,dv,ok", [(152, 8, True), (156, 8, False), (256, 4, False), (256, 12, True), (256, 16, True), (8, 4, False)])
+def test_group_sizes_that_are_taken_run(dk, dv, ok):
+    """Few columns have few threads, which copy the pieces of a group of wide keys no longer: such heads go token by token. What is taken
+    runs."""
+    o = ops()
+    assert o.channel_delta_groups_ok(dk, dv) == ok
+    if not ok:
+        return
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    rec, sc, dec = torch.zeros(5, 1, 3, dk, device=DEV), torch.zeros(5, 1, o.GROUP_SCALARS, device=DEV), torch.ones(5, dk, device=DEV)
+    state = torch.ones(1, o.delta_state_floats(dk, dv), device=DEV)
+    o.channel_delta_group_scan(rec, sc, dec, torch.zeros(5, 2 * dk + dv, device=DEV), state, torch.empty(5, dv, device=DEV), i32([0, 5]), i32([7]), i32([0]),
+                               1, 1, 1, dk, dv)
+    assert bool((state <= 1).all()) and float(state.sum()) == dk * dv      # (entries behind dk are written as zeros)
