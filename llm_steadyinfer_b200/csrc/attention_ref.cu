@@ -83,7 +83,7 @@ paged_attention_ref_kernel(const T* __restrict__ q, long long q_row_stride,
       dot[u] = warp_sum(s) * scale;
       if (have[u]) m_new = fmaxf(m_new, dot[u]);
     }
-    if (m_new == -INFINITY) continue;    // no key of the run could be read
+    if (!__any_sync(0xffffffffu, at >= 0)) continue;      // no key of the run could be read
     const float corr = expf(m - m_new);
     l *= corr;
 #pragma unroll

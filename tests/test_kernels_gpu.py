@@ -1684,3 +1684,25 @@ def test_group_sizes_that_are_taken_run(dk, dv, ok):
     o.channel_delta_group_scan(rec, sc, dec, torch.zeros(5, 2 * dk + dv, device=DEV), state, torch.empty(5, dv, device=DEV), i32([0, 5]), i32([7]), i32([0]),
                                1, 1, 1, dk, dv)
     assert bool((state <= 1).all()) and float(state.sum()) == dk * dv      # (entries behind dk are written as zeros)
+
+
+@pytest.mark.parametrize("odd", [math.nan, math.inf])
+@pytest.mark.parametrize("at", [0, 7, 8, 16])
+def test_plain_attention_keeps_no_result_that_is_not_finite_from_sight(at, odd):
+    """A key that is not finite (here the only one of its warp's run, or one of eight) spoils the rows that see it: they come out as zeros,
+    the mark of a row without a finite sum, and never as the weighted sum of the other keys. Rows before it are what they were."""
+    o = ops()
+    g = torch.Generator().manual_seed(at)
+    T, hs = 17, 32
+    q, k, v = (torch.randn(T, hs, generator=g) for _ in range(3))
+    q = q.abs() + 0.1                                 # an infinite key gives infinite scores, not NaN
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    outs = []
+    for x in (0.5, odd):
+        k[at] = x
+        out = torch.full((T, hs), 7.0, device=DEV)
+        o.paged_attention_ref(q.to(DEV), k.view(T, 1, 1, hs).to(DEV), v.view(T, 1, 1, hs).to(DEV), i32(list(range(T))).view(1, -1), i32([0] * T),
+                              i32(list(range(T))), out, 1, 1, 1, 1, hs, hs ** -0.5)
+        outs.append(out.cpu())
+    assert torch.equal(outs[0][:at], outs[1][:at]) and bool(outs[0].abs().amax(1).min() > 0)
+    assert bool((outs[1][at:] == 0).all() | torch.isnan(outs[1][at:]).all())
