@@ -2084,7 +2084,7 @@ def moe_combine(y, place_of, wts, out, shared=None, gate=None, ids=None, real: i
     T, d = out.shape
     top = wts.shape[1]
     _need(y.shape[1] == d and y.stride(1) == 1 and out.stride(1) == 1 and y.dtype in (out.dtype, torch.float32), "moe_combine: y [P, d]")
-    _need(y.shape[0] >= T * top, "moe_combine: y [P, d]")
+    _need(place_of is not None or y.shape[0] >= T * top, "moe_combine: y [P, d]")
     _need((place_of is None or place_of.shape == (T, top)) and wts.shape == (T, top) and wts.dtype == torch.float32 and wts.is_contiguous(), "moe_combine: wts, place_of")
     if shared is not None:
         _need(shared.shape == (T, d) and shared.stride(1) == 1 and shared.dtype == out.dtype, "moe_combine: shared must be [T, d]")

@@ -1706,3 +1706,16 @@ def test_plain_attention_keeps_no_result_that_is_not_finite_from_sight(at, odd):
         outs.append(out.cpu())
     assert torch.equal(outs[0][:at], outs[1][:at]) and bool(outs[0].abs().amax(1).min() > 0)
     assert bool((outs[1][at:] == 0).all() | torch.isnan(outs[1][at:]).all())
+
+
+def test_experts_results_with_no_rows_for_identity_experts():
+    """The combining sum with results of the experts that have weights only: places of identity experts have no row."""
+    o = ops()
+    g = torch.Generator().manual_seed(1)
+    y, x, wts = torch.randn(3, 40, generator=g), torch.randn(2, 40, generator=g), torch.rand(2, 2, generator=g)
+    ids = torch.tensor([[0, 5], [1, 2]], dtype=torch.int32)
+    place = torch.tensor([[1, 3], [0, 2]], dtype=torch.int32)         # place 3 is the identity expert's: y has no such row
+    out = torch.empty(2, 40, device=DEV)
+    o.moe_combine(y.to(DEV), place.to(DEV), wts.to(DEV), out, ids=ids.to(DEV), real=4, x=x.to(DEV))
+    want = torch.stack([wts[0, 0] * y[1] + wts[0, 1] * x[0], wts[1, 0] * y[0] + wts[1, 1] * y[2]])
+    assert (out.cpu() - want).abs().max().item() <= 1e-6
