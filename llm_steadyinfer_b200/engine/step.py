@@ -106,7 +106,7 @@ class _PinnedRing:
             ev = self.events[self.turn]
             if ev is None:
                 ev = self.events[self.turn] = torch.cuda.Event()
-            ev.record()
+            ev.record(torch.cuda.current_stream(self.dev.device))      # where the copy is, whatever device the calling thread is at
 
 
 class ModelRunner:

@@ -56,7 +56,7 @@ class Sampler:
         d.copy_(self._hosts[turn], non_blocking=True)
         if self._host_events[turn] is None:
             self._host_events[turn] = torch.cuda.Event()
-        self._host_events[turn].record()
+        self._host_events[turn].record(torch.cuda.current_stream(d.device))      # where the copy is, whatever device the calling thread is at
         v = self._device_views.get(R)
         if v is None:
             v = self._device_views[R] = (d[0:R].view(torch.float32), d[n:n + R].view(torch.float32), d[2 * n:2 * n + R],
