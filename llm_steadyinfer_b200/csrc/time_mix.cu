@@ -170,26 +170,25 @@ SI_EXPORT int si_shift_mix(const void* x, int dtype, long long x_stride, const f
 // r, k, v: rows of C values each in the compute dtype; z [T, L] likewise; w2t fp32 [L, C] (the second low-rank matrix,
 // transposed); w0 fp32 [C]; xs fp32 [T, 4C] = [r | k | v | decay]. A block takes ROWS rows and 256 channels (blockIdx.y),
 // a thread one channel: it walks the L rows of w2t once for all its rows, in the order l = 0, 1, ... whatever ROWS is, so a
-// row's decay does not depend on how many rows the step has. A single row is a chain of loads: the first PREP_AHEAD rows of w2t, which
-// do not depend on the kernel before, are on their way before the wait for it, then the row's r, k and v while its low-rank values
-// come in: three rows, C = 2,048, L = 64, 9.0 us before and 3.9 so.
-#define PREP_AHEAD 64
-template <typename T, int ROWS>
+// row's decay does not depend on how many rows the step has. A single row is a chain of loads: with AHEAD the first AHEAD rows of w2t,
+// which do not depend on the kernel before, are on their way before the wait for it, then the row's r, k and v while its low-rank values
+// come in (a launch behind a launch, 3 rows, C = 2,048, L = 64: 4.0 us without and 3.4 so; L = 160: 7.3 and 5.1). That is for one wave of
+// blocks: a later wave has nothing to wait for and fewer blocks a multiprocessor (300 rows: 13.2 us without, 28.5 so).
+template <typename T, int ROWS, int AHEAD>
 __global__ void __launch_bounds__(256) time_mix_prepare_kernel(const T* __restrict__ r, long long r_stride, const T* __restrict__ k,
     long long k_stride, const T* __restrict__ v, long long v_stride, const T* __restrict__ z, long long z_stride,
     const float* __restrict__ w2t, const float* __restrict__ w0, float* __restrict__ xs, int rows, int C, int L) {
   extern __shared__ float th[];                      // [L][ROWS]: tanh of the rows' low-rank values
   const int t0 = blockIdx.x * ROWS;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
-  constexpr int AHEAD = ROWS == 1 ? PREP_AHEAD : 1;
-  float ahead[AHEAD], rkv[3];
-  if (ROWS == 1 && c < C) {
+  static_assert(AHEAD == 0 || ROWS == 1, "a single row's loads");
+  float ahead[AHEAD > 0 ? AHEAD : 1], rkv[3];
+  if (AHEAD > 0 && c < C) {                          // (AHEAD rows at least)
 #pragma unroll
-    for (int l = 0; l < AHEAD; ++l) ahead[l] = l < L ? w2t[(size_t)l * C + c] : 0.f;
+    for (int l = 0; l < AHEAD; ++l) ahead[l] = w2t[(size_t)l * C + c];
   }
-  const float b = c < C ? w0[c] : 0.f;
   pdl_wait();
-  if (ROWS == 1 && c < C) {
+  if (AHEAD > 0 && c < C) {
     rkv[0] = to_f32<T>(r[(size_t)t0 * r_stride + c]);
     rkv[1] = to_f32<T>(k[(size_t)t0 * k_stride + c]);
     rkv[2] = to_f32<T>(v[(size_t)t0 * v_stride + c]);
@@ -203,35 +202,33 @@ __global__ void __launch_bounds__(256) time_mix_prepare_kernel(const T* __restri
   float acc[ROWS];
 #pragma unroll
   for (int rr = 0; rr < ROWS; ++rr) acc[rr] = 0.f;
-  if (ROWS == 1) {
 #pragma unroll
-    for (int l = 0; l < AHEAD; ++l)
-      if (l < L) acc[0] = fmaf(ahead[l], th[l], acc[0]);
-  }
-#pragma unroll(ROWS == 1 ? 16 : 4)
-  for (int l = ROWS == 1 ? AHEAD : 0; l < L; ++l) {
+  for (int l = 0; l < AHEAD; ++l) acc[0] = fmaf(ahead[l], th[l], acc[0]);
+#pragma unroll(ROWS == 1 ? 16 : 4)                   // a single row's walk: many loads in flight
+  for (int l = AHEAD; l < L; ++l) {
     const float w = w2t[(size_t)l * C + c];
 #pragma unroll
     for (int rr = 0; rr < ROWS; ++rr) acc[rr] = fmaf(w, th[l * ROWS + rr], acc[rr]);
   }
+  const float b = w0[c];
 #pragma unroll
   for (int rr = 0; rr < ROWS; ++rr) {
     const int t = t0 + rr;
     if (t >= rows) break;
     float* o = xs + (size_t)t * 4 * C;
-    o[c] = ROWS == 1 ? rkv[0] : to_f32<T>(r[(size_t)t * r_stride + c]);
-    o[C + c] = ROWS == 1 ? rkv[1] : to_f32<T>(k[(size_t)t * k_stride + c]);
-    o[2 * C + c] = ROWS == 1 ? rkv[2] : to_f32<T>(v[(size_t)t * v_stride + c]);
+    o[c] = AHEAD > 0 ? rkv[0] : to_f32<T>(r[(size_t)t * r_stride + c]);
+    o[C + c] = AHEAD > 0 ? rkv[1] : to_f32<T>(k[(size_t)t * k_stride + c]);
+    o[2 * C + c] = AHEAD > 0 ? rkv[2] : to_f32<T>(v[(size_t)t * v_stride + c]);
     o[3 * C + c] = expf(-expf(acc[rr] + b));
   }
 }
 
-template <typename T, int ROWS>
+template <typename T, int ROWS, int AHEAD = 0>
 static void time_mix_prepare_launch(const void* r, long long r_stride, const void* k, long long k_stride, const void* v,
                                     long long v_stride, const void* z, long long z_stride, const float* w2t, const float* w0,
                                     float* xs, int rows, int C, int L, cudaStream_t stream) {
   const dim3 grid((rows + ROWS - 1) / ROWS, (C + 255) / 256), block(256);
-  si_launch(time_mix_prepare_kernel<T, ROWS>, grid, block, (size_t)ROWS * L * sizeof(float), stream, (const T*)r, r_stride,
+  si_launch(time_mix_prepare_kernel<T, ROWS, AHEAD>, grid, block, (size_t)ROWS * L * sizeof(float), stream, (const T*)r, r_stride,
             (const T*)k, k_stride, (const T*)v, v_stride, (const T*)z, z_stride, w2t, w0, xs, rows, C, L);
 }
 
@@ -241,10 +238,12 @@ SI_EXPORT int si_time_mix_prepare(const void* r, long long r_stride, const void*
   if (rows <= 0) return 0;
   if (C <= 0 || L <= 0 || L > 2048 || (C + 255) / 256 > 65535) return -2;
   // few rows: a row a block, so that the blocks are many; many rows: 16 a block, so that w2t is read once for all of them
-  const bool many = (long long)rows * ((C + 255) / 256) >= 16LL * 4 * si_sm_count();
+  const long long blocks = (long long)rows * ((C + 255) / 256);
+  const bool many = blocks >= 16LL * 4 * si_sm_count(), ahead = L >= 64 && blocks <= si_sm_count();
 #define PREP_LAUNCH(T)                                                                                              \
   if (many && L <= 768) time_mix_prepare_launch<T, 16>(r, r_stride, k, k_stride, v, v_stride, z, z_stride, w2t, w0, xs, rows, C, L, stream); \
   else if (many) time_mix_prepare_launch<T, 4>(r, r_stride, k, k_stride, v, v_stride, z, z_stride, w2t, w0, xs, rows, C, L, stream); \
+  else if (ahead) time_mix_prepare_launch<T, 1, 64>(r, r_stride, k, k_stride, v, v_stride, z, z_stride, w2t, w0, xs, rows, C, L, stream); \
   else time_mix_prepare_launch<T, 1>(r, r_stride, k, k_stride, v, v_stride, z, z_stride, w2t, w0, xs, rows, C, L, stream);
   if (dtype == SI_BF16) { PREP_LAUNCH(__nv_bfloat16) } else { PREP_LAUNCH(float) }
 #undef PREP_LAUNCH
