@@ -544,9 +544,12 @@ static int scan_launch(const float* xbc, long long xbc_stride, const void* dt_ra
   // layout does not depend on the cut.
   int Pb = P;
   while (Pb % 2 == 0 && Pb / 2 >= 8 && 2LL * num_seqs * heads * (P / Pb) <= si_sm_count()) Pb /= 2;
-  // portions, and a state of up to 128 rows: two columns a thread
+  // Portions, and a state of up to 128 rows: two columns a thread. Half the threads hide less latency, so the portions have to be long
+  // enough: eight rows a sequence on average (64 heads of 64 columns: three sequences of 4 rows 10.6 us with one column and 11.3 with two,
+  // of 8 rows 13.1 and 12.7), more where the columns are cut over blocks (one sequence, cut in two: 32 rows 10.1 and 10.4, 48 rows 13.9 and
+  // 13.3; 16 heads, cut in eight: 64 rows 13.9 and 14.7, 200 rows 35.6 and 33.7).
   constexpr int WIDE = NPT == 8 || NPT == 16 ? NPT : 8;
-  const bool two = WIDE == NPT && NS == 8 && Pb % 2 == 0 && Pb <= 64 && num_tokens >= 4LL * num_seqs;
+  const bool two = WIDE == NPT && NS == 8 && Pb % 2 == 0 && Pb <= 64 && num_tokens >= (long long)num_seqs * (Pb == P ? 8 : 20 * (P / Pb));
   const int threads = (Pb / (two ? 2 : 1) * NS + 31) / 32 * 32;
   const size_t smem = (size_t)2 * (2 * SCAN_CHUNK * NS * NPT + SCAN_CHUNK * ((Pb + 3) / 4 * 4) + 2 * SCAN_CHUNK) * sizeof(float);
   if (smem > 200 * 1024) return -2;
