@@ -10,6 +10,9 @@
 // sixteenth and less of the work, so that a small product spreads over more SMs) where they do not: a small product is bound by one
 // block's chain of K dependent sums and the first fetch.
 // Measured at six rows, N and K of 96 to 1,000: 3.5 us a launch, where tiles of 64 x 64 alone, one k tile at a time, took 11.3.
+// Rows that are not in 16-byte words go entry by entry, where a small tile's fetches outweigh its sums: large tiles from half the SMs on
+// (700 x 780, K = 333: 44.3 us in small tiles, 26.3 in large ones; 300 x 1,700, K = 700, in words: 42.4 in small ones, where the large ones of
+// before took 53.5).
 #include "common.cuh"
 
 template <int BM, int BN, int TM, int TN, int BK, int STAGES, bool VEC>
@@ -89,11 +92,12 @@ SI_EXPORT int si_gemm_f32(const float* A, long long lda, const float* W, long lo
   if (M <= 0 || N <= 0) return 0;
   const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
   const long long big = (long long)((N + 63) / 64) * ((M + 63) / 64);
-  const dim3 grid = big >= si_sm_count() ? dim3((N + 63) / 64, (M + 63) / 64) : dim3((N + 31) / 32, (M + 15) / 16);
+  const bool large = big >= (vec ? si_sm_count() : si_sm_count() / 2);
+  const dim3 grid = large ? dim3((N + 63) / 64, (M + 63) / 64) : dim3((N + 31) / 32, (M + 15) / 16);
   if (grid.y > 65535) return -2;
-  if (big >= si_sm_count()) {
+  if (large) {
     if (vec) si_launch(gemm_f32_kernel<64, 64, 4, 4, 32, 2, true>, grid, dim3(256), 0, stream, A, lda, W, ldw, C, ldc, M, N, K);
-    else si_launch(gemm_f32_kernel<64, 64, 4, 4, 32, 2, false>, grid, dim3(256), 0, stream, A, lda, W, ldw, C, ldc, M, N, K);
+    else si_launch(gemm_f32_kernel<64, 64, 4, 4, 16, 3, false>, grid, dim3(256), 0, stream, A, lda, W, ldw, C, ldc, M, N, K);
   } else {
     if (vec) si_launch(gemm_f32_kernel<16, 32, 2, 2, 64, 3, true>, grid, dim3(128), 0, stream, A, lda, W, ldw, C, ldc, M, N, K);
     else si_launch(gemm_f32_kernel<16, 32, 2, 2, 64, 3, false>, grid, dim3(128), 0, stream, A, lda, W, ldw, C, ldc, M, N, K);
