@@ -56,8 +56,7 @@ __device__ __forceinline__ void mma16816(float (&d)[4], unsigned a0, unsigned a1
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-struct true_type { static constexpr bool value = true; };
-struct false_type { static constexpr bool value = false; };
+template <int V> struct int_c { static constexpr int value = V; };
 
 template <typename TO> __device__ __forceinline__ void store_out(TO* p, float v);
 template <> __device__ __forceinline__ void store_out<float>(float* p, float v) { *p = v; }
@@ -103,15 +102,16 @@ gemm_skinny_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __rest
   const bf16* xr[MT];
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) xr[mt] = x + (size_t)(mt * 8 + g < M ? mt * 8 + g : 0) * ldx + t * 8;
-  // UNROLL chunks of a warp with all their loads in flight. A round that is not whole (ALL false) loads only what is there: lanes
-  // past the end feed zeros, and every lane of the warp issues the same mma (mma.sync must not sit in a divergent branch).
-  // (A tail of single chunks instead, a round trip to memory each: two rows and K = 704, 1,408 and 2,816 took
-  // 3.5, 4.0 and 5.9 us, so 2.7, 3.3 and 5.3; K = 4,096, whole rounds, 6.0 either way)
+  // Chunks of a warp go in rounds with all their loads in flight: UNROLL whole ones, then four whole ones, then up to four of which a round
+  // that is not whole loads only what is there: lanes past the end feed zeros, and every lane of the warp issues the same mma
+  // (mma.sync must not sit in a divergent branch). A launch behind a launch, against single chunks behind the rounds of UNROLL (which the
+  // compiler takes four at a time), two rows of 2,048 columns: K = 704 2.6 us before, 2.1 so; 1,408 3.2 and 2.6; 2,816 4.9 and 3.4;
+  // 5,632 7.0 and 5.8. 16 rows: 704 3.1 and 3.0, 2,816 6.0 and 5.6. 28,672 columns, K = 4,096: 34.5 and 34.6 us, 16 rows 46.3 and 46.2.
   // The weights do not depend on the kernel before this one: the first round of their loads is in flight
   // before this kernel waits for that kernel's results (x).
-  auto round = [&](int c, bool first, auto all) {
+  auto round = [&](int c, auto chunks, auto all, bool first) {
+    constexpr int U = decltype(chunks)::value;
     constexpr bool ALL = decltype(all)::value;
-    constexpr int U = ALL || MT == 1 ? UNROLL : UNROLL / 2;      // (two row tiles and the tests: half the loads fit the registers)
     uint4 a_lo[U], a_hi[U], xb[U][MT];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -143,18 +143,55 @@ gemm_skinny_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __rest
         }
       }
   };
-  constexpr int STEP = WARPS * (MT == 1 ? UNROLL : UNROLL / 2);
   int c = warp;
-  if (c + (UNROLL - 1) * WARPS < full) {
-    round(c, true, true_type());
-    c += WARPS * UNROLL;
-    for (; c + (UNROLL - 1) * WARPS < full; c += WARPS * UNROLL) round(c, false, true_type());
+  if constexpr (MT == 1) {
+    // one copy of each kind of round, the wait behind a branch; a copy of its own for the only round where blocks are very many
+    bool first = true;
+    if (c + (2 * UNROLL - 1) * WARPS < full || gridDim.x < 4096) {
+#pragma unroll 1
+      for (; c + (UNROLL - 1) * WARPS < full; c += WARPS * UNROLL) {
+        round(c, int_c<UNROLL>(), int_c<true>(), first);
+        first = false;
+      }
+    } else if (c + (UNROLL - 1) * WARPS < full) {
+      round(c, int_c<UNROLL>(), int_c<true>(), true);
+      first = false;
+      c += WARPS * UNROLL;
+    }
+    if (trigger == 2) pdl_trigger();
+    if (c + 3 * WARPS < full) {
+      round(c, int_c<4>(), int_c<true>(), first);
+      first = false;
+      c += WARPS * 4;
+    }
+    if (c < nchunks) {                                       // at most three whole ones and the part of one
+      round(c, int_c<4>(), int_c<false>(), first);
+      first = false;
+    }
+    if (first) pdl_wait();                                   // a warp without any chunk waits like the others
   } else {
-    round(c, true, false_type());        // (also where a warp has no chunk at all: it waits like the others)
-    c += STEP;
+    // the loads of two row tiles fill the registers: rounds that cannot be the first ones without the branch
+    if (c + (UNROLL - 1) * WARPS < full) {
+      round(c, int_c<UNROLL>(), int_c<true>(), true);
+      c += WARPS * UNROLL;
+#pragma unroll 1
+      for (; c + (UNROLL - 1) * WARPS < full; c += WARPS * UNROLL) round(c, int_c<UNROLL>(), int_c<true>(), false);
+      if (trigger == 2) pdl_trigger();
+      if (c + 3 * WARPS < full) {
+        round(c, int_c<4>(), int_c<true>(), false);
+        c += WARPS * 4;
+      }
+      if (c < nchunks) round(c, int_c<4>(), int_c<false>(), false);      // at most three whole ones and the part of one
+    } else if (c + 3 * WARPS < full) {
+      round(c, int_c<4>(), int_c<true>(), true);
+      c += WARPS * 4;
+      if (trigger == 2) pdl_trigger();
+      if (c < nchunks) round(c, int_c<4>(), int_c<false>(), false);
+    } else {
+      round(c, int_c<4>(), int_c<false>(), true);      // (also where a warp has no chunk at all: it waits like the others)
+      if (trigger == 2) pdl_trigger();
+    }
   }
-  if (trigger == 2) pdl_trigger();
-  for (; c < nchunks; c += STEP) round(c, false, false_type());
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
