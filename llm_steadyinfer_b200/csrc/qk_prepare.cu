@@ -64,8 +64,8 @@ __device__ __forceinline__ void norm_rotate_vector(const T* __restrict__ src, T*
   }
 }
 
-template <typename T, int ITEMS>
-__global__ void __launch_bounds__(1024) qk_prepare_kernel(T* __restrict__ rows, long long row_stride, const float* __restrict__ q_w,
+template <typename T, int ITEMS, int THREADS>
+__global__ void __launch_bounds__(THREADS) qk_prepare_kernel(T* __restrict__ rows, long long row_stride, const float* __restrict__ q_w,
     const float* __restrict__ k_w, float eps, const float* __restrict__ inv_freq, int rd, int interleaved,
     const int* __restrict__ positions, const int* __restrict__ row_seq, const int* __restrict__ block_table, int table_width,
     T* __restrict__ k_cache, T* __restrict__ v_cache, int num_pages, int page_size, int num_seqs, int NQ, int NK, int NV,
@@ -104,12 +104,20 @@ __global__ void __launch_bounds__(1024) qk_prepare_kernel(T* __restrict__ rows, 
   if (whole) {                                       // one norm over all of the row's q vectors, one over all its k vectors
     float sq = 0.f, sk = 0.f;
     // (256 threads whatever the block, so that a row's sums have one order)
-    const int n = min((int)blockDim.x, 256);
-    if (threadIdx.x < n) {
-#pragma unroll 8
-      for (int i = threadIdx.x; i < NQ * dk; i += n) { const float x = to_f32<T>(row[i]); sq = fmaf(x, x, sq); }
-#pragma unroll 4
-      for (int i = threadIdx.x; i < NK * dk; i += n) { const float x = to_f32<T>(row[(size_t)NQ * dk + i]); sk = fmaf(x, x, sk); }
+    const int n = THREADS > 256 ? 256 : blockDim.x;
+    auto add = [&](const T* src, int entries) {
+      float s = 0.f;
+      int i = threadIdx.x;
+      for (; i + 3 * n < entries; i += 4 * n) {      // four loads in flight, added in the same order
+        const float a = to_f32<T>(src[i]), b = to_f32<T>(src[i + n]), c = to_f32<T>(src[i + 2 * n]), d = to_f32<T>(src[i + 3 * n]);
+        s = fmaf(a, a, s); s = fmaf(b, b, s); s = fmaf(c, c, s); s = fmaf(d, d, s);
+      }
+      for (; i < entries; i += n) { const float x = to_f32<T>(src[i]); s = fmaf(x, x, s); }
+      return s;
+    };
+    if (THREADS <= 256 || threadIdx.x < 256) {
+      sq = add(row, NQ * dk);
+      sk = add(row + (size_t)NQ * dk, NK * dk);
     }
     inv_q = q_w ? rsqrtf(block_sum(sq, red) / (float)(NQ * dk) + eps) : 1.f;
     inv_k = k_w ? rsqrtf(block_sum(sk, red) / (float)(NK * dk) + eps) : 1.f;
@@ -152,11 +160,12 @@ SI_EXPORT int si_qk_prepare(void* rows, int dtype, long long row_stride, const f
   // for every vector, up to 32, while the rows are no more than the SMs: a vector is a chain of a load, a sum over the warp and a
   // store, and a decode row waits for as many of them as its warps take in turn (four rows, 20
   // vectors of 128: eight warps 13.6 us, a warp each 9.7)
+  // (that instance has 64 registers a thread; many rows keep one with more: 600 rows of 20 vectors 12.6 us in the one, 12.2 in the other)
   int threads = NQ + NK >= 8 ? 256 : 128;
   if (num_tokens <= si_sm_count() && NQ + NK > 8) threads = NQ + NK >= 32 ? 1024 : (NQ + NK + 7) / 8 * 256;
   const dim3 grid(num_tokens), block(threads);
 #define QK_LAUNCH(T, ITEMS)                                                                                              \
-  si_launch(qk_prepare_kernel<T, ITEMS>, grid, block, smem, stream, (T*)rows, row_stride, q_w, k_w, eps, inv_freq, rd,      \
+  si_launch(threads <= 256 ? qk_prepare_kernel<T, ITEMS, 256> : qk_prepare_kernel<T, ITEMS, 1024>, grid, block, smem, stream, (T*)rows, row_stride, q_w, k_w, eps, inv_freq, rd,      \
             interleaved, positions, row_seq, block_table, table_width, (T*)k_cache, (T*)v_cache, num_pages, page_size,   \
             num_seqs, NQ, NK, NV, dk, dv, (T*)q_out, q_out_stride, maps, whole, rot_scale, status)
   if (dtype == SI_BF16) {
