@@ -10,7 +10,8 @@
 // the rest of the batch: the warps take runs of KEYS keys in turn with a running max, and
 // their partial results are merged at the end. Bound by latency: a warp's table entries, then all key and value loads of
 // a run are in flight at once, so that a run costs two round trips instead of two a key.
-// Measured at one row each of six sequences of up to 216 keys, 3 heads of 32: 7.8 us, where a key at a time took 36.
+// Measured at one row each of six sequences of up to 216 keys, 3 heads of 32: 7.8 us, where a key at a time took 36. Heads above 128 have
+// runs of two keys, which leave room for more warps (1,000 rows of two heads of 256: four keys 554 us, two 357, a key at a time 448).
 #include "common.cuh"
 #include <math.h>
 
@@ -143,7 +144,7 @@ SI_EXPORT int si_paged_attention_ref(const void* q, int dtype, long long q_row_s
   if (hs <= 32) REF_LAUNCH(T, 1, 8);            \
   else if (hs <= 64) REF_LAUNCH(T, 2, 8);       \
   else if (hs <= 128) REF_LAUNCH(T, 4, 8);      \
-  else REF_LAUNCH(T, REF_MAX_PER_LANE, 4)
+  else REF_LAUNCH(T, REF_MAX_PER_LANE, 2)
   if (dtype == SI_BF16) { REF_BY_SIZE(__nv_bfloat16); }
   else { REF_BY_SIZE(float); }
 #undef REF_BY_SIZE
