@@ -34,7 +34,7 @@ import torch
 from ..csrc import ops
 from .base import Mixer, StateNeed, register_mixer
 from .linear import linear
-from .step_rows import portions, row_kinds
+from .step_rows import longest, portions, row_kinds
 
 
 class GatedDeltaRule(Mixer):
@@ -98,6 +98,14 @@ class GatedDeltaRule(Mixer):
     def kernel_files(self, page_size):
         return ("ssm", "delta_rule") + (("gemm_f32",) if self.dtype == torch.float32 else ("gemm_skinny", "gemm_rows", "gemm_tc05"))
 
+    def by_groups(self, ctx, T: int) -> bool:
+        """The recurrence four tokens at a time, which takes a launch more and twice the loads a token. It pays for long portions, and for
+        shorter ones once they are many (16 heads of 128, us by the token and by groups: one portion of 32 rows 12.4 and 14.3, of 64 21.5
+        and 18.7; three of 48 25.9 and 27.3; eight of 16 25.1 and 24.5, of 8 16.2 and 18.0; 32 of 4 40.4 and 39.0, of 2 33.7 and 36.5)."""
+        if not (row_kinds(ctx) & 2 and USE_GROUPS and ops.channel_delta_groups_ok(self.dk, self.dv)):
+            return False
+        return longest(ctx) >= 64 or (ctx.num_seqs >= 4 and T >= max(160, 4 * ctx.num_seqs))
+
     def forward(self, x, ctx, cache):
         T = x.shape[0]
         H, G, dk, dv, C = self.H, self.G, self.dk, self.dv, self.channels
@@ -110,7 +118,7 @@ class GatedDeltaRule(Mixer):
         bg = ctx.buf("delta_bg", (T, 2 * H + G), torch.float32)
         ops.delta_prepare(xc, u, self.b_off, self.a_off, self.a_log, self.dt_bias, bg, G, H, dk, dk ** -0.5)
         y = ctx.buf("delta_y", (T, self.nv), torch.float32)
-        if row_kinds(ctx) & 2 and USE_GROUPS and ops.channel_delta_groups_ok(dk, dv):
+        if self.by_groups(ctx, T):
             # portions: the recurrence with a decay per channel, all channels of a head alike, four tokens at a time
             dec = ctx.buf("delta_decay", (T, H * dk), torch.float32)
             rec = ctx.buf("delta_groups", (T, H, 3, dk), torch.float32)

@@ -27,3 +27,13 @@ def row_kinds(ctx) -> int:
         n = np.diff(ctx.h_q_start)
         got = ctx.plans["row_kinds"] = (1 if (n == 1).any() else 0) | (2 if (n > 1).any() else 0)
     return got
+
+
+def longest(ctx) -> int:
+    """Most rows of any of the step's sequences."""
+    if ctx.seq_cap is not None:
+        return 1
+    got = ctx.plans.get("longest")
+    if got is None:
+        got = ctx.plans["longest"] = int(np.diff(ctx.h_q_start).max())
+    return got

@@ -20,7 +20,7 @@ import torch
 from ..csrc import ops
 from .base import Mixer, StateNeed, register_mixer
 from .linear import linear, linear_batched
-from .step_rows import row_kinds
+from .step_rows import longest, row_kinds
 
 MIXES = ("r", "k", "v", "g", "w")
 
@@ -82,6 +82,14 @@ class TimeMix(Mixer):
     def kernel_files(self, page_size):
         return ("time_mix", "delta_rule") + (("gemm_f32",) if self.dtype == torch.float32 else ("gemm_skinny", "gemm_rows", "gemm_tc05"))
 
+    def by_groups(self, ctx, T: int) -> bool:
+        """The recurrence four tokens at a time, a launch more: for long portions, and for shorter ones where sequences and heads fill half
+        the device (32 heads of 64, us by the token and by groups: one portion of 24 rows 6.4 and 6.7, of 32 7.8 and 7.3; two of 16 5.9 and
+        6.8; three of 8 7.0 and 6.2; sixteen of 2 14.6 and 12.5)."""
+        if not (row_kinds(ctx) & 2 and ops.decay_groups_ok(self.n)):
+            return False
+        return longest(ctx) >= 28 or (T >= max(28, 2 * ctx.num_seqs) and 2 * ctx.num_seqs * self.H > ops.sm_count(self.device))
+
     def forward_heads(self, x, ctx, cache, out, scale: float = 1.0):
         """The normalised, gated read-out, times ``scale``, into ``out`` [T, C] (a view with a row stride): everything but W_o."""
         T = x.shape[0]
@@ -97,7 +105,7 @@ class TimeMix(Mixer):
         xs = ctx.buf("tmix_xs", (T, 4 * C), torch.float32)
         ops.time_mix_prepare(proj[0], proj[1], proj[2], z[:, :self.L], self.w2t, self.w0, xs)
         y = ctx.buf("tmix_y", (T, C), torch.float32)
-        if row_kinds(ctx) & 2 and ops.decay_groups_ok(n):       # portions: four tokens at a time
+        if self.by_groups(ctx, T):                              # portions: four tokens at a time
             sc = ctx.buf("tmix_factors", (T, H, 4), torch.float32)
             ops.decay_group_scan(xs, self.u, sc, state, y, ctx.row_seq, ctx.q_start, ctx.ctx_len, ctx.slots, ctx.seq_slots, H, n)
         else:
