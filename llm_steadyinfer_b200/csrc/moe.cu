@@ -13,7 +13,7 @@
 //   moe_gemm     C[place] = act(A[row of place] W_e^T) for every place of expert e: a grouped product whose row tiles are
 //                found from the offsets by every block itself (blocks beyond the last tile leave). bf16 on mma.sync
 //                m16n8k16 with fp32 sums: few places an expert stream its weights (moe_stream_kernel), more go by tiles of 64
-//                rows x 64 columns, three cp.async stages; fp32 on FFMA.
+//                rows x 64 columns, three cp.async stages (16 rows, four stages, where few are not in 16-byte pieces); fp32 on FFMA.
 //                act "glu_limited": W_e holds gate and up rows in turn (row 2i the gate of entry i, row 2i + 1 its up), and
 //                C[place, i] = g sigmoid(alpha g) (u + shift) with g = min(gate sum, limit), u = clamp(up sum, -limit, limit)
 //                (no limit, alpha 1 and shift 0: silu(gate) * up).
@@ -390,8 +390,8 @@ __global__ void __launch_bounds__(128) moe_gemm_bf16_kernel(const bf16* __restri
   __syncthreads();
   const bf16* We = W + (size_t)e * N * K;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
-  constexpr int NT = BN / 8;                         // n-tiles of 8 columns a warp; warps over the rows
-  const int wr0 = warp * 16, wn0 = 0;
+  constexpr int NT = BM == 64 ? BN / 8 : BN / 32;    // n-tiles of 8 columns a warp: warps over the rows, or over the columns
+  const int wr0 = BM == 64 ? warp * 16 : 0, wn0 = BM == 64 ? 0 : warp * (BN / 4);
   float acc[NT][4];
 #pragma unroll
   for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
@@ -727,6 +727,11 @@ SI_EXPORT int si_moe_gemm(const void* A, int dtype, long long a_stride, const in
     if (tiles > 65535) return -2;
     si_launch(moe_stream_kernel, dim3((N + 15) / 16, (unsigned)tiles), dim3(STREAM_WARPS * 32), 0, stream, (const bf16*)A, a_stride, a_rows,
               nullptr, 1, (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, offsets, P, E, N, K, act, limit, alpha, shift);
+  } else if (P < 32LL * E && !wide) {
+    // few rows an expert, and sizes or rows that are not in 16-byte pieces: tiles of 16 places (one row of two experts of 1,408 x 1,034:
+    // 134 us, 176 in tiles of 64)
+    si_launch(moe_gemm_bf16_kernel<16, 64, 64, 4>, dim3((P + 15) / 16 + E, ny), dim3(128), 0, stream, (const bf16*)A, a_stride, a_rows,
+              (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, offsets, E, N, K, act, wide, limit, alpha, shift);
   } else {
     const dim3 grid((P + 63) / 64 + E, ny), block(128);
     si_launch(moe_gemm_bf16_kernel<64, 64, 32, 3>, grid, block, 0, stream, (const bf16*)A, a_stride, a_rows, (const bf16*)W, C, c_stride,
