@@ -29,96 +29,83 @@ typedef __nv_bfloat16 bf16;
 
 // ---- router -------------------------------------------------------------------------------------------------------------
 // x [T, d]; w [E + extra, d] (router rows, then `extra` gate rows) in the compute dtype; ids int32 [T, top]; wts fp32
-// [T, top]; gates fp32 [T, extra]. mode 0: sigmoid scores; 1: softmax over the experts. A block takes RB rows, a warp a weight
-// row at a time for all of them. Few rows: one a block, as many warps as weight rows, and a warp's first 256 x ROUTE_AHEAD
-// weights, which do not depend on the kernel before, are in flight before the block waits for x. Many rows: four a block, so that
-// the weight rows are read from L2 a quarter as often. A row's sums run over k in the same order either way. Both are bound by
-// latency (a round trip for the weights, one for the row, the choice by one warp): measured
-// for four rows of 32 to 64 experts, d = 1,536 to 2,048: 5.8 to 6.7 us, where eight warps that read the weights after the wait took 15 to 18.
+// [T, top]; gates fp32 [T, extra]. mode 0: sigmoid scores; 1: softmax over the experts. A block takes a row, a warp a weight row at a time.
+// EARLY (no more rows than SMs): as many warps as weight rows, up to 32, and a warp's first 256 x ROUTE_AHEAD weights, which do not depend
+// on the kernel before, are in flight before the block waits for x. A row's sums run over k in the same order either way. Bound by latency
+// (a round trip for the weights, one for the row, the choice by one warp): four rows, a launch behind a launch, d = 2,048 and 64 experts
+// 20.7 us with eight warps that read the weights behind the wait and 12.0 so, d = 1,536 and 32 experts 10.1 and 5.8. With more rows than
+// SMs the eight warps serve (591 rows, d = 2,048, 64 experts: 31.0 us; four rows a block took 32.4, and 97 against 89 at 2,048 rows).
 #define ROUTE_AHEAD 4
-template <typename T, int RB>
-__global__ void __launch_bounds__(RB == 1 ? 1024 : 256) moe_route_kernel(const T* __restrict__ x, long long x_stride, const T* __restrict__ w,
-    int E, int extra, int d, int top, float scale, int mode, int renorm, float renorm_eps, int groups, int keep, int rows,
+template <typename T, bool EARLY>
+__global__ void __launch_bounds__(EARLY ? 1024 : 256) moe_route_kernel(const T* __restrict__ x, long long x_stride, const T* __restrict__ w,
+    int E, int extra, int d, int top, float scale, int mode, int renorm, float renorm_eps, int groups, int keep,
     const float* __restrict__ choice_bias, int* __restrict__ ids, float* __restrict__ wts, float* __restrict__ gates) {
-  extern __shared__ float rsm[];                       // rows [RB, d]; a row's scores [E + extra], used [E], choice keys [E] (and groups' scores)
+  extern __shared__ float rsm[];                       // the row [d], scores [E + extra], used [E], choice keys [E] (and groups' scores)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const long long t0 = (long long)blockIdx.x * RB;
-  const int per = 3 * E + extra + (groups > 1 ? groups : 0);
-  float* const scores = rsm + (size_t)RB * d;
+  const long long t = blockIdx.x;
+  float* xr = rsm;
+  float* sc = rsm + d;
+  float* used = sc + E + extra;
+  float* key = used + E;
   const bool wide = sizeof(T) == 2 && d % 8 == 0 && ((uintptr_t)w & 15) == 0;      // rows of 16-byte pieces: eight entries a load
   uint4 ahead[ROUTE_AHEAD];
-  if (RB == 1 && wide && warp < E + extra) {
+  if (EARLY && wide && warp < E + extra) {
 #pragma unroll
     for (int u = 0; u < ROUTE_AHEAD; ++u)
       if (lane * 8 + u * 256 < d) ahead[u] = *reinterpret_cast<const uint4*>(w + (size_t)warp * d + lane * 8 + u * 256);
   }
   pdl_wait();
-  if (wide && x_stride % 8 == 0 && ((uintptr_t)x & 15) == 0) {
-    for (int i = threadIdx.x; i < RB * (d / 8); i += blockDim.x) {
-      const int r = i / (d / 8), at = (i - r * (d / 8)) * 8;
-      uint4 raw = make_uint4(0, 0, 0, 0);
-      if (t0 + r < rows) raw = *reinterpret_cast<const uint4*>(x + (t0 + r) * x_stride + at);
+  if (EARLY && wide && x_stride % 8 == 0 && ((uintptr_t)x & 15) == 0) {
+    for (int at = threadIdx.x * 8; at < d; at += blockDim.x * 8) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(x + t * x_stride + at);
       const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) reinterpret_cast<float2*>(rsm + (size_t)r * d + at)[j] = __bfloat1622float2(h2[j]);
+      for (int j = 0; j < 4; ++j) reinterpret_cast<float2*>(xr + at)[j] = __bfloat1622float2(h2[j]);
     }
   } else {
-    for (int i = threadIdx.x; i < RB * d; i += blockDim.x) {
-      const int r = i / d;
-      rsm[i] = t0 + r < rows ? to_f32<T>(x[(t0 + r) * x_stride + (i - r * d)]) : 0.f;
-    }
+    for (int i = threadIdx.x; i < d; i += blockDim.x) xr[i] = to_f32<T>(x[t * x_stride + i]);
   }
-  for (int i = threadIdx.x; i < RB * E; i += blockDim.x) scores[(i / E) * per + E + extra + i % E] = 0.f;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) used[e] = 0.f;
   __syncthreads();
   for (int e = warp; e < E + extra; e += nwarps) {
     const T* we = w + (size_t)e * d;
-    float acc[RB];
-#pragma unroll
-    for (int r = 0; r < RB; ++r) acc[r] = 0.f;
-    auto piece = [&](const uint4& raw, int i) {
-      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-      for (int j = 0; j < 4; j += 2) {
-        const float2 f = __bfloat1622float2(h2[j]), h = __bfloat1622float2(h2[j + 1]);
-#pragma unroll
-        for (int r = 0; r < RB; ++r) {
-          const float4 xv = *reinterpret_cast<const float4*>(rsm + (size_t)r * d + i + 2 * j);
-          acc[r] = fmaf(f.x, xv.x, acc[r]);
-          acc[r] = fmaf(f.y, xv.y, acc[r]);
-          acc[r] = fmaf(h.x, xv.z, acc[r]);
-          acc[r] = fmaf(h.y, xv.w, acc[r]);
-        }
-      }
-    };
+    float acc = 0.f;
     if (wide) {
-      int from = 0;
-      if (RB == 1 && e == warp) {
+      int from = lane * 8;
+      if (EARLY && e == warp) {
 #pragma unroll
         for (int u = 0; u < ROUTE_AHEAD; ++u)
-          if (lane * 8 + u * 256 < d) piece(ahead[u], lane * 8 + u * 256);
-        from = ROUTE_AHEAD * 256;
+          if (lane * 8 + u * 256 < d) {
+            const int i = lane * 8 + u * 256;
+            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&ahead[u]);
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {
+              const float2 f = __bfloat1622float2(h2[j]), h = __bfloat1622float2(h2[j + 1]);
+              const float4 xv = *reinterpret_cast<const float4*>(xr + i + 2 * j);
+              acc = fmaf(f.x, xv.x, acc); acc = fmaf(f.y, xv.y, acc);
+              acc = fmaf(h.x, xv.z, acc); acc = fmaf(h.y, xv.w, acc);
+            }
+          }
+        from += ROUTE_AHEAD * 256;
       }
-#pragma unroll 4
-      for (int i = from + lane * 8; i < d; i += 256) piece(*reinterpret_cast<const uint4*>(we + i), i);
+      for (int i = from; i < d; i += 256) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(we + i);
+        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __bfloat1622float2(h2[j]);
+          acc = fmaf(f.x, xr[i + 2 * j], acc);
+          acc = fmaf(f.y, xr[i + 2 * j + 1], acc);
+        }
+      }
     } else {
-      for (int i = lane; i < d; i += 32) {
-        const float f = to_f32<T>(we[i]);
-#pragma unroll
-        for (int r = 0; r < RB; ++r) acc[r] = fmaf(f, rsm[(size_t)r * d + i], acc[r]);
-      }
+      for (int i = lane; i < d; i += 32) acc = fmaf(to_f32<T>(we[i]), xr[i], acc);
     }
-#pragma unroll
-    for (int r = 0; r < RB; ++r) {
-      const float s = warp_sum(acc[r]);
-      if (lane == 0) scores[r * per + e] = s;
-    }
+    acc = warp_sum(acc);
+    if (lane == 0) sc[e] = acc;
   }
   __syncthreads();
-  if (warp >= RB || t0 + warp >= rows) return;           // a warp chooses for a row
-  const long long t = t0 + warp;
-  float* sc = scores + warp * per;
-  float* used = sc + E + extra;
-  float* key = used + E;
+  if (warp != 0) return;                               // one warp chooses
   for (int e = lane; e < extra; e += 32) gates[t * extra + e] = 1.f / (1.f + expf(-sc[E + e]));
   float zmax = -INFINITY, zsum = 0.f;
   if (mode == 1) {
@@ -200,22 +187,21 @@ SI_EXPORT int si_moe_route(const void* x, int dtype, long long x_stride, const v
   if (E <= 0 || top <= 0 || top > E || top > 32 || extra < 0 || d <= 0 || mode < 0 || mode > 1) return -2;
   if (groups > 1 && (E % groups || keep < 1 || keep > groups || !choice_bias)) return -2;      // groups go by choice scores
   if (groups > 1 && (long long)keep * (E / groups) < top) return -2;
-  // Four rows a block from the rows on that give every SM a block of four, where they fit (a fp32 copy of a row each).
-  const size_t per_row = (size_t)(d + 3 * E + extra + (groups > 1 ? groups : 0)) * sizeof(float);
-  const int rb = rows >= 4 * si_sm_count() && 4 * per_row <= 48 * 1024 ? 4 : 1;
-  const size_t smem = rb * per_row;
+  const size_t smem = (size_t)(d + 3 * E + extra + (groups > 1 ? groups : 0)) * sizeof(float);
   if (smem > 160 * 1024) return -2;
+  const bool early = rows <= si_sm_count();
   const int warps = E + extra < 32 ? E + extra : 32;
-  const dim3 grid((rows + rb - 1) / rb), block(rb == 4 ? 256 : 32 * (rows <= si_sm_count() ? warps : (warps < 8 ? warps : 8)));
+  const dim3 grid(rows), block(early ? 32 * warps : E + extra >= 8 ? 256 : 128);
 #define ROUTE_LAUNCH(T)                                                                                                \
   {                                                                                                                  \
     static size_t configured = 0;                                                                                    \
     if (smem > 48 * 1024 && smem > configured) {                                                                     \
-      if (cudaFuncSetAttribute(moe_route_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -2; \
+      if (cudaFuncSetAttribute(moe_route_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess       \
+          || cudaFuncSetAttribute(moe_route_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -2; \
       configured = smem;                                                                                             \
     }                                                                                                                \
-    si_launch(rb == 4 ? moe_route_kernel<T, 4> : moe_route_kernel<T, 1>, grid, block, smem, stream, (const T*)x, x_stride, (const T*)w, E, extra, d, top, scale, \
-              mode, renorm, renorm_eps, groups, keep, rows, choice_bias, ids, wts, gates);                                             \
+    si_launch(early ? moe_route_kernel<T, true> : moe_route_kernel<T, false>, grid, block, smem, stream, (const T*)x, x_stride, (const T*)w, E, extra, d, top, scale, \
+              mode, renorm, renorm_eps, groups, keep, choice_bias, ids, wts, gates);                                                           \
   }
   if (dtype == SI_BF16) ROUTE_LAUNCH(bf16) else ROUTE_LAUNCH(float)
 #undef ROUTE_LAUNCH
