@@ -42,6 +42,9 @@
 // is bounded; when one runs out the block sets SI_WAIT_LIMIT and leaves without storing.
 #include "attention_common.cuh"
 #include "tma_common.cuh"
+#include <algorithm>
+#include <functional>
+#include <vector>
 #include <limits.h>
 
 // Packed fp32 arithmetic of sm_100 in the softmax (two scores an instruction) and three-input maxima.
@@ -672,6 +675,87 @@ static int launch(const AttnParams& p, const CUtensorMap& km, const CUtensorMap&
   if (e != cudaSuccess) return (int)e;
   si_launch(k, dim3(p.KV, num_items, (p.vs + NV * 64 - 1) / (NV * 64)), dim3(320), smem, stream, p, km, vm, log2_page, x);
   return si_last_error();
+}
+
+// The cut of a step's items into shares (host arithmetic only; called before every long prompt step, so in native code: some 3,000 steps of
+// a heap). `tiles[i]`: key tiles of item i, which runs for `copies` key/value heads; `blocks` run at once. Longest shares are tried from the
+// longest item down and the shortest schedule is taken (longest share first to the block that is free first; a share costs its tiles and
+// about two for its start, a cut item's share three more for handing over). No share is below `least` tiles; at most `most` shares are
+// partial results. entries [cap][4] receives (item, share, shares, first slot), longest first, cut [n][4] (item, shares, first slot, 0),
+// counts (entries, cut items, slots). Returns 1, 0 where whole items are within a twentieth of the best, or -2.
+SI_EXPORT int si_cut_portions(const int* tiles, int n, int copies, int blocks, int least, long long most, int* entries, int cap, int* cut, int* counts) {
+  if (n <= 0 || copies <= 0 || blocks <= 0 || least <= 0) return -2;
+  long long longest = 0, total = 0;
+  for (int i = 0; i < n; ++i) {
+    longest = std::max<long long>(longest, tiles[i]);
+    total += (long long)tiles[i] * copies;
+  }
+  if (longest < 2LL * least || (long long)n * copies > 8LL * blocks) return 0;
+  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  std::vector<long long> cost, heap;
+  auto schedule = [&](long long limit) {
+    cost.clear();
+    for (int i = 0; i < n; ++i) {
+      if (tiles[i] <= 0) continue;
+      const long long shares = up(tiles[i], limit), each = up(tiles[i], shares) + 2 + (shares > 1 ? 3 : 0);
+      cost.insert(cost.end(), (size_t)shares, each);
+    }
+    std::sort(cost.begin(), cost.end(), std::greater<long long>());
+    heap.assign((size_t)blocks, 0);                        // every block's end, the earliest on top
+    long long end = 0;
+    for (const long long c : cost)
+      for (int k = 0; k < copies; ++k) {
+        const long long v = heap[0] + c;
+        end = std::max(end, v);
+        size_t at = 0;
+        for (;;) {
+          size_t kid = 2 * at + 1;
+          if (kid >= heap.size()) break;
+          if (kid + 1 < heap.size() && heap[kid + 1] < heap[kid]) ++kid;
+          if (heap[kid] >= v) break;
+          heap[at] = heap[kid];
+          at = kid;
+        }
+        heap[at] = v;
+      }
+    return end;
+  };
+  const long long whole = schedule(longest);
+  if ((double)whole * 0.95 <= (double)total / blocks) return 0;
+  std::vector<long long> limits;
+  for (const int k : {2, 3, 4, 6, 9, 13, 18}) {
+    const long long limit = std::max<long long>(least, up(longest, k));
+    long long shares = 0;
+    for (int i = 0; i < n; ++i) shares += tiles[i] > limit ? up(tiles[i], limit) : 0;
+    if ((k <= 6 || (long long)n * copies * k <= 4LL * blocks) && limit < longest && shares * copies <= most) limits.push_back(limit);
+  }
+  std::sort(limits.begin(), limits.end());
+  limits.erase(std::unique(limits.begin(), limits.end()), limits.end());
+  long long best = -1, limit = 0;
+  for (const long long l : limits) {
+    const long long end = schedule(l);
+    if (best < 0 || end < best) { best = end; limit = l; }
+  }
+  if (best < 0 || (double)best > 0.95 * (double)whole) return 0;
+  int num = 0, num_cut = 0, slots = 0;
+  struct Share { long long length; int v[4]; };
+  std::vector<Share> all;
+  for (int i = 0; i < n; ++i) {
+    if (tiles[i] <= 0) continue;
+    const int shares = (int)up(tiles[i], limit);
+    if (shares > 32 || num + shares > cap) return -2;      // (a merging warp's lanes; never with 18 shares at most)
+    for (int k = 0; k < shares; ++k) all.push_back(Share{up(tiles[i], shares), {i, k, shares, shares > 1 ? slots : 0}});
+    num += shares;
+    if (shares > 1) {
+      const int e[4] = {i, shares, slots, 0};
+      std::copy(e, e + 4, cut + 4 * (num_cut++));
+      slots += shares;
+    }
+  }
+  std::stable_sort(all.begin(), all.end(), [](const Share& x, const Share& y) { return x.length > y.length; });
+  for (int i = 0; i < num; ++i) std::copy(all[i].v, all[i].v + 4, entries + 4 * i);
+  counts[0] = num; counts[1] = num_cut; counts[2] = slots;
+  return 1;
 }
 
 // Floats of partial results of `slots` shares.

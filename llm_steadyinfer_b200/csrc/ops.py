@@ -1031,44 +1031,32 @@ def attn_portion_share_floats(slots: int, KV: int, hs: int, vs: int) -> int:
     return lib.si_attn_portion_share_floats(_c_int(slots), _c_int(KV), _c_int(hs), _c_int(vs))
 
 
-def cut_portions(tiles, copies: int, blocks: int, least: int = 16):
+SHARE_ROUNDS = 3        # blocks' worth of partial results at most: what the cut gives beyond (contexts above 60,000 tokens) is less than the scratch
+
+
+def cut_slots(copies: int, blocks: int) -> int:
+    """Most slots of partial results that ``cut_portions`` gives."""
+    return SHARE_ROUNDS * blocks // copies
+
+
+CUT_LEAST = 16          # key tiles of a share; items of fewer than two shares' worth are never cut
+
+
+def cut_portions(tiles, copies: int, blocks: int, least: int = CUT_LEAST):
     """Cut work items (``tiles[i]`` key tiles each, every item run for ``copies`` key/value heads) so that ``blocks`` blocks that run at
-    once end together: a long prompt's portion is a few items more than the blocks, and the last ones would run alone. Tries longest
-    shares from the longest item down and takes the shortest schedule (longest share first to the block that is free first; a share
-    costs its tiles and about two for its start, a cut item's share three more for handing over). No share is below ``least`` tiles.
-    Returns (entries int32 [n, 4] of (item, share, shares, first slot), longest first, cut int32 [m, 4] of (item, shares, first slot, 0),
-    slots), or None where whole items are within a twentieth of the best."""
-    import heapq
+    once end together: a long prompt's portion is a few items more than the blocks, and the last ones would run alone. No share is below
+    ``least`` tiles. Returns (entries int32 [n, 4] of (item, share, shares, first slot), longest first, cut int32 [m, 4] of (item, shares,
+    first slot, 0), slots), or None where whole items are within a twentieth of the best."""
+    if max(tiles) < 2 * least or len(tiles) * copies > 8 * blocks:
+        return None
     import numpy as np
-
-    def schedule(limit):
-        cost = sorted((sh + 2 + (3 if n > 1 else 0) for t in tiles for n in (-(-t // limit),) for sh in [-(-t // n)] * n), reverse=True)
-        heap = [0] * blocks
-        for c in cost:
-            for _ in range(copies):
-                heapq.heapreplace(heap, heap[0] + c)
-        return max(heap)
-
-    longest = max(tiles)
-    total = sum(tiles) * copies
-    if longest < 2 * least or len(tiles) * copies > 8 * blocks:
-        return None
-    whole = schedule(longest)
-    if whole * 0.95 <= total / blocks:
-        return None
-    limits = sorted({max(least, -(-longest // n)) for n in (2, 3, 4, 6, 9, 13, 18) if n <= 6 or len(tiles) * copies * n <= 4 * blocks})
-    best, limit = min((schedule(l), l) for l in limits if l < longest)
-    if best > 0.95 * whole:
-        return None
-    entries, cut, slots = [], [], 0
-    for i, t in enumerate(tiles):
-        n = min(32, -(-t // limit))
-        entries += [(-(-t // n), i, s, n, slots if n > 1 else 0) for s in range(n)]
-        if n > 1:
-            cut.append((i, n, slots, 0))
-            slots += n
-    entries.sort(key=lambda e: -e[0])
-    return np.asarray([e[1:] for e in entries], dtype=np.int32), np.asarray(cut, dtype=np.int32).reshape(-1, 4), slots
+    n, cap = len(tiles), len(tiles) + cut_slots(copies, blocks)
+    t = np.asarray(tiles, dtype=np.int32)
+    entries, cut, counts = np.empty((cap, 4), dtype=np.int32), np.empty((n, 4), dtype=np.int32), np.zeros(3, dtype=np.int32)
+    f = _fn("attention_tc05", "si_cut_portions", [_c_p, _c_int, _c_int, _c_int, _c_int, _c_llr, _c_p, _c_int, _c_p, _c_p])
+    rc = f(t.ctypes.data, n, int(copies), int(blocks), int(least), SHARE_ROUNDS * int(blocks), entries.ctypes.data, cap, cut.ctypes.data, counts.ctypes.data)
+    _need(rc >= 0, "cut_portions: sizes")
+    return (entries[:counts[0]], cut[:counts[1]], int(counts[2])) if rc else None
 
 
 @_of_sizes
