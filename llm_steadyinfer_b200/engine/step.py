@@ -64,6 +64,7 @@ class StepContext:
         self.status = runner.status
         self.plans: Dict = {}             # per-step host-side plans of parts, cleared each step
         self.alias: Dict[str, str] = {}   # scratch keys that stand for another buffer for the time being (set by arrangements)
+        self.max_seq_len = runner.max_seq_len     # tokens a request may have
         self.seq_cap: Optional[int] = None    # fixed-shape (graph) steps: sequences the shapes are for
         # device int32 views
         self.tokens = self.positions = self.row_seq = None

@@ -505,19 +505,23 @@ class Attention(Mixer):
                 n = ops.attn_decode_scratch_floats(len(dec), self.H, self.KV, self.hs, nsplit)
                 plan["scratch"] = ctx.buf("attn_split", (n,), torch.float32)
         if por:
-            shares = None
+            shares, room = None, 4 * len(por)
             if tc05:
                 tiles = [-(-(pos0 + n - first_visible_key(pos0, self.window, self.chunk) // 128 * 128) // 128) for _, _, n, pos0 in por]
-                shares = ops.cut_portions(tiles, self.KV, ops.sm_count(self.device))
-            if shares is None:
-                plan["por"] = ctx.upload_ints(f"attn_por_{self._tag()}", np.asarray(por, dtype=np.int32)).view(-1, 4)
-            else:
-                entries, cut, slots = shares
-                ints = ctx.upload_ints(f"attn_por_{self._tag()}", np.concatenate([np.asarray(por, dtype=np.int32), entries, cut])).view(-1, 4)
-                a, b = len(por), len(por) + len(entries)
-                plan["por"] = ints[:a]
-                plan["shares"] = (ints[a:b], ints[b:], slots,
-                                  ctx.buf("attn_shares", (ops.attn_portion_share_floats(slots, self.KV, self.hs, self.vs),), torch.float32))
+                blocks = ops.sm_count(self.device)
+                shares = ops.cut_portions(tiles, self.KV, blocks)
+                # Room for the most that a cut gives, with the first portion of a run whose contexts may become long enough, so that no
+                # later step asks for more (a buffer that grows drops the recorded steps).
+                if shares is not None or ctx.max_seq_len > (2 * ops.CUT_LEAST - 1) * 128:
+                    most = ops.cut_slots(self.KV, blocks)
+                    scratch = ctx.buf("attn_shares", (ops.attn_portion_share_floats(most, self.KV, self.hs, self.vs),), torch.float32)
+                    room = 4 * (3 * len(por) + most)
+            lists = [np.asarray(por, dtype=np.int32)] + (list(shares[:2]) if shares is not None else [])
+            ints = ctx.upload_ints(f"attn_por_{self._tag()}", np.concatenate(lists), capacity=room).view(-1, 4)
+            plan["por"] = ints[:len(por)]
+            if shares is not None:
+                b = len(por) + len(shares[0])
+                plan["shares"] = (ints[len(por):b], ints[b:], shares[2], scratch)
         ctx.plans[key] = plan
 
     def attend(self, q, cache, ctx, out):

@@ -590,3 +590,21 @@ def test_another_block_arrangement_is_registered_and_replayed(tmp_path, dtype):
         llm = LLM(folder, dtype="float32", max_batch=2, max_seq_len=64, max_gen_len=12)
         assert [g.token_ids for g in llm.generate(prompts, SamplingParams(ignore_eos=True))] == greedy
         assert llm.stats["graph_steps"] > 0
+
+
+def test_growing_contexts_ask_for_no_more_scratch(folders):
+    """A request prompted in portions up to 9,000 tokens: once its first portions have run, no step asks for a larger buffer (which would
+    drop the recorded steps), although the cut of its work items begins on the way."""
+    from llm_steadyinfer_b200.engine.step import ModelRunner, StepEntry
+    from llm_steadyinfer_b200.weights import load_model
+    runner = ModelRunner(load_model(folders["C"], torch.bfloat16, DEV), page_size=16, num_pages=600, max_requests=2, max_step_tokens=512)
+    toks = ru.random_tokens(777, 9000, 3)
+    generations, cut = [], []
+    for a in range(0, 9000, 500):
+        runner.step([StepEntry("r", toks[a:a + 500], [499])])
+        generations.append(runner._generation)
+        plan = [p for k, p in runner.ctx.plans.items() if isinstance(k, tuple) and k[0] == "attention"]
+        cut.append(any(p.get("shares") is not None for p in plan))
+    runner.check_status()
+    assert not cut[0] and cut[-1], "the cut begins on the way"
+    assert len(set(generations[1:])) == 1, generations
