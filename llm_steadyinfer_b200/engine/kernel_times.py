@@ -25,17 +25,17 @@ KINDS = {
     "embedding_gather": "embedding", "add_rmsnorm": "add_rmsnorm", "rope_kv_write": "rope_kv_write",
     "paged_attention_ref": "attention_ref", "swiglu": "swiglu", "gemm_f32": "gemm_f32",
     "sample": "sampling", "argmax": "sampling", "attn_portion": "attn_portion_mma", "attn_decode": "attn_decode_mma",
-    "attn_decode_tma": "attn_decode_tma", "attn_portion_tc05": "attn_portion_tc05", "gemm_skinny": "gemm_skinny",
-    "gemm_skinny_swiglu": "gemm_skinny_swiglu", "gemm_skinny_qkv_rope": "gemm_skinny_qkv_rope", "gemm_tc05": "gemm_tc05", "gemm_tc05_swiglu": "gemm_tc05_swiglu",
+    "attn_decode_tma": "attn_decode_tma", "attn_portion_tc05": "attn_portion_tc05", "attn_portion_gen": "attn_portion_gen", "gemm_skinny": "gemm_skinny",
+    "gemm_skinny_swiglu": "gemm_skinny_swiglu", "gemm_skinny_qkv_rope": "gemm_skinny_qkv_rope", "gemm_tc05": "gemm_tc05", "gemm_tc05_add": "gemm_tc05_add", "gemm_tc05_swiglu": "gemm_tc05_swiglu",
     "gemm_rows": "gemm_rows", "gemm_rows_swiglu": "gemm_rows_swiglu",
     "embedding_pair": "embedding", "rmsnorm_rows": "rmsnorm_rows", "attention_general": "attention_general",
     "attn_flex": "attn_flex", "kv_store": "kv_store", "latent_prepare": "latent_prepare", "activation": "activation",
     "gemm_heads": "gemm_heads", "gemm_skinny_relu2": "gemm_skinny_relu2", "gemm_tc05_relu2": "gemm_tc05_relu2", "latent_gather": "latent_gather", "latent_expand_keys": "latent_expand_keys", "causal_conv": "causal_conv", "ssm_scan": "ssm_scan", "gated_part_norm": "gated_part_norm",
     "add_norm": "add_norm", "qk_prepare": "qk_prepare", "diff_combine": "diff_combine", "delta_prepare": "delta_prepare",
     "delta_scan": "delta_scan", "head_norm_gate": "head_norm_gate", "softcap": "softcap", "add_bias": "add_bias",
-    "talk_combine": "talk_combine", "shift_mix": "shift_mix", "time_mix_prepare": "time_mix_prepare", "decay_scan": "decay_scan",
+    "talk_combine": "talk_combine", "shift_mix": "shift_mix", "time_mix_prepare": "time_mix_prepare", "decay_scan": "decay_scan", "decay_group_scan": "decay_group_scan",
     "moe_route": "moe_route", "moe_plan": "moe_plan", "moe_gather": "moe_gather", "moe_gemm_tc05": "moe_gemm_tc05",
-    "moe_gemm_tiles": "moe_gemm_tiles", "moe_combine": "moe_combine", "gated_add": "gated_add", "gemm_skinny_batched": "gemm_skinny_batched",
+    "moe_gemm_tiles": "moe_gemm_tiles", "moe_gemm_pairs": "moe_gemm_pairs", "moe_combine": "moe_combine", "gated_add": "gated_add", "gemm_skinny_batched": "gemm_skinny_batched",
     "stream_norm": "stream_norm", "qkv_conv": "qkv_conv", "conv_rows": "conv_rows", "stream_add": "stream_add",
     "channel_delta_prepare": "channel_delta_prepare", "channel_delta_scan": "channel_delta_scan", "channel_delta_groups": "channel_delta_groups", "channel_delta_group_scan": "channel_delta_group_scan", "gated_linear": "gated_linear",
     "token_gate": "token_gate", "gemm_skinny_token_gate": "gemm_skinny_token_gate",
