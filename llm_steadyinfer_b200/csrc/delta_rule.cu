@@ -724,8 +724,9 @@ SI_EXPORT int si_channel_delta_groups(const float* xc, long long xc_stride, cons
 // the eight that the triangular system needs and solves it for both columns. Shared memory: two buffers of GROUP_AHEAD groups of
 // 4 x [c k | c q | s k: RPT * 16 each | v: cols | scalars] and C; every thread knows its pieces of a group once and for all.
 #define GROUP_AHEAD 4
+// (Three or four pieces a thread come with blocks of at most 128 threads, of which few run at once: they have the registers of two.)
 template <int RPT, int SLOTS>
-__global__ void __launch_bounds__(256, RPT <= 8 && SLOTS <= 4 ? 2 : 1) channel_delta_group_scan_kernel(const float* __restrict__ rec,
+__global__ void __launch_bounds__(RPT <= 8 && SLOTS == 4 ? 128 : 256, RPT <= 8 && SLOTS <= 4 ? 2 : 1) channel_delta_group_scan_kernel(const float* __restrict__ rec,
     const float* __restrict__ sc, const float* __restrict__ dec, long long dec_stride, const float* __restrict__ xc, long long xc_stride,
     float* __restrict__ state, long long state_stride, float* __restrict__ y, long long y_stride, const int* __restrict__ q_start,
     const int* __restrict__ ctx_len, const int* __restrict__ slots, int G, int H, int dk, int dv, int cols) {
