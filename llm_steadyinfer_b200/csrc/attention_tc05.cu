@@ -30,10 +30,10 @@
 // says what a score gets beside its scale: nothing, the extended form (slopes by distance, a query temperature, an output gate), a
 // bias by distance from a table, or a soft limit (see AttnExtras). All of it is fp32 arithmetic on the scores in registers, which
 // costs issue slots of the softmax threads: they, and their exponentials, bound the kernel, not the tensor cores.
-// Measured, a portion of 2,000 to 2,048 tokens, 16 query heads, in place of the mma.sync kernel: bias by distance 291 -> 62 us, 192-wide
-// latent keys 291 -> 51, a soft limit over 64-wide keys and 128-wide values 225 -> 46, four key heads a value head 264 -> 63. Keys of
-// one item cut over blocks (2,043 tokens at the end of 16,128, 24 query and 8 key heads, where 200 blocks were 1.4 waves of SMs): 564 ->
-// 457 us and 18 for the merge.
+// Measured, a portion of 2,048 tokens in place of the mma.sync kernel: bias by distance (16 query, 4 key heads of 128) 285 -> 59 us, 192-wide
+// latent keys (16 heads) 297 -> 49, a soft limit over 64-wide keys and 128-wide values (32 query, 8 key heads) 501 -> 63, four key heads a
+// 512-wide value head 752 -> 99; 32 tokens behind 16,000 with the bias 1,333 -> 279. Keys of one item cut over blocks (2,043 tokens at the end of
+// 16,128, 24 query and 8 key heads, where 200 blocks were 1.4 waves of SMs): 622 -> 518 us with the merge.
 //
 // The reference computes prompt attention row by row with its scalar split kernel
 // (src/source/op/kernels/cuda/paged_kernels.cu:96-206). Conditions here: key sizes up to 192 and value sizes in multiples of 8

@@ -580,8 +580,8 @@ SI_EXPORT int si_channel_delta_scan(const float* xc, long long xc_stride, const 
 // which is the token-by-token recurrence written out, all in fp32 and with products of decays alone (nothing is divided). The sums over
 // the key channels of all four tokens read the same state, so they are formed and added up over the lanes together, and what is left
 // of the chain from token to token is a triangular system of a few scalars.
-// One decay a head (SCALAR) is the same with all channels alike: two portions of up to 1,500 rows, 16 heads of 128, took 270 us by the token,
-// 156 so and 18 for the preparation.
+// One decay a head (SCALAR) is the same with all channels alike: two portions of 1,500 and 700 rows, 16 heads of 128, take 475 us by the token
+// and 312 so with the preparation (a launch behind a launch).
 #define GROUP_TOKENS 4
 #define GROUP_SCALARS 8                                   // a token's beta, kk_i0 .. kk_i2, qk_i0 .. qk_i3
 

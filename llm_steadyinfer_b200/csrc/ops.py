@@ -2040,7 +2040,7 @@ def moe_pairs_ok(x, w_up, w_down, T: int, top: int) -> bool:
 def moe_gemm_pairs(a, ids, w, out, by_row: bool, act: str = "none", limit: float = 0.0, alpha: float = 1.702, shift: float = 1.0) -> None:
     """The grouped product without a plan, for few pairs: out[p, :] = act(a[row, :] @ w[e]^T) for the pair p of ``ids`` int32
     [T, top] that chose expert e, row = p / top (``by_row``: ``a`` [T, K]) or p (``a`` [T * top, K]). Pairs whose id is not below
-    E are left alone. ``out`` and ``act`` as for ``moe_gemm``."""
+    E are left alone; a row's choices are different experts (at most 16 pairs an expert). ``out`` and ``act`` as for ``moe_gemm``."""
     _cuda(a, ids, w, out)
     _i32(ids, "ids")
     _need(act in MOE_ACTS, f"moe_gemm_pairs: act {act!r} is not one of {sorted(MOE_ACTS)}")

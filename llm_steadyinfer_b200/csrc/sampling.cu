@@ -172,8 +172,9 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int vocab,
 // decides alike. The range for top-p starts at max - T (ln(vocab / (1 - top_p)) + 1): what lies below weighs less than 1 - top_p
 // of the maximum alone. A group of 128 logits (a warp's loads) without a key between the bounds is added up once and then left.
 // Bound by the exchanges' latency (some ten of 1 to 2 us) and, from 37 rows of 128,256 logits on, by the second round of clusters
-// over the SMs, not by memory. Rows of 128,256 logits, temperature 0.7, top_p 0.9: 64 rows 1,146 us with a block a row that reads
-// it some 40 times, 74 us here; 8 rows 30 us; top_k 50 instead 62 and 24 us; no restriction 28 and 11 us.
+// over the SMs, not by memory. Rows of 128,256 logits, temperature 0.7, top_p 0.9, a launch behind a launch: 64 rows 1,142 us with a block a
+// row that reads it some 40 times, 77 us here (86 with the rows in memory); 8 rows 30 us (47); top_k 50 instead 64 and 25 us; no restriction 31
+// and 11 us.
 #define SC_THREADS 512
 #define SC_WARPS (SC_THREADS / 32)
 #define SC_MAX_CLUSTER 8

@@ -485,7 +485,7 @@ SI_EXPORT int si_decay_scan(const float* xs, long long xs_stride, const float* u
 //   o_i = (c_i r_i) . S + sum_(j<i) (r_i . diag(w_(j+1) .. w_(i-1)) k_j) v_j + (r_i . diag(u) k_i) v_i;   S <- C S + sum_i (s_i k_i) v_i^T
 // which is the token-by-token recurrence written out, in fp32 and with products of decays alone. The reads of the state and the sums over
 // the lanes of four tokens and two columns go together, and what is a chain is one update of the state in four tokens.
-// Measured, three portions of up to 1,200 rows, 32 heads of 64: 240 us by the token, 157 so and 10 for the preparation.
+// Measured, three portions of 1,200, 900 and 500 rows, 32 heads of 64: 270 us by the token, 186 so with the preparation (a launch behind a launch).
 // Heads of 36 to 64 rows, where a thread's rows are four of one column as in decay_scan_kernel (the slot's layout is the same).
 #define DECAY_GROUP 4
 #define DECAY_GROUP_AHEAD 4

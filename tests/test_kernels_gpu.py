@@ -1335,8 +1335,7 @@ def test_portions_in_the_general_form_on_tcgen05(H, KV, dk, dv, share, page, bia
     a pool whose other pages hold numbers that would show. Probabilities meet the values as bf16 (2^-9 relative each) and results
     are stored in bf16 or fp32: 2^-7 of the largest value is allowed, the plain kernels' bound."""
     o = ops()
-    if not o.attn_portion_gen_ok(H, KV, dk, dv, share, page, bias > 0, cap > 0):
-        pytest.skip("no tensor-map encoder")
+    assert o.attn_portion_gen_ok(H, KV, dk, dv, share, page, bias > 0, cap > 0)
     g = torch.Generator().manual_seed(H * 1000 + dk + n)
     KVv, scale, ends = KV // share, 2.0 * dk ** -0.5, [pos0 + n, pos0 + n + 35]
     starts = [pos0, pos0 + 35]
@@ -1445,8 +1444,7 @@ def test_gated_delta_portions_in_groups_of_four(G, H, dk, dv):
     rows beside each other, from position 0 and going on from a slot. Unit keys and decays below one keep the state of the values'
     size, so the two orders of the sums differ by some 1e-6 a token: 2e-5 of the largest value is allowed."""
     o = ops()
-    if not o.channel_delta_groups_ok(dk, dv):
-        pytest.skip("sizes that go token by token")
+    assert o.channel_delta_groups_ok(dk, dv)
     g = torch.Generator().manual_seed(dk)
     lens, starts = [9, 1, 4, 7, 2], [0, 5, 0, 3, 11]
     T, S, C = sum(lens), len(lens), 2 * G * dk + H * dv
