@@ -44,6 +44,7 @@
 #include "tma_common.cuh"
 #include <algorithm>
 #include <functional>
+#include <new>
 #include <vector>
 #include <limits.h>
 
@@ -683,7 +684,7 @@ static int launch(const AttnParams& p, const CUtensorMap& km, const CUtensorMap&
 // about two for its start, a cut item's share three more for handing over). No share is below `least` tiles; at most `most` shares are
 // partial results. entries [cap][4] receives (item, share, shares, first slot), longest first, cut [n][4] (item, shares, first slot, 0),
 // counts (entries, cut items, slots). Returns 1, 0 where whole items are within a twentieth of the best, or -2.
-SI_EXPORT int si_cut_portions(const int* tiles, int n, int copies, int blocks, int least, long long most, int* entries, int cap, int* cut, int* counts) {
+static int cut_portions(const int* tiles, int n, int copies, int blocks, int least, long long most, int* entries, int cap, int* cut, int* counts) {
   if (n <= 0 || copies <= 0 || blocks <= 0 || least <= 0) return -2;
   long long longest = 0, total = 0;
   for (int i = 0; i < n; ++i) {
@@ -756,6 +757,14 @@ SI_EXPORT int si_cut_portions(const int* tiles, int n, int copies, int blocks, i
   for (int i = 0; i < num; ++i) std::copy(all[i].v, all[i].v + 4, entries + 4 * i);
   counts[0] = num; counts[1] = num_cut; counts[2] = slots;
   return 1;
+}
+
+SI_EXPORT int si_cut_portions(const int* tiles, int n, int copies, int blocks, int least, long long most, int* entries, int cap, int* cut, int* counts) {
+  try {
+    return cut_portions(tiles, n, copies, blocks, least, most, entries, cap, cut, counts);
+  } catch (const std::bad_alloc&) {                        // no memory for the search: whole items serve as well
+    return 0;
+  }
 }
 
 // Floats of partial results of `slots` shares.

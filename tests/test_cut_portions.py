@@ -1,11 +1,16 @@
 """The cut of long prompts' work items into shares (host arithmetic of the tcgen05 prompt attention)."""
 import heapq
+import os
 import random
+import subprocess
+import sys
 
 import numpy as np
 import pytest
 
 from llm_steadyinfer_b200.csrc import ops
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def plain(tiles, copies, blocks, least, most):
@@ -59,3 +64,17 @@ def test_a_cut_follows_the_rule_and_covers_every_item_once():
 @pytest.mark.parametrize("tiles,copies,blocks", [([31], 1, 148), ([1], 8, 148), ([400] * 149, 8, 148)])
 def test_short_and_many_items_stay_whole(tiles, copies, blocks):
     assert ops.cut_portions(tiles, copies, blocks) is None
+
+
+def test_no_memory_for_the_search_leaves_items_whole():
+    # (a child process, whose address space is limited to little more than what it has)
+    code = """
+import resource
+from llm_steadyinfer_b200.csrc import ops
+ops.cut_portions([400] * 20, 8, 148)                     # (loads the library)
+pages = int(open("/proc/self/statm").read().split()[0])
+resource.setrlimit(resource.RLIMIT_AS, (pages * resource.getpagesize() + (1 << 30),) * 2)
+assert ops.cut_portions([400], 1 << 20, 2**31 - 1) is None       # asks for 17 GB
+"""
+    got = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert got.returncode == 0, got.stderr[-500:]
