@@ -14,6 +14,12 @@
 // tile is token r / Gb, head r % Gb; warp w owns rows 16w..16w+15 and walks all keys of the share. K tiles of
 // BLOCK_N keys x dk come through cp.async into XOR-swizzled shared memory, two stages deep; the values are a
 // second tile (own values: only the block's slice) or columns of the key tile itself.
+// A share of a decode row's keys is a chain of latencies (page, keys, queries, scores, merge) for a few kilobytes: what does not need the
+// kernel before (pages, the first two tiles of keys that are older than the step, biases) is fetched before the wait for it, the four warps
+// merge and store a quarter of the columns each, warps that are slices share one score product, shares without a tile store nothing, and
+// the merge is launched while the last shares store. Behind the kernel that stores the newest key, one row (us, attention / merge, before
+// and now): 2,060 keys of 4 x 128 with biases 11.1 / 3.8 and 8.2 / 3.2; a latent of 576 and 16 heads 13.3 / 5.4 and 10.2 / 4.7. (The merge
+// or the product behind it launched from the start instead: 13.7 / 6.5, its loads slow the attention's.)
 // Sizes are run-time values: the loops over dk are not unrolled by the compiler, only the value slice (DVB, the
 // accumulators) and the key tile (BLOCK_N) are template parameters.
 #include "attention_common.cuh"
@@ -40,6 +46,9 @@ struct FlexParams {
                             // value slice of its own, so that a block serves four slices from one key tile
   float scale_log2;         // scale * log2(e)
   int window, chunk, nsplit;
+  int own_rows;             // every item holds all the rows that its sequence has in this step: the keys before its first position are older than the step
+  int block_n;              // keys of a tile
+  int trigger;              // the merge is launched while the last shares store theirs
   int* status;
 };
 
@@ -47,6 +56,14 @@ struct FlexParams {
 
 __device__ __forceinline__ bf16* ftile(bf16* base, int pitch_chunks, int row, int chunk) {
   return base + ((size_t)row * pitch_chunks + (chunk ^ (row & 7))) * 8;
+}
+
+// The tiles of an item's keys and how many of them each of its shares takes; shares behind the last tile have none.
+__device__ __forceinline__ int flex_tiles(const FlexParams& p, const AttnItem& item, int block_n, int* per_share) {
+  const int first = first_visible_key(item.pos0, p.window, p.chunk) / block_n * block_n;
+  const int tiles = (item.pos0 + item.ntok - first + block_n - 1) / block_n;
+  *per_share = (tiles + p.nsplit - 1) / p.nsplit;
+  return tiles;
 }
 
 // KSPLIT 4: items of at most 16 rows; every warp takes rows 0..15 and a quarter of each tile's keys, and the four
@@ -68,30 +85,37 @@ attn_flex_kernel(const FlexParams p) {
   // [2][BLOCK_N + 64 / Gb][Gb] biases of the distances that the rows of this block have to the keys of a tile
   float* Bs = reinterpret_cast<float*>(Vs + (own_v ? (size_t)2 * BLOCK_N * DVB : 0));
   const int bwin = BLOCK_N + FLEX_M / p.Gb;
+  // Warps that are slices have the same rows and keys: each takes a quarter of the key size for the scores, which meet in shared memory
+  // [4][NT * 4][32] (the whole product a warp is a chain of 36 steps at 576)
+  const bool shared_scores = KSPLIT == 1 && p.warps_are_slices;
+  float* Ss = Bs + (p.bias_in_smem ? (size_t)2 * bwin * p.Gb : 0);
 
   const int item_idx = blockIdx.x / p.nsplit, split = blockIdx.x % p.nsplit;
-  const AttnItem item = p.items[item_idx];                 // copied in before the step's first kernel
-  pdl_wait();
+  const AttnItem item = p.items[item_idx];                 // copied in before the step's first kernel, like the block table
   const int g = blockIdx.y / p.hparts, hpart = blockIdx.y % p.hparts;
   const int warp = threadIdx.x >> 5;
   const int wrow = (p.warps_are_slices || KSPLIT > 1) ? 0 : warp * 16;        // first tile row of this warp
   const int krow0 = KSPLIT > 1 ? warp * KEYS_W : 0;                           // first key row of a tile for this warp
   const int v0 = (p.warps_are_slices ? blockIdx.z * 4 + (threadIdx.x >> 5) : blockIdx.z) * DVB;   // first value column
   const int lane = threadIdx.x & 31;
-  if (item.ntok <= 0) return;
-  if (item.seq < 0 || item.seq >= p.num_seqs) {
-    if (threadIdx.x == 0) set_status(p.status, SI_BAD_SEQ);
+  if (item.ntok <= 0 || item.seq < 0 || item.seq >= p.num_seqs) {
+    pdl_wait();
+    if (item.ntok > 0 && threadIdx.x == 0) set_status(p.status, SI_BAD_SEQ);
     return;
   }
   const int* table = p.block_table + (size_t)item.seq * p.table_width;
   const int kv_end_all = item.pos0 + item.ntok;
   const int kv_lo = first_visible_key(item.pos0, p.window, p.chunk);
   const int kv_begin_all = kv_lo / BLOCK_N * BLOCK_N;
-  const int tiles_all = (kv_end_all - kv_begin_all + BLOCK_N - 1) / BLOCK_N;
-  const int tiles_per = (tiles_all + p.nsplit - 1) / p.nsplit;
+  int tiles_per;
+  const int tiles_all = flex_tiles(p, item, BLOCK_N, &tiles_per);
   const int t_begin = split * tiles_per;
   const int t_end = min(tiles_all, t_begin + tiles_per);
   const int ntiles = max(0, t_end - t_begin);
+  if (ntiles == 0 && p.nsplit > 1) {                       // a share behind the item's last tile: the merge does not ask for it
+    pdl_wait();
+    return;
+  }
   const int kv_begin = kv_begin_all + t_begin * BLOCK_N;
   const int kv_end = min(kv_end_all, kv_begin_all + t_end * BLOCK_N);
   const int head0 = g * p.G + hpart * p.Gb;
@@ -134,7 +158,9 @@ attn_flex_kernel(const FlexParams p) {
         cp_async16(ftile(Vt, DT, row, c), valid ? vrow + c * 8 : p.v_cache, valid);
       }
     }
-    if (p.bias_in_smem) {                     // entry (d - dlo, head) with dlo the least distance of the tile
+  };
+  auto load_bias = [&](int j0, int stage) {   // entry (d - dlo, head) with dlo the least distance of the tile
+    if (p.bias_in_smem) {
       float* Bt = Bs + (size_t)stage * bwin * p.Gb;
       const int dlo = item.pos0 - (j0 + BLOCK_N - 1);
       const int total = bwin * p.Gb;
@@ -153,6 +179,16 @@ attn_flex_kernel(const FlexParams p) {
     }
   };
 
+  // Two tiles are on their way from the start. Those whose keys are older than the step are fetched before this kernel waits for the one that
+  // makes the queries and the newest keys; the biases are weights.
+  auto older = [&](int t) { return p.own_rows && t < ntiles && min(kv_begin + (t + 1) * BLOCK_N, kv_end) <= item.pos0; };
+  const bool early0 = older(0), early1 = older(1);
+  if (early0) load_kv(kv_begin, 0);
+  if (early1) load_kv(kv_begin + BLOCK_N, 1);
+  cp_async_commit();
+  if (ntiles > 0) load_bias(kv_begin, 0);
+  if (ntiles > 1) load_bias(kv_begin + BLOCK_N, 1);
+  pdl_wait();
   if (ntiles > 0) {
     for (int id = threadIdx.x; id < q_rows * kch; id += THREADS) {
       const int row = id / kch, c = id % kch;
@@ -162,8 +198,10 @@ attn_flex_kernel(const FlexParams p) {
       if (valid) src = p.q + (size_t)(item.row0 + tok) * p.q_stride + (size_t)(head0 + hh) * p.dk + c * 8;
       cp_async16(ftile(Qs, kch, row, c), src, valid);
     }
-    load_kv(kv_begin, 0);
+    if (!early0) load_kv(kv_begin, 0);
   }
+  cp_async_commit();
+  if (ntiles > 1 && !early1) load_kv(kv_begin + BLOCK_N, 1);
   cp_async_commit();
 
   const int r_lo = wrow + (lane >> 2), r_hi = r_lo + 8;
@@ -179,9 +217,11 @@ attn_flex_kernel(const FlexParams p) {
   const float sl_lo = p.slopes ? p.slopes[head_lo] * LOG2E : 0.f, sl_hi = p.slopes ? p.slopes[head_hi] * LOG2E : 0.f;
   const int warp_last_tok = min(item.ntok - 1, (wrow + 15) / p.Gb);
   const int warp_first_tok = wrow / p.Gb;
-  const bool warp_active = warp_first_tok < item.ntok && v0 < p.dv;
+  const bool warp_active = warp_first_tok < item.ntok && (v0 < p.dv || shared_scores);
   const int warp_max_pos = item.pos0 + warp_last_tok;
   const int warp_first_key = first_visible_key(item.pos0 + warp_first_tok, p.window, p.chunk);
+
+  const int kk0 = shared_scores ? kt_steps * warp / 4 : 0, kk1 = shared_scores ? kt_steps * (warp + 1) / 4 : kt_steps;
 
   float o[DT][4];
 #pragma unroll
@@ -191,13 +231,7 @@ attn_flex_kernel(const FlexParams p) {
   for (int t = 0; t < ntiles; ++t) {
     const int j0 = kv_begin + t * BLOCK_N;
     bf16* Kt = Ks + (size_t)(t & 1) * BLOCK_N * p.dk_pitch;
-    if (t + 1 < ntiles) {
-      load_kv(j0 + BLOCK_N, (t + 1) & 1);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
+    cp_async_wait<1>();
     __syncthreads();
     bool skip = !warp_active || j0 + krow0 > warp_max_pos;
     if (j0 + krow0 + KEYS_W - 1 < warp_first_key) skip = true;
@@ -206,7 +240,7 @@ attn_flex_kernel(const FlexParams p) {
 #pragma unroll
       for (int i = 0; i < NT; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
 #pragma unroll 4
-      for (int kk = 0; kk < kt_steps; ++kk) {
+      for (int kk = kk0; kk < kk1; ++kk) {
         unsigned a0, a1, a2, a3;
         ldsm_x4(a0, a1, a2, a3, ftile(Qs, kch, wrow + (lane & 7) + 8 * ((lane >> 3) & 1), kk * 2 + (lane >> 4)));
 #pragma unroll
@@ -216,6 +250,21 @@ attn_flex_kernel(const FlexParams p) {
           mma_bf16(s[nt], a0, a1, a2, a3, b0, b1);
           mma_bf16(s[nt + 1], a0, a1, a2, a3, b2, b3);
         }
+      }
+      if (shared_scores) {                      // every warp has summed up its quarter of the key size
+        float* mine = Ss + (size_t)warp * NT * 4 * 32 + lane;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) mine[(nt * 4 + e) * 32] = s[nt][e];
+        __syncthreads();
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float* at = Ss + (nt * 4 + e) * 32 + lane;
+            s[nt][e] = (at[0] + at[NT * 4 * 32]) + (at[2 * NT * 4 * 32] + at[3 * NT * 4 * 32]);
+          }
       }
       float mx_lo = m_lo, mx_hi = m_hi;
       const float* Bt = Bs + (size_t)(t & 1) * bwin * p.Gb;
@@ -282,48 +331,53 @@ attn_flex_kernel(const FlexParams p) {
         }
       }
     }
-    __syncthreads();       // everyone is done with this stage before it is refilled
+    if (t + 1 < ntiles) {
+      __syncthreads();     // everyone is done with this stage before it is refilled
+      if (t + 2 < ntiles) { load_kv(j0 + 2 * BLOCK_N, t & 1); load_bias(j0 + 2 * BLOCK_N, t & 1); }
+    }
+    cp_async_commit();
   }
-  if (KSPLIT > 1) {
-    // The warps hold partial results for the same rows and columns, lane by lane: warps 1.. hand theirs to warp 0
-    // through shared memory (the tiles are done with), which weighs them by their maxima and goes on alone.
+  if (p.trigger) pdl_trigger();
+  constexpr int DO = DT / KSPLIT;              // column tiles whose results a warp ends up with, from dt0 on
+  const int dt0 = KSPLIT > 1 ? warp * DO : 0;
+  if constexpr (KSPLIT > 1) {
+    // The warps hold partial results for the same rows and columns, lane by lane: they meet in shared memory, and every warp adds up its
+    // part of the columns, weighed by the maxima.
     constexpr int W = DT * 4 + 4;
     float* X = reinterpret_cast<float*>(smem_raw);
-    if (warp > 0) {
-      float* mine = X + (size_t)(warp - 1) * W * 32 + lane;
+    cp_async_wait<0>();
+    __syncthreads();                          // the tiles are done with
+    float* mine = X + (size_t)warp * W * 32 + lane;
 #pragma unroll
-      for (int i = 0; i < DT; ++i)
+    for (int i = 0; i < DT; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) mine[(i * 4 + e) * 32] = o[i][e];
-      mine[(DT * 4 + 0) * 32] = m_lo; mine[(DT * 4 + 1) * 32] = m_hi;
-      mine[(DT * 4 + 2) * 32] = l_lo; mine[(DT * 4 + 3) * 32] = l_hi;
-    }
+      for (int e = 0; e < 4; ++e) mine[(i * 4 + e) * 32] = o[i][e];
+    mine[(DT * 4 + 0) * 32] = m_lo; mine[(DT * 4 + 1) * 32] = m_hi;
+    mine[(DT * 4 + 2) * 32] = l_lo; mine[(DT * 4 + 3) * 32] = l_hi;
     __syncthreads();
-    if (warp > 0) return;
-    float M_lo = m_lo, M_hi = m_hi;
+    m_lo = m_hi = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < KSPLIT - 1; ++w) {
-      M_lo = fmaxf(M_lo, X[((size_t)w * W + DT * 4 + 0) * 32 + lane]);
-      M_hi = fmaxf(M_hi, X[((size_t)w * W + DT * 4 + 1) * 32 + lane]);
+    for (int w = 0; w < KSPLIT; ++w) {
+      m_lo = fmaxf(m_lo, X[((size_t)w * W + DT * 4 + 0) * 32 + lane]);
+      m_hi = fmaxf(m_hi, X[((size_t)w * W + DT * 4 + 1) * 32 + lane]);
     }
-    const float b_lo = M_lo == -INFINITY ? 0.f : M_lo, b_hi = M_hi == -INFINITY ? 0.f : M_hi;
-    const float f_lo = exp2f(m_lo - b_lo), f_hi = exp2f(m_hi - b_hi);
-    l_lo *= f_lo; l_hi *= f_hi;
+    const float b_lo = m_lo == -INFINITY ? 0.f : m_lo, b_hi = m_hi == -INFINITY ? 0.f : m_hi;
+    l_lo = l_hi = 0.f;
 #pragma unroll
-    for (int i = 0; i < DT; ++i) { o[i][0] *= f_lo; o[i][1] *= f_lo; o[i][2] *= f_hi; o[i][3] *= f_hi; }
+    for (int i = 0; i < DO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
 #pragma unroll
-    for (int w = 0; w < KSPLIT - 1; ++w) {
+    for (int w = 0; w < KSPLIT; ++w) {
       const float* theirs = X + (size_t)w * W * 32 + lane;
       const float g_lo = exp2f(theirs[(DT * 4 + 0) * 32] - b_lo), g_hi = exp2f(theirs[(DT * 4 + 1) * 32] - b_hi);
       l_lo = fmaf(theirs[(DT * 4 + 2) * 32], g_lo, l_lo);
       l_hi = fmaf(theirs[(DT * 4 + 3) * 32], g_hi, l_hi);
 #pragma unroll
-      for (int i = 0; i < DT; ++i) {
-        o[i][0] = fmaf(theirs[(i * 4 + 0) * 32], g_lo, o[i][0]); o[i][1] = fmaf(theirs[(i * 4 + 1) * 32], g_lo, o[i][1]);
-        o[i][2] = fmaf(theirs[(i * 4 + 2) * 32], g_hi, o[i][2]); o[i][3] = fmaf(theirs[(i * 4 + 3) * 32], g_hi, o[i][3]);
+      for (int i = 0; i < DO; ++i) {
+        const float* at = theirs + (size_t)(dt0 + i) * 4 * 32;
+        o[i][0] = fmaf(at[0], g_lo, o[i][0]); o[i][1] = fmaf(at[32], g_lo, o[i][1]);
+        o[i][2] = fmaf(at[64], g_hi, o[i][2]); o[i][3] = fmaf(at[96], g_hi, o[i][3]);
       }
     }
-    m_lo = M_lo; m_hi = M_hi;
   }
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1); l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1); l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
@@ -336,13 +390,13 @@ attn_flex_kernel(const FlexParams p) {
     for (int half = 0; half < 2; ++half) {
       const int r = half ? r_hi : r_lo;
       if (r / p.Gb >= item.ntok) continue;
-      if ((lane & 3) == 0 && v0 == 0) {
+      if ((lane & 3) == 0 && v0 == 0 && dt0 == 0) {
         pml[r * 2] = half ? m_hi : m_lo;
         pml[r * 2 + 1] = half ? l_hi : l_lo;
       }
 #pragma unroll
-      for (int dt = 0; dt < DT; ++dt) {
-        const int d = v0 + dt * 8 + (lane & 3) * 2;
+      for (int dt = 0; dt < DO; ++dt) {
+        const int d = v0 + (dt0 + dt) * 8 + (lane & 3) * 2;
         if (d < p.dv) *reinterpret_cast<float2*>(po + (size_t)r * p.dv + d) = make_float2(o[dt][half * 2], o[dt][half * 2 + 1]);
       }
     }
@@ -364,8 +418,8 @@ attn_flex_kernel(const FlexParams p) {
     const size_t at = (size_t)(item.row0 + tok) * p.out_stride + (size_t)(head0 + hh) * p.dv;
     const bf16* grow = p.gate ? p.gate + (size_t)(item.row0 + tok) * p.gate_stride + (size_t)(head0 + hh) * p.dv : nullptr;
 #pragma unroll
-    for (int dt = 0; dt < DT; ++dt) {
-      const int d = v0 + dt * 8 + (lane & 3) * 2;
+    for (int dt = 0; dt < DO; ++dt) {
+      const int d = v0 + (dt0 + dt) * 8 + (lane & 3) * 2;
       if (d >= p.dv) continue;
       float r0 = o[dt][half * 2] * inv, r1 = o[dt][half * 2 + 1] * inv;
       if (grow) {
@@ -392,18 +446,20 @@ __global__ void __launch_bounds__(128) attn_flex_merge_kernel(const FlexParams p
   const int g = blockIdx.y / p.hparts, hpart = blockIdx.y % p.hparts;
   const int tok = r / p.Gb, head = g * p.G + hpart * p.Gb + r % p.Gb;
   const size_t slab0 = ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * p.nsplit;
+  int per_share;
+  const int tiles = flex_tiles(p, item, p.block_n, &per_share), shares = (tiles + per_share - 1) / per_share;      // shares with keys
   constexpr int FLY = 32;
   const float* col = p.part_o + (slab0 * FLEX_M + r) * p.dv + d;        // share s: FLEX_M * dv further on
   const size_t step = (size_t)FLEX_M * p.dv;
   float v[FLY];
 #pragma unroll
-  for (int u = 0; u < FLY; ++u) v[u] = (u < p.nsplit && d < p.dv) ? col[u * step] : 0.f;
+  for (int u = 0; u < FLY; ++u) v[u] = (u < shares && d < p.dv) ? col[u * step] : 0.f;
   if (threadIdx.x < 32) {                                 // nsplit <= 64: two shares a lane
     const int s0 = threadIdx.x, s1 = threadIdx.x + 32;
-    const float m0 = s0 < p.nsplit ? p.part_ml[((slab0 + s0) * FLEX_M + r) * 2] : -INFINITY;
-    const float m1 = s1 < p.nsplit ? p.part_ml[((slab0 + s1) * FLEX_M + r) * 2] : -INFINITY;
-    const float l0 = s0 < p.nsplit ? p.part_ml[((slab0 + s0) * FLEX_M + r) * 2 + 1] : 0.f;
-    const float l1 = s1 < p.nsplit ? p.part_ml[((slab0 + s1) * FLEX_M + r) * 2 + 1] : 0.f;
+    const float m0 = s0 < shares ? p.part_ml[((slab0 + s0) * FLEX_M + r) * 2] : -INFINITY;
+    const float m1 = s1 < shares ? p.part_ml[((slab0 + s1) * FLEX_M + r) * 2] : -INFINITY;
+    const float l0 = s0 < shares ? p.part_ml[((slab0 + s0) * FLEX_M + r) * 2 + 1] : 0.f;
+    const float l1 = s1 < shares ? p.part_ml[((slab0 + s1) * FLEX_M + r) * 2 + 1] : 0.f;
     const float sk = p.sink ? p.sink[head] * LOG2E : -INFINITY;
     const float M = fmaxf(warp_max(fmaxf(m0, m1)), sk);
     const float w0 = m0 == -INFINITY ? 0.f : exp2f(m0 - M), w1 = m1 == -INFINITY ? 0.f : exp2f(m1 - M);
@@ -415,13 +471,13 @@ __global__ void __launch_bounds__(128) attn_flex_merge_kernel(const FlexParams p
   __syncthreads();
   if (d >= p.dv) return;
   float acc = 0.f;
-  for (int s0 = 0;;) {                                    // a share without keys has written zeros and weighs nothing
+  for (int s0 = 0;;) {                                    // a share that no row sees a key of weighs nothing
 #pragma unroll
-    for (int u = 0; u < FLY; ++u) if (s0 + u < p.nsplit && w[s0 + u] > 0.f) acc = fmaf(v[u], w[s0 + u], acc);
+    for (int u = 0; u < FLY; ++u) if (s0 + u < shares && w[s0 + u] > 0.f) acc = fmaf(v[u], w[s0 + u], acc);
     s0 += FLY;
-    if (s0 >= p.nsplit) break;
+    if (s0 >= shares) break;
 #pragma unroll
-    for (int u = 0; u < FLY; ++u) v[u] = s0 + u < p.nsplit ? col[(s0 + u) * step] : 0.f;
+    for (int u = 0; u < FLY; ++u) v[u] = s0 + u < shares ? col[(s0 + u) * step] : 0.f;
   }
   const size_t at = (size_t)(item.row0 + tok) * p.out_stride + (size_t)head * p.dv;
   float res = acc * s_inv;
@@ -452,14 +508,18 @@ SI_EXPORT long long si_attn_flex_scratch_floats(int num_items, int H, int KV, in
 template <int BLOCK_N, int DVB, int KSPLIT>
 static int flex_launch(const FlexParams& p, int dslices, size_t smem, cudaStream_t stream) {
   static size_t configured = 0;
-  if (KSPLIT > 1 && smem < (size_t)(KSPLIT - 1) * 32 * (DVB / 2 + 4) * sizeof(float))
-    smem = (size_t)(KSPLIT - 1) * 32 * (DVB / 2 + 4) * sizeof(float);          // room for the warps' merge
+  if (KSPLIT > 1 && smem < (size_t)KSPLIT * 32 * (DVB / 2 + 4) * sizeof(float))
+    smem = (size_t)KSPLIT * 32 * (DVB / 2 + 4) * sizeof(float);                // room for the warps' merge
   if (smem > 48 * 1024 && smem > configured) {
     if (cudaFuncSetAttribute(attn_flex_kernel<BLOCK_N, DVB, KSPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return -2;
     configured = smem;
   }
-  si_launch(attn_flex_kernel<BLOCK_N, DVB, KSPLIT>, dim3(p.num_items * p.nsplit, p.KV * p.hparts, dslices), dim3(128), smem, stream, p);
+  const dim3 grid(p.num_items * p.nsplit, p.KV * p.hparts, dslices);
+  FlexParams q = p;
+  q.block_n = BLOCK_N;
+  q.trigger = p.nsplit > 1 && si_pdl_trigger_enabled();
+  si_launch(attn_flex_kernel<BLOCK_N, DVB, KSPLIT>, grid, dim3(128), smem, stream, q);
   return 0;
 }
 
@@ -490,6 +550,8 @@ SI_EXPORT int si_attn_flex(const void* q, long long q_stride, const void* k_cach
   p.H = H; p.KV = KV; p.G = H / KV; p.Gb = flex_heads_per_block(p.G); p.hparts = p.G / p.Gb;
   p.dk = dk; p.dv = dv; p.dk_pitch = (dk + 63) / 64 * 64;
   p.scale_log2 = scale * LOG2E; p.window = window; p.chunk = chunk; p.nsplit = nsplit; p.status = status;
+  p.own_rows = max_rows > 0;
+  p.trigger = 0;
   const long long slabs = (long long)num_items * KV * p.hparts * nsplit;
   p.part_o = scratch;
   p.part_ml = scratch ? scratch + slabs * FLEX_M * dv : nullptr;
@@ -509,6 +571,10 @@ SI_EXPORT int si_attn_flex(const void* q, long long q_stride, const void* k_cach
   const size_t bias_bytes = (size_t)2 * (block_n + FLEX_M / p.Gb) * p.Gb * sizeof(float);
   p.bias_in_smem = dist_bias && smem + bias_bytes <= 227 * 1024 ? 1 : 0;       // else each score fetches its own
   if (p.bias_in_smem) smem += bias_bytes;
+  if (p.warps_are_slices) {
+    smem += (size_t)4 * (block_n / 8) * 4 * 32 * sizeof(float);
+    if (smem > 227 * 1024) return -2;
+  }
   int rc;
   if (ksplit) rc = dvb == 128 ? flex_launch<64, 128, 4>(p, zblocks, smem, stream) : flex_launch<64, 64, 4>(p, zblocks, smem, stream);
   else if (block_n == 64) rc = dvb == 128 ? flex_launch<64, 128, 1>(p, zblocks, smem, stream) : flex_launch<64, 64, 1>(p, zblocks, smem, stream);
@@ -516,6 +582,7 @@ SI_EXPORT int si_attn_flex(const void* q, long long q_stride, const void* k_cach
   if (rc) return rc;
   if (nsplit > 1) {
     const int rows = max_rows > 0 && max_rows < FLEX_M ? max_rows : FLEX_M, col_blocks = (dv + 127) / 128;
+    p.block_n = block_n;
     si_launch(attn_flex_merge_kernel, dim3(num_items, KV * p.hparts, rows * col_blocks), dim3(128), 0, stream, p, col_blocks);
   }
   return si_last_error();

@@ -188,7 +188,7 @@ __global__ void kv_store_kernel(const T* __restrict__ qkv, long long row_stride,
                                 const int* __restrict__ row_seq, const int* __restrict__ block_table,
                                 int table_width, T* __restrict__ k_cache, T* __restrict__ v_cache, int num_pages,
                                 int page_size, int num_seqs, int H, int KV, int dk, int dv, int* status) {
-  pdl_prologue();
+  pdl_prologue_small();
   const int t = blockIdx.x;
   const int pos = positions[t];
   const long long page = page_of(block_table, table_width, num_pages, page_size, num_seqs, row_seq[t], pos, status);
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(1024) latent_prepare_kernel(const T* __restric
                                       int num_pages, int page_size, int num_seqs, int H, int dq, int dr, int rk,
                                       int interleaved, float rot_scale, int* status) {
   __shared__ float red[33];
-  pdl_prologue();
+  pdl_prologue_small();
   const int t = blockIdx.x;
   const int pos = positions[t];
   const int seq = row_seq[t];

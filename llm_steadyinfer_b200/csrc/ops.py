@@ -1384,6 +1384,8 @@ def attn_flex(q, k_cache, v_cache, block_table, items, out, page_size: int, num_
     many shares (decode rows over long contexts); ``scratch`` then holds ``attn_flex_scratch_floats`` floats.
     ``max_rows``: the most rows (tokens x query heads of a key head served together) of any item when the caller knows it
     (0: unknown); at most 16 rows over keys that are their own values let a block's warps take a value slice each.
+    Given, it also says that an item holds all the rows of its sequence that the kernels of this step write: keys before its first position
+    are read before the kernel before this one is waited for.
     ``softcap``, ``v_share``, ``slopes``, ``q_temp``, ``gate``, ``chunk`` as in ``attention_general``; ``out`` may be fp32."""
     _cuda(q, k_cache, v_cache, block_table, items, out, dist_bias, sink, scratch, slopes, gate, status)
     _need(gate is None or (gate.dtype == torch.bfloat16 and gate.shape == (q.shape[0], H * dv) and gate.stride(1) == 1

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(THREADS) qk_prepare_kernel(T* __restrict__ row
     int dk, int dv, T* __restrict__ q_out, long long q_out_stride, int maps, int whole, float rot_scale, int* status) {
   extern __shared__ float sc_table[];                  // the row's sines, then its cosines: rd / 2 each, once for all vectors
   __shared__ float red[33];
-  pdl_prologue();
+  pdl_prologue_small();
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int pos = positions[t];

@@ -16,7 +16,7 @@ from .base import first_visible_key
 
 MAX_SPLITS = 32
 MIN_KEYS_PER_SPLIT = 256
-BLOCKS_PER_SM = 2
+BLOCKS_PER_SM = 3         # shares start with two tiles on their way; two blocks: a Nufasun pass of two requests 11.01 ms, three 10.94, four 11.03
 GEN_MIN_ROWS = 128        # rows (tokens x query heads of a key head) of a sequence from which on the tcgen05 prompt kernel serves it
 
 

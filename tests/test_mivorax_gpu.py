@@ -294,6 +294,34 @@ def test_tensor_core_attention_sizes(H, KV, dk, dv, own_v):
     assert (got.float() - want.float()).abs().max().item() <= 2e-2
 
 
+@pytest.mark.parametrize("H,KV,dk,dv,own_v,window", [(16, 4, 128, 128, True, 0), (8, 8, 64, 64, True, 100), (16, 1, 576, 512, False, 0),
+                                                     (4, 1, 320, 264, False, 70)])
+def test_tensor_core_attention_shares_without_keys(H, KV, dk, dv, own_v, window):
+    """Rows at the edges of key tiles with more shares than tiles: shares behind the last tile leave their partial results as they are (here
+    not a number), and the merge does not ask for them. Keys before a row's own are fetched before the wait for the kernel before. Both
+    sides round the same 32-bit result to 8 bits of mantissa, from weights rounded to as many: 2^-7 of values up to some 3."""
+    from llm_steadyinfer_b200.csrc import ops
+    dev = "cuda:0"
+    torch.manual_seed(dk)
+    n, ps = 330, 16
+    k = (torch.randn(n, KV, dk) * 0.5).bfloat16()
+    v = torch.randn(n, KV, dv).bfloat16() if own_v else None
+    kc, table = _paged(k, ps, 5)
+    kc, table, vc = kc.to(dev), table.to(dev), _paged(v, ps, 5)[0].to(dev) if own_v else None
+    at = [0, 1, 30, 31, 32, 63, 64, 65, 127, 128, 191, 192, 255, 256, 329]
+    q = (torch.randn(len(at), H * dk) * 0.5).bfloat16().to(dev)
+    bias = torch.randn(40, H, device=dev)
+    pos, seqs = torch.tensor(at, dtype=torch.int32, device=dev), torch.zeros(len(at), dtype=torch.int32, device=dev)
+    want, got = (torch.zeros(len(at), H * dv, dtype=torch.bfloat16, device=dev) for _ in range(2))
+    ops.attention_general(q, kc, vc, table, seqs, pos, want, ps, 1, H, KV, dk, dv, dk ** -0.5, window, dist_bias=bias)
+    items = torch.tensor([(0, r, 1, j) for r, j in enumerate(at)], dtype=torch.int32, device=dev)
+    for nsplit in (2, 5, 32, 64):
+        scratch = torch.full((ops.attn_flex_scratch_floats(len(at), H, KV, dv, nsplit),), float("nan"), device=dev)
+        ops.attn_flex(q, kc, vc, table, items, got, ps, 1, H, KV, dk, dv, dk ** -0.5, window, dist_bias=bias, nsplit=nsplit, scratch=scratch,
+                      max_rows=H // KV)
+        assert (got.float() - want.float()).abs().max().item() <= 2e-2, nsplit
+
+
 def test_bias_table_is_spread_as_the_plain_bucket_says():
     from llm_steadyinfer_b200.parts.attention import spread_by_distance
     for rows, dmax in ((2, 5.0), (6, 9.0), (12, 300.0), (32, 120.0), (16, 17.5), (10, 1000.0)):
