@@ -40,6 +40,7 @@ template <typename T, bool EARLY>
 __global__ void __launch_bounds__(EARLY ? 1024 : 256) moe_route_kernel(const T* __restrict__ x, long long x_stride, const T* __restrict__ w,
     int E, int extra, int d, int top, float scale, int mode, int renorm, float renorm_eps, int groups, int keep,
     const float* __restrict__ choice_bias, int* __restrict__ ids, float* __restrict__ wts, float* __restrict__ gates) {
+  if (EARLY) pdl_trigger();
   extern __shared__ float rsm[];                       // the row [d], scores [E + extra], used [E], choice keys [E] (and groups' scores)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const long long t = blockIdx.x;
@@ -473,10 +474,7 @@ __global__ void __launch_bounds__(128) moe_gemm_bf16_kernel(const bf16* __restri
 // matrix. A block takes 16 columns of one expert for up to 16 of its places; its eight warps take the 32-wide chunks of k in turn,
 // with a warp's loads of four chunks (both operands, 16 bytes a lane) in flight at once, straight into the fragments of
 // mma.sync m16n8k16 (the weights are its 16 rows, the places its 8 columns), and their sums are added in warp order. The places come
-// from the plan (offsets and rows), or, where a step has at most 32 (row, choice) pairs, straight from the ids: a pair is then a
-// place of its own, every block finds its expert's pairs by one warp instruction, and no plan is made.
-// Measured, an average of the two products of 2,048 columns and experts of 1,408: one row of two experts 22.3 -> 6.2 us, three rows
-// 24.2 -> 11.3, two rows of four experts 29.1 -> 15.7 (before: tiles of 16 places, a chain of K steps a block).
+// from the plan (offsets and rows); steps of at most 32 (row, choice) pairs have a kernel of their own (moe_pairs_kernel).
 __device__ __forceinline__ void moe_mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -537,10 +535,9 @@ __device__ __forceinline__ void moe_stream_tile(const bf16* __restrict__ A, long
     for (int i = 0; i < 4; ++i) red[warp][mt][lane][i] = acc[mt][i];
 }
 
-// ids given: at most 32 pairs of at most 16 rows, `choices` a row, a pair's row of A is pair / a_div; else offsets and a_rows.
 __global__ void __launch_bounds__(STREAM_WARPS * 32, 3) moe_stream_kernel(const bf16* __restrict__ A, long long a_stride,
-    const int* __restrict__ a_rows, const int* __restrict__ ids, int a_div, const bf16* __restrict__ W, void* __restrict__ C,
-    long long c_stride, int c_f32, const int* __restrict__ offsets, int P, int E, int N, int K, int act, float limit, float alpha,
+    const int* __restrict__ a_rows, const bf16* __restrict__ W, void* __restrict__ C,
+    long long c_stride, int c_f32, const int* __restrict__ offsets, int E, int N, int K, int act, float limit, float alpha,
     float shift) {
   __shared__ float red[STREAM_WARPS][2][32][4];
   __shared__ int place[16], src_row[16], info[2];
@@ -548,48 +545,34 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32, 3) moe_stream_kernel(const 
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < 32) {
     int e = -1, rows = 0, mine = -1;                     // lane l < 16: the tile's place l
-    if (ids) {
-      int id = lane < P ? ids[lane] : -1;
-      if (id < 0 || id >= E) id = -1;                    // (identity experts and none: no product)
-      const unsigned same = __match_any_sync(0xffffffffu, id);
-      const unsigned leaders = __ballot_sync(0xffffffffu, id >= 0 && __ffs(same) - 1 == lane);
-      if ((int)blockIdx.y < __popc(leaders)) {
-        const int lead = __fns(leaders, 0, blockIdx.y + 1);
-        e = __shfl_sync(0xffffffffu, id, lead);
-        const unsigned members = __shfl_sync(0xffffffffu, same, lead);
-        rows = min(__popc(members), 16);
-        if (lane < rows) mine = (int)__fns(members, 0, lane + 1);
-      }
-    } else {
-      int before = 0, first = 0;
-      for (int base = 0; base < E && e < 0; base += 32) {
-        const int x = base + lane;
-        const int a = x < E ? offsets[x] : 0, n = x < E ? offsets[x + 1] - a : 0;
-        const int tiles = (n + 15) / 16;
-        int upto = tiles;
+    int before = 0, first = 0;
+    for (int base = 0; base < E && e < 0; base += 32) {
+      const int x = base + lane;
+      const int a = x < E ? offsets[x] : 0, n = x < E ? offsets[x + 1] - a : 0;
+      const int tiles = (n + 15) / 16;
+      int upto = tiles;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, upto, o);
-          if (lane >= o) upto += v;
-        }
-        upto += before;
-        const unsigned past = __ballot_sync(0xffffffffu, (int)blockIdx.y < upto);
-        if (past) {
-          const int at = __ffs(past) - 1;
-          const int skip = ((int)blockIdx.y - (upto - tiles)) * 16;      // of lane `at`: places of the expert before this tile
-          first = __shfl_sync(0xffffffffu, a + skip, at);
-          rows = __shfl_sync(0xffffffffu, min(n - skip, 16), at);
-          e = base + at;
-        }
-        before = __shfl_sync(0xffffffffu, upto, 31);
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
       }
-      if (e >= 0 && lane < rows) mine = first + lane;
+      upto += before;
+      const unsigned past = __ballot_sync(0xffffffffu, (int)blockIdx.y < upto);
+      if (past) {
+        const int at = __ffs(past) - 1;
+        const int skip = ((int)blockIdx.y - (upto - tiles)) * 16;      // of lane `at`: places of the expert before this tile
+        first = __shfl_sync(0xffffffffu, a + skip, at);
+        rows = __shfl_sync(0xffffffffu, min(n - skip, 16), at);
+        e = base + at;
+      }
+      before = __shfl_sync(0xffffffffu, upto, 31);
     }
+    if (e >= 0 && lane < rows) mine = first + lane;
     const int head = __shfl_sync(0xffffffffu, mine, 0);
     if (lane < 16) {                                     // places that are not there stand for the first one: never stored
       const int p = mine >= 0 ? mine : head;
       place[lane] = mine;
-      src_row[lane] = p < 0 ? 0 : ids ? p / a_div : a_rows ? a_rows[p] : p;
+      src_row[lane] = p < 0 ? 0 : a_rows ? a_rows[p] : p;
     }
     if (lane == 0) { info[0] = e; info[1] = rows; }
   }
@@ -626,6 +609,168 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32, 3) moe_stream_kernel(const 
     }
     if (c_f32) reinterpret_cast<float*>(C)[at + n] = v;
     else reinterpret_cast<bf16*>(C)[at + n] = __float2bfloat16_rn(v);
+  }
+}
+
+// ---- few pairs ------------------------------------------------------------------------------------------------------------
+// A matrix that every row takes, beside the chosen ones (the shared expert's): C[t] = form(A[t] W^T) for `rows` rows, at most 16.
+// form 0 the sum; 1 the square of relu; 2 silu(gate) * up; 3 the limited form with biases (fp32 in the rows' order, or null). The latter two
+// have gates and ups in groups of 8 rows. The sums are rounded to bf16 before a form, as the few-row product does that serves it alone.
+struct MoeShared {
+  const bf16* A; long long a_stride;
+  const bf16* W;
+  bf16* C; long long c_stride;
+  const float* bias;
+  int rows, N, K, form;
+  float limit, alpha;
+};
+
+__device__ __forceinline__ uint4 moe_ld_if(const bf16* p, bool take, bool stream) {      // without a branch; not taken: zeros
+  uint4 v;
+  if (stream)
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+                 "@q ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}\n"
+                 : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((int)take));
+  else
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+                 "@q ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}\n"
+                 : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((int)take));
+  return v;
+}
+
+// At most 32 (row, choice) pairs of at most 16 rows: a pair is a place of its own, and no plan is made; pair p reads row p / a_div of A.
+// Tiles of 16 columns, first the shared matrix's, then expert by expert as they are first chosen, go in turn to two blocks an SM. A block's
+// warps take the 32-wide chunks of k in turn, UP of them at once with both operands, straight into the fragments of mma.sync; the next
+// round's loads (of this tile or the next) are on their way while the warps' sums are added, so that a block's start and the latency of a round
+// are paid once, and blocks that begin with the shared matrix ask for its weights before the wait for the router. Bound by the stream of
+// weights. Both products of 2,048 columns, in us, as launches of their own with a block a tile and the shared expert behind them, and so: one
+// row of two experts of 1,408 and a shared one of 2,816 (69 MB) 23.1, 14.3; three rows of six without gates (69 MB) 28.4, 18.1; two rows of
+// eight and none shared (138 MB) 31.3, 25.5.
+template <int MT>
+__global__ void __launch_bounds__(STREAM_WARPS * 32, 2) moe_pairs_kernel(const bf16* __restrict__ A, long long a_stride,
+    const int* __restrict__ ids, int a_div, const bf16* __restrict__ W, void* __restrict__ C, long long c_stride, int c_f32, int P, int E,
+    int N, int K, int act, float limit, float alpha, float shift, const MoeShared sh) {
+  constexpr int UP = MT == 1 ? 8 : 4;
+  __shared__ float red[2][STREAM_WARPS][MT][32][4];
+  __shared__ int place[32][16], count[32], expert[32], distinct;
+  pdl_trigger();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int nx = (N + 15) / 16, ns = (sh.N + 15) / 16;
+  // The tiles go to the blocks forwards and backwards in turn: the first ones (the shared matrix's) may be the longer ones.
+  int q = blockIdx.x, pass = 0, r = 0, y = 0, n0 = 0, width = 0, depth = 0;      // the tile and round whose loads were asked for last
+  uint4 lo[UP], hi[UP], xb[UP][MT];
+  auto load_w = [&]() {
+    const bf16* w;
+    if (q < ns) {
+      n0 = q * 16; w = sh.W; width = sh.N; depth = sh.K;
+    } else {
+      y = (q - ns) / nx;
+      n0 = (q - ns - y * nx) * 16; w = W + (size_t)expert[y] * N * K; width = N; depth = K;
+    }
+    const bf16* w0 = w + (size_t)min(n0 + g, width - 1) * depth;       // rows beyond the matrix stand for the last one: never stored
+    const bf16* w1 = w + (size_t)min(n0 + 8 + g, width - 1) * depth;
+#pragma unroll
+    for (int u = 0; u < UP; ++u) {
+      const int k = (warp + (r * UP + u) * STREAM_WARPS) * 32 + t * 8;
+      lo[u] = moe_ld_if(w0 + k, k < depth, true);
+      hi[u] = moe_ld_if(w1 + k, k < depth, true);
+    }
+  };
+  auto load_x = [&]() {
+    const bool shared = q < ns;
+    const int rows = shared ? sh.rows : count[y];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const int i = mt * 8 + g;
+      const bool in = i < rows;
+      const bf16* xr = shared ? sh.A + (long long)(in ? i : 0) * sh.a_stride : A + (long long)(place[y][in ? i : 0] / a_div) * a_stride;
+#pragma unroll
+      for (int u = 0; u < UP; ++u) {
+        const int k = (warp + (r * UP + u) * STREAM_WARPS) * 32 + t * 8;
+        xb[u][mt] = moe_ld_if(xr + k, in && k < depth, false);
+      }
+    }
+  };
+  if (q < ns) load_w();                                  // the shared matrix does not depend on the choice before this kernel
+  pdl_wait();
+  if (warp == 0) {
+    int id = lane < P ? ids[lane] : -1;
+    if (id < 0 || id >= E) id = -1;                      // (identity experts and none: no product)
+    const unsigned same = __match_any_sync(0xffffffffu, id), below = (1u << lane) - 1;
+    const unsigned leaders = __ballot_sync(0xffffffffu, id >= 0 && __ffs(same) - 1 == lane);
+    if (id >= 0) {
+      const int at = __popc(leaders & ((1u << (__ffs(same) - 1)) - 1)), rank = __popc(same & below);
+      if (rank < 16) place[at][rank] = lane;             // (a row's choices are different experts: at most 16)
+      if (rank == 0) { expert[at] = id; count[at] = min(__popc(same), 16); }
+    }
+    if (lane == 0) distinct = __popc(leaders);
+  }
+  __syncthreads();
+  const int total = ns + distinct * nx;
+  if (q < total) {
+    if (q >= ns) load_w();
+    load_x();
+  }
+  int par = 0;
+  while (q < total) {
+    float acc[MT][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
+    const bool shared = q < ns;
+    const int rows = shared ? sh.rows : count[y], tile_y = y, tile_n0 = n0, tile_width = width;
+    const int rounds = (depth + STREAM_WARPS * UP * 32 - 1) / (STREAM_WARPS * UP * 32);
+    for (int round = 0; round < rounds; ++round) {
+#pragma unroll
+      for (int u = 0; u < UP; ++u)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          moe_mma(acc[mt], lo[u].x, hi[u].x, lo[u].y, hi[u].y, xb[u][mt].x, xb[u][mt].y);
+          moe_mma(acc[mt], lo[u].z, hi[u].z, lo[u].w, hi[u].w, xb[u][mt].z, xb[u][mt].w);
+        }
+      if (++r == rounds) {
+        r = 0;
+        ++pass;
+        q = pass * gridDim.x + ((pass & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+      }
+      if (q < total) { load_w(); load_x(); }
+    }
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+      *reinterpret_cast<float4*>(red[par][warp][mt][lane]) = make_float4(acc[mt][0], acc[mt][1], acc[mt][2], acc[mt][3]);
+    __syncthreads();
+    // a thread adds the warps' sums of one column (or of a gate and its up) of one place
+    const bool gated = shared ? sh.form >= 2 : act == MOE_ACT_GLU_LIMITED;
+    const int per_place = gated ? 8 : 16, gap = shared ? 8 : 1;        // the shared matrix has gates and ups in eights, the experts' in turn
+    for (int i = threadIdx.x; i < rows * per_place; i += STREAM_WARPS * 32) {
+      const int row = i / per_place, c = i % per_place, mt = row >> 3;
+      auto sum = [&](int col) {                          // column of the 16: fragment (lane (col % 8, row % 8 / 2), element)
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < STREAM_WARPS; ++w) v += red[par][w][mt][(col & 7) * 4 + ((row & 7) >> 1)][(col >> 3) * 2 + (row & 1)];
+        return v;
+      };
+      const int first = gated && !shared ? 2 * c : c;
+      if (tile_n0 + first + (gated ? gap : 0) >= tile_width) continue;
+      float v = sum(first), up = gated ? sum(first + gap) : 0.f;
+      const int n = gated ? (tile_n0 >> 1) + c : tile_n0 + c;
+      if (shared) {
+        v = __bfloat162float(__float2bfloat16_rn(v));
+        up = __bfloat162float(__float2bfloat16_rn(up));
+        if (sh.form == 3) {
+          if (sh.bias) { v += sh.bias[tile_n0 + c]; up += sh.bias[tile_n0 + 8 + c]; }
+          v = moe_glu_limited(v, up, sh.limit, sh.alpha, 1.f);
+        } else {
+          v = sh.form == 2 ? silu_mul(v, up) : moe_act(v, sh.form);
+        }
+        sh.C[(size_t)row * sh.c_stride + n] = __float2bfloat16_rn(v);
+      } else {
+        v = gated ? moe_glu_limited(v, up, limit, alpha, shift) : moe_act(v, act);
+        const size_t at = (size_t)place[tile_y][row] * c_stride + n;
+        if (c_f32) reinterpret_cast<float*>(C)[at] = v;
+        else reinterpret_cast<bf16*>(C)[at] = __float2bfloat16_rn(v);
+      }
+    }
+    par ^= 1;
   }
 }
 
@@ -712,7 +857,7 @@ SI_EXPORT int si_moe_gemm(const void* A, int dtype, long long a_stride, const in
     const long long tiles = P < (P + 15) / 16 + E ? P : (P + 15) / 16 + E;       // no more can there be
     if (tiles > 65535) return -2;
     si_launch(moe_stream_kernel, dim3((N + 15) / 16, (unsigned)tiles), dim3(STREAM_WARPS * 32), 0, stream, (const bf16*)A, a_stride, a_rows,
-              nullptr, 1, (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, offsets, P, E, N, K, act, limit, alpha, shift);
+              (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, offsets, E, N, K, act, limit, alpha, shift);
   } else if (P < 32LL * E && !wide) {
     // few rows an expert, and sizes or rows that are not in 16-byte pieces: tiles of 16 places (one row of two experts of 1,408 x 1,034:
     // 134 us, 176 in tiles of 64)
@@ -727,16 +872,29 @@ SI_EXPORT int si_moe_gemm(const void* A, int dtype, long long a_stride, const in
 }
 
 // The grouped product without a plan: P = rows x choices pairs, at most 32 of at most 16 rows; pair p of expert ids[p] reads row
-// p / a_div of A and writes row p of C. Pairs whose id is not below E are left alone. bf16; returns -2 for what it does not take.
+// p / a_div of A and writes row p of C. Pairs whose id is not below E are left alone. With sW the shared matrix's product (see MoeShared) for
+// the P / choices rows of sA runs in the same launch. bf16; returns -2 for what it does not take.
 SI_EXPORT int si_moe_gemm_pairs(const void* A, long long a_stride, int a_div, const int* ids, const void* W, void* C, int c_dtype,
                                 long long c_stride, int P, int choices, int E, int N, int K, int act, float limit, float alpha,
-                                float shift, cudaStream_t stream) {
+                                float shift, const void* sA, long long sa_stride, const void* sW, void* sC, long long sc_stride,
+                                int sN, int sK, int s_form, const float* s_bias, float s_limit, float s_alpha, cudaStream_t stream) {
   if (P <= 0) return 0;
   if (E <= 0 || N <= 0 || K <= 0 || act < 0 || act > MOE_ACT_GLU_LIMITED || choices <= 0 || P % choices || P > 32 || P / choices > 16 || a_div <= 0) return -2;
   if (act == MOE_ACT_GLU_LIMITED && (N % 2 || !(limit > 0.f))) return -2;
   if (K % 8 || a_stride % 8 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return -2;
-  si_launch(moe_stream_kernel, dim3((N + 15) / 16, P < E ? P : E), dim3(STREAM_WARPS * 32), 0, stream, (const bf16*)A, a_stride, nullptr, ids, a_div,
-            (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, nullptr, P, E, N, K, act, limit, alpha, shift);
+  MoeShared sh = {};
+  long long tiles = (long long)((N + 15) / 16) * (P < E ? P : E);
+  const int T = P / choices;
+  if (sW) {
+    if (sN <= 0 || sK <= 0 || sK % 8 || sa_stride % 8 || ((uintptr_t)sA & 15) || ((uintptr_t)sW & 15) || s_form < 0 || s_form > 3 || !sC) return -2;
+    if (s_form >= 2 && sN % 16) return -2;
+    sh.A = (const bf16*)sA; sh.a_stride = sa_stride; sh.W = (const bf16*)sW; sh.C = (bf16*)sC; sh.c_stride = sc_stride;
+    sh.bias = s_bias; sh.rows = T; sh.N = sN; sh.K = sK; sh.form = s_form; sh.limit = s_limit; sh.alpha = s_alpha;
+    tiles += (sN + 15) / 16;
+  }
+  const long long slots = 2LL * si_sm_count();
+  si_launch(T <= 8 ? moe_pairs_kernel<1> : moe_pairs_kernel<2>, dim3((unsigned)(tiles < slots ? tiles : slots)), dim3(STREAM_WARPS * 32), 0, stream,
+            (const bf16*)A, a_stride, ids, a_div, (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, P, E, N, K, act, limit, alpha, shift, sh);
   return si_last_error();
 }
 

@@ -2039,25 +2039,46 @@ def moe_pairs_ok(x, w_up, w_down, T: int, top: int) -> bool:
             and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
 
 
-def moe_gemm_pairs(a, ids, w, out, by_row: bool, act: str = "none", limit: float = 0.0, alpha: float = 1.702, shift: float = 1.0) -> None:
+# what ``moe_gemm_pairs`` does to the sums of a shared matrix
+MOE_SHARED_FORMS = {"none": 0, "relu2": 1, "silu_glu": 2, "glu_limited": 3}
+
+
+def moe_gemm_pairs(a, ids, w, out, by_row: bool, act: str = "none", limit: float = 0.0, alpha: float = 1.702, shift: float = 1.0,
+                   shared=None) -> None:
     """The grouped product without a plan, for few pairs: out[p, :] = act(a[row, :] @ w[e]^T) for the pair p of ``ids`` int32
     [T, top] that chose expert e, row = p / top (``by_row``: ``a`` [T, K]) or p (``a`` [T * top, K]). Pairs whose id is not below
-    E are left alone; a row's choices are different experts (at most 16 pairs an expert). ``out`` and ``act`` as for ``moe_gemm``."""
+    E are left alone; a row's choices are different experts (at most 16 pairs an expert). ``out`` and ``act`` as for ``moe_gemm``.
+    ``shared`` {"a" [T, K'], "w" [N', K'], "out", "form" one of ``MOE_SHARED_FORMS``, "bias", "limit", "alpha"}: a product that every row
+    takes, in the same launch, as ``gemm_skinny`` and its gated forms (rows of w in groups of 8 gates and 8 ups) give it."""
     _cuda(a, ids, w, out)
     _i32(ids, "ids")
     _need(act in MOE_ACTS, f"moe_gemm_pairs: act {act!r} is not one of {sorted(MOE_ACTS)}")
     E, N, K = w.shape
     T, top = ids.shape
     P = T * top
+    also = (None, 0, None, None, 0, 0, 0, 0, None, 0.0, 0.0)
+    if shared is not None:
+        sa, sw, so, form = shared["a"], shared["w"], shared["out"], shared["form"]
+        bias = shared.get("bias")
+        _cuda(sa, sw, so, bias)
+        glu = form in ("silu_glu", "glu_limited")
+        _need(form in MOE_SHARED_FORMS and gemm_skinny_ok(sa, sw, so) and so.dtype == torch.bfloat16 and sw.is_contiguous()
+              and sa.shape == (T, sw.shape[1]) and so.shape == (T, sw.shape[0] // 2 if glu else sw.shape[0])
+              and (not glu or sw.shape[0] % 16 == 0) and (form != "glu_limited" or shared["limit"] > 0),
+              "moe_gemm_pairs: shared a [T, K], w [N, K], out [T, N] (gated: [T, N / 2], N a multiple of 16), bf16")
+        _f32v(bias, "bias", sw.shape[0])
+        also = (_ptr(sa), sa.stride(0), _ptr(sw), _ptr(so), so.stride(0), sw.shape[0], sw.shape[1], MOE_SHARED_FORMS[form], _ptr(bias),
+                float(shared.get("limit", 0.0)), float(shared.get("alpha", 1.0)))
     pair = act == "glu_limited"
     _need(not pair or (N % 2 == 0 and limit > 0), "moe_gemm_pairs: glu_limited needs an even N and a positive limit")
     _need(a.dtype == torch.bfloat16 and a.shape == (T if by_row else P, K) and a.stride(1) == 1 and w.is_contiguous() and w.dtype == a.dtype
           and ids.is_contiguous(), "moe_gemm_pairs: a [rows, K], w [E, N, K]")
     _need(out.shape == (P, N // 2 if pair else N) and out.stride(1) == 1 and out.dtype in (a.dtype, torch.float32), "moe_gemm_pairs: out must be [P, N]")
     f = _fn("moe", "si_moe_gemm_pairs", [_c_p, _c_ll, _c_int, _c_p, _c_p, _c_p, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int,
-                                         _c_int, _c_f, _c_f, _c_f, _c_p])
+                                         _c_int, _c_f, _c_f, _c_f,
+                                         _c_p, _c_ll, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_p, _c_f, _c_f, _c_p])
     _check(f(_ptr(a), a.stride(0), top if by_row else 1, _ptr(ids), _ptr(w), _ptr(out), _dt(out), out.stride(0), P, top, E, N, K,
-             MOE_ACTS[act], float(limit), float(alpha), float(shift), _stream()), f"moe_gemm_pairs(experts={E}, N={N}, K={K})")
+             MOE_ACTS[act], float(limit), float(alpha), float(shift), *also, _stream()), f"moe_gemm_pairs(experts={E}, N={N}, K={K})")
 
 
 def moe_combine(y, place_of, wts, out, shared=None, gate=None, ids=None, real: int = 0, x=None) -> None:

@@ -241,6 +241,11 @@ class FeedForward(Part):
     def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
         raise NotImplementedError
 
+    def streamed(self, x: torch.Tensor) -> Optional[dict]:
+        """For few rows: the two products that ``forward`` is, {"up", "down", "inter", "form" (one of ``ops.MOE_SHARED_FORMS``), and its
+        "bias", "limit", "alpha"}, for a caller that runs them beside others of its own. None: ``forward`` alone."""
+        return None
+
 
 class Embedder(Part):
     """Turns the step's tokens into rows of the fp32 residual stream. ``table`` is the [vocab, hidden] matrix that a

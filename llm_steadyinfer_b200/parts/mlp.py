@@ -57,6 +57,11 @@ class GatedMLP(FeedForward):
             return ("gemm_f32", "swiglu")
         return ("gemm_skinny", "swiglu", "gemm_tc05", "gemm_rows")
 
+    def streamed(self, x):
+        if self.group != INTERLEAVE or self.dtype != torch.bfloat16 or not linear_mod.USE_SKINNY:
+            return None
+        return {"up": self.gate_up, "down": self.down, "inter": self.inter, "form": "silu_glu"}
+
     def forward(self, x, ctx, resid=None):
         T = x.shape[0]
         act = ctx.buf("ffn_act", (T, self.inter), self.dtype)
@@ -113,6 +118,11 @@ class DenseMLP(FeedForward):
 
     def kernel_files(self, page_size):
         return ("gemm_f32", "activation") if self.dtype == torch.float32 else ("gemm_skinny", "gemm_tc05", "gemm_rows", "activation")
+
+    def streamed(self, x):
+        if self.activation != "relu2" or self.dtype != torch.bfloat16 or not linear_mod.USE_SKINNY:
+            return None
+        return {"up": self.up, "down": self.down, "inter": self.inter, "form": "relu2"}
 
     def forward(self, x, ctx):
         T = x.shape[0]
@@ -195,6 +205,12 @@ class LimitedGatedMLP(FeedForward):
     def kernel_files(self, page_size):
         return ("gemm_f32", "swiglu", "activation") if self.dtype == torch.float32 else \
             ("gemm_skinny", "swiglu", "activation", "gemm_tc05", "gemm_rows")
+
+    def streamed(self, x):
+        if self.group != INTERLEAVE or self.dtype != torch.bfloat16 or not linear_mod.USE_SKINNY or self.output_bias is not None:
+            return None
+        return {"up": self.gate_up, "down": self.down, "inter": self.inter, "form": "glu_limited", "bias": self.gate_up_bias, "limit": self.limit,
+                "alpha": self.alpha}
 
     def forward(self, x, ctx, add_bias=True):
         T = x.shape[0]

@@ -25,7 +25,8 @@ On the device, with nothing read back: ``moe_route`` (scores, choice, weights, t
 by expert), two grouped products over the ordered places (the first reads its rows through the order and applies the
 activation in its epilogue; true 32-bit in float32; in bfloat16 on the tensor cores: mma.sync tiles for few places, and
 from 128 places on the TMA-fed tcgen05 grouped kernel behind a gather of the rows), ``moe_combine`` (weighted sum in each
-row's own order of choices, in fp32, the shared expert included). Within a kernel a row's result does not depend on what
+row's own order of choices, in fp32, the shared expert included). Steps of few pairs make no plan, and their two products take the shared
+expert's beside them in one launch each, where its form is one that kernel knows. Within a kernel a row's result does not depend on what
 else is in the batch: places only decide where a row lies in a tile, never the order of its sums; which kernel runs
 depends on the number of places, as for every product of the package, and changes the rounding of bfloat16 sums only.
 
@@ -128,6 +129,20 @@ class RoutedMLP(FeedForward):
     def kernel_files(self, page_size):
         return ("moe",) + (("gemm_tc05",) if self.dtype == torch.bfloat16 else ()) + (self.shared.kernel_files(page_size) if self.shared is not None else ())
 
+    def _shared_products(self, x, ctx):
+        """(first product, second product, result) of the shared expert as ``ops.moe_gemm_pairs`` takes them, or three times None."""
+        st = self.shared.streamed(x) if self.shared is not None else None
+        if st is None:
+            return None, None, None
+        T = x.shape[0]
+        act = ctx.buf("moe_shared_act", (T, st["inter"]), self.dtype)
+        out = ctx.buf("moe_shared", (T, self.hidden), self.dtype)
+        if not ops.gemm_skinny_ok(x, st["up"], act) or not ops.gemm_skinny_ok(act, st["down"], out):
+            return None, None, None
+        first = {"a": x, "w": st["up"], "out": act, "form": st["form"], "bias": st.get("bias"), "limit": st.get("limit", 0.0),
+                 "alpha": st.get("alpha", 1.0)}
+        return first, {"a": act, "w": st["down"], "out": out, "form": "none"}, out
+
     def forward(self, x, ctx):
         T = x.shape[0]
         E, top, P = self.E, self.top, x.shape[0] * self.top
@@ -139,10 +154,11 @@ class RoutedMLP(FeedForward):
                       choice_bias=self.choice_bias, renorm_eps=self.renorm_eps, groups=self.groups)
         act = ctx.buf("moe_act", (P, self.inter), self.dtype)
         y = ctx.buf("moe_y", (P, self.hidden), torch.float32)
-        place_of = None
+        place_of = shared = None
         if ops.moe_pairs_ok(x, self.w_up, self.w_down, T, top):  # few pairs: each its own place, no plan
-            ops.moe_gemm_pairs(x, ids, self.w_up, act, True, act=self.act, limit=self.limit, alpha=self.alpha, shift=self.shift)
-            ops.moe_gemm_pairs(act, ids, self.w_down, y, False)
+            first, second, shared = self._shared_products(x, ctx)         # the shared expert's products beside the chosen ones'
+            ops.moe_gemm_pairs(x, ids, self.w_up, act, True, act=self.act, limit=self.limit, alpha=self.alpha, shift=self.shift, shared=first)
+            ops.moe_gemm_pairs(act, ids, self.w_down, y, False, shared=second)
         else:
             scratch = ctx.buf("moe_plan", (ops.moe_plan_ints(P, R),), torch.int32)
             offsets = ctx.buf("moe_offsets", (R + 1,), torch.int32)
@@ -154,7 +170,8 @@ class RoutedMLP(FeedForward):
             ops.moe_gemm(x, row_of, self.w_up, act, offsets, act=self.act, gathered=gathered, status=ctx.status,
                          limit=self.limit, alpha=self.alpha, shift=self.shift)
             ops.moe_gemm(act, None, self.w_down, y, offsets, status=ctx.status)
-        shared = self.shared.forward(x, ctx) if self.shared is not None else None
+        if self.shared is not None and shared is None:
+            shared = self.shared.forward(x, ctx)
         out = ctx.buf("moe_out", (T, self.hidden), self.dtype)
         ops.moe_combine(y, place_of, wts, out, shared=shared, gate=gates[:, 0] if gates is not None else None,
                         ids=ids if self.identity else None, real=E, x=x if self.identity else None)

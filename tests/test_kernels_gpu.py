@@ -1306,6 +1306,37 @@ def test_experts_weights_streamed_for_few_places(T, top, E, N, K, act):
         assert torch.equal(planned[place_of.view(-1)[p]], out[p])
 
 
+@pytest.mark.parametrize("form", ["none", "relu2", "silu_glu", "glu_limited"])
+@pytest.mark.parametrize("T,top,N,K,sN,sK", [(1, 1, 16, 8, 16, 8), (3, 2, 40, 264, 304, 520), (9, 2, 64, 520, 16, 2056), (16, 2, 48, 264, 1008, 264)])
+def test_shared_product_beside_the_experts(T, top, N, K, sN, sK, form):
+    """The shared matrix's blocks in the experts' launch, from fewer column tiles than the experts have to many more: the experts' results to
+    the bit what they are alone, the shared ones what the few-row product gives (its warps may be four: sums in another order, so a sum may
+    round to the neighbouring bf16 number, 2^-8, which the square of relu doubles and the last rounding adds to)."""
+    g = torch.Generator().manual_seed(T + sN)
+    o, E = ops(), 4
+    rand = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).to(DEV)                      # noqa: E731
+    a, w = rand(T, K), rand(E, N, K) / K ** 0.5
+    sa, sw = rand(T, sK), rand(sN, sK) / sK ** 0.5
+    ids = torch.stack([torch.randperm(E + 1, generator=g)[:top] for _ in range(T)]).int().to(DEV)
+    glu = form in ("silu_glu", "glu_limited")
+    alone, out = (torch.full((T * top, N), 7.0, device=DEV) for _ in range(2))
+    want, got = (torch.full((T, sN // 2 if glu else sN), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    bias = torch.randn(sN, generator=g).to(DEV) if form == "glu_limited" else None
+    o.moe_gemm_pairs(a, ids, w, alone, True)
+    o.moe_gemm_pairs(a, ids, w, out, True, shared={"a": sa, "w": sw, "out": got, "form": form, "bias": bias, "limit": 0.9, "alpha": 1.7})
+    assert torch.equal(alone, out)
+    if form == "none":
+        o.gemm_skinny(sa, sw, want)
+    elif form == "relu2":
+        o.gemm_skinny_relu2(sa, sw, want)
+    elif form == "silu_glu":
+        o.gemm_skinny_swiglu(sa, sw, want)
+    else:
+        o.gemm_skinny_glu_limited(sa, sw, bias, want, 0.9, 1.7)
+    d = (got.double() - want.double()).abs()
+    assert bool((d <= 2 ** -6 * want.double().abs() + 2 ** -7).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 48, 8), (3, 40, 264), (8, 96, 1408), (9, 64, 1416), (16, 128, 2816), (8, 64, 5632), (2, 5000, 768)])
 def test_few_row_product_at_ragged_k(M, N, K):
     """The few-row product where k fills no whole round of a block's loads, against float64 (fp32 sums of K products)."""
