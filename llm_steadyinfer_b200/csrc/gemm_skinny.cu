@@ -9,7 +9,7 @@
 //   x[g][k .. k+8). The sum over k does not care in which order k is visited, so the 8
 //   consecutive k of a lane are fed as logical columns (2t, 2t+1, 2t+8, 2t+9) of two mma steps,
 //   the same mapping for A and B.
-// A block owns 16 output columns; its warps take the 32-wide k chunks in turn (adjacent warps
+// A tile is 16 output columns; a block's warps take the 32-wide k chunks in turn (adjacent warps
 // read adjacent 64 bytes of a row) and their partial sums are added in a fixed order.
 //
 // With SWIGLU the product is the stacked gate/up projection with gates and ups interleaved in
@@ -62,7 +62,7 @@ template <typename TO> __device__ __forceinline__ void store_out(TO* p, float v)
 template <> __device__ __forceinline__ void store_out<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void store_out<bf16>(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 
-__device__ __forceinline__ uint4 ld_stream(const bf16* p) {      // weights: read once, keep out of L1
+__device__ __forceinline__ uint4 ld_stream_nc(const bf16* p) {      // weights: read once, keep out of L1
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -73,141 +73,39 @@ __device__ __forceinline__ uint4 ld_cached(const bf16* p) {      // x: small, sh
   asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
+// Loads without a branch: what is not taken becomes zeros. Weights are read once and kept out of L1; not by the read-only path, whose loads the assembler
+// moves behind the wait for the kernel before where a loop around them uses the registers again (2,048 x 2,048, one row: 3.7 us so, 2.2 as it is).
+__device__ __forceinline__ uint4 ld_stream_if(const bf16* p, bool take) {
+  uint4 v;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+               "@q ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}\n"
+               : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((int)take) : "memory");
+  return v;
+}
+// x: small, shared by every block; written by the kernel before: not by the read-only path
+__device__ __forceinline__ uint4 ld_cached_if(const bf16* p, bool take) {
+  uint4 v;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+               "@q ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}\n"
+               : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((int)take) : "memory");
+  return v;
+}
 
-// Rows of W or x beyond N or M are replaced by row 0: their products land in output elements
-// that are never stored, so the loads need no predicate.
-template <int MT, int WARPS, int UNROLL, typename TO, bool SWIGLU = false, bool ROPE = false>
-__global__ void __launch_bounds__(WARPS * 32, 512 / (WARPS * 32))
-gemm_skinny_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ W, long long ldw,
-                   TO* __restrict__ out, long long ldo, int M, int N, int K, int trigger, const SkinnyRope rope,
-                   long long batch_x, long long batch_w, long long batch_o) {
-  __shared__ float red[WARPS][MT][32][4];
-  if (trigger == 1) pdl_trigger();
-  x += blockIdx.y * batch_x;                    // a batch of products of one shape: blockIdx.y names the product
-  W += blockIdx.y * batch_w;
-  out += blockIdx.y * batch_o;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  // the block's 16 rows of W: n0 .. n0+7 and n1 .. n1+7 (next to each other, or a rotation's two halves)
-  const int per_head = ROPE ? rope.hs / 16 : 1;
-  const int n0 = ROPE ? (blockIdx.x / per_head) * rope.hs + (blockIdx.x % per_head) * 8 : blockIdx.x * 16;
-  const int n1 = ROPE ? n0 + rope.hs / 2 : n0 + 8;
-  const bf16* w0 = W + (size_t)(n0 + g < N ? n0 + g : 0) * ldw + t * 8;
-  const bf16* w1 = W + (size_t)(n1 + g < N ? n1 + g : 0) * ldw + t * 8;
-  float acc[MT][4];
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
-
-  const int full = K >> 5, nchunks = (K + 31) >> 5;      // whole 32-wide chunks; with the part of one (K is a multiple of 8)
-  const bf16* xr[MT];
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt) xr[mt] = x + (size_t)(mt * 8 + g < M ? mt * 8 + g : 0) * ldx + t * 8;
-  // Chunks of a warp go in rounds with all their loads in flight: UNROLL whole ones, then four whole ones, then up to four of which a round
-  // that is not whole loads only what is there: lanes past the end feed zeros, and every lane of the warp issues the same mma
-  // (mma.sync must not sit in a divergent branch). A launch behind a launch, against single chunks behind the rounds of UNROLL (which the
-  // compiler takes four at a time), two rows of 2,048 columns: K = 704 2.6 us before, 2.1 so; 1,408 3.2 and 2.6; 2,816 4.9 and 3.4;
-  // 5,632 7.0 and 5.8. 16 rows: 704 3.1 and 3.0, 2,816 6.0 and 5.6. 28,672 columns, K = 4,096: 34.5 and 34.6 us, 16 rows 46.3 and 46.2.
-  // The weights do not depend on the kernel before this one: the first round of their loads is in flight
-  // before this kernel waits for that kernel's results (x).
-  auto round = [&](int c, auto chunks, auto all, bool first) {
-    constexpr int U = decltype(chunks)::value;
-    constexpr bool ALL = decltype(all)::value;
-    uint4 a_lo[U], a_hi[U], xb[U][MT];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = (c + u * WARPS) * 32;
-      if (!ALL) a_lo[u] = a_hi[u] = make_uint4(0, 0, 0, 0);
-      if (ALL || k + t * 8 < K) {
-        a_lo[u] = ld_stream(w0 + k);
-        a_hi[u] = ld_stream(w1 + k);
-      }
-    }
-    if (first) pdl_wait();
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = (c + u * WARPS) * 32;
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        if (!ALL) xb[u][mt] = make_uint4(0, 0, 0, 0);
-        if (ALL || k + t * 8 < K) xb[u][mt] = ld_cached(xr[mt] + k);
-      }
-    }
-    if (!ALL) __syncwarp();
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (ALL || c + u * WARPS < nchunks) {
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          mma16816(acc[mt], a_lo[u].x, a_hi[u].x, a_lo[u].y, a_hi[u].y, xb[u][mt].x, xb[u][mt].y);
-          mma16816(acc[mt], a_lo[u].z, a_hi[u].z, a_lo[u].w, a_hi[u].w, xb[u][mt].z, xb[u][mt].w);
-        }
-      }
-  };
-  int c = warp;
-  if constexpr (MT == 1) {
-    // one copy of each kind of round, the wait behind a branch; a copy of its own for the only round where blocks are very many
-    bool first = true;
-    if (c + (2 * UNROLL - 1) * WARPS < full || gridDim.x < 4096) {
-#pragma unroll 1
-      for (; c + (UNROLL - 1) * WARPS < full; c += WARPS * UNROLL) {
-        round(c, int_c<UNROLL>(), int_c<true>(), first);
-        first = false;
-      }
-    } else if (c + (UNROLL - 1) * WARPS < full) {
-      round(c, int_c<UNROLL>(), int_c<true>(), true);
-      first = false;
-      c += WARPS * UNROLL;
-    }
-    if (trigger == 2) pdl_trigger();
-    if (c + 3 * WARPS < full) {
-      round(c, int_c<4>(), int_c<true>(), first);
-      first = false;
-      c += WARPS * 4;
-    }
-    if (c < nchunks) {                                       // at most three whole ones and the part of one
-      round(c, int_c<4>(), int_c<false>(), first);
-      first = false;
-    }
-    if (first) pdl_wait();                                   // a warp without any chunk waits like the others
-  } else {
-    // the loads of two row tiles fill the registers: rounds that cannot be the first ones without the branch
-    if (c + (UNROLL - 1) * WARPS < full) {
-      round(c, int_c<UNROLL>(), int_c<true>(), true);
-      c += WARPS * UNROLL;
-#pragma unroll 1
-      for (; c + (UNROLL - 1) * WARPS < full; c += WARPS * UNROLL) round(c, int_c<UNROLL>(), int_c<true>(), false);
-      if (trigger == 2) pdl_trigger();
-      if (c + 3 * WARPS < full) {
-        round(c, int_c<4>(), int_c<true>(), false);
-        c += WARPS * 4;
-      }
-      if (c < nchunks) round(c, int_c<4>(), int_c<false>(), false);      // at most three whole ones and the part of one
-    } else if (c + 3 * WARPS < full) {
-      round(c, int_c<4>(), int_c<true>(), true);
-      c += WARPS * 4;
-      if (trigger == 2) pdl_trigger();
-      if (c < nchunks) round(c, int_c<4>(), int_c<false>(), false);
-    } else {
-      round(c, int_c<4>(), int_c<false>(), true);      // (also where a warp has no chunk at all: it waits like the others)
-      if (trigger == 2) pdl_trigger();
-    }
-  }
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) red[warp][mt][lane][e] = acc[mt][e];
-  __syncthreads();
+// A tile's sums of the warps, [WARPS][MT][32] fragments, added in warp order, and what the product's form does with them.
+template <int MT, int WARPS, typename TO, bool SWIGLU, bool ROPE>
+__device__ __forceinline__ void skinny_store(const float (*red)[4], int tile, int n0, int per_head, TO* __restrict__ out, long long ldo, int M, int N,
+                                             const SkinnyRope& rope) {
   if constexpr (ROPE) {
     // threads (mt, lane, e) add the partial sums of the two elements of one rotation pair of one row
-    const int head = blockIdx.x / per_head, half = rope.hs / 2;
+    const int head = tile / per_head, half = rope.hs / 2;
     for (int idx = threadIdx.x; idx < MT * 32 * 2; idx += WARPS * 32) {
       const int mt = idx / 64, ln = (idx >> 1) & 31, e = idx & 1;
       float a = 0.f, b = 0.f;
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w) { a += red[w][mt][ln][e]; b += red[w][mt][ln][e + 2]; }
+      for (int w = 0; w < WARPS; ++w) { a += red[(w * MT + mt) * 32 + ln][e]; b += red[(w * MT + mt) * 32 + ln][e + 2]; }
       const int m = mt * 8 + (ln & 3) * 2 + e;
       if (m >= M) continue;
-      const int i = (blockIdx.x % per_head) * 8 + (ln >> 2);       // index in the head's first half
+      const int i = (tile % per_head) * 8 + (ln >> 2);       // index in the head's first half
       const float x0 = __bfloat162float(__float2bfloat16_rn(a)), x1 = __bfloat162float(__float2bfloat16_rn(b));
       float y0 = x0, y1 = x1;
       const int pos = rope.positions[m];
@@ -242,13 +140,13 @@ gemm_skinny_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __rest
       const int mt = idx / 64, ln = (idx >> 1) & 31, e = idx & 1;
       float gs = 0.f, us = 0.f;
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w) { gs += red[w][mt][ln][e]; us += red[w][mt][ln][e + 2]; }
-      const int f = blockIdx.x * 8 + (ln >> 2);
+      for (int w = 0; w < WARPS; ++w) { gs += red[(w * MT + mt) * 32 + ln][e]; us += red[(w * MT + mt) * 32 + ln][e + 2]; }
+      const int f = tile * 8 + (ln >> 2);
       const int m = mt * 8 + (ln & 3) * 2 + e;
       if (2 * f < N && m < M) {
         float gv = __bfloat162float(__float2bfloat16_rn(gs)), uv = __bfloat162float(__float2bfloat16_rn(us));
         if (rope.glu) {
-          const int gc = blockIdx.x * 16 + (ln >> 2);             // the gate's place among the stacked columns; its up: 8 on
+          const int gc = tile * 16 + (ln >> 2);             // the gate's place among the stacked columns; its up: 8 on
           if (rope.glu_bias) { gv += rope.glu_bias[gc]; uv += rope.glu_bias[gc + 8]; }
           gv = fminf(gv, rope.glu_limit);
           uv = fminf(fmaxf(uv, -rope.glu_limit), rope.glu_limit);
@@ -264,7 +162,7 @@ gemm_skinny_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __rest
       const int mt = idx / 128, ln = (idx >> 2) & 31, e = idx & 3;
       float s = 0.f;
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w) s += red[w][mt][ln][e];
+      for (int w = 0; w < WARPS; ++w) s += red[(w * MT + mt) * 32 + ln][e];
       const int n = n0 + (ln >> 2) + ((e >> 1) ? 8 : 0);
       const int m = mt * 8 + (ln & 3) * 2 + (e & 1);
       if (rope.act == 1) {
@@ -282,31 +180,214 @@ gemm_skinny_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __rest
   }
 }
 
-// Eight warps a block (two blocks an SM) unless the blocks would then make more than one round but no more than
-// two: with four warps a block, four blocks fit an SM and all of them run at once, sharing the memory bandwidth,
-// instead of a full round followed by a part of one.
-static inline bool skinny_four_warps(unsigned blocks) {
-  const unsigned sms = (unsigned)si_sm_count();
-  return blocks > 2 * sms && blocks <= 4 * sms;
+// A block takes tiles of 16 columns, WARPS warps the 32-wide chunks of k in turn, U chunks of a warp at once with both operands. The rounds of
+// a block's tiles follow one another: the next round's loads, of this tile or the next, are asked for as soon as the operands are used, and
+// are on their way while the warps' sums are added and stored. Rows of W beyond N stand for row 0 (never stored); x beyond M and what is
+// beyond K are zeros; no load sits behind a branch, as mma.sync must not. The weights do not depend on the kernel before this one: the
+// first round of their loads is in flight before this kernel waits for that kernel's results (x).
+template <int MT, int WARPS, int U, typename TO, bool SWIGLU = false, bool ROPE = false>
+__global__ void __launch_bounds__(WARPS * 32, 512 / (WARPS * 32))
+gemm_skinny_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ W, long long ldw,
+                   TO* __restrict__ out, long long ldo, int M, int N, int K, int tiles, int trigger, const SkinnyRope rope,
+                   long long batch_x, long long batch_w, long long batch_o) {
+  __shared__ float red[2][WARPS * MT * 32][4];
+  if (trigger) pdl_trigger();
+  x += blockIdx.y * batch_x;                    // a batch of products of one shape: blockIdx.y names the product
+  W += blockIdx.y * batch_w;
+  out += blockIdx.y * batch_o;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int per_head = ROPE ? rope.hs / 16 : 1;
+  // a tile's 16 rows of W: n0 .. n0+7 and n1 .. n1+7 (next to each other, or a rotation's two halves)
+  auto first_row = [&](int tile) { return ROPE ? (tile / per_head) * rope.hs + (tile % per_head) * 8 : tile * 16; };
+  const int rounds = (K + 32 * WARPS * U - 1) / (32 * WARPS * U);
+  int tile = blockIdx.x, r = 0;                 // whose loads were asked for last
+  uint4 lo[U], hi[U], xb[U][MT];
+  auto load_w = [&]() {
+    const int n0 = first_row(tile), n1 = ROPE ? n0 + rope.hs / 2 : n0 + 8;
+    const bf16* w0 = W + (size_t)(n0 + g < N ? n0 + g : 0) * ldw;
+    const bf16* w1 = W + (size_t)(n1 + g < N ? n1 + g : 0) * ldw;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (warp + (r * U + u) * WARPS) * 32 + t * 8;
+      lo[u] = ld_stream_if(w0 + k, k < K);
+      hi[u] = ld_stream_if(w1 + k, k < K);
+    }
+  };
+  auto load_x = [&]() {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const bool in = mt * 8 + g < M;
+      const bf16* xr = x + (size_t)(in ? mt * 8 + g : 0) * ldx;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = (warp + (r * U + u) * WARPS) * 32 + t * 8;
+        xb[u][mt] = ld_cached_if(xr + k, in && k < K);
+      }
+    }
+  };
+  load_w();
+  pdl_wait();
+  load_x();
+  for (int par = 0; tile < tiles; par ^= 1) {
+    const int now = tile;
+    float acc[MT][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
+#pragma unroll 1
+    for (int round = 0; round < rounds; ++round) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          mma16816(acc[mt], lo[u].x, hi[u].x, lo[u].y, hi[u].y, xb[u][mt].x, xb[u][mt].y);
+          mma16816(acc[mt], lo[u].z, hi[u].z, lo[u].w, hi[u].w, xb[u][mt].z, xb[u][mt].w);
+        }
+      if (++r == rounds) { r = 0; tile += gridDim.x; }
+      if (tile < tiles) { load_w(); load_x(); }
+    }
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+      *reinterpret_cast<float4*>(red[par][(warp * MT + mt) * 32 + lane]) = make_float4(acc[mt][0], acc[mt][1], acc[mt][2], acc[mt][3]);
+    __syncthreads();
+    skinny_store<MT, WARPS, TO, SWIGLU, ROPE>(red[par], now, first_row(now), per_head, out, ldo, M, N, rope);
+  }
 }
 
-template <int WARPS, typename TO, bool SWIGLU, bool ROPE>
-static void skinny_launch(unsigned blocks, cudaStream_t stream, const bf16* xp, long long ldx, const bf16* wp, long long ldw,
-                          TO* out, long long ldo, int M, int N, int K, const SkinnyRope& r, int batch = 1, long long bx = 0,
-                          long long bw = 0, long long bo = 0) {
-  constexpr int UNROLL = 8;
-  const int trig = si_pdl_trigger_mode(blocks * batch, (512 / (WARPS * 32)) * si_sm_count());
-  const dim3 grid(blocks, batch);
-  if (M <= 8) si_launch(gemm_skinny_kernel<1, WARPS, UNROLL, TO, SWIGLU, ROPE>, grid, dim3(WARPS * 32), 0, stream, xp, ldx, wp, ldw, out, ldo, M, N, K, trig, r, bx, bw, bo);
-  else si_launch(gemm_skinny_kernel<2, WARPS, UNROLL, TO, SWIGLU, ROPE>, grid, dim3(WARPS * 32), 0, stream, xp, ldx, wp, ldw, out, ldo, M, N, K, trig, r, bx, bw, bo);
+// At most eight rows, a block a tile.
+// Rows of W or x beyond N or M are replaced by row 0: their products land in output elements
+// that are never stored, so the loads need no predicate.
+template <int WARPS, typename TO, bool SWIGLU = false, bool ROPE = false>
+__global__ void __launch_bounds__(WARPS * 32, 512 / (WARPS * 32))
+gemm_skinny_once_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ W, long long ldw,
+                   TO* __restrict__ out, long long ldo, int M, int N, int K, int trigger, const SkinnyRope rope,
+                   long long batch_x, long long batch_w, long long batch_o) {
+  constexpr int MT = 1, UNROLL = 8;
+  __shared__ float red[WARPS * 32][4];
+  if (trigger) pdl_trigger();
+  x += blockIdx.y * batch_x;                    // a batch of products of one shape: blockIdx.y names the product
+  W += blockIdx.y * batch_w;
+  out += blockIdx.y * batch_o;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  // the block's 16 rows of W: n0 .. n0+7 and n1 .. n1+7 (next to each other, or a rotation's two halves)
+  const int per_head = ROPE ? rope.hs / 16 : 1;
+  const int n0 = ROPE ? (blockIdx.x / per_head) * rope.hs + (blockIdx.x % per_head) * 8 : blockIdx.x * 16;
+  const int n1 = ROPE ? n0 + rope.hs / 2 : n0 + 8;
+  const bf16* w0 = W + (size_t)(n0 + g < N ? n0 + g : 0) * ldw + t * 8;
+  const bf16* w1 = W + (size_t)(n1 + g < N ? n1 + g : 0) * ldw + t * 8;
+  float acc[MT][4];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
+
+  const int full = K >> 5, nchunks = (K + 31) >> 5;      // whole 32-wide chunks; with the part of one (K is a multiple of 8)
+  const bf16* xr[MT];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) xr[mt] = x + (size_t)(mt * 8 + g < M ? mt * 8 + g : 0) * ldx + t * 8;
+  // Chunks of a warp go in rounds with all their loads in flight: UNROLL whole ones, then four whole ones, then up to four of which a round
+  // that is not whole loads only what is there: lanes past the end feed zeros, and every lane of the warp issues the same mma
+  // (mma.sync must not sit in a divergent branch). A launch behind a launch, against single chunks behind the rounds of UNROLL (which the
+  // compiler takes four at a time), two rows of 2,048 columns: K = 704 2.6 us before, 2.1 so; 1,408 3.2 and 2.6. 28,672 columns, K = 4,096:
+  // 34.5 and 34.6 us.
+  // The weights do not depend on the kernel before this one: the first round of their loads is in flight
+  // before this kernel waits for that kernel's results (x).
+  auto round = [&](int c, auto chunks, auto all, bool first) {
+    constexpr int U = decltype(chunks)::value;
+    constexpr bool ALL = decltype(all)::value;
+    uint4 a_lo[U], a_hi[U], xb[U][MT];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (c + u * WARPS) * 32;
+      if (!ALL) a_lo[u] = a_hi[u] = make_uint4(0, 0, 0, 0);
+      if (ALL || k + t * 8 < K) {
+        a_lo[u] = ld_stream_nc(w0 + k);
+        a_hi[u] = ld_stream_nc(w1 + k);
+      }
+    }
+    if (first) pdl_wait();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = (c + u * WARPS) * 32;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        if (!ALL) xb[u][mt] = make_uint4(0, 0, 0, 0);
+        if (ALL || k + t * 8 < K) xb[u][mt] = ld_cached(xr[mt] + k);
+      }
+    }
+    if (!ALL) __syncwarp();
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (ALL || c + u * WARPS < nchunks) {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          mma16816(acc[mt], a_lo[u].x, a_hi[u].x, a_lo[u].y, a_hi[u].y, xb[u][mt].x, xb[u][mt].y);
+          mma16816(acc[mt], a_lo[u].z, a_hi[u].z, a_lo[u].w, a_hi[u].w, xb[u][mt].z, xb[u][mt].w);
+        }
+      }
+  };
+  int c = warp;
+  // one copy of each kind of round, the wait behind a branch
+  bool first = true;
+#pragma unroll 1
+  for (; c + (UNROLL - 1) * WARPS < full; c += WARPS * UNROLL) {
+    round(c, int_c<UNROLL>(), int_c<true>(), first);
+    first = false;
+  }
+  if (c + 3 * WARPS < full) {
+    round(c, int_c<4>(), int_c<true>(), first);
+    first = false;
+    c += WARPS * 4;
+  }
+  if (c < nchunks) {                                       // at most three whole ones and the part of one
+    round(c, int_c<4>(), int_c<false>(), first);
+    first = false;
+  }
+  if (first) pdl_wait();                                   // a warp without any chunk waits like the others
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) red[warp * 32 + lane][e] = acc[mt][e];
+  __syncthreads();
+  skinny_store<1, WARPS, TO, SWIGLU, ROPE>(red, blockIdx.x, n0, per_head, out, ldo, M, N, rope);
 }
 
+// Which kernel, and how many warps a block. In us, one and eight rows, a launch behind a launch:
+// * no more tiles than SMs and K above 2,048 (more than one round of eight warps): sixteen warps share a tile's chunks. 2,048 x 5,632: a block
+//   of eight, round by round, 6.8 and 7.4; so 5.3 and 5.7. At one round sixteen have nothing to share.
+// * more tiles than four blocks an SM and K up to 2,048: as many blocks as run at once go through the tiles. 11,264 x 2,048: a block a tile 9.4 and
+//   9.8, so 8.1 and 8.6; 32,000 x 2,048: 21.1 and 22.1, so 20.1 and 21.3. With more rounds a tile, blocks that start anew keep more loads in
+//   flight beside what runs before and behind: a step of the 8B shape (28,672 x 4,096) 25.4 ms for eight, with tiles in turn 25.8.
+// * more tiles than two blocks an SM but no more than four: four warps a block, so that all run at once, sharing the memory
+//   bandwidth, instead of a full round followed by a part of one.
+// * else a block of eight warps a tile.
+// Nine to sixteen rows take the first kernel always (2,048 x 2,048 4.5 -> 3.9 us, 11,264 x 2,048 12.3 -> 10.8, 4,096 x 14,336 23.2 -> 22.6,
+// 28,672 x 4,096 48.2 -> 43.7 against a block a tile, whose loads of two row tiles took all registers).
 template <typename TO, bool SWIGLU, bool ROPE>
-static void skinny_dispatch(unsigned blocks, cudaStream_t stream, const bf16* xp, long long ldx, const bf16* wp, long long ldw,
+static void skinny_dispatch(unsigned tiles, cudaStream_t stream, const bf16* xp, long long ldx, const bf16* wp, long long ldw,
                             TO* out, long long ldo, int M, int N, int K, const SkinnyRope& r, int batch = 1, long long bx = 0,
                             long long bw = 0, long long bo = 0) {
-  if (skinny_four_warps(blocks * batch)) skinny_launch<4, TO, SWIGLU, ROPE>(blocks, stream, xp, ldx, wp, ldw, out, ldo, M, N, K, r, batch, bx, bw, bo);
-  else skinny_launch<8, TO, SWIGLU, ROPE>(blocks, stream, xp, ldx, wp, ldw, out, ldo, M, N, K, r, batch, bx, bw, bo);
+  const long long sms = si_sm_count(), all = (long long)tiles * batch;
+  const bool one_round = K <= 8 * 8 * 32;
+  const int warps = all <= sms && !one_round ? 16 : all > 2 * sms && all <= 4 * sms ? 4 : 8;
+  const long long slots = 512 / (warps * 32) * sms;
+  const bool in_turn = batch == 1 && all > slots && (one_round || M > 8);
+  const dim3 grid((unsigned)(in_turn ? slots : tiles), batch), block(warps * 32);
+  const int trig = si_pdl_trigger_mode((long long)grid.x * batch, slots) == 1;
+#define SK_TILES(MT, WARPS, U) si_launch(gemm_skinny_kernel<MT, WARPS, U, TO, SWIGLU, ROPE>, grid, block, 0, stream, xp, ldx, wp, ldw, out, ldo, M, N, K, (int)tiles, trig, r, bx, bw, bo)
+#define SK_ONCE(WARPS) si_launch(gemm_skinny_once_kernel<WARPS, TO, SWIGLU, ROPE>, grid, block, 0, stream, xp, ldx, wp, ldw, out, ldo, M, N, K, trig, r, bx, bw, bo)
+  if (M > 8) {
+    if (warps == 16) SK_TILES(2, 16, 4); else if (warps == 4) SK_TILES(2, 4, 4); else SK_TILES(2, 8, 4);
+  } else if (warps == 16) {
+    SK_TILES(1, 16, 8);
+  } else if (in_turn) {
+    SK_TILES(1, 8, 8);
+  } else if (warps == 4) {
+    SK_ONCE(4);
+  } else {
+    SK_ONCE(8);
+  }
+#undef SK_ONCE
+#undef SK_TILES
 }
 
 // Largest M this kernel takes.

@@ -1337,7 +1337,9 @@ def test_shared_product_beside_the_experts(T, top, N, K, sN, sK, form):
     assert bool((d <= 2 ** -6 * want.double().abs() + 2 ** -7).all())
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 48, 8), (3, 40, 264), (8, 96, 1408), (9, 64, 1416), (16, 128, 2816), (8, 64, 5632), (2, 5000, 768)])
+@pytest.mark.parametrize("M,N,K", [(1, 48, 8), (3, 40, 264), (8, 96, 1408), (9, 64, 1416), (16, 128, 2816), (8, 64, 5632), (2, 5000, 768),
+                                   (1, 9480, 8), (5, 9490, 2040), (8, 14300, 264), (9, 9490, 2056), (16, 5000, 72),      # tiles in turn
+                                   (2, 40, 2056), (8, 2368, 2088), (12, 2360, 4104), (1, 2376, 2056)])                  # sixteen warps a tile, and one tile too many
 def test_few_row_product_at_ragged_k(M, N, K):
     """The few-row product where k fills no whole round of a block's loads, against float64 (fp32 sums of K products)."""
     g = torch.Generator().manual_seed(K + M)
