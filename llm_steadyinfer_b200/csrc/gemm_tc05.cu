@@ -315,11 +315,12 @@ gemm_tc05_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
 // Barriers: full[s] (leader: one arrival with the bytes of all four boxes), empty[s] (each CTA: the commit
 // after the stage's instructions), acc_full[b] (each CTA: the commit after a tile's last instruction),
 // acc_empty[b] (leader: the eight epilogue warps of both CTAs).
-template <int STAGES, typename TO, int EPI>
+template <int STAGES, typename TO, int EPI, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192)
 gemm_tc05_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap,
                       TO* __restrict__ out, long long ldo, int M, int N, int K, int* status, const EpiArgs epi) {
-  constexpr int BM = 128, BN = 256, BK = 64;             // BM, and BN / 2 rows of W, per CTA
+  constexpr int BM = 128, BK = 64;                       // BM, and BN / 2 rows of W, per CTA
+  constexpr int CW = BN < 128 ? BN : 128;                // columns that an epilogue thread holds at once
   constexpr int A_BYTES = BM * BK * 2, B_BYTES = (BN / 2) * BK * 2;
   extern __shared__ unsigned char smem_dyn[];
   __shared__ __align__(8) uint64_t full_bar[STAGES];
@@ -431,19 +432,19 @@ gemm_tc05_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_con
       const int row = m0 + q * 32 + lane;
       const unsigned src = tmem + ((unsigned)(q * 32) << 16) + (unsigned)(buf * BN);
 #pragma unroll 1
-      for (int h = 0; h < BN / 128; ++h) {
-        float v[4][32];
+      for (int h = 0; h < BN / CW; ++h) {
+        float v[CW / 32][32];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld_32x32_issue(src + h * 128 + c * 32, v[c]);
+        for (int c = 0; c < CW / 32; ++c) tmem_ld_32x32_issue(src + h * CW + c * 32, v[c]);
         tmem_ld_wait();
-        if (h == BN / 128 - 1) {                // in registers: the leader's issuer may have the accumulator back
+        if (h == BN / CW - 1) {                // in registers: the leader's issuer may have the accumulator back
           tc05_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(cluster_map_u32(&acc_empty[buf], 0));
         }
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int n = n0 + h * 128 + c * 32;
+        for (int c = 0; c < CW / 32; ++c) {
+          const int n = n0 + h * CW + c * 32;
           if (row < M && n < N) {
             if (EPI == EPI_SWIGLU) store_swiglu16((bf16*)out + (size_t)row * ldo + n / 2, v[c], min(16, (N - n) / 2), vec);
             else if (EPI == EPI_GLU_LIMITED)
@@ -474,15 +475,31 @@ static bool pair_enabled() {
   return on == 1;
 }
 
-template <typename TO, int EPI>
+// Columns of a pair's tile: 256, or 128 or 64 where tiles of 256 leave most of the SMs idle. A tile then takes as long as its pair fetches
+// 128 rows of x and BN / 2 of W a CTA and k step, so the width with the fewest rows fetched in turn is taken, if it saves a fifth: a wider
+// tile costs less in all. Behind one another, us, tiles of 256 and as chosen here: PAIR_FIGURES
+static int pair_columns(int M, int N) {
+  const long long slots = si_sm_count() / 2, m_tiles = (M + 255) / 256;
+  if (m_tiles * ((N + 255) / 256) > slots) return 256;
+  long long least = 128 + 256 / 2;
+  int best = 256;
+  for (int bn = 128; bn >= 64; bn /= 2) {
+    const long long tiles = m_tiles * ((N + bn - 1) / bn), cost = (tiles + slots - 1) / slots * (128 + bn / 2);
+    if (cost < least && cost * 5 <= (128 + 256 / 2) * 4) { least = cost; best = bn; }
+  }
+  return best;
+}
+SI_EXPORT int si_gemm_tc05_columns(int M, int N) { return pair_columns(M, N); }
+
+template <typename TO, int EPI, int BN = 256>
 static int launch_pair(const CUtensorMap& am, const CUtensorMap& bm_half, void* out, long long ldo, int M, int N, int K,
                        int* status, cudaStream_t stream, EpiArgs epi = EpiArgs()) {
-  constexpr int STAGES = 6;
-  const size_t smem = (size_t)STAGES * (128 * 64 * 2 + 128 * 64 * 2) + 1024;
-  auto k = gemm_tc05_pair_kernel<STAGES, TO, EPI>;
+  constexpr int STAGES = BN == 256 ? 6 : BN == 128 ? 8 : 10;
+  const size_t smem = (size_t)STAGES * (128 * 64 * 2 + BN / 2 * 64 * 2) + 1024;
+  auto k = gemm_tc05_pair_kernel<STAGES, TO, EPI, BN>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  const int tiles = ((M + 255) / 256) * ((N + 255) / 256);
+  const int tiles = ((M + 255) / 256) * ((N + BN - 1) / BN);
   const int pairs = tiles < si_sm_count() / 2 ? tiles : si_sm_count() / 2;
   if (pairs < 1) return -2;
   si_launch(k, dim3(2 * pairs), dim3(192), smem, stream, am, bm_half, (TO*)out, ldo, M, N, K, status, epi);
@@ -506,9 +523,9 @@ static int launch(const CUtensorMap& am, const CUtensorMap& bm, void* out, long 
 SI_EXPORT int si_gemm_tc05_ok() { return si_encode_fn() != nullptr; }
 
 // The weight's tensor map (boxes of [256, 64]); made once per weight. `map_out`: 128 bytes, 64-byte aligned.
-// `box_rows`: 256 for the one-CTA kernel, 128 for the kernel of CTA pairs (each CTA fetches half of the tile's rows).
+// `box_rows`: 256 for the one-CTA kernel, half the columns of the tile for the kernel of CTA pairs (each CTA fetches half of them).
 SI_EXPORT int si_gemm_tc05_encode_weight(void* map_out, const void* W, int N, int K, long long ldw, int box_rows) {
-  if ((K % 8) || (ldw % 8) || ((uintptr_t)W % 16) || (box_rows != 128 && box_rows != 256)) return -2;
+  if ((K % 8) || (ldw % 8) || ((uintptr_t)W % 16) || (box_rows != 32 && box_rows != 64 && box_rows != 128 && box_rows != 256)) return -2;
   return si_encode_bf16_2d((CUtensorMap*)map_out, W, (unsigned long long)N, (unsigned long long)K,
                            (unsigned long long)ldw, (unsigned)box_rows);
 }
@@ -734,7 +751,7 @@ SI_EXPORT int si_gemm_tc05_grouped(const void* x, long long ldx, const void* wma
 }
 
 // out_dtype: SI_BF16 or SI_F32. x: [M, K] bf16 rows `ldx` apart. Returns -2 for unsupported sizes.
-// `wmap`: the weight's map with boxes of 256 rows; `wmap_half` (may be null): the one with boxes of 128 rows.
+// `wmap`: the weight's map with boxes of 256 rows; `wmap_half` (may be null): the one with boxes of si_gemm_tc05_columns(M, N) / 2 rows.
 SI_EXPORT int si_gemm_tc05(const void* x, long long ldx, const void* wmap, const void* wmap_half, void* out, long long ldo,
                            int out_dtype, int M, int N, int K, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
@@ -743,8 +760,13 @@ SI_EXPORT int si_gemm_tc05(const void* x, long long ldx, const void* wmap, const
   if (rc) return rc;
   if (use_pair(M, wmap_half)) {
     const CUtensorMap& bh = *(const CUtensorMap*)wmap_half;
-    if (out_dtype == SI_BF16) return launch_pair<bf16, EPI_STORE>(am, bh, out, ldo, M, N, K, status, stream);
-    return launch_pair<float, EPI_STORE>(am, bh, out, ldo, M, N, K, status, stream);
+    const int columns = pair_columns(M, N);
+#define TC05_PAIR(BN) return out_dtype == SI_BF16 ? launch_pair<bf16, EPI_STORE, BN>(am, bh, out, ldo, M, N, K, status, stream) \
+                                                  : launch_pair<float, EPI_STORE, BN>(am, bh, out, ldo, M, N, K, status, stream)
+    if (columns == 64) TC05_PAIR(64);
+    if (columns == 128) TC05_PAIR(128);
+    TC05_PAIR(256);
+#undef TC05_PAIR
   }
   const CUtensorMap& bm = *(const CUtensorMap*)wmap;
   if (out_dtype == SI_BF16) return launch<4, bf16, EPI_STORE>(am, bm, out, ldo, M, N, K, status, stream);

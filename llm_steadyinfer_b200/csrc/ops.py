@@ -841,7 +841,7 @@ def gemm_tc05_ok(a, w, out) -> bool:
 
 
 def _weight_map(w: torch.Tensor, box_rows: int = 256):
-    """The weight's TMA descriptor with boxes of ``box_rows`` rows (256: one CTA a tile; 128: a pair of CTAs)."""
+    """The weight's TMA descriptor with boxes of ``box_rows`` rows (256: one CTA a tile; half the tile's columns: a pair of CTAs)."""
     key = (w.device.index, w.data_ptr(), tuple(w.shape), w.stride(0), box_rows)
     ent = _weight_maps.get(key)
     if ent is None:
@@ -856,6 +856,14 @@ def _weight_map(w: torch.Tensor, box_rows: int = 256):
     return _c_p(ent[1])
 
 
+@_of_sizes
+def gemm_tc05_columns(M: int, N: int) -> int:
+    """Columns of the tile that a pair of CTAs takes of a product of M rows and N columns."""
+    lib = build.load("gemm_tc05")
+    lib.si_gemm_tc05_columns.restype = _c_int
+    return lib.si_gemm_tc05_columns(_c_int(M), _c_int(N))
+
+
 def gemm_tc05(a, w, out, status=None) -> None:
     """out[M,N] = a[M,K] @ w[N,K]^T on the tcgen05 tensor cores (TMA-fed, accumulators in tensor memory)."""
     _cuda(a, w, out, status)
@@ -865,7 +873,7 @@ def gemm_tc05(a, w, out, status=None) -> None:
     _need(gemm_tc05_ok(a, w, out), "gemm_tc05: bf16 inputs, K a multiple of 8, 16-byte aligned rows")
     f = _fn("gemm_tc05", "si_gemm_tc05",
             [_c_p, _c_ll, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_p, _c_p])
-    half = _weight_map(w, 128) if M > 128 else None          # more than one tile of rows: pairs of CTAs take tiles together
+    half = _weight_map(w, gemm_tc05_columns(M, N) // 2) if M > 128 else None     # more than one tile of rows: pairs of CTAs take tiles together
     _check(f(_ptr(a), a.stride(0), _weight_map(w), half, _ptr(out), out.stride(0), _dt(out), M, N, K, _ptr(status),
              _stream()), f"gemm_tc05(M={M}, N={N}, K={K})")
 

@@ -1337,6 +1337,23 @@ def test_shared_product_beside_the_experts(T, top, N, K, sN, sK, form):
     assert bool((d <= 2 ** -6 * want.double().abs() + 2 ** -7).all())
 
 
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K,columns", [(129, 8, 72, 64), (203, 2048, 2048, 64), (256, 200, 64, 64), (257, 2312, 1096, 64), (300, 2400, 8, 128),
+                                           (938, 2048, 136, 128), (513, 3000, 520, 128), (2048, 2048, 72, 256), (129, 9600, 200, 256)])
+def test_pairs_tiles_of_fewer_columns(M, N, K, columns, out_dtype):
+    """The pair kernel's tiles of 64, 128 and 256 columns, at remainders of rows, columns and k, against float64: K / 16 instructions that each
+    add to a sum of at most some 6 in 32 bits, rounding by up to 2^-23 of it, and where the result is bf16 its rounding (2^-8 of it)."""
+    g = torch.Generator().manual_seed(M + N)
+    x, w = torch.randn(M, K, generator=g).to(torch.bfloat16).to(DEV), (torch.randn(N, K, generator=g) / K ** 0.5).to(torch.bfloat16).to(DEV)
+    assert ops().gemm_tc05_columns(M, N) == columns
+    wide = torch.full((M, N + 8), 7.0, dtype=out_dtype, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops().gemm_tc05(x, w, wide[:, :N], status)
+    assert int(status) == 0 and bool((wide[:, N:] == 7.0).all())
+    err = (wide[:, :N].double() - x.double() @ w.double().t()).abs().max().item()
+    assert err <= -(-K // 16) * 6 * 2 ** -23 + (6 * 2 ** -8 if out_dtype == torch.bfloat16 else 0.0)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 48, 8), (3, 40, 264), (8, 96, 1408), (9, 64, 1416), (16, 128, 2816), (8, 64, 5632), (2, 5000, 768),
                                    (1, 9480, 8), (5, 9490, 2040), (8, 14300, 264), (9, 9490, 2056), (16, 5000, 72),      # tiles in turn
                                    (2, 40, 2056), (8, 2368, 2088), (12, 2360, 4104), (1, 2376, 2056)])                  # sixteen warps a tile, and one tile too many
