@@ -438,6 +438,7 @@ attn_flex_kernel(const FlexParams p) {
 __global__ void __launch_bounds__(128) attn_flex_merge_kernel(const FlexParams p, int col_blocks) {
   __shared__ float w[64];
   __shared__ float s_inv;
+  if (p.out_f32) pdl_trigger();
   const AttnItem item = p.items[blockIdx.x];
   pdl_wait();
   if (item.ntok <= 0 || item.seq < 0 || item.seq >= p.num_seqs) return;

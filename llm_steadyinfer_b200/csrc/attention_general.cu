@@ -188,10 +188,11 @@ __global__ void kv_store_kernel(const T* __restrict__ qkv, long long row_stride,
                                 const int* __restrict__ row_seq, const int* __restrict__ block_table,
                                 int table_width, T* __restrict__ k_cache, T* __restrict__ v_cache, int num_pages,
                                 int page_size, int num_seqs, int H, int KV, int dk, int dv, int* status) {
-  pdl_prologue_small();
+  pdl_trigger_small();
   const int t = blockIdx.x;
-  const int pos = positions[t];
+  const int pos = positions[t];                     // copied in before the step's first kernel, like the pages
   const long long page = page_of(block_table, table_width, num_pages, page_size, num_seqs, row_seq[t], pos, status);
+  pdl_wait();
   if (page < 0) return;
   const int off = pos % page_size;
   const T* krow = qkv + (size_t)t * row_stride + (size_t)H * dk;
@@ -211,12 +212,13 @@ SI_EXPORT int si_kv_store(const void* qkv, int dtype, long long row_stride, cons
                           int page_size, int num_tokens, int num_seqs, int H, int KV, int dk, int dv, int* status,
                           cudaStream_t stream) {
   if (num_tokens <= 0) return 0;
+  const int threads = num_tokens <= si_sm_count() ? 512 : 128;      // a decode row's entries all at once
   if (dtype == SI_BF16)
-    si_launch(kv_store_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(128), 0, stream, (const __nv_bfloat16*)qkv,
+    si_launch(kv_store_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), 0, stream, (const __nv_bfloat16*)qkv,
               row_stride, positions, row_seq, block_table, table_width, (__nv_bfloat16*)k_cache,
               (__nv_bfloat16*)v_cache, num_pages, page_size, num_seqs, H, KV, dk, dv, status);
   else
-    si_launch(kv_store_kernel<float>, dim3(num_tokens), dim3(128), 0, stream, (const float*)qkv, row_stride,
+    si_launch(kv_store_kernel<float>, dim3(num_tokens), dim3(threads), 0, stream, (const float*)qkv, row_stride,
               positions, row_seq, block_table, table_width, (float*)k_cache, (float*)v_cache, num_pages,
               page_size, num_seqs, H, KV, dk, dv, status);
   return si_last_error();
@@ -229,10 +231,7 @@ SI_EXPORT int si_kv_store(const void* qkv, int dtype, long long row_stride, cons
 //   q_exp[h]  = [ q[h, :dq] | rotate(q[h, dq:dq + dr]) ]                                       (optional)
 // rotate(): the first rd of the dr entries in pairs (i, i + rd/2), or (2i, 2i + 1) when `interleaved`, angle
 // pos * inv_freq[i] in fp32, cosine and sine times `rot_scale`; the other dr - rd entries pass.
-__device__ __forceinline__ float rotated_entry(float u, float v, bool second, float angle, float rot_scale) {
-  float s, c;
-  sincosf(angle, &s, &c);
-  s *= rot_scale; c *= rot_scale;
+__device__ __forceinline__ float rotated_entry(float u, float v, bool second, float s, float c) {
   return second ? v * c + u * s : u * c - v * s;
 }
 template <typename T>
@@ -244,12 +243,22 @@ __global__ void __launch_bounds__(1024) latent_prepare_kernel(const T* __restric
                                       int num_pages, int page_size, int num_seqs, int H, int dq, int dr, int rk,
                                       int interleaved, float rot_scale, int* status) {
   __shared__ float red[33];
-  pdl_prologue_small();
+  extern __shared__ float sc_table[];              // the row's sines, then its cosines: rd / 2 each
+  pdl_trigger_small();
   const int t = blockIdx.x;
-  const int pos = positions[t];
+  const int pos = positions[t];                    // copied in before the step's first kernel, like the pages
   const int seq = row_seq[t];
   const int half = rd / 2;
   const float fpos = (float)pos;
+  for (int f = threadIdx.x; f < half; f += blockDim.x) {
+    float sn, cs;
+    sincosf(fpos * inv_freq[f], &sn, &cs);
+    sc_table[f] = sn * rot_scale;
+    sc_table[half + f] = cs * rot_scale;
+  }
+  const long long page = k_cache ? page_of(block_table, table_width, num_pages, page_size, num_seqs, seq, pos, status) : -1;
+  __syncthreads();
+  pdl_wait();
   // the queries' rotated parts
   const T* qrow = q + (size_t)t * q_stride;
   T* qf = q_full + (size_t)t * qf_stride;
@@ -260,7 +269,7 @@ __global__ void __launch_bounds__(1024) latent_prepare_kernel(const T* __restric
     if (i < rd) {
       const int f = interleaved ? i >> 1 : (i < half ? i : i - half);
       const int iu = interleaved ? 2 * f : f, iv = interleaved ? 2 * f + 1 : f + half;
-      y = rotated_entry(to_f32<T>(src[iu]), to_f32<T>(src[iv]), i == iv, fpos * inv_freq[f], rot_scale);
+      y = rotated_entry(to_f32<T>(src[iu]), to_f32<T>(src[iv]), i == iv, sc_table[f], sc_table[half + f]);
     } else {
       y = to_f32<T>(src[i]);
     }
@@ -282,7 +291,6 @@ __global__ void __launch_bounds__(1024) latent_prepare_kernel(const T* __restric
     }
   }
   ss = block_sum(ss, red);
-  const long long page = page_of(block_table, table_width, num_pages, page_size, num_seqs, seq, pos, status);
   if (page < 0) return;
   T* dst = k_cache + ((size_t)page * page_size + pos % page_size) * (rk + dr);
   const float rs = 1.f / sqrtf(ss / (float)rk + eps);
@@ -292,7 +300,7 @@ __global__ void __launch_bounds__(1024) latent_prepare_kernel(const T* __restric
     if (i < rd) {
       const int f = interleaved ? i >> 1 : (i < half ? i : i - half);
       const int iu = interleaved ? 2 * f : f, iv = interleaved ? 2 * f + 1 : f + half;
-      y = rotated_entry(to_f32<T>(row[rk + iu]), to_f32<T>(row[rk + iv]), i == iv, fpos * inv_freq[f], rot_scale);
+      y = rotated_entry(to_f32<T>(row[rk + iu]), to_f32<T>(row[rk + iv]), i == iv, sc_table[f], sc_table[half + f]);
     } else {
       y = to_f32<T>(row[rk + i]);
     }
@@ -314,13 +322,13 @@ SI_EXPORT int si_latent_prepare(const void* kv, int dtype, long long kv_stride, 
   // 6.1)
   const int threads = num_tokens <= si_sm_count() ? (H * dr >= 1024 ? 1024 : H * dr >= 512 ? 512 : 256) : 128;
   if (dtype == SI_BF16)
-    si_launch(latent_prepare_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), 0, stream, (const __nv_bfloat16*)kv,
+    si_launch(latent_prepare_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), (size_t)rd * sizeof(float), stream, (const __nv_bfloat16*)kv,
               kv_stride, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)q_full, qf_stride, (__nv_bfloat16*)q_exp,
               qe_stride, norm_w, eps, inv_freq,
               rd, positions, row_seq, block_table, table_width, (__nv_bfloat16*)k_cache, num_pages, page_size,
               num_seqs, H, dq, dr, rk, interleaved, rot_scale, status);
   else
-    si_launch(latent_prepare_kernel<float>, dim3(num_tokens), dim3(threads), 0, stream, (const float*)kv, kv_stride,
+    si_launch(latent_prepare_kernel<float>, dim3(num_tokens), dim3(threads), (size_t)rd * sizeof(float), stream, (const float*)kv, kv_stride,
               (const float*)q, q_stride, (float*)q_full, qf_stride, (float*)q_exp, qe_stride, norm_w, eps, inv_freq, rd,
               positions, row_seq,
               block_table, table_width, (float*)k_cache, num_pages, page_size, num_seqs, H, dq, dr, rk, interleaved,

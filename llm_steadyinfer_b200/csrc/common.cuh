@@ -111,11 +111,10 @@ __device__ __forceinline__ void l2_prefetch_share(const void* base, long long by
 // places of their own later blocks.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-// The same for a kernel with a handful of blocks (a decode step's rows): the kernel behind it, which reads the cache, starts on the keys that
-// are older than the step.
-__device__ __forceinline__ void pdl_prologue_small() {
+// For a kernel with a handful of blocks (a decode step's rows) that stores the newest keys: the kernel behind it, which reads the cache,
+// starts on the keys that are older than the step.
+__device__ __forceinline__ void pdl_trigger_small() {
   if (gridDim.x * gridDim.y * gridDim.z <= 64u) pdl_trigger();
-  pdl_wait();
 }
 
 // SI_PDL_TRIGGER: 0 no kernel triggers; 1 the small kernels; 2 (default) also every kernel of one wave of

@@ -990,7 +990,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) head_norm_gate_kernel(const float* __restrict__ o, long long o_stride, const T* __restrict__ z,
     long long z_stride, const float* __restrict__ w, T* __restrict__ out, long long out_stride, long long pairs, int H, int dv,
     float eps, long long w_head_stride, float post, int sigmoid) {
-  pdl_prologue();
+  pdl_trigger_small();
+  pdl_wait();
   const long long wi = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (wi >= pairs) return;
   const int lane = threadIdx.x & 31;

@@ -11,26 +11,31 @@
 __global__ void __launch_bounds__(GH_WARPS * 32)
 gemm_heads_kernel(const __nv_bfloat16* __restrict__ a, long long a_row, long long a_head,
                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out, long long o_row,
-                  long long o_head, int M, int N, int K) {
+                  long long o_head, int M, int N, int K, int trigger) {
   extern __shared__ __align__(16) unsigned char gh_smem[];
   __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(gh_smem);          // [M][K]
-  pdl_prologue();
+  if (trigger) pdl_trigger();
   const int h = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kc = K / 8;
+  const int n = blockIdx.x * GH_WARPS + warp;
+  const __nv_bfloat16* wr = w + ((size_t)h * N + (n < N ? n : 0)) * K;
+  // the column's first weights are on their way before the wait for the rows (a load of this kind stays before it)
+  uint4 first = make_uint4(0, 0, 0, 0);
+  if (lane < kc)
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(first.x), "=r"(first.y), "=r"(first.z), "=r"(first.w) : "l"(wr + lane * 8) : "memory");
+  pdl_wait();
   for (int id = threadIdx.x; id < M * kc; id += blockDim.x) {
     const int m = id / kc, c = id % kc;
     reinterpret_cast<uint4*>(As)[id] = *reinterpret_cast<const uint4*>(a + (size_t)m * a_row + (size_t)h * a_head + c * 8);
   }
   __syncthreads();
-  const int n = blockIdx.x * GH_WARPS + warp;
   if (n >= N) return;
-  const __nv_bfloat16* wr = w + ((size_t)h * N + n) * K;
   float acc[GH_MAX_ROWS];
 #pragma unroll
   for (int m = 0; m < GH_MAX_ROWS; ++m) acc[m] = 0.f;
   for (int c = lane; c < kc; c += 32) {
-    const uint4 wv = *reinterpret_cast<const uint4*>(wr + c * 8);
+    const uint4 wv = c == lane ? first : *reinterpret_cast<const uint4*>(wr + c * 8);
     const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(&wv);
     float wf[8];
 #pragma unroll
@@ -62,7 +67,9 @@ SI_EXPORT int si_gemm_heads(const void* a, long long a_row, long long a_head, co
   if (M > GH_MAX_ROWS || K % 8 || K <= 0 || H > 65535) return -2;
   const size_t smem = (size_t)M * K * sizeof(__nv_bfloat16);
   if (smem > 48 * 1024) return -2;
-  si_launch(gemm_heads_kernel, dim3((N + GH_WARPS - 1) / GH_WARPS, H), dim3(GH_WARPS * 32), smem, stream,
-            (const __nv_bfloat16*)a, a_row, a_head, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, o_row, o_head, M, N, K);
+  const dim3 grid((N + GH_WARPS - 1) / GH_WARPS, H);
+  const int trigger = si_pdl_trigger_mode((long long)grid.x * grid.y, 8LL * si_sm_count()) == 1;
+  si_launch(gemm_heads_kernel, grid, dim3(GH_WARPS * 32), smem, stream,
+            (const __nv_bfloat16*)a, a_row, a_head, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, o_row, o_head, M, N, K, trigger);
   return si_last_error();
 }

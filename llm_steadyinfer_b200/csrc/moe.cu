@@ -941,7 +941,8 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const TY* __restrict__
     const float* __restrict__ wts, int top, const T* __restrict__ shared, long long shared_stride, const float* __restrict__ gate,
     int gate_stride, T* __restrict__ out, long long out_stride, int d, const int* __restrict__ ids, int real,
     const T* __restrict__ x, long long x_stride) {
-  pdl_prologue();
+  pdl_trigger_small();
+  pdl_wait();
   const long long t = blockIdx.x;
   for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < d; i += blockDim.x * gridDim.y) {
     float acc = 0.f;

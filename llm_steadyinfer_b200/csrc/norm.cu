@@ -199,7 +199,8 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const TX* __restrict_
                                                            const TW* __restrict__ weight, long long num_rows, int n, int inner,
                                                            long long x_outer, long long x_inner, long long o_outer,
                                                            long long o_inner, float eps) {
-  pdl_prologue();
+  pdl_trigger_small();
+  pdl_wait();
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= num_rows) return;
   const int lane = threadIdx.x & 31;
