@@ -71,6 +71,23 @@ def _stream():
     return torch.cuda.current_stream().cuda_stream
 
 
+_stream_objects: dict = {}
+
+
+def stream_object(device):
+    """``torch.cuda.current_stream(device)`` without building its object every time: the objects are kept by device and handle (an object
+    is its handle; a handle that is used anew names the stream that has it then)."""
+    if _raw_stream is None or device.type != "cuda" or device.index is None:
+        return torch.cuda.current_stream(device)
+    key = (device.index, _raw_stream(device.index))
+    stream = _stream_objects.get(key)
+    if stream is None:
+        if len(_stream_objects) >= 64:
+            _stream_objects.clear()
+        stream = _stream_objects[key] = torch.cuda.current_stream(device)
+    return stream
+
+
 def _need(cond: bool, msg: str) -> None:
     if not cond:
         raise KernelError(msg)

@@ -107,7 +107,7 @@ class _PinnedRing:
             ev = self.events[self.turn]
             if ev is None:
                 ev = self.events[self.turn] = torch.cuda.Event()
-            ev.record(torch.cuda.current_stream(self.dev.device))      # where the copy is, whatever device the calling thread is at
+            ev.record(ops.stream_object(self.dev.device))      # where the copy is, whatever device the calling thread is at
 
 
 class ModelRunner:
@@ -150,10 +150,12 @@ class ModelRunner:
         self._uploads: Dict[str, _PinnedRing] = {}
         G = max(1, len(self.manager.groups))
         T, S, W = self.max_step_tokens, max_requests, self.max_width
-        self._stage = _PinnedRing(4 * (T + 4) + 3 * (S + 4) + 8 + G * S * W, self.device)
+        self._stage = _PinnedRing(4 * (T + 4) + 4 * (S + 4) + 8 + G * S * W, self.device)
         self._table_arrays: Dict[Tuple[int, Hashable], Tuple[int, np.ndarray]] = {}
         self._graphs: Dict[Tuple[int, int], dict] = {}
         self._stage_views: Dict[Tuple[int, int], tuple] = {}      # of fixed-shape steps: their inputs lie in the same places
+        self._counting = np.arange(S, dtype=np.int32)
+        self._stage_rows: Dict[Tuple[int, int], np.ndarray] = {}  # of fixed-shape steps: their inputs as they are without any values
         # Shapes whose recording failed: they run directly from then on, as the reference marks a batch size
         # capture_failed and keeps to its direct path (src/source/model/model.cpp:189-227, 251).
         self.capture_failed: Dict[Tuple[int, int], str] = {}
@@ -216,7 +218,7 @@ class ModelRunner:
         ``dst[i]`` of the batch is not known on the host yet (its entry holds a placeholder) and is
         taken on the device from ``ids[src[i]]`` (int32 tensor, lists)."""
         with tracing.span("prepare"):
-            ctx = self._prepare(entries)
+            ctx = self._prepare(entries, feed=feed)
             if feed is not None:
                 self._feed_tokens(ctx, feed)
             self.storage.zero_new_slots(self.upload_ints)
@@ -232,9 +234,10 @@ class ModelRunner:
     def _feed_tokens(self, ctx, feed) -> None:
         ids, dst, src = feed
         n = len(dst)
-        if list(dst) == list(range(n)):                                  # the first n rows: one gather into place
-            idx = self.upload_ints("token_feed", np.asarray(src, dtype=np.int32), capacity=self.max_requests)
-            torch.index_select(ids, 0, idx, out=ctx.tokens[:n])
+        if n == 0:
+            return
+        if self._feed_rows is not None:                                  # the first n rows: one gather into place
+            torch.index_select(ids, 0, self._feed_rows, out=ctx.tokens[:n])
             return
         both = self.upload_ints("token_feed_some", np.asarray(list(src) + list(dst), dtype=np.int32),
                                 capacity=2 * self.max_requests)
@@ -262,7 +265,7 @@ class ModelRunner:
             cap = self.max_requests
         if S > cap:
             raise StepError(f"{S} sequences exceed the limit of {self.max_requests}")
-        ctx = self._prepare(entries, seq_cap=cap, width_cap=self.max_width)
+        ctx = self._prepare(entries, seq_cap=cap, width_cap=self.max_width, feed=feed)
         if feed is not None:
             self._feed_tokens(ctx, feed)
         self.storage.zero_new_slots(self.upload_ints)
@@ -315,8 +318,146 @@ class ModelRunner:
         if captured is not None and gen == self._generation:      # no buffer moved while recording
             self._graphs[key] = {"graph": graph, "logits": captured, "launches": launches}
 
+    def _decode_rows(self, entries: Sequence[StepEntry]):
+        """(tokens, positions, slots) of a step whose entries are one wanted row each, of live requests whose next place lies in a page that
+        they hold alone: such a step takes no pages and has nothing to be refused for. None: anything else, which is looked at entry by
+        entry."""
+        mgr, ps = self.manager, self.page_size
+        requests, groups, most = mgr.requests, mgr.groups, self.max_width * self.page_size
+        if not 0 < len(entries) <= min(self.max_requests, self.max_step_tokens):
+            return None
+        seen, toks, pos, slots = set(), [], [], []
+        for e in entries:
+            req, tokens, want = e.req, e.tokens, e.want
+            rc = requests.get(req)
+            if rc is None or req in seen or len(tokens) != 1 or len(want) != 1 or want[0] != 0 or rc.length >= most:
+                return None
+            seen.add(req)
+            b = rc.length // ps
+            for grp in groups:
+                table = grp.tables[req]
+                if b >= len(table) or (table[b] >= 0 and grp.pool.refcount(table[b]) != 1):
+                    return None
+            toks.append(tokens[0])
+            pos.append(rc.length)
+            slots.append(rc.slot)
+        return toks, pos, slots
+
     def _prepare(self, entries: Sequence[StepEntry], seq_cap: Optional[int] = None,
-                 width_cap: Optional[int] = None) -> StepContext:
+                 width_cap: Optional[int] = None, feed=None) -> StepContext:
+        mgr = self.manager
+        rows = self._decode_rows(entries)
+        if rows is None:
+            self._admit(entries)
+        else:
+            self._new_lengths = [p + 1 for p in rows[1]]
+        S = len(entries)
+        T = S if rows is not None else sum(len(e.tokens) for e in entries)
+        R = S if rows is not None else sum(len(e.want) for e in entries)
+        G = len(mgr.groups)
+        W = width_cap or max([1] + [len(mgr.table(g, e.req)) for g in range(G) for e in entries])   # pages may be reserved ahead
+        fixed = seq_cap is not None
+        S_cap = seq_cap or S
+        T_cap = S_cap if fixed else T          # fixed-shape steps: one row per sequence slot
+        R_cap = S_cap if fixed else R
+        # layout (ints): tokens | positions | row_seq | logit_rows | q_start | ctx_len | slots | tables
+        offs = {}
+        o = 0
+        for name, n in (("tokens", T_cap), ("positions", T_cap), ("row_seq", T_cap), ("logit_rows", max(R_cap, 1)),
+                        ("q_start", S_cap + 1), ("ctx_len", S_cap), ("slots", S_cap)):
+            offs[name] = o
+            o += (n + 3) // 4 * 4                     # 16-byte aligned regions
+        table_off = o
+        o += G * S_cap * W
+        # tokens that are known on the device alone: which of them goes to which of the first rows
+        feed_off, feed_rows = (o + 3) // 4 * 4, 0
+        if feed is not None and list(feed[1]) == list(range(len(feed[1]))):
+            feed_rows = len(feed[1])
+            o = feed_off + feed_rows
+        if o > self._stage.cap:
+            raise StepError(f"step inputs of {o} integers exceed the staging buffer of {self._stage.cap}")
+        h = self._stage.next_host()
+        dev = self._stage.dev
+        b_tok, b_pos, b_seq = offs["tokens"], offs["positions"], offs["row_seq"]
+        b_lr, b_qs, b_cl, b_sl = offs["logit_rows"], offs["q_start"], offs["ctx_len"], offs["slots"]
+        blank = self._stage_rows.get((S_cap, S)) if fixed else None
+        if blank is not None:
+            h[:table_off] = blank
+        else:
+            if fixed:
+                h[:table_off] = 0
+                h[b_seq:b_seq + T_cap] = -1           # padding rows store nothing
+                h[b_lr:b_lr + R_cap] = np.arange(R_cap, dtype=np.int32)
+            h[b_qs:b_qs + S_cap + 1] = T
+            h[b_cl:b_cl + S_cap] = 0
+            h[b_sl:b_sl + S_cap] = 0
+            if fixed:
+                if len(self._stage_rows) >= 1024:
+                    self._stage_rows.clear()
+                self._stage_rows[(S_cap, S)] = h[:table_off].copy()
+        if rows is not None:
+            h[b_tok:b_tok + T] = np.asarray(rows[0], dtype=np.int64).astype(np.int32)   # an id beyond 32 bits wraps and is flagged by the kernel
+            h[b_pos:b_pos + T] = rows[1]
+            h[b_seq:b_seq + T] = h[b_qs:b_qs + T] = h[b_lr:b_lr + T] = self._counting[:T]
+            h[b_cl:b_cl + S] = self._new_lengths
+            h[b_sl:b_sl + S] = rows[2]
+        else:
+            # one assignment a region: the per-entry values are gathered in lists first (a step of 64 decode rows
+            # would otherwise pay for several hundred small array writes)
+            toks, pos, seqs, qs, cl, sl, lr = [], [], [], [], [], [], []
+            row = 0
+            for s, e in enumerate(entries):
+                n = len(e.tokens)
+                start = mgr.length(e.req)
+                if n == 1:
+                    toks.append(e.tokens[0]); pos.append(start); seqs.append(s)
+                else:
+                    toks.extend(e.tokens); pos.extend(range(start, start + n)); seqs.extend([s] * n)
+                qs.append(row); cl.append(start + n); sl.append(mgr.slot(e.req))
+                for w in e.want:
+                    lr.append(row + w)
+                row += n
+            h[b_tok:b_tok + T] = np.asarray(toks, dtype=np.int64).astype(np.int32)   # an id beyond 32 bits wraps and is flagged by the kernel
+            h[b_pos:b_pos + T] = pos
+            h[b_seq:b_seq + T] = seqs
+            h[b_qs:b_qs + S] = qs
+            h[b_cl:b_cl + S] = cl
+            h[b_sl:b_sl + S] = sl
+            if lr:
+                h[b_lr:b_lr + len(lr)] = lr
+        tabs = h[table_off:table_off + G * S_cap * W].reshape(G, S_cap, W)
+        tabs[:] = -1
+        for g in range(G):
+            for s, e in enumerate(entries):
+                t = self._table_array(g, e.req)
+                tabs[g, s, :t.size] = t
+        if feed_rows:
+            h[feed_off:o] = feed[2]
+        self._stage.send(o)
+        self._feed_rows = dev[feed_off:o] if feed_rows else None
+        self.h2d_bytes_last_step = 4 * o       # parts add their uploads in prepare()
+
+        ctx = self.ctx
+        ctx.plans.clear()
+        ctx.seq_cap = seq_cap
+        ctx.num_tokens, ctx.num_seqs, ctx.num_logit_rows = T_cap, S, R_cap
+        ctx.seq_slots = S_cap
+        views = self._stage_views.get((S_cap, W)) if fixed else None
+        if views is None:
+            dtabs = dev[table_off:table_off + G * S_cap * W].view(G, S_cap, W)
+            views = (dev[b_tok:b_tok + T_cap], dev[b_pos:b_pos + T_cap], dev[b_seq:b_seq + T_cap], dev[b_lr:b_lr + R_cap],
+                     dev[b_qs:b_qs + S_cap + 1], dev[b_cl:b_cl + S_cap], dev[b_sl:b_sl + S_cap], [dtabs[g] for g in range(G)])
+            if fixed:
+                self._stage_views[(S_cap, W)] = views
+        (ctx.tokens, ctx.positions, ctx.row_seq, ctx.logit_rows, ctx.q_start, ctx.ctx_len, ctx.slots, self._tables) = views
+        ctx.h_positions = h[b_pos:b_pos + T].copy()
+        ctx.h_q_start = h[b_qs:b_qs + S + 1].copy()
+        ctx.h_ctx_len = h[b_cl:b_cl + S].copy()
+        ctx.h_slots = h[b_sl:b_sl + S].copy()
+        return ctx
+
+    def _admit(self, entries: Sequence[StepEntry]) -> None:
+        """Checks a step's entries and takes the pages that their tokens need, in every group or in none."""
         mgr = self.manager
         if not entries:
             raise StepError("a step needs at least one entry")
@@ -357,88 +498,6 @@ class ModelRunner:
             mgr.grow(e.req, new_len)
             self._new_lengths.append(new_len)
         self._check_pages_written(entries)
-
-        R = sum(len(e.want) for e in entries)
-        G = len(mgr.groups)
-        W = max([1] + [len(mgr.table(g, e.req)) for g in range(G) for e in entries])   # pages may be reserved ahead
-        fixed = seq_cap is not None
-        S_cap = seq_cap or S
-        W_cap = width_cap or W
-        T_cap = S_cap if fixed else T          # fixed-shape steps: one row per sequence slot
-        R_cap = S_cap if fixed else R
-        # layout (ints): tokens | positions | row_seq | logit_rows | q_start | ctx_len | slots | tables
-        offs = {}
-        o = 0
-        for name, n in (("tokens", T_cap), ("positions", T_cap), ("row_seq", T_cap), ("logit_rows", max(R_cap, 1)),
-                        ("q_start", S_cap + 1), ("ctx_len", S_cap), ("slots", S_cap)):
-            offs[name] = o
-            o += (n + 3) // 4 * 4                     # 16-byte aligned regions
-        table_off = o
-        o += G * S_cap * W_cap
-        if o > self._stage.cap:
-            raise StepError(f"step inputs of {o} integers exceed the staging buffer of {self._stage.cap}")
-        h = self._stage.next_host()
-        dev = self._stage.dev
-        b_tok, b_pos, b_seq = offs["tokens"], offs["positions"], offs["row_seq"]
-        b_lr, b_qs, b_cl, b_sl = offs["logit_rows"], offs["q_start"], offs["ctx_len"], offs["slots"]
-        if fixed:
-            h[b_tok:b_tok + T_cap] = 0
-            h[b_pos:b_pos + T_cap] = 0
-            h[b_seq:b_seq + T_cap] = -1               # padding rows store nothing
-            h[b_lr:b_lr + R_cap] = np.arange(R_cap, dtype=np.int32)
-        h[b_qs:b_qs + S_cap + 1] = T
-        h[b_cl:b_cl + S_cap] = 0
-        h[b_sl:b_sl + S_cap] = 0
-        # one assignment a region: the per-entry values are gathered in lists first (a step of 64 decode rows
-        # would otherwise pay for several hundred small array writes)
-        toks, pos, seqs, qs, cl, sl, lr = [], [], [], [], [], [], []
-        row = 0
-        for s, e in enumerate(entries):
-            n = len(e.tokens)
-            start = mgr.length(e.req)
-            if n == 1:
-                toks.append(e.tokens[0]); pos.append(start); seqs.append(s)
-            else:
-                toks.extend(e.tokens); pos.extend(range(start, start + n)); seqs.extend([s] * n)
-            qs.append(row); cl.append(start + n); sl.append(mgr.slot(e.req))
-            for w in e.want:
-                lr.append(row + w)
-            row += n
-        h[b_tok:b_tok + T] = np.asarray(toks, dtype=np.int64).astype(np.int32)   # an id beyond 32 bits wraps and is flagged by the kernel
-        h[b_pos:b_pos + T] = pos
-        h[b_seq:b_seq + T] = seqs
-        h[b_qs:b_qs + S] = qs
-        h[b_cl:b_cl + S] = cl
-        h[b_sl:b_sl + S] = sl
-        if lr:
-            h[b_lr:b_lr + len(lr)] = lr
-        tabs = h[table_off:table_off + G * S_cap * W_cap].reshape(G, S_cap, W_cap)
-        tabs[:] = -1
-        for g in range(G):
-            for s, e in enumerate(entries):
-                t = self._table_array(g, e.req)
-                tabs[g, s, :t.size] = t
-        self._stage.send(o)
-        self.h2d_bytes_last_step = 4 * o       # parts add their uploads in prepare()
-
-        ctx = self.ctx
-        ctx.plans.clear()
-        ctx.seq_cap = seq_cap
-        ctx.num_tokens, ctx.num_seqs, ctx.num_logit_rows = T_cap, S, R_cap
-        ctx.seq_slots = S_cap
-        views = self._stage_views.get((S_cap, W_cap)) if fixed else None
-        if views is None:
-            dtabs = dev[table_off:table_off + G * S_cap * W_cap].view(G, S_cap, W_cap)
-            views = (dev[b_tok:b_tok + T_cap], dev[b_pos:b_pos + T_cap], dev[b_seq:b_seq + T_cap], dev[b_lr:b_lr + R_cap],
-                     dev[b_qs:b_qs + S_cap + 1], dev[b_cl:b_cl + S_cap], dev[b_sl:b_sl + S_cap], [dtabs[g] for g in range(G)])
-            if fixed:
-                self._stage_views[(S_cap, W_cap)] = views
-        (ctx.tokens, ctx.positions, ctx.row_seq, ctx.logit_rows, ctx.q_start, ctx.ctx_len, ctx.slots, self._tables) = views
-        ctx.h_positions = h[b_pos:b_pos + T].copy()
-        ctx.h_q_start = h[b_qs:b_qs + S + 1].copy()
-        ctx.h_ctx_len = h[b_cl:b_cl + S].copy()
-        ctx.h_slots = h[b_sl:b_sl + S].copy()
-        return ctx
 
     def _check_pages_written(self, entries: Sequence[StepEntry]) -> None:
         """A step may store keys and values only into pages that its request holds alone. A page with more
