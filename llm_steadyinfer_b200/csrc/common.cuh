@@ -91,6 +91,10 @@ __device__ __forceinline__ void pdl_wait() {
 }
 __device__ __forceinline__ void pdl_prologue() { pdl_wait(); }
 
+// A decode row's norm weights have left L2 since the step before (all weights passed through it): a hint at a thread's own, given before the wait
+// for the kernel before, brings them while the row is still being made. Many rows find them in L2.
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];\n" :: "l"(p) : "memory"); }
+
 // A hint that [base, base + bytes) will be streamed soon: block `part` of `parts` asks the memory system
 // to bring its share into L2, one prefetch per 128-byte line. Kernels that wait on latency while HBM
 // idles (the norms of a decode step) call this for the first weights of the matrix product after them.
@@ -117,24 +121,19 @@ __device__ __forceinline__ void pdl_trigger_small() {
   if (gridDim.x * gridDim.y * gridDim.z <= 64u) pdl_trigger();
 }
 
-// SI_PDL_TRIGGER: 0 no kernel triggers; 1 the small kernels; 2 (default) also every kernel of one wave of
-// blocks, at its start; 3 also kernels of several waves, once their main loop is done.
+// SI_PDL_TRIGGER (the kernels above, the tcgen05 kernels and the experts of few rows trigger whatever it says): 0 no other kernel triggers;
+// 1 the small kernels; 2 (default) also every kernel of one wave of blocks, at its start.
 static inline int si_pdl_trigger_level() {
   static int level = -1;
   if (level < 0) {
     const char* e = getenv("SI_PDL_TRIGGER");
-    level = (e && e[0] >= '0' && e[0] <= '3') ? e[0] - '0' : 2;
+    level = (e && e[0] >= '0' && e[0] <= '2') ? e[0] - '0' : 2;
   }
   return level;
 }
 static inline bool si_pdl_trigger_enabled() { return si_pdl_trigger_level() >= 1; }
-// What a kernel of `blocks` blocks, `slots` of which run at once, is told: 0 do not trigger, 1 at the
-// start, 2 after the main loop.
-static inline int si_pdl_trigger_mode(long long blocks, long long slots) {
-  const int level = si_pdl_trigger_level();
-  if (blocks <= slots) return level >= 2 ? 1 : 0;
-  return level >= 3 ? 2 : 0;
-}
+// Whether a kernel of `blocks` blocks, `slots` of which run at once, triggers at its start: 1 or 0.
+static inline int si_pdl_trigger_mode(long long blocks, long long slots) { return blocks <= slots && si_pdl_trigger_level() >= 2 ? 1 : 0; }
 
 // Streaming multiprocessors of the current device, asked once per device. Grid sizes that should fill the
 // device once ("one wave") are derived from it; no kernel's result depends on it.

@@ -56,13 +56,18 @@ __global__ void __launch_bounds__(512) add_rmsnorm_vec_kernel(float* __restrict_
     l2_prefetch_share(ahead, ahead_bytes, blockIdx.x - num_rows, gridDim.x - num_rows);
     return;
   }
-  pdl_prologue();
+  const int nchunks = hidden >> 3;
+  if (trigger) {
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c)
+      if ((int)(threadIdx.x + c * blockDim.x) < nchunks) prefetch_l1(weight + (threadIdx.x + c * blockDim.x) * 8);
+  }
+  pdl_wait();
   const int r = blockIdx.x;
   const int src = rows ? rows[r] : r;
   float* h = resid + (size_t)src * hidden;
   const TX* dl = delta ? delta + (size_t)src * hidden : nullptr;
   const TX* dl2 = (delta && delta2) ? delta2 + (size_t)src * hidden : nullptr;     // a second result of the same block
-  const int nchunks = hidden >> 3;
   Vec8<float> x[CHUNKS];
   Vec8<TX> dv[CHUNKS], dv2[CHUNKS];
 #pragma unroll
@@ -303,11 +308,20 @@ __global__ void __launch_bounds__(512) add_norm_general_vec_kernel(float* __rest
     const float* __restrict__ extra, const float* __restrict__ vec, const int* __restrict__ rows,
     const TW* __restrict__ weight, TX* __restrict__ out, int hidden, float eps) {
   __shared__ float scratch[33];
-  pdl_prologue();
+  pdl_trigger_small();
+  const int nchunks = hidden >> 3;
+  if (gridDim.x <= 64) {
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int ch = threadIdx.x + c * blockDim.x;
+      if (ch < nchunks && out) prefetch_l1(weight + ch * 8);
+      if (ch < nchunks && delta_weight) prefetch_l1(delta_weight + ch * 8);
+    }
+  }
+  pdl_wait();
   const int r = blockIdx.x;
   const int src = rows ? rows[r] : r;
   float* h = resid + (size_t)src * hidden;
-  const int nchunks = hidden >> 3;
   Vec8<float> x[CHUNKS], d[CHUNKS];
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {

@@ -80,10 +80,22 @@ template <typename T, int CHUNKS>
 __global__ void __launch_bounds__(512) stream_add_vec_kernel(const StreamAdd p) {
   __shared__ float scratch[33];
   if (p.trigger) pdl_trigger();
+  const int nchunks = p.hidden >> 3, first = blockIdx.y * blockDim.x + threadIdx.x, step = blockDim.x * gridDim.y;
+  if (p.trigger) {
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int i = first + c * step;
+      if (i < nchunks) {
+        if (p.delta && p.dn.w) prefetch_l1(p.dn.w + i * 8);
+        if (p.delta && p.dn.b) prefetch_l1(p.dn.b + i * 8);
+        if (p.out && p.on.w) prefetch_l1(p.on.w + i * 8);
+        if (p.out && p.on.b) prefetch_l1(p.on.b + i * 8);
+      }
+    }
+  }
   pdl_wait();
   const int r = blockIdx.x, src = p.rows ? p.rows[r] : r;
   float* h = p.resid + (size_t)src * p.hidden;
-  const int nchunks = p.hidden >> 3, first = blockIdx.y * blockDim.x + threadIdx.x, step = blockDim.x * gridDim.y;
   float x[CHUNKS][8], d[CHUNKS][8];
 #pragma unroll
   for (int c = 0; c < CHUNKS; ++c) {

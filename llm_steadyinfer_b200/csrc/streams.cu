@@ -74,10 +74,17 @@ __global__ void __launch_bounds__(512) stream_norm_vec_kernel(const StreamArgs p
     coef[SM * SM + i] = (moved && i < S) ? p.write[i] : 0.f;
     coef[SM * SM + SM + i] = i < S ? (p.read ? p.read[i] : 1.f) : 0.f;
   }
-  pdl_wait();
-  const int row = p.rows ? p.rows[r] : r;
   const int pieces = p.width / 4, per = (pieces + parts - 1) / parts;
   const int c0 = rank * per, c1 = min(pieces, c0 + per);
+  if (p.trigger) {
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const int c = c0 + threadIdx.x + v * blockDim.x;
+      if (c < c1) prefetch_l1((const char*)p.weight + (size_t)c * (p.weight_bf16 ? 8 : 16));
+    }
+  }
+  pdl_wait();
+  const int row = p.rows ? p.rows[r] : r;
   const float* src = p.src + (size_t)row * p.src_row;
   const T* y = (const T*)p.y + (size_t)row * p.width;
   float4 x[V][SM], yv[V];
