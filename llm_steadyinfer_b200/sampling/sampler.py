@@ -37,14 +37,9 @@ class Sampler:
         if R != len(rows) or R > self.max_rows:
             raise ValueError(f"sampler got {R} logits rows for {len(rows)} requests (limit {self.max_rows})")
         out = self._out[:R]
-        one = rows[0][0] if R else None
-        if all(r[0] is one for r in rows):                      # the rows of one call's requests mostly share their parameters
-            temperature, top_p, top_k = (one.temperature, one.top_p, one.top_k) if R else (0.0, 1.0, 0)
-            greedy = not temperature > 0
-        else:
-            temperature, top_p, top_k = ([r[0].temperature for r in rows], [r[0].top_p for r in rows], [r[0].top_k for r in rows])
-            greedy = not any(t > 0 for t in temperature)
-        if greedy:
+        params = [r[0] for r in rows]
+        temperature = [p.temperature for p in params]
+        if not any(t > 0 for t in temperature):
             ops.argmax(logits, out, self._argmax_scratch)
             return out
         turn = self._host_turn = (self._host_turn + 1) % 4
@@ -53,15 +48,15 @@ class Sampler:
         h = self._arrays[turn]
         n = self.max_rows
         h[0:R].view(np.float32)[:] = temperature
-        h[n:n + R].view(np.float32)[:] = top_p
-        h[2 * n:2 * n + R] = top_k
+        h[n:n + R].view(np.float32)[:] = [p.top_p for p in params]
+        h[2 * n:2 * n + R] = [p.top_k for p in params]
         h[4 * n:4 * n + 2 * R].view(np.uint64)[:] = [r[1] & 0xFFFFFFFFFFFFFFFF for r in rows]
         h[6 * n:6 * n + 2 * R].view(np.int64)[:] = [r[2] for r in rows]
         d = self._dev
         d.copy_(self._hosts[turn], non_blocking=True)
         if self._host_events[turn] is None:
             self._host_events[turn] = torch.cuda.Event()
-        self._host_events[turn].record(ops.stream_object(d.device))      # where the copy is, whatever device the calling thread is at
+        self._host_events[turn].record(torch.cuda.current_stream(d.device))      # where the copy is, whatever device the calling thread is at
         v = self._device_views.get(R)
         if v is None:
             v = self._device_views[R] = (d[0:R].view(torch.float32), d[n:n + R].view(torch.float32), d[2 * n:2 * n + R],
