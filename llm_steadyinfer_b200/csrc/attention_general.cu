@@ -231,8 +231,10 @@ SI_EXPORT int si_kv_store(const void* qkv, int dtype, long long row_stride, cons
 //   q_exp[h]  = [ q[h, :dq] | rotate(q[h, dq:dq + dr]) ]                                       (optional)
 // rotate(): the first rd of the dr entries in pairs (i, i + rd/2), or (2i, 2i + 1) when `interleaved`, angle
 // pos * inv_freq[i] in fp32, cosine and sine times `rot_scale`; the other dr - rd entries pass.
+// The roundings are written out (the product with the sine first, the other joined to it by one fma): left to the compiler, which product
+// is rounded alone changes with what stands around the expression, and a quarter of the 32-bit entries with it by their last place.
 __device__ __forceinline__ float rotated_entry(float u, float v, bool second, float s, float c) {
-  return second ? v * c + u * s : u * c - v * s;
+  return second ? fmaf(v, c, __fmul_rn(u, s)) : fmaf(u, c, -__fmul_rn(v, s));
 }
 template <typename T>
 __global__ void __launch_bounds__(1024) latent_prepare_kernel(const T* __restrict__ kv, long long kv_stride, const T* __restrict__ q,

@@ -562,6 +562,41 @@ def test_latent_rotation_pairs_and_magnitude(interleaved):
     assert (got_q - want_q).abs().max() < 1e-4
 
 
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_latent_rotation_rounds_the_product_with_the_sine_first(interleaved):
+    """Every rotated entry is fma(one, cosine, round(other * sine)), to the bit, in queries and key: the kernel's own sines and cosines are read
+    off from pairs (1, 0); a product of two 32-bit numbers is exact in 64 bits, and so, but for one entry in 2^29, is its rounded sum."""
+    from llm_steadyinfer_b200.csrc import ops
+    torch.manual_seed(7)
+    T, H, dq, dr, rk, ps = 3, 4, 8, 64, 16, 4
+    first, second = (slice(0, dr, 2), slice(1, dr, 2)) if interleaved else (slice(0, dr // 2), slice(dr // 2, dr))
+    norm_w = torch.ones(rk, device=DEV)
+    freqs = (10000.0 ** (-torch.arange(dr // 2) / (dr // 2))).float().to(DEV)
+    pos = torch.tensor([5, 1799, 3001], dtype=torch.int32, device=DEV)
+    seqs = torch.zeros(T, dtype=torch.int32, device=DEV)
+    table = torch.arange(800, dtype=torch.int32, device=DEV).view(1, -1)
+
+    def rotated(parts):                                 # [T, H + 1, dr]: the queries' rotated parts, then the key's
+        q = torch.zeros(T, H, dq + dr, device=DEV)
+        q[:, :, dq:] = parts[:, :H]
+        kv = torch.cat([torch.ones(T, rk, device=DEV), parts[:, H]], 1).contiguous()
+        q_full, cache = torch.zeros(T, H * (rk + dr), device=DEV), torch.zeros(800, 1, ps, rk + dr, device=DEV)
+        ops.latent_prepare(kv, q.view(T, -1), q_full, norm_w, 1e-5, freqs, dr, pos, seqs, table, cache, ps, 1, H, dq, dr, rk,
+                           interleaved=interleaved, rot_scale=1.07)
+        p = pos.long()
+        return torch.cat([q_full.view(T, H, rk + dr)[:, :, rk:], cache[p // ps, 0, p % ps, rk:].unsqueeze(1)], 1)
+
+    unit = torch.zeros(T, H + 1, dr, device=DEV)
+    unit[..., first] = 1.0
+    got = rotated(unit)
+    c, s = got[..., first], got[..., second]
+    x = torch.randn(T, H + 1, dr, device=DEV)
+    u, v = x[..., first], x[..., second]
+    got = rotated(x)
+    assert torch.equal(got[..., first], (u.double() * c.double() - (v * s).double()).float())
+    assert torch.equal(got[..., second], (v.double() * c.double() + (u * s).double()).float())
+
+
 # ---- the entry point ----------------------------------------------------------------------------------------
 
 def greedy(cfg, w, prompt, new):
