@@ -14,8 +14,9 @@
 // tile is token r / Gb, head r % Gb; warp w owns rows 16w..16w+15 and walks all keys of the share. K tiles of
 // BLOCK_N keys x dk come through cp.async into XOR-swizzled shared memory, two stages deep; the values are a
 // second tile (own values: only the block's slice) or columns of the key tile itself.
-// A share of a decode row's keys is a chain of latencies (page, keys, queries, scores, merge) for a few kilobytes: what does not need the
-// kernel before (pages, the first two tiles of keys that are older than the step, biases) is fetched before the wait for it, the four warps
+// A share of a decode row's keys is a chain of latencies (page, keys, queries, scores, merge) for a few kilobytes: where the caller says so
+// (`ahead`), what does not need the kernel before (pages, the first two tiles of keys that are older than the step, biases) is fetched before
+// the wait for it; the four warps
 // merge and store a quarter of the columns each, warps that are slices share one score product, shares without a tile store nothing, and
 // the merge is launched while the last shares store. Behind the kernel that stores the newest key, one row (us, attention / merge, before
 // and now): 2,060 keys of 4 x 128 with biases 11.1 / 3.8 and 8.2 / 3.2; a latent of 576 and 16 heads 13.3 / 5.4 and 10.2 / 4.7. (The merge
@@ -46,7 +47,7 @@ struct FlexParams {
                             // value slice of its own, so that a block serves four slices from one key tile
   float scale_log2;         // scale * log2(e)
   int window, chunk, nsplit;
-  int own_rows;             // every item holds all the rows that its sequence has in this step: the keys before its first position are older than the step
+  int ahead;                // the caller's word that keys before an item's first position, pages and biases are older than the kernel before this one
   int block_n;              // keys of a tile
   int trigger;              // the merge is launched while the last shares store theirs
   int* status;
@@ -91,6 +92,7 @@ attn_flex_kernel(const FlexParams p) {
   float* Ss = Bs + (p.bias_in_smem ? (size_t)2 * bwin * p.Gb : 0);
 
   const int item_idx = blockIdx.x / p.nsplit, split = blockIdx.x % p.nsplit;
+  if (!p.ahead) pdl_wait();                                // (a second wait returns at once)
   const AttnItem item = p.items[item_idx];                 // copied in before the step's first kernel, like the block table
   const int g = blockIdx.y / p.hparts, hpart = blockIdx.y % p.hparts;
   const int warp = threadIdx.x >> 5;
@@ -179,9 +181,9 @@ attn_flex_kernel(const FlexParams p) {
     }
   };
 
-  // Two tiles are on their way from the start. Those whose keys are older than the step are fetched before this kernel waits for the one that
-  // makes the queries and the newest keys; the biases are weights.
-  auto older = [&](int t) { return p.own_rows && t < ntiles && min(kv_begin + (t + 1) * BLOCK_N, kv_end) <= item.pos0; };
+  // Two tiles are on their way from the start. With the caller's word those whose keys are older than the step are fetched before this kernel
+  // waits for the one that makes the queries and the newest keys, and the biases, which are weights.
+  auto older = [&](int t) { return p.ahead && t < ntiles && min(kv_begin + (t + 1) * BLOCK_N, kv_end) <= item.pos0; };
   const bool early0 = older(0), early1 = older(1);
   if (early0) load_kv(kv_begin, 0);
   if (early1) load_kv(kv_begin + BLOCK_N, 1);
@@ -528,7 +530,7 @@ SI_EXPORT int si_attn_flex(const void* q, long long q_stride, const void* k_cach
                            const int* block_table, int table_width, const int* items, int num_items, void* out,
                            long long out_stride, int num_pages, int page_size, int num_seqs, int H, int KV, int dk,
                            int dv, float scale, int window, const float* dist_bias, int nd, const float* sink,
-                           int nsplit, float* scratch, int max_rows, float softcap, int v_share, int out_is_f32, int chunk,
+                           int nsplit, float* scratch, int max_rows, int ahead, float softcap, int v_share, int out_is_f32, int chunk,
                            const float* slopes, float qt_coef, int qt_every, const void* gate, long long gate_stride,
                            int* status, cudaStream_t stream) {
   if (num_items <= 0) return 0;
@@ -551,7 +553,7 @@ SI_EXPORT int si_attn_flex(const void* q, long long q_stride, const void* k_cach
   p.H = H; p.KV = KV; p.G = H / KV; p.Gb = flex_heads_per_block(p.G); p.hparts = p.G / p.Gb;
   p.dk = dk; p.dv = dv; p.dk_pitch = (dk + 63) / 64 * 64;
   p.scale_log2 = scale * LOG2E; p.window = window; p.chunk = chunk; p.nsplit = nsplit; p.status = status;
-  p.own_rows = max_rows > 0;
+  p.ahead = ahead;
   p.trigger = 0;
   const long long slabs = (long long)num_items * KV * p.hparts * nsplit;
   p.part_o = scratch;

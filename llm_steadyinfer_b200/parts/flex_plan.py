@@ -89,10 +89,10 @@ def attend(pl: dict, q, k_cache, v_cache, block_table, out, page_size, seq_slots
            dist_bias=None, sink=None, status=None, softcap: float = 0.0, v_share: int = 1, slopes=None, q_temp=None,
            gate=None, chunk=None) -> None:
     args = (page_size, seq_slots, H, KV, dk, dv, scale, window or 0)
-    if pl["dec"] is not None:
+    if pl["dec"] is not None:                         # one item a sequence: all its rows of the step
         ops.attn_flex(q, k_cache, v_cache, block_table, pl["dec"], out, *args, dist_bias=dist_bias, sink=sink,
                       nsplit=pl["nsplit"], scratch=pl["scratch"], status=status, max_rows=pl["dec_rows"], softcap=softcap,
-                      v_share=v_share, slopes=slopes, q_temp=q_temp, gate=gate, chunk=chunk or 0)
+                      v_share=v_share, slopes=slopes, q_temp=q_temp, gate=gate, chunk=chunk or 0, ahead=True)
     if pl["por"] is not None:
         ops.attn_flex(q, k_cache, v_cache, block_table, pl["por"], out, *args, dist_bias=dist_bias, sink=sink, status=status,
                       softcap=softcap, v_share=v_share, slopes=slopes, q_temp=q_temp, gate=gate, chunk=chunk or 0)

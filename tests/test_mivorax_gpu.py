@@ -316,10 +316,58 @@ def test_tensor_core_attention_shares_without_keys(H, KV, dk, dv, own_v, window)
     ops.attention_general(q, kc, vc, table, seqs, pos, want, ps, 1, H, KV, dk, dv, dk ** -0.5, window, dist_bias=bias)
     items = torch.tensor([(0, r, 1, j) for r, j in enumerate(at)], dtype=torch.int32, device=dev)
     for nsplit in (2, 5, 32, 64):
-        scratch = torch.full((ops.attn_flex_scratch_floats(len(at), H, KV, dv, nsplit),), float("nan"), device=dev)
-        ops.attn_flex(q, kc, vc, table, items, got, ps, 1, H, KV, dk, dv, dk ** -0.5, window, dist_bias=bias, nsplit=nsplit, scratch=scratch,
+        for ahead in (False, True):
+            scratch = torch.full((ops.attn_flex_scratch_floats(len(at), H, KV, dv, nsplit),), float("nan"), device=dev)
+            ops.attn_flex(q, kc, vc, table, items, got, ps, 1, H, KV, dk, dv, dk ** -0.5, window, dist_bias=bias, nsplit=nsplit, scratch=scratch,
+                          max_rows=H // KV, ahead=ahead)
+            assert (got.float() - want.float()).abs().max().item() <= 2e-2, (nsplit, ahead)
+
+
+@pytest.mark.parametrize("H,KV,dk,dv,own_v", [(16, 4, 128, 128, True), (16, 1, 576, 512, False)])
+def test_tensor_core_attention_reads_rows_that_the_kernel_before_stores(H, KV, dk, dv, own_v):
+    """Sixteen rows of one sequence, stored and attended to with one item a row and the most rows of an item given: every row sees the keys
+    that the kernel before has just stored for the rows ahead of it. The cache holds not-a-numbers in their places, and the product that makes
+    the rows lets the store, and the store the attention, start early. Weights and result are rounded to 8 bits: 2^-7 of the largest value."""
+    from llm_steadyinfer_b200.csrc import ops
+    dev = "cuda:0"
+    torch.manual_seed(dk)
+    old, new, ps, K = 200, 16, 16, 1024
+    n, vw = old + new, KV * dv if own_v else 0
+    k = (torch.randn(n, KV, dk) * 0.5).bfloat16()
+    v = torch.randn(n, KV, dv).bfloat16() if own_v else None
+    kc, table = _paged(k, ps, 5)
+    kc, table, vc = kc.to(dev), table.to(dev), _paged(v, ps, 5)[0].to(dev) if own_v else None
+    x = torch.randn(new, K, device=dev).bfloat16()
+    w = (torch.randn(H * dk + KV * dk + vw, K, device=dev) / K ** 0.5).bfloat16()
+    rows = torch.zeros(new, w.shape[0], dtype=torch.bfloat16, device=dev)
+    ops.gemm_skinny(x, w, rows)
+    q = rows[:, :H * dk].double().view(new, H, dk)
+    keys, vals = k.to(dev).double(), (v if own_v else k[..., :dv]).to(dev).double()
+    keys[old:] = rows[:, H * dk:(H + KV) * dk].double().view(new, KV, dk)
+    vals[old:] = rows[:, (H + KV) * dk:].double().view(new, KV, dv) if own_v else keys[old:, :, :dv]
+    want = torch.zeros(new, H, dv, dtype=torch.float64, device=dev)
+    for r in range(new):
+        for h in range(H):
+            g = h // (H // KV)
+            want[r, h] = torch.softmax(keys[:old + r + 1, g] @ q[r, h] * dk ** -0.5, 0) @ vals[:old + r + 1, g]
+    pos = torch.arange(old, n, dtype=torch.int32, device=dev)
+    seqs, status = torch.zeros(new, dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    items = torch.tensor([(0, r, 1, old + r) for r in range(new)], dtype=torch.int32, device=dev)
+    got = torch.zeros(new, H * dv, dtype=torch.bfloat16, device=dev)
+    places = [(int(table[0, j // ps]), j % ps) for j in range(old, n)]
+    for nsplit in (1, 3):
+        scratch = torch.zeros(ops.attn_flex_scratch_floats(new, H, KV, dv, nsplit), device=dev)
+        for page, at in places:
+            for cache in (kc, vc) if own_v else (kc,):
+                cache[page, :, at] = float("nan")
+        rows.zero_()
+        torch.cuda.synchronize()
+        ops.gemm_skinny(x, w, rows)
+        ops.kv_store(rows, pos, seqs, table, kc, vc, ps, 1, H, KV, dk, dv if own_v else 0, status)
+        ops.attn_flex(rows[:, :H * dk], kc, vc, table, items, got, ps, 1, H, KV, dk, dv, dk ** -0.5, nsplit=nsplit, scratch=scratch,
                       max_rows=H // KV)
-        assert (got.float() - want.float()).abs().max().item() <= 2e-2, nsplit
+        assert int(status) == 0
+        assert (got.double().view(new, H, dv) - want).abs().max() <= 2 ** -7 * vals.abs().max(), nsplit
 
 
 def test_bias_table_is_spread_as_the_plain_bucket_says():
