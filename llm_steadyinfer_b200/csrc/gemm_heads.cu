@@ -11,7 +11,7 @@
 __global__ void __launch_bounds__(GH_WARPS * 32)
 gemm_heads_kernel(const __nv_bfloat16* __restrict__ a, long long a_row, long long a_head,
                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out, long long o_row,
-                  long long o_head, int M, int N, int K, int trigger) {
+                  long long o_head, int M, int N, int K, int trigger, int ahead) {
   extern __shared__ __align__(16) unsigned char gh_smem[];
   __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(gh_smem);          // [M][K]
   if (trigger) pdl_trigger();
@@ -20,7 +20,9 @@ gemm_heads_kernel(const __nv_bfloat16* __restrict__ a, long long a_row, long lon
   const int kc = K / 8;
   const int n = blockIdx.x * GH_WARPS + warp;
   const __nv_bfloat16* wr = w + ((size_t)h * N + (n < N ? n : 0)) * K;
-  // the column's first weights are on their way before the wait for the rows (a load of this kind stays before it)
+  // with the caller's word that w is older than the kernel before, the column's first weights are on their way before the wait for the rows (a
+  // load of this kind stays before it)
+  if (!ahead) pdl_wait();
   uint4 first = make_uint4(0, 0, 0, 0);
   if (lane < kc)
     asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(first.x), "=r"(first.y), "=r"(first.z), "=r"(first.w) : "l"(wr + lane * 8) : "memory");
@@ -62,7 +64,7 @@ gemm_heads_kernel(const __nv_bfloat16* __restrict__ a, long long a_row, long lon
 }
 
 SI_EXPORT int si_gemm_heads(const void* a, long long a_row, long long a_head, const void* w, void* out, long long o_row,
-                            long long o_head, int M, int H, int N, int K, cudaStream_t stream) {
+                            long long o_head, int M, int H, int N, int K, int ahead, cudaStream_t stream) {
   if (M <= 0 || H <= 0 || N <= 0) return 0;
   if (M > GH_MAX_ROWS || K % 8 || K <= 0 || H > 65535) return -2;
   const size_t smem = (size_t)M * K * sizeof(__nv_bfloat16);
@@ -70,6 +72,6 @@ SI_EXPORT int si_gemm_heads(const void* a, long long a_row, long long a_head, co
   const dim3 grid((N + GH_WARPS - 1) / GH_WARPS, H);
   const int trigger = si_pdl_trigger_mode((long long)grid.x * grid.y, 8LL * si_sm_count()) == 1;
   si_launch(gemm_heads_kernel, grid, dim3(GH_WARPS * 32), smem, stream,
-            (const __nv_bfloat16*)a, a_row, a_head, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, o_row, o_head, M, N, K, trigger);
+            (const __nv_bfloat16*)a, a_row, a_head, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, o_row, o_head, M, N, K, trigger, ahead);
   return si_last_error();
 }

@@ -1477,16 +1477,17 @@ def gemm_heads_ok(a, w, out, H: int, a_head: int, o_head: int) -> bool:
             and w.data_ptr() % 16 == 0 and a.shape[0] * w.shape[2] * 2 <= 48 * 1024)
 
 
-def gemm_heads(a, w, out, a_head: int, o_head: int) -> None:
+def gemm_heads(a, w, out, a_head: int, o_head: int, ahead: bool = False) -> None:
     """out[t, h*o_head : h*o_head + N] = a[t, h*a_head : h*a_head + K] @ w[h]^T for every head h of w [H, N, K], at
-    most 16 rows, in one launch (``a_head``, ``o_head``: distance between heads within a row, in elements)."""
+    most 16 rows, in one launch (``a_head``, ``o_head``: distance between heads within a row, in elements). ``ahead``: the caller's word that
+    no kernel of the step writes ``w``, which is then read before the kernel before this one is waited for."""
     _cuda(a, w, out)
     H, N, K = w.shape
     M = a.shape[0]
     _need(gemm_heads_ok(a, w, out, H, a_head, o_head), "gemm_heads: bf16, at most 16 rows, K a multiple of 8, aligned heads")
     _need(out.shape[0] == M and a.shape[1] >= (H - 1) * a_head + K and out.shape[1] >= (H - 1) * o_head + N, "gemm_heads: shapes")
-    f = _fn("gemm_heads", "si_gemm_heads", [_c_p, _c_ll, _c_ll, _c_p, _c_p, _c_ll, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_p])
-    _check(f(_ptr(a), a.stride(0), int(a_head), _ptr(w), _ptr(out), out.stride(0), int(o_head), M, H, N, K, _stream()),
+    f = _fn("gemm_heads", "si_gemm_heads", [_c_p, _c_ll, _c_ll, _c_p, _c_p, _c_ll, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_p])
+    _check(f(_ptr(a), a.stride(0), int(a_head), _ptr(w), _ptr(out), out.stride(0), int(o_head), M, H, N, K, 1 if ahead else 0, _stream()),
            f"gemm_heads(M={M}, heads={H}, N={N}, K={K})")
 
 

@@ -201,7 +201,7 @@ class LatentAttention(Mixer):
         if not absorbed:
             pass
         elif ops.gemm_heads_ok(q, self.ukT, q_full, H, dq + dr, rk + dr):          # few rows: all heads in one launch
-            ops.gemm_heads(q, self.ukT, q_full, dq + dr, rk + dr)
+            ops.gemm_heads(q, self.ukT, q_full, dq + dr, rk + dr, ahead=True)
         else:
             for i in range(H):
                 linear(q[:, i * (dq + dr): i * (dq + dr) + dq], self.ukT[i], q_full[:, i * (rk + dr): i * (rk + dr) + rk], ctx.status)
@@ -251,7 +251,7 @@ class LatentAttention(Mixer):
                                   ctx.seq_slots, H, 1, rk + dr, rk, self.scale, self.window or 0, sink=self.sink,
                                   status=ctx.status)
         if ops.gemm_heads_ok(o_lat, self.uv, attn, H, rk, dv):
-            ops.gemm_heads(o_lat, self.uv, attn, rk, dv)
+            ops.gemm_heads(o_lat, self.uv, attn, rk, dv, ahead=True)
         else:
             for i in range(H):
                 linear(o_lat[:, i * rk:(i + 1) * rk], self.uv[i], attn[:, i * dv:(i + 1) * dv], ctx.status)

@@ -508,6 +508,23 @@ def test_per_head_product(M, H, N, K, a_head, o_head):
         assert (out[:, N:o_head] == 7.0).all()            # nothing written between the heads
 
 
+def test_per_head_product_reads_matrices_that_the_kernel_before_makes():
+    """The matrices of sixteen heads, each a row of a product that lets the next kernel start early: without the caller's word the product a
+    head waits for them (their place holds not-a-numbers before). Sums of 32 in fp32 and one rounding to 8 bits: 2^-8 of the result."""
+    from llm_steadyinfer_b200.csrc import ops
+    torch.manual_seed(3)
+    H, N, K, deep = 16, 8, 32, 2048
+    x, big = torch.randn(H, deep, device="cuda:0").bfloat16(), (torch.randn(N * K, deep, device="cuda:0") / deep ** 0.5).bfloat16()
+    a = torch.randn(4, H * K, device="cuda:0").bfloat16()
+    w = torch.full((H, N * K), float("nan"), device="cuda:0").bfloat16()
+    out = torch.zeros(4, H * N, device="cuda:0").bfloat16()
+    torch.cuda.synchronize()
+    ops.gemm_skinny(x, big, w)
+    ops.gemm_heads(a, w.view(H, N, K), out, K, N)
+    want = torch.einsum("mhk,hnk->mhn", a.double().view(4, H, K), w.double().view(H, N, K)).reshape(4, H * N)
+    assert ((out.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5).all()
+
+
 def test_command_line_serves_the_design(folders, tmp_path):
     """The serving program on a Mivorax folder: requests of random lengths arriving over time, sampling, a pool that
     is used again; and once more on random weights drawn from a configuration file."""
