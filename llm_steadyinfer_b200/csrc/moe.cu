@@ -650,9 +650,9 @@ template <int MT>
 __global__ void __launch_bounds__(STREAM_WARPS * 32, 2) moe_pairs_kernel(const bf16* __restrict__ A, long long a_stride,
     const int* __restrict__ ids, int a_div, const bf16* __restrict__ W, void* __restrict__ C, long long c_stride, int c_f32, int P, int E,
     int N, int K, int act, float limit, float alpha, float shift, const MoeShared sh) {
-  constexpr int UP = MT == 1 ? 8 : 4;
+  constexpr int UP = MT == 1 ? 8 : 4, PLACES = MT * 8;  // places that a tile's sums have room for
   __shared__ float red[2][STREAM_WARPS][MT][32][4];
-  __shared__ int place[32][16], count[32], expert[32], distinct;
+  __shared__ int place[32][PLACES], count[32], expert[32], entries;
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nx = (N + 15) / 16, ns = (sh.N + 15) / 16;
@@ -696,17 +696,21 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32, 2) moe_pairs_kernel(const b
   if (warp == 0) {
     int id = lane < P ? ids[lane] : -1;
     if (id < 0 || id >= E) id = -1;                      // (identity experts and none: no product)
+    // An expert is one entry, as a row's choices are different experts; ids that name one more often than its rows make an entry of every
+    // PLACES places.
     const unsigned same = __match_any_sync(0xffffffffu, id), below = (1u << lane) - 1;
-    const unsigned leaders = __ballot_sync(0xffffffffu, id >= 0 && __ffs(same) - 1 == lane);
+    const int rank = __popc(same & below), first = rank - rank % PLACES;
+    const unsigned leaders = __ballot_sync(0xffffffffu, id >= 0 && rank == first);
     if (id >= 0) {
-      const int at = __popc(leaders & ((1u << (__ffs(same) - 1)) - 1)), rank = __popc(same & below);
-      if (rank < 16) place[at][rank] = lane;             // (a row's choices are different experts: at most 16)
-      if (rank == 0) { expert[at] = id; count[at] = min(__popc(same), 16); }
+      const int leader = first == 0 ? __ffs(same) - 1 : (int)__fns(same, 0, first + 1);
+      const int at = __popc(leaders & ((1u << leader) - 1));
+      place[at][rank - first] = lane;
+      if (rank == first) { expert[at] = id; count[at] = min(__popc(same) - first, PLACES); }
     }
-    if (lane == 0) distinct = __popc(leaders);
+    if (lane == 0) entries = __popc(leaders);
   }
   __syncthreads();
-  const int total = ns + distinct * nx;
+  const int total = ns + entries * nx;
   if (q < total) {
     if (q >= ns) load_w();
     load_x();

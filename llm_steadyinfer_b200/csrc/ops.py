@@ -2088,7 +2088,7 @@ def moe_gemm_pairs(a, ids, w, out, by_row: bool, act: str = "none", limit: float
                    shared=None) -> None:
     """The grouped product without a plan, for few pairs: out[p, :] = act(a[row, :] @ w[e]^T) for the pair p of ``ids`` int32
     [T, top] that chose expert e, row = p / top (``by_row``: ``a`` [T, K]) or p (``a`` [T * top, K]). Pairs whose id is not below
-    E are left alone; a row's choices are different experts (at most 16 pairs an expert). ``out`` and ``act`` as for ``moe_gemm``.
+    E are left alone; a row's choices are different experts (where they are not, the expert's weights are read again for what its tile has no room for). ``out`` and ``act`` as for ``moe_gemm``.
     ``shared`` {"a" [T, K'], "w" [N', K'], "out", "form" one of ``MOE_SHARED_FORMS``, "bias", "limit", "alpha"}: a product that every row
     takes, in the same launch, as ``gemm_skinny`` and its gated forms (rows of w in groups of 8 gates and 8 ups) give it."""
     _cuda(a, ids, w, out)

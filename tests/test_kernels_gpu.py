@@ -1306,6 +1306,20 @@ def test_experts_weights_streamed_for_few_places(T, top, E, N, K, act):
         assert torch.equal(planned[place_of.view(-1)[p]], out[p])
 
 
+@pytest.mark.parametrize("T,ids", [(2, [[0] * 16, [0] * 16]), (8, [[0, 0, 1, 0]] * 8), (3, [[1, 0, 1, 1, 1, 1]] * 3), (1, [[2] * 32]), (16, [[1, 1]] * 16)])
+def test_pairs_that_name_an_expert_more_often_than_there_are_rows(T, ids):
+    """Ids that no router makes, an expert named up to 32 times, against float64: more places than one tile has sums for. Sums of K products of
+    bf16 numbers of size one in fp32, the weights divided by sqrt(K): 2e-6 sqrt(K)."""
+    g = torch.Generator().manual_seed(T)
+    o, E, N, K = ops(), 3, 40, 264
+    a, w = torch.randn(T, K, generator=g).to(torch.bfloat16), (torch.randn(E, N, K, generator=g) / K ** 0.5).to(torch.bfloat16)
+    ids = torch.tensor(ids, dtype=torch.int32)
+    out = torch.full((ids.numel(), N), 7.0, device=DEV)
+    o.moe_gemm_pairs(a.to(DEV), ids.to(DEV), w.to(DEV), out, True)
+    want = torch.einsum("pk,pnk->pn", a.double().repeat_interleave(ids.shape[1], 0), w.double()[ids.flatten().long()])
+    assert (out.cpu().double() - want).abs().max().item() <= 2e-6 * K ** 0.5 * max(1.0, want.abs().max().item())
+
+
 @pytest.mark.parametrize("form", ["none", "relu2", "silu_glu", "glu_limited"])
 @pytest.mark.parametrize("T,top,N,K,sN,sK", [(1, 1, 16, 8, 16, 8), (3, 2, 40, 264, 304, 520), (9, 2, 64, 520, 16, 2056), (16, 2, 48, 264, 1008, 264)])
 def test_shared_product_beside_the_experts(T, top, N, K, sN, sK, form):
