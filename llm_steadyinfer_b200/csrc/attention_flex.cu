@@ -49,7 +49,7 @@ struct FlexParams {
   int window, chunk, nsplit;
   int ahead;                // the caller's word that keys before an item's first position, pages and biases are older than the kernel before this one
   int block_n;              // keys of a tile
-  int trigger;              // the merge is launched while the last shares store theirs
+  int trigger;              // the merge is launched while the last shares store theirs; a merge whose kernel behind is a small one lets that start
   int* status;
 };
 
@@ -440,7 +440,7 @@ attn_flex_kernel(const FlexParams p) {
 __global__ void __launch_bounds__(128) attn_flex_merge_kernel(const FlexParams p, int col_blocks) {
   __shared__ float w[64];
   __shared__ float s_inv;
-  if (p.out_f32) pdl_trigger();
+  if (p.trigger) pdl_trigger();
   const AttnItem item = p.items[blockIdx.x];
   pdl_wait();
   if (item.ntok <= 0 || item.seq < 0 || item.seq >= p.num_seqs) return;
@@ -586,6 +586,7 @@ SI_EXPORT int si_attn_flex(const void* q, long long q_stride, const void* k_cach
   if (nsplit > 1) {
     const int rows = max_rows > 0 && max_rows < FLEX_M ? max_rows : FLEX_M, col_blocks = (dv + 127) / 128;
     p.block_n = block_n;
+    p.trigger = p.out_f32 && si_pdl_trigger_enabled();
     si_launch(attn_flex_merge_kernel, dim3(num_items, KV * p.hparts, rows * col_blocks), dim3(128), 0, stream, p, col_blocks);
   }
   return si_last_error();

@@ -187,8 +187,8 @@ template <typename T>
 __global__ void kv_store_kernel(const T* __restrict__ qkv, long long row_stride, const int* __restrict__ positions,
                                 const int* __restrict__ row_seq, const int* __restrict__ block_table,
                                 int table_width, T* __restrict__ k_cache, T* __restrict__ v_cache, int num_pages,
-                                int page_size, int num_seqs, int H, int KV, int dk, int dv, int* status) {
-  pdl_trigger_small();
+                                int page_size, int num_seqs, int H, int KV, int dk, int dv, int trigger, int* status) {
+  if (trigger) pdl_trigger();
   const int t = blockIdx.x;
   const int pos = positions[t];                     // copied in before the step's first kernel, like the pages
   const long long page = page_of(block_table, table_width, num_pages, page_size, num_seqs, row_seq[t], pos, status);
@@ -213,14 +213,15 @@ SI_EXPORT int si_kv_store(const void* qkv, int dtype, long long row_stride, cons
                           cudaStream_t stream) {
   if (num_tokens <= 0) return 0;
   const int threads = num_tokens <= si_sm_count() ? 512 : 128;      // a decode row's entries all at once
+  const int trigger = si_pdl_trigger_small(num_tokens);
   if (dtype == SI_BF16)
     si_launch(kv_store_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), 0, stream, (const __nv_bfloat16*)qkv,
               row_stride, positions, row_seq, block_table, table_width, (__nv_bfloat16*)k_cache,
-              (__nv_bfloat16*)v_cache, num_pages, page_size, num_seqs, H, KV, dk, dv, status);
+              (__nv_bfloat16*)v_cache, num_pages, page_size, num_seqs, H, KV, dk, dv, trigger, status);
   else
     si_launch(kv_store_kernel<float>, dim3(num_tokens), dim3(threads), 0, stream, (const float*)qkv, row_stride,
               positions, row_seq, block_table, table_width, (float*)k_cache, (float*)v_cache, num_pages,
-              page_size, num_seqs, H, KV, dk, dv, status);
+              page_size, num_seqs, H, KV, dk, dv, trigger, status);
   return si_last_error();
 }
 
@@ -243,10 +244,10 @@ __global__ void __launch_bounds__(1024) latent_prepare_kernel(const T* __restric
                                       int rd, const int* __restrict__ positions, const int* __restrict__ row_seq,
                                       const int* __restrict__ block_table, int table_width, T* __restrict__ k_cache,
                                       int num_pages, int page_size, int num_seqs, int H, int dq, int dr, int rk,
-                                      int interleaved, float rot_scale, int* status) {
+                                      int interleaved, float rot_scale, int trigger, int* status) {
   __shared__ float red[33];
   extern __shared__ float sc_table[];              // the row's sines, then its cosines: rd / 2 each
-  pdl_trigger_small();
+  if (trigger) pdl_trigger();
   const int t = blockIdx.x;
   const int pos = positions[t];                    // copied in before the step's first kernel, like the pages
   const int seq = row_seq[t];
@@ -322,19 +323,20 @@ SI_EXPORT int si_latent_prepare(const void* kv, int dtype, long long kv_stride, 
   // a thread an entry of the queries' rotated parts while the rows are no more than the SMs: a decode row waits for as many sines as
   // a thread takes in turn (four rows of 16 heads and a rotated part of 64: 128 threads 9.6 us, 1,024
   // 6.1)
+  const int trigger = si_pdl_trigger_small(num_tokens);
   const int threads = num_tokens <= si_sm_count() ? (H * dr >= 1024 ? 1024 : H * dr >= 512 ? 512 : 256) : 128;
   if (dtype == SI_BF16)
     si_launch(latent_prepare_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), (size_t)rd * sizeof(float), stream, (const __nv_bfloat16*)kv,
               kv_stride, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)q_full, qf_stride, (__nv_bfloat16*)q_exp,
               qe_stride, norm_w, eps, inv_freq,
               rd, positions, row_seq, block_table, table_width, (__nv_bfloat16*)k_cache, num_pages, page_size,
-              num_seqs, H, dq, dr, rk, interleaved, rot_scale, status);
+              num_seqs, H, dq, dr, rk, interleaved, rot_scale, trigger, status);
   else
     si_launch(latent_prepare_kernel<float>, dim3(num_tokens), dim3(threads), (size_t)rd * sizeof(float), stream, (const float*)kv, kv_stride,
               (const float*)q, q_stride, (float*)q_full, qf_stride, (float*)q_exp, qe_stride, norm_w, eps, inv_freq, rd,
               positions, row_seq,
               block_table, table_width, (float*)k_cache, num_pages, page_size, num_seqs, H, dq, dr, rk, interleaved,
-              rot_scale, status);
+              rot_scale, trigger, status);
   return si_last_error();
 }
 

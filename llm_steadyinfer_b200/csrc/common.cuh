@@ -115,23 +115,19 @@ __device__ __forceinline__ void l2_prefetch_share(const void* base, long long by
 // places of their own later blocks.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-// For a kernel with a handful of blocks (a decode step's rows) that stores the newest keys: the kernel behind it, which reads the cache,
-// starts on the keys that are older than the step.
-__device__ __forceinline__ void pdl_trigger_small() {
-  if (gridDim.x * gridDim.y * gridDim.z <= 64u) pdl_trigger();
-}
-
-// SI_PDL_TRIGGER (the kernels above, the tcgen05 kernels and the experts of few rows trigger whatever it says): 0 no other kernel triggers;
-// 1 the small kernels; 2 (default) also every kernel of one wave of blocks, at its start.
+// SI_PDL_TRIGGER: 0 no kernel triggers but the tcgen05 ones, which always do; 1 the small kernels too; 2 (default; higher levels are the same)
+// also every kernel of one wave of blocks, at its start.
 static inline int si_pdl_trigger_level() {
   static int level = -1;
   if (level < 0) {
     const char* e = getenv("SI_PDL_TRIGGER");
-    level = (e && e[0] >= '0' && e[0] <= '2') ? e[0] - '0' : 2;
+    level = (e && (e[0] == '0' || e[0] == '1')) ? e[0] - '0' : 2;
   }
   return level;
 }
 static inline bool si_pdl_trigger_enabled() { return si_pdl_trigger_level() >= 1; }
+// Whether a small kernel of `blocks` blocks, a handful as a decode step's rows make them, triggers: 1 or 0.
+static inline int si_pdl_trigger_small(long long blocks) { return blocks <= 64 && si_pdl_trigger_enabled() ? 1 : 0; }
 // Whether a kernel of `blocks` blocks, `slots` of which run at once, triggers at its start: 1 or 0.
 static inline int si_pdl_trigger_mode(long long blocks, long long slots) { return blocks <= slots && si_pdl_trigger_level() >= 2 ? 1 : 0; }
 

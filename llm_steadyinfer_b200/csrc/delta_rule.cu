@@ -989,8 +989,8 @@ SI_EXPORT int si_channel_delta_group_scan(const float* rec, const float* sc, con
 template <typename T>
 __global__ void __launch_bounds__(256) head_norm_gate_kernel(const float* __restrict__ o, long long o_stride, const T* __restrict__ z,
     long long z_stride, const float* __restrict__ w, T* __restrict__ out, long long out_stride, long long pairs, int H, int dv,
-    float eps, long long w_head_stride, float post, int sigmoid) {
-  pdl_trigger_small();
+    float eps, long long w_head_stride, float post, int sigmoid, int trigger) {
+  if (trigger) pdl_trigger();
   pdl_wait();
   const long long wi = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (wi >= pairs) return;
@@ -1017,11 +1017,12 @@ SI_EXPORT int si_head_norm_gate(const float* o, long long o_stride, const void* 
   if (H <= 0 || dv <= 0) return -2;
   const long long pairs = (long long)rows * H;
   const dim3 grid((unsigned)((pairs + 7) / 8)), block(256);
+  const int trigger = si_pdl_trigger_small(grid.x);
   if (dtype == SI_BF16)
     si_launch(head_norm_gate_kernel<__nv_bfloat16>, grid, block, 0, stream, o, o_stride, (const __nv_bfloat16*)z, z_stride, w,
-              (__nv_bfloat16*)out, out_stride, pairs, H, dv, eps, w_head_stride, post, sigmoid);
+              (__nv_bfloat16*)out, out_stride, pairs, H, dv, eps, w_head_stride, post, sigmoid, trigger);
   else
     si_launch(head_norm_gate_kernel<float>, grid, block, 0, stream, o, o_stride, (const float*)z, z_stride, w, (float*)out,
-              out_stride, pairs, H, dv, eps, w_head_stride, post, sigmoid);
+              out_stride, pairs, H, dv, eps, w_head_stride, post, sigmoid, trigger);
   return si_last_error();
 }

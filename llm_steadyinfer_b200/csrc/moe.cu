@@ -39,8 +39,8 @@ typedef __nv_bfloat16 bf16;
 template <typename T, bool EARLY>
 __global__ void __launch_bounds__(EARLY ? 1024 : 256) moe_route_kernel(const T* __restrict__ x, long long x_stride, const T* __restrict__ w,
     int E, int extra, int d, int top, float scale, int mode, int renorm, float renorm_eps, int groups, int keep,
-    const float* __restrict__ choice_bias, int* __restrict__ ids, float* __restrict__ wts, float* __restrict__ gates) {
-  if (EARLY) pdl_trigger();
+    const float* __restrict__ choice_bias, int* __restrict__ ids, float* __restrict__ wts, float* __restrict__ gates, int trigger) {
+  if (trigger) pdl_trigger();
   extern __shared__ float rsm[];                       // the row [d], scores [E + extra], used [E], choice keys [E] (and groups' scores)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const long long t = blockIdx.x;
@@ -191,6 +191,7 @@ SI_EXPORT int si_moe_route(const void* x, int dtype, long long x_stride, const v
   const size_t smem = (size_t)(d + 3 * E + extra + (groups > 1 ? groups : 0)) * sizeof(float);
   if (smem > 160 * 1024) return -2;
   const bool early = rows <= si_sm_count();
+  const int trigger = early ? si_pdl_trigger_mode(rows, si_sm_count()) : 0;
   const int warps = E + extra < 32 ? E + extra : 32;
   const dim3 grid(rows), block(early ? 32 * warps : E + extra >= 8 ? 256 : 128);
 #define ROUTE_LAUNCH(T)                                                                                                \
@@ -202,7 +203,7 @@ SI_EXPORT int si_moe_route(const void* x, int dtype, long long x_stride, const v
       configured = smem;                                                                                             \
     }                                                                                                                \
     si_launch(early ? moe_route_kernel<T, true> : moe_route_kernel<T, false>, grid, block, smem, stream, (const T*)x, x_stride, (const T*)w, E, extra, d, top, scale, \
-              mode, renorm, renorm_eps, groups, keep, choice_bias, ids, wts, gates);                                                           \
+              mode, renorm, renorm_eps, groups, keep, choice_bias, ids, wts, gates, trigger);                                                        \
   }
   if (dtype == SI_BF16) ROUTE_LAUNCH(bf16) else ROUTE_LAUNCH(float)
 #undef ROUTE_LAUNCH
@@ -649,11 +650,11 @@ __device__ __forceinline__ uint4 moe_ld_if(const bf16* p, bool take, bool stream
 template <int MT>
 __global__ void __launch_bounds__(STREAM_WARPS * 32, 2) moe_pairs_kernel(const bf16* __restrict__ A, long long a_stride,
     const int* __restrict__ ids, int a_div, const bf16* __restrict__ W, void* __restrict__ C, long long c_stride, int c_f32, int P, int E,
-    int N, int K, int act, float limit, float alpha, float shift, const MoeShared sh) {
+    int N, int K, int act, float limit, float alpha, float shift, int trigger, const MoeShared sh) {
   constexpr int UP = MT == 1 ? 8 : 4, PLACES = MT * 8;  // places that a tile's sums have room for
   __shared__ float red[2][STREAM_WARPS][MT][32][4];
   __shared__ int place[32][PLACES], count[32], expert[32], entries;
-  pdl_trigger();
+  if (trigger) pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nx = (N + 15) / 16, ns = (sh.N + 15) / 16;
   // The tiles go to the blocks forwards and backwards in turn: the first ones (the shared matrix's) may be the longer ones.
@@ -896,9 +897,10 @@ SI_EXPORT int si_moe_gemm_pairs(const void* A, long long a_stride, int a_div, co
     sh.bias = s_bias; sh.rows = T; sh.N = sN; sh.K = sK; sh.form = s_form; sh.limit = s_limit; sh.alpha = s_alpha;
     tiles += (sN + 15) / 16;
   }
-  const long long slots = 2LL * si_sm_count();
-  si_launch(T <= 8 ? moe_pairs_kernel<1> : moe_pairs_kernel<2>, dim3((unsigned)(tiles < slots ? tiles : slots)), dim3(STREAM_WARPS * 32), 0, stream,
-            (const bf16*)A, a_stride, ids, a_div, (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, P, E, N, K, act, limit, alpha, shift, sh);
+  const long long slots = 2LL * si_sm_count(), grid = tiles < slots ? tiles : slots;
+  si_launch(T <= 8 ? moe_pairs_kernel<1> : moe_pairs_kernel<2>, dim3((unsigned)grid), dim3(STREAM_WARPS * 32), 0, stream,
+            (const bf16*)A, a_stride, ids, a_div, (const bf16*)W, C, c_stride, c_dtype == SI_F32 ? 1 : 0, P, E, N, K, act, limit, alpha, shift,
+            si_pdl_trigger_mode(grid, slots), sh);
   return si_last_error();
 }
 
@@ -944,8 +946,8 @@ template <typename TY, typename T>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const TY* __restrict__ Y, long long y_stride, const int* __restrict__ place_of,
     const float* __restrict__ wts, int top, const T* __restrict__ shared, long long shared_stride, const float* __restrict__ gate,
     int gate_stride, T* __restrict__ out, long long out_stride, int d, const int* __restrict__ ids, int real,
-    const T* __restrict__ x, long long x_stride) {
-  pdl_trigger_small();
+    const T* __restrict__ x, long long x_stride, int trigger) {
+  if (trigger) pdl_trigger();
   pdl_wait();
   const long long t = blockIdx.x;
   for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < d; i += blockDim.x * gridDim.y) {
@@ -968,15 +970,16 @@ SI_EXPORT int si_moe_combine(const void* Y, int y_dtype, long long y_stride, con
   if (top <= 0 || d <= 0 || (ids && !x)) return -2;
   const dim3 block(d >= 1024 ? 256 : 128);
   const dim3 grid(rows, si_row_shares(rows, d, block.x));
+  const int trigger = si_pdl_trigger_small((long long)grid.x * grid.y);
   if (dtype == SI_BF16 && y_dtype == SI_F32)
     si_launch(moe_combine_kernel<float, bf16>, grid, block, 0, stream, (const float*)Y, y_stride, place_of, wts, top,
-              (const bf16*)shared, shared_stride, gate, gate_stride, (bf16*)out, out_stride, d, ids, real, (const bf16*)x, x_stride);
+              (const bf16*)shared, shared_stride, gate, gate_stride, (bf16*)out, out_stride, d, ids, real, (const bf16*)x, x_stride, trigger);
   else if (dtype == SI_BF16 && y_dtype == SI_BF16)
     si_launch(moe_combine_kernel<bf16, bf16>, grid, block, 0, stream, (const bf16*)Y, y_stride, place_of, wts, top,
-              (const bf16*)shared, shared_stride, gate, gate_stride, (bf16*)out, out_stride, d, ids, real, (const bf16*)x, x_stride);
+              (const bf16*)shared, shared_stride, gate, gate_stride, (bf16*)out, out_stride, d, ids, real, (const bf16*)x, x_stride, trigger);
   else if (dtype == SI_F32 && y_dtype == SI_F32)
     si_launch(moe_combine_kernel<float, float>, grid, block, 0, stream, (const float*)Y, y_stride, place_of, wts, top,
-              (const float*)shared, shared_stride, gate, gate_stride, (float*)out, out_stride, d, ids, real, (const float*)x, x_stride);
+              (const float*)shared, shared_stride, gate, gate_stride, (float*)out, out_stride, d, ids, real, (const float*)x, x_stride, trigger);
   else
     return -2;
   return si_last_error();

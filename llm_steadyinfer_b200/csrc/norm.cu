@@ -203,8 +203,8 @@ template <typename TX, typename TW>
 __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const TX* __restrict__ x, TX* __restrict__ out,
                                                            const TW* __restrict__ weight, long long num_rows, int n, int inner,
                                                            long long x_outer, long long x_inner, long long o_outer,
-                                                           long long o_inner, float eps) {
-  pdl_trigger_small();
+                                                           long long o_inner, float eps, int trigger) {
+  if (trigger) pdl_trigger();
   pdl_wait();
   const long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= num_rows) return;
@@ -228,7 +228,7 @@ static int rows_launch(const void* x, void* out, const void* weight, long long n
   const long long blocks = (num_rows + 7) / 8;
   if (blocks > 0x7fffffffLL) return -2;
   si_launch(rmsnorm_rows_kernel<TX, TW>, dim3((unsigned)blocks), dim3(256), 0, stream, (const TX*)x, (TX*)out, (const TW*)weight,
-            num_rows, n, inner, x_outer, x_inner, o_outer, o_inner, eps);
+            num_rows, n, inner, x_outer, x_inner, o_outer, o_inner, eps, si_pdl_trigger_small(blocks));
   return si_last_error();
 }
 
@@ -306,9 +306,9 @@ template <typename TX, typename TW, int CHUNKS>
 __global__ void __launch_bounds__(512) add_norm_general_vec_kernel(float* __restrict__ resid, const TX* __restrict__ delta,
     const float* __restrict__ delta_bias, const TW* __restrict__ delta_weight, float delta_eps,
     const float* __restrict__ extra, const float* __restrict__ vec, const int* __restrict__ rows,
-    const TW* __restrict__ weight, TX* __restrict__ out, int hidden, float eps) {
+    const TW* __restrict__ weight, TX* __restrict__ out, int hidden, float eps, int trigger) {
   __shared__ float scratch[33];
-  pdl_trigger_small();
+  if (trigger) pdl_trigger();
   const int nchunks = hidden >> 3;
   if (gridDim.x <= 64) {
 #pragma unroll
@@ -418,7 +418,8 @@ static int general_launch(float* resid, const void* delta, const float* delta_bi
     const int per = (nchunks + threads - 1) / threads;
 #define SI_GENERAL_VEC(C)                                                                                             \
     si_launch(add_norm_general_vec_kernel<TX, TW, C>, dim3(num_rows), dim3(threads), 0, stream, resid, (const TX*)delta,   \
-              delta_bias, (const TW*)delta_weight, delta_eps, extra, vec, rows, (const TW*)weight, (TX*)out, hidden, eps)
+              delta_bias, (const TW*)delta_weight, delta_eps, extra, vec, rows, (const TW*)weight, (TX*)out, hidden, eps,      \
+              si_pdl_trigger_small(num_rows))
     if (per <= 1) SI_GENERAL_VEC(1);
     else if (per <= 2) SI_GENERAL_VEC(2);
     else SI_GENERAL_VEC(4);

@@ -72,12 +72,12 @@ __global__ void __launch_bounds__(THREADS) qk_prepare_kernel(T* __restrict__ row
     const float* __restrict__ k_w, float eps, const float* __restrict__ inv_freq, int rd, int interleaved,
     const int* __restrict__ positions, const int* __restrict__ row_seq, const int* __restrict__ block_table, int table_width,
     T* __restrict__ k_cache, T* __restrict__ v_cache, int num_pages, int page_size, int num_seqs, int NQ, int NK, int NV,
-    int dk, int dv, T* __restrict__ q_out, long long q_out_stride, int maps, int whole, float rot_scale, int* status) {
+    int dk, int dv, T* __restrict__ q_out, long long q_out_stride, int maps, int whole, float rot_scale, int trigger, int* status) {
   extern __shared__ float sc_table[];                  // the row's sines, then its cosines: rd / 2 each, once for all vectors
   __shared__ float red[33];
   // Positions, sequences and pages were copied in before the step's first kernel: the row's place and its sines are ready before the wait
   // for the projection. (Behind it: two rows of 48 vectors 4.5 us, now 4.3; three of 20 with one norm over all 7.0, now 5.0.)
-  pdl_trigger_small();
+  if (trigger) pdl_trigger();
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int pos = positions[t];
@@ -173,7 +173,7 @@ SI_EXPORT int si_qk_prepare(void* rows, int dtype, long long row_stride, const f
 #define QK_LAUNCH(T, ITEMS)                                                                                              \
   si_launch(threads <= 256 ? qk_prepare_kernel<T, ITEMS, 256> : qk_prepare_kernel<T, ITEMS, 1024>, grid, block, smem, stream, (T*)rows, row_stride, q_w, k_w, eps, inv_freq, rd,      \
             interleaved, positions, row_seq, block_table, table_width, (T*)k_cache, (T*)v_cache, num_pages, page_size,   \
-            num_seqs, NQ, NK, NV, dk, dv, (T*)q_out, q_out_stride, maps, whole, rot_scale, status)
+            num_seqs, NQ, NK, NV, dk, dv, (T*)q_out, q_out_stride, maps, whole, rot_scale, si_pdl_trigger_small(grid.x), status)
   if (dtype == SI_BF16) {
     if (dk <= 64) QK_LAUNCH(__nv_bfloat16, 1);
     else if (dk <= 128) QK_LAUNCH(__nv_bfloat16, 2);
@@ -197,8 +197,8 @@ SI_EXPORT int si_qk_prepare(void* rows, int dtype, long long row_stride, const f
 template <typename TA, typename T>
 __global__ void __launch_bounds__(256) diff_combine_kernel(const TA* __restrict__ a, long long a_stride, const T* __restrict__ gate,
     long long gate_stride, T* __restrict__ out, long long out_stride, long long pairs, int H, int dv, int ratio, float lambda,
-    float eps, float post) {
-  pdl_trigger_small();
+    float eps, float post, int trigger) {
+  if (trigger) pdl_trigger();
   pdl_wait();
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= pairs) return;
@@ -226,15 +226,16 @@ SI_EXPORT int si_diff_combine(const void* a, int a_dtype, long long a_stride, co
   if (H <= 0 || dv <= 0 || ratio <= 0 || H % ratio) return -2;
   const long long pairs = (long long)rows * H;
   const dim3 grid((unsigned)((pairs + 7) / 8)), block(256);
+  const int trigger = si_pdl_trigger_small(grid.x);
   if (dtype == SI_BF16 && a_dtype == SI_F32)
     si_launch(diff_combine_kernel<float, __nv_bfloat16>, grid, block, 0, stream, (const float*)a, a_stride,
-              (const __nv_bfloat16*)gate, gate_stride, (__nv_bfloat16*)out, out_stride, pairs, H, dv, ratio, lambda, eps, post);
+              (const __nv_bfloat16*)gate, gate_stride, (__nv_bfloat16*)out, out_stride, pairs, H, dv, ratio, lambda, eps, post, trigger);
   else if (dtype == SI_BF16 && a_dtype == SI_BF16)
     si_launch(diff_combine_kernel<__nv_bfloat16, __nv_bfloat16>, grid, block, 0, stream, (const __nv_bfloat16*)a, a_stride,
-              (const __nv_bfloat16*)gate, gate_stride, (__nv_bfloat16*)out, out_stride, pairs, H, dv, ratio, lambda, eps, post);
+              (const __nv_bfloat16*)gate, gate_stride, (__nv_bfloat16*)out, out_stride, pairs, H, dv, ratio, lambda, eps, post, trigger);
   else if (dtype == SI_F32 && a_dtype == SI_F32)
     si_launch(diff_combine_kernel<float, float>, grid, block, 0, stream, (const float*)a, a_stride, (const float*)gate,
-              gate_stride, (float*)out, out_stride, pairs, H, dv, ratio, lambda, eps, post);
+              gate_stride, (float*)out, out_stride, pairs, H, dv, ratio, lambda, eps, post, trigger);
   else
     return -2;
   return si_last_error();

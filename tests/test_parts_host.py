@@ -1,5 +1,9 @@
 """What the parts tell the engine about themselves, checked on the host (no kernel runs): which steps may be
-recorded in a CUDA graph, which weights a part streams first, which norms take a hint to fetch ahead."""
+recorded in a CUDA graph, which weights a part streams first, which norms take a hint to fetch ahead. And what the kernels' sources promise
+of the switch for early launches."""
+import os
+import re
+
 import torch
 
 from llm_steadyinfer_b200.config import config_from_dict
@@ -71,3 +75,20 @@ def test_block_arrangements_are_a_registry():
     b = Block(None, None, None, None, "host_test_order")
     assert b.forward(None, None, None, None) == "out" and calls == [b] and b.capturable is False
     assert Block(None, None, None, None).capturable is True          # the built-in arrangement can be recorded
+
+
+def test_early_launches_go_by_the_switch_but_for_the_tcgen05_kernels():
+    """SI_PDL_TRIGGER=0 leaves no other kernel that lets the next one start early: every trigger stands behind an argument, and every such
+    argument comes from the functions that read the switch."""
+    from llm_steadyinfer_b200.csrc import build
+    guarded = 0
+    for name in build.kernel_sources():
+        with open(os.path.join(build.CSRC_DIR, name + ".cu"), encoding="utf-8") as f:
+            code = [line.split("//")[0] for line in f]
+        for line in code:
+            if "pdl_trigger()" in line and name not in ("gemm_tc05", "attention_tc05"):
+                assert re.search(r"if \((p\.)?trigger\) pdl_trigger\(\);", line), f"{name}: {line}"
+                guarded += 1
+            if re.search(r"\btrig(ger)? = ", line):
+                assert "si_pdl_trigger_" in line or line.strip() == "p.trigger = 0;", f"{name}: {line}"
+    assert guarded >= 20
