@@ -483,8 +483,8 @@ class Attention(Mixer):
             if max(self.hs, self.vs) <= 64 and plan["dec_rows"] <= 8 and budget < len(dec) <= 2 * self.target_blocks() // self.KV:
                 budget = 2 * self.target_blocks() // self.KV
             # Many items that all start at once, four blocks a multiprocessor, have room for a second round of short shares: beside 60 short
-            # sequences a long one is else cut in two or three. 61 sequences of 32 to 2,016 keys, 32 heads of 64: 17.1 us in one round,
-            # 16.1 so; a pass of 8 steps 9.43 ms, 9.30.
+            # sequences a long one is else cut in two or three (figures beside the cut). A pass of 8 steps of 61 sequences of 32 to 2,016
+            # keys, 32 heads of 64: 9.44 ms in one round, 9.28 so.
             many = max(self.hs, self.vs) <= 64 and plan["dec_rows"] <= 8 and budget // 2 < len(dec) <= budget
             entries = (budget + (budget // 2 if many else 0)) if len(dec) <= budget else budget + len(dec) + min(3 * len(dec), 2 * budget)
             work = ops.split_work(tiles, budget, entries, MAX_SPLITS, MIN_TILES_PER_SPLIT, second_round=many)

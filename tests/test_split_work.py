@@ -18,7 +18,7 @@ def test_every_share_is_listed_once_and_slots_do_not_overlap():
         tiles = [rng.choice([0, 1, 2, 3, 5, 17, 64, 128, 500]) for _ in range(n)]
         budget = rng.choice([1, 5, 37, 148])
         entries = budget + n
-        work = split_work(tiles, budget, entries, 32, rng.choice([1, 2, 4]))
+        work = split_work(tiles, budget, entries, 32, rng.choice([1, 2, 4]), second_round=rng.random() < 0.5)
         assert work.shape == (entries, 4) and work.dtype == np.int32
         sp, live = _shares(work)
         assert set(sp) == {i for i, t in enumerate(tiles) if t > 0}
@@ -78,3 +78,36 @@ def test_shares_that_run_at_once_need_no_more_entries():
         tiles = [rng.choice([0, 1, rng.randint(1, 40), rng.randint(1, 2000)]) for _ in range(rng.randint(1, budget))]
         sp, live = _shares(split_work(tiles, budget, budget, 32, 2))
         assert len(live) <= budget and all((sp.get(i, 0) >= 1) == (t > 0) for i, t in enumerate(tiles))
+
+
+def test_a_second_round_is_cut_by_the_longest_share_it_leaves():
+    """Finer cuts than one round holds: only where the longest share shrinks by a quarter at least, with no more shares than that share needs
+    (an item at its most cuts stays as long however short the others' shares are), and within the entries."""
+    rng = random.Random(5)
+    taken = clamped = 0
+    for _ in range(300):
+        n = rng.randint(38, 74)
+        tiles = [max(1, int(32 ** rng.random())) for _ in range(n)]
+        if rng.random() < 0.5:
+            tiles[rng.randrange(n)] = rng.randint(100, 2000)
+        entries = rng.choice([80, 111, 148])
+        one, _ = _shares(split_work(tiles, 74, entries, 32, 2))
+        two, live = _shares(split_work(tiles, 74, entries, 32, 2, second_round=True))
+        longest = lambda sp: max(-(-tiles[i] // k) for i, k in sp.items())                       # noqa: E731
+        assert len(live) <= entries and max(two.values()) <= 32 and all(k <= max(1, -(-tiles[i] // 2)) for i, k in two.items())
+        if two == one:
+            continue
+        taken += 1
+        clamped += max(two.values()) == 32
+        assert longest(two) + 0.5 < 0.75 * (longest(one) + 0.5)
+        assert len(live) == min(sum(min(32, -(-t // L)) for t in tiles) for L in range(2, max(tiles) + 1)
+                                if max(-(-t // min(32, -(-t // L))) for t in tiles) <= longest(two))
+    assert taken > 45 and clamped > 8
+
+
+def test_sequences_of_one_length_class_stay_in_one_round():
+    """A cut whose shares are hardly shorter than those of one round is not taken, whatever length was asked for."""
+    rng = random.Random(6)
+    for _ in range(200):
+        tiles = [rng.randint(16, 32) for _ in range(61)]
+        assert (split_work(tiles, 74, 111, 32, 2) == split_work(tiles, 74, 111, 32, 2, second_round=True)).all()
