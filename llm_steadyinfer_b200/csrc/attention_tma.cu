@@ -46,7 +46,8 @@ __device__ __forceinline__ unsigned movmatrix_trans(unsigned v) {
 template <int NH, int MT, int STAGES, bool SWAP>
 __global__ void __launch_bounds__(160, SWAP ? (NH == 1 ? 4 : 2) : 1)
 attn_decode_tma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap kmap,
-                       const __grid_constant__ CUtensorMap vmap, int log2_page, const int4* __restrict__ work) {
+                       const __grid_constant__ CUtensorMap vmap, int log2_page, const int4* __restrict__ work,
+                       int num_work) {
   constexpr int NWARPS = 4, THREADS = 128, BLOCK_N = 64, ROWS = 16 * MT, HS_PAD = NH * 64;   // consumer warps/threads
   constexpr int KT = HS_PAD / 16, DT = HS_PAD / 8;
   constexpr int TILE = NH * BLOCK_N * 64;             // elements of one K (or V) tile
@@ -62,13 +63,15 @@ attn_decode_tma_kernel(const AttnParams p, const __grid_constant__ CUtensorMap k
 
   // Until its pdl_wait() below no thread reads what the kernel before this one writes (the queries and the
   // newest keys and values): the work list, the items and the block table were copied in before it began.
-  // Which share of which item: with a work list, entry blockIdx.y = (item, split, splits of the item, first
-  // partial-result slot of the item), so that long sequences are cut into more shares than short ones, and
+  // Which share of which item: with a work list, entry blockIdx.y (65,535 on for each blockIdx.z) = (item, split, splits of the
+  // item, first partial-result slot of the item), so that long sequences are cut into more shares than short ones, and
   // head blockIdx.x: the longest shares of all heads start first, entries without work come last;
   // without one, item blockIdx.x, head blockIdx.y and split blockIdx.z of p.nsplit.
   int item_idx = blockIdx.x, split = blockIdx.z, nsplit = p.nsplit, slot0 = blockIdx.x * p.nsplit;
   if (work) {
-    const int4 w = work[blockIdx.y];
+    const int entry = blockIdx.y + blockIdx.z * 65535;
+    if (entry >= num_work) return;
+    const int4 w = work[entry];
     if (w.x < 0) return;                           // entries behind the step's last one
     item_idx = w.x; split = w.y; nsplit = w.z; slot0 = w.w;
   }
@@ -553,11 +556,10 @@ static int launch(const AttnParams& p, const CUtensorMap& km, const CUtensorMap&
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  if (work && num_work > 65535) return -2;
-  const dim3 grid = work ? dim3(p.KV, num_work, 1) : dim3(num_items, p.KV, p.nsplit);
+  const dim3 grid = work ? dim3(p.KV, num_work < 65535 ? num_work : 65535, (num_work + 65534) / 65535) : dim3(num_items, p.KV, p.nsplit);
   // (No early trigger: with one, the kernels behind it are resident beside it and a step of 8 sequences and 32 layers took 4.9 ms
   // instead of 3.3.)
-  si_launch(k, grid, dim3(160), smem, stream, p, km, vm, log2_page, work);
+  si_launch(k, grid, dim3(160), smem, stream, p, km, vm, log2_page, work, num_work);
   return si_last_error();
 }
 

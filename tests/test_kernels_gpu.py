@@ -605,6 +605,27 @@ def test_decode_with_shares_of_equal_length(H, KV, hs, page_size, window, budget
         assert (out.double().cpu() - want).abs().max().item() <= 2 ** -8 * vmax, turn
 
 
+def test_decode_with_more_work_entries_than_65535():
+    """A work list of any length: the entries with work first, the others leave. Outputs to the bit those of the short list."""
+    o = ops()
+    H, KV, hs, ps, lengths = 8, 2, 64, 16, [700, 3, 129]
+    if not o.attn_decode_tma_ok(H, KV, hs, ps):
+        pytest.skip("the TMA decode kernel does not take this layout")
+    seqs, table, kc, vc = build_cache(torch.bfloat16, lengths, H, KV, hs, ps, seed=5)
+    items = torch.tensor([(s, s, 1, n - 1) for s, n in enumerate(lengths)], dtype=torch.int32, device=DEV)
+    q = torch.stack([seqs[s][0][n - 1].reshape(-1) for s, n in enumerate(lengths)]).to(torch.bfloat16).to(DEV)
+    outs = []
+    for entries in (12, 65535, 70001):
+        work = torch.tensor(o.split_work([-(-n // 64) for n in lengths], 9, entries, 32, 2), dtype=torch.int32, device=DEV)
+        scratch = torch.zeros(o.attn_decode_tma_work_floats(entries, H, KV, hs), device=DEV)
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        outs.append(torch.full_like(q, float("nan")))
+        o.attn_decode_tma(q, kc.to(DEV), vc.to(DEV), table.to(DEV), items, outs[-1], ps, len(lengths), H, KV, hs, hs ** -0.5, work=work,
+                          scratch=scratch, status=status, max_rows=H // KV)
+        assert status.item() == 0
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and not torch.isnan(outs[0]).any()
+
+
 @pytest.mark.parametrize("tma", [False, True], ids=["cp_async", "tma"])
 def test_split_decode_shares_its_scratch_between_shapes(tma):
     """One scratch buffer serves launches with different numbers of items and splits, as the engine's does
