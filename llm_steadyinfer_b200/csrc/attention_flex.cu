@@ -508,6 +508,27 @@ SI_EXPORT long long si_attn_flex_scratch_floats(int num_items, int H, int KV, in
   return (long long)num_items * gy * nsplit * FLEX_M * (dv + 2);
 }
 
+// How a launch whose items have at most `max_rows` rows (0: unknown) goes about them, and the shared memory of a block without biases.
+struct FlexForm { int block_n, dvb, slices, ksplit, q_rows; size_t smem; };
+static FlexForm flex_form(int dk, int dv, bool own_v, int max_rows) {
+  FlexForm f;
+  const int pitch = (dk + 63) / 64 * 64, few = max_rows > 0 && max_rows <= 16;
+  f.block_n = pitch > 256 ? 32 : 64;                     // the two key stages and the queries share 227 KB
+  f.dvb = dv > 64 ? 128 : 64;
+  // few rows over keys that are their own values: the four warps take a value slice each instead of 16 rows each; few rows otherwise: a
+  // quarter of each tile's keys (tiles of 64 keys only)
+  f.slices = !own_v && dv > f.dvb && few;
+  f.ksplit = !f.slices && f.block_n == 64 && few;
+  f.q_rows = f.slices || f.ksplit ? 16 : FLEX_M;
+  f.smem = ((size_t)(f.q_rows + 2 * f.block_n) * pitch + (own_v ? (size_t)2 * f.block_n * f.dvb : 0)) * sizeof(bf16)
+           + (f.slices ? (size_t)4 * (f.block_n / 8) * 4 * 32 * sizeof(float) : 0);
+  return f;
+}
+// Blocks a multiprocessor that few rows' keys are cut for: three where shared memory has room for them, else two.
+SI_EXPORT int si_attn_flex_blocks(int dk, int dv, int own_v, int max_rows) {
+  return 3 * (flex_form(dk, dv, own_v != 0, max_rows).smem + 1024) <= 228 * 1024 ? 3 : 2;
+}
+
 template <int BLOCK_N, int DVB, int KSPLIT>
 static int flex_launch(const FlexParams& p, int dslices, size_t smem, cudaStream_t stream) {
   static size_t configured = 0;
@@ -559,27 +580,17 @@ SI_EXPORT int si_attn_flex(const void* q, long long q_stride, const void* k_cach
   p.part_o = scratch;
   p.part_ml = scratch ? scratch + slabs * FLEX_M * dv : nullptr;
   const bool own_v = v_cache != nullptr;
-  const int block_n = p.dk_pitch > 256 ? 32 : 64;        // the two key stages and the queries share 227 KB
-  const int dvb = dv > 64 ? 128 : 64;
-  const int dslices = (dv + dvb - 1) / dvb;
-  // items of at most 16 rows (max_rows, 0: unknown) over keys that are their own values: the four warps take a value
-  // slice each instead of 16 rows each
-  p.warps_are_slices = (!own_v && dslices > 1 && max_rows > 0 && max_rows <= 16) ? 1 : 0;
+  const FlexForm form = flex_form(dk, dv, own_v, max_rows);
+  const int block_n = form.block_n, dvb = form.dvb, dslices = (dv + dvb - 1) / dvb;
+  p.warps_are_slices = form.slices;
   const int zblocks = p.warps_are_slices ? (dslices + 3) / 4 : dslices;
-  // items of at most 16 rows otherwise: the four warps take a quarter of each tile's keys (tiles of 64 keys only)
-  const bool ksplit = !p.warps_are_slices && block_n == 64 && max_rows > 0 && max_rows <= 16;
-  const int q_rows = p.warps_are_slices || ksplit ? 16 : FLEX_M;
-  size_t smem = ((size_t)(q_rows + 2 * block_n) * p.dk_pitch + (own_v ? (size_t)2 * block_n * dvb : 0)) * sizeof(bf16);
+  size_t smem = form.smem;
   if (smem > 227 * 1024) return -2;
   const size_t bias_bytes = (size_t)2 * (block_n + FLEX_M / p.Gb) * p.Gb * sizeof(float);
   p.bias_in_smem = dist_bias && smem + bias_bytes <= 227 * 1024 ? 1 : 0;       // else each score fetches its own
   if (p.bias_in_smem) smem += bias_bytes;
-  if (p.warps_are_slices) {
-    smem += (size_t)4 * (block_n / 8) * 4 * 32 * sizeof(float);
-    if (smem > 227 * 1024) return -2;
-  }
   int rc;
-  if (ksplit) rc = dvb == 128 ? flex_launch<64, 128, 4>(p, zblocks, smem, stream) : flex_launch<64, 64, 4>(p, zblocks, smem, stream);
+  if (form.ksplit) rc = dvb == 128 ? flex_launch<64, 128, 4>(p, zblocks, smem, stream) : flex_launch<64, 64, 4>(p, zblocks, smem, stream);
   else if (block_n == 64) rc = dvb == 128 ? flex_launch<64, 128, 1>(p, zblocks, smem, stream) : flex_launch<64, 64, 1>(p, zblocks, smem, stream);
   else rc = dvb == 128 ? flex_launch<32, 128, 1>(p, zblocks, smem, stream) : flex_launch<32, 64, 1>(p, zblocks, smem, stream);
   if (rc) return rc;

@@ -1424,6 +1424,14 @@ def attn_flex_tokens(H: int, KV: int) -> int:
 
 
 @_of_sizes
+def attn_flex_blocks(dk: int, dv: int, own_v: bool, max_rows: int) -> int:
+    """Blocks a multiprocessor that items of at most ``max_rows`` rows have their keys cut for: three where it has room for them, else two."""
+    lib = build.load("attention_flex")
+    lib.si_attn_flex_blocks.restype = _c_int
+    return lib.si_attn_flex_blocks(_c_int(dk), _c_int(dv), _c_int(1 if own_v else 0), _c_int(max_rows))
+
+
+@_of_sizes
 def attn_flex_scratch_floats(num_items: int, H: int, KV: int, dv: int, nsplit: int) -> int:
     lib = build.load("attention_flex")
     lib.si_attn_flex_scratch_floats.restype = _c_llr

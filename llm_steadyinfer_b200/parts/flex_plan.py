@@ -16,7 +16,6 @@ from .base import first_visible_key
 
 MAX_SPLITS = 32
 MIN_KEYS_PER_SPLIT = 256
-BLOCKS_PER_SM = 3         # shares start with two tiles on their way; two blocks: a Nufasun pass of two requests 11.01 ms, three 10.94, four 11.03
 GEN_MIN_ROWS = 128        # rows (tokens x query heads of a key head) of a sequence from which on the tcgen05 prompt kernel serves it
 
 
@@ -65,7 +64,12 @@ def plan(ctx, device, H: int, KV: int, dk: int, dv: int, own_v: bool, window, sk
             slices = -(-slices // 4)                  # a block's four warps take a slice each
         per = KV * ((H // KV) // gb) * slices
         # keys that are their own values are wide (a latent): a tile is 32 of them, so a share may be half as many keys
-        nsplit = max(1, min(MAX_SPLITS if own_v else 2 * MAX_SPLITS, BLOCKS_PER_SM * ops.sm_count(device) // (len(dec) * per)))
+        # As many shares as blocks run at once. Where a multiprocessor has no room for three blocks, a cut for three begins a second round. Rows
+        # of 8,000 keys in us, the store of the newest keys before it, cut for two and for three: 16 rows of a latent of 576 with 16 heads 65.2,
+        # 83.9, 8 rows of one with 64 heads 230.8, 243.3; 8 rows of 2 x 256 with 8 heads 62.2, 85.0, of 4 x 192 with 16 heads 53.9, 71.1. Where
+        # three fit: 8 rows of 4 x 128 with 16 heads and biases 62.3, 50.1 (for four 64.1), of 2 x 128 that are their own values 25.8, 22.0 (28.8).
+        nsplit = max(1, min(MAX_SPLITS if own_v else 2 * MAX_SPLITS,
+                            ops.attn_flex_blocks(dk, dv, own_v, out["dec_rows"]) * ops.sm_count(device) // (len(dec) * per)))
         if not fixed:
             longest = max(d[3] + d[2] - first_visible_key(d[3], window, chunk) for d in dec)
             nsplit = min(nsplit, max(1, longest // MIN_KEYS_PER_SPLIT))

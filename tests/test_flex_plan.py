@@ -96,3 +96,19 @@ def test_a_layer_whose_scores_the_extended_form_does_not_know_gets_no_items_ther
     got = {ok: Attention._plan_general_tc05(layers[ok], ctx, 16) for ok in (first, not first)}
     assert got[False] == {"skip": frozenset(), "all": False, "items": None}
     assert got[True]["all"] and sum(n for _, _, n, _ in got[True]["items"].items()) == 400
+
+
+@pytest.mark.parametrize("H,KV,dk,dv,own_v,rows", [(16, 1, 576, 512, False, 16), (64, 1, 576, 512, False, 8), (8, 2, 256, 256, True, 8), (16, 4, 192, 128, True, 8),
+                                                   (16, 4, 128, 128, True, 8), (16, 2, 128, 128, False, 8), (32, 8, 64, 64, True, 4), (8, 2, 320, 128, True, 3)])
+def test_long_rows_are_cut_for_the_blocks_that_run_at_once(H, KV, dk, dv, own_v, rows):
+    """No more blocks than three a multiprocessor where its 228 KB hold three (two stages of keys and, where they are others, of values, the
+    query rows, the exchanged scores, 1 KB of the system's), two elsewhere; and no fewer than half of them."""
+    p = flex_plan.plan(Ctx([(1, 8000)] * rows), None, H, KV, dk, dv, own_v, None)
+    pitch, few = -(-dk // 64) * 64, p["dec_rows"] <= 16
+    tile, columns = 64 if pitch <= 256 else 32, 128 if dv > 64 else 64
+    slices = not own_v and few and dv > columns
+    q_rows = 16 if slices or (few and tile == 64) else 64
+    block = (q_rows + 2 * tile) * pitch * 2 + (2 * tile * columns * 2 if own_v else 0) + (tile * 256 if slices else 0) + 1024
+    most = (3 if 3 * block <= 228 * 1024 else 2) * 148
+    blocks = rows * p["nsplit"] * KV * (-(-dv // (4 * columns)) if slices else -(-dv // columns))
+    assert most // 2 < blocks <= most or p["nsplit"] == 31
