@@ -126,7 +126,8 @@ def test_swiglu_interleaved(dtype, T, F, group):
     assert (out.double().cpu() - want).abs().max().item() <= tol
 
 
-@pytest.mark.parametrize("M,F,K", [(1, 64, 96), (8, 1336, 320), (11, 40, 1000), (16, 256, 72)])
+@pytest.mark.parametrize("M,F,K", [(1, 64, 96), (8, 1336, 320), (11, 40, 1000), (16, 256, 72), (3, 4760, 2048), (8, 9600, 40), (12, 4760, 328),   # tiles in turn
+                                   (5, 1184, 2088), (13, 1176, 4104), (2, 8, 2056)])                                                             # sixteen warps a tile
 def test_gemm_skinny_swiglu(M, F, K):
     """The few-row gate/up product with the activation in its epilogue equals the product stored in bf16
     followed by the activation kernel."""
@@ -777,7 +778,9 @@ def test_gemm_skinny(M, N, K, out_dtype):
 
 
 @pytest.mark.parametrize("M,H,KV,hs,K,page_size", [(1, 4, 2, 64, 256, 16), (8, 32, 8, 128, 4096, 16), (16, 3, 1, 32, 96, 8),
-                                                   (11, 6, 3, 16, 136, 4), (5, 2, 2, 96, 320, 32)])
+                                                   (11, 6, 3, 16, 136, 4), (5, 2, 2, 96, 320, 32),
+                                                   (4, 59, 8, 128, 264, 16), (10, 64, 6, 128, 2048, 16),         # tiles in turn
+                                                   (3, 10, 4, 128, 2120, 16), (14, 12, 3, 128, 4104, 8)])        # sixteen warps a tile
 def test_gemm_skinny_qkv_rope(M, H, KV, hs, K, page_size):
     """The q/k/v product with the rotation and the cache store in its epilogue against the three kernels it
     stands for (product, then rotation and store): rotated q, and the pages of k and v, a padding row included."""
@@ -1346,7 +1349,8 @@ def test_pairs_that_name_an_expert_more_often_than_there_are_rows(T, ids):
 def test_shared_product_beside_the_experts(T, top, N, K, sN, sK, form):
     """The shared matrix's blocks in the experts' launch, from fewer column tiles than the experts have to many more: the experts' results to
     the bit what they are alone, the shared ones what the few-row product gives (its warps may be four: sums in another order, so a sum may
-    round to the neighbouring bf16 number, 2^-8, which the square of relu doubles and the last rounding adds to)."""
+    round to the neighbouring bf16 number, 2^-8, which the square of relu doubles and the last rounding adds to), and against float64: a sum
+    is off by its rounding, 2^-8 of it, which the form multiplies by its slope (a tenth more for its curve), and the result is rounded so."""
     g = torch.Generator().manual_seed(T + sN)
     o, E = ops(), 4
     rand = lambda *s: torch.randn(*s, generator=g).to(torch.bfloat16).to(DEV)                      # noqa: E731
@@ -1370,6 +1374,22 @@ def test_shared_product_beside_the_experts(T, top, N, K, sN, sK, form):
         o.gemm_skinny_glu_limited(sa, sw, bias, want, 0.9, 1.7)
     d = (got.double() - want.double()).abs()
     assert bool((d <= 2 ** -6 * want.double().abs() + 2 ** -7).all())
+    s = sa.double() @ sw.double().t()
+    gate, up = s.view(T, -1, 2, 8).unbind(2) if glu else (s, s)
+    gate, up = gate.reshape(T, -1), up.reshape(T, -1)
+    if form == "none":
+        exact, slope = s, s.abs()
+    elif form == "relu2":
+        exact, slope = s.clamp(min=0) ** 2, 2 * s.clamp(min=0) * s.abs()
+    else:
+        alpha, zg, zu = 1.0, gate, up
+        if form == "glu_limited":
+            b = bias.double().view(-1, 2, 8)
+            alpha, zg, zu = 1.7, (gate + b[:, 0].reshape(-1)).clamp(max=0.9), (up + b[:, 1].reshape(-1)).clamp(-0.9, 0.9) + 1.0
+        sig = torch.sigmoid(alpha * zg)
+        exact = zg * sig * zu
+        slope = (gate * zu).abs() * (sig * (1 + alpha * zg * (1 - sig))).abs() + (up * zg * sig).abs()
+    assert bool(((got.double() - exact).abs() <= 2 ** -8 * (1.1 * slope + exact.abs()) + 1e-4).all())
 
 
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
@@ -1390,7 +1410,7 @@ def test_pairs_tiles_of_fewer_columns(M, N, K, columns, out_dtype):
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 48, 8), (3, 40, 264), (8, 96, 1408), (9, 64, 1416), (16, 128, 2816), (8, 64, 5632), (2, 5000, 768),
-                                   (1, 9480, 8), (5, 9490, 2040), (8, 14300, 264), (9, 9490, 2056), (16, 5000, 72),      # tiles in turn
+                                   (1, 9480, 8), (5, 9490, 2040), (8, 14300, 264), (9, 9490, 2056), (16, 9490, 72),      # tiles in turn
                                    (2, 40, 2056), (8, 2368, 2088), (12, 2360, 4104), (1, 2376, 2056)])                  # sixteen warps a tile, and one tile too many
 def test_few_row_product_at_ragged_k(M, N, K):
     """The few-row product where k fills no whole round of a block's loads, against float64 (fp32 sums of K products)."""

@@ -298,8 +298,9 @@ def test_tensor_core_attention_sizes(H, KV, dk, dv, own_v):
                                                      (4, 1, 320, 264, False, 70)])
 def test_tensor_core_attention_shares_without_keys(H, KV, dk, dv, own_v, window):
     """Rows at the edges of key tiles with more shares than tiles: shares behind the last tile leave their partial results as they are (here
-    not a number), and the merge does not ask for them. Keys before a row's own are fetched before the wait for the kernel before. Both
-    sides round the same 32-bit result to 8 bits of mantissa, from weights rounded to as many: 2^-7 of values up to some 3."""
+    not a number), and the merge does not ask for them. Keys before a row's own are fetched before the wait for the kernel before, or behind
+    it. Against the plain kernel, where both sides round the same 32-bit result to 8 bits of mantissa, from weights rounded to as many: 2^-7
+    of values up to some 3; and against float64: 2^-7 of the largest value."""
     from llm_steadyinfer_b200.csrc import ops
     dev = "cuda:0"
     torch.manual_seed(dk)
@@ -315,12 +316,22 @@ def test_tensor_core_attention_shares_without_keys(H, KV, dk, dv, own_v, window)
     want, got = (torch.zeros(len(at), H * dv, dtype=torch.bfloat16, device=dev) for _ in range(2))
     ops.attention_general(q, kc, vc, table, seqs, pos, want, ps, 1, H, KV, dk, dv, dk ** -0.5, window, dist_bias=bias)
     items = torch.tensor([(0, r, 1, j) for r, j in enumerate(at)], dtype=torch.int32, device=dev)
+    keys, vals = k.double(), v.double() if own_v else k[..., :dv].double()
+    exact = torch.zeros(len(at), H, dv, dtype=torch.float64)
+    for r, j in enumerate(at):
+        first = max(0, j - window + 1) if window else 0
+        d = (j - torch.arange(first, j + 1)).clamp(max=39)
+        for h in range(H):
+            g = h // (H // KV)
+            s = keys[first:j + 1, g] @ q[r, h * dk:(h + 1) * dk].double().cpu() * dk ** -0.5 + bias.double().cpu()[d, h]
+            exact[r, h] = torch.softmax(s, 0) @ vals[first:j + 1, g]
     for nsplit in (2, 5, 32, 64):
         for ahead in (False, True):
             scratch = torch.full((ops.attn_flex_scratch_floats(len(at), H, KV, dv, nsplit),), float("nan"), device=dev)
             ops.attn_flex(q, kc, vc, table, items, got, ps, 1, H, KV, dk, dv, dk ** -0.5, window, dist_bias=bias, nsplit=nsplit, scratch=scratch,
                           max_rows=H // KV, ahead=ahead)
             assert (got.float() - want.float()).abs().max().item() <= 2e-2, (nsplit, ahead)
+            assert (got.double().cpu().view(len(at), H, dv) - exact).abs().max().item() <= 2 ** -7 * vals.abs().max().item(), (nsplit, ahead)
 
 
 @pytest.mark.parametrize("H,KV,dk,dv,own_v", [(16, 4, 128, 128, True), (16, 1, 576, 512, False)])

@@ -161,6 +161,39 @@ def test_graph_decode_logits(folders, plains, name):
     print(f"{name} graph decode: worst difference {worst:.2e}, batch sizes {sorted(buckets)}")
 
 
+@pytest.mark.parametrize("dst,src", [([0, 1, 2, 3, 4], [4, 0, 3, 1, 2]), ([0, 1, 2], [2, 2, 6]), ([4, 1], [0, 5]), ([3], [6]), ([], [])])
+@pytest.mark.parametrize("short", [True, False], ids=["short way", "general way"])
+def test_tokens_from_the_device_are_those_from_the_host(folders, monkeypatch, short, dst, src):
+    """Decode steps some or all of whose tokens lie on the device alone, direct and recorded, beside the same steps with the tokens given: the
+    same logits to the bit, by the short way through the preparation and by the general one."""
+    from llm_steadyinfer_b200.engine.step import ModelRunner, StepEntry
+    from llm_steadyinfer_b200.weights import load_model
+    if not short:
+        monkeypatch.setattr(ModelRunner, "_decode_rows", lambda self, entries: None)
+    cfg, _, page = CONFIGS["C"]
+    model = load_model(folders["C"], torch.bfloat16, "cuda:0")
+    lengths = [15, 16, 31, 100, 3]
+    prompts = [ru.random_tokens(cfg["vocab_size"], n, 60 + n) for n in lengths]
+    tokens = ru.random_tokens(cfg["vocab_size"], 7 * 4, 9)
+    logits = []
+    for fed in (False, True):
+        rn = ModelRunner(model, page_size=page, num_pages=64, max_requests=5, max_step_tokens=256)
+        for i, p in enumerate(prompts):
+            rn.step([StepEntry(i, p, [])])
+        rows = []
+        for turn in range(4):                             # twice directly, then recorded and replayed
+            ids = tokens[7 * turn:7 * turn + 7]
+            toks = [ids[i] for i in range(5)]
+            for d, s in zip(dst, src):
+                toks[d] = 0 if fed else ids[s]
+            entries = [StepEntry(i, [t], [0]) for i, t in enumerate(toks)]
+            feed = (torch.tensor(ids, dtype=torch.int32, device="cuda:0"), dst, src) if fed else None
+            rows.append((rn.step(entries, feed=feed) if turn < 2 else rn.step_decode_graph(entries, feed=feed)).clone())
+        rn.check_status()
+        logits.append(torch.stack(rows))
+    assert torch.equal(logits[0], logits[1])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["fp32", "bf16"])
 @pytest.mark.parametrize("name,seed", [("B", 1), ("C", 2), ("C", 3)])
 def test_random_serving_through_the_runner(folders, plains, name, seed, dtype):
