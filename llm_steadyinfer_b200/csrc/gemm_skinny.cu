@@ -73,8 +73,9 @@ __device__ __forceinline__ uint4 ld_cached(const bf16* p) {      // x: small, sh
   asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
-// Loads without a branch: what is not taken becomes zeros. Weights are read once and kept out of L1; not by the read-only path, whose loads the assembler
-// moves behind the wait for the kernel before where a loop around them uses the registers again (2,048 x 2,048, one row: 3.7 us so, 2.2 as it is).
+// Loads without a branch: what is not taken becomes zeros. Weights are read once and kept out of L1; by plain loads: with the read-only path's in
+// their place the kernel took 3.7 us, so 2.2 (2,048 x 2,048, one row, behind a launch), as if those loads waited for the kernel before. Loads
+// ahead of that wait in a loop are therefore plain ones.
 __device__ __forceinline__ uint4 ld_stream_if(const bf16* p, bool take) {
   uint4 v;
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"

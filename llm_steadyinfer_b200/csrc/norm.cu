@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(512) add_norm_general_vec_kernel(float* __rest
   __shared__ float scratch[33];
   if (trigger) pdl_trigger();
   const int nchunks = hidden >> 3;
-  if (gridDim.x <= 64) {
+  if (gridDim.x <= 64) {                                 // rows of a decode step; many rows find the weights in L2 (hints for all: no faster)
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
       const int ch = threadIdx.x + c * blockDim.x;

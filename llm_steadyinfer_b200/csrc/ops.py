@@ -679,7 +679,9 @@ def attn_decode_tma(q, k_cache, v_cache, block_table, items, out, page_size: int
                     hs: int, scale: float, window: int = 0, nsplit: int = 1, scratch=None, status=None,
                     max_rows: int = 0, work=None, chunk: int = 0, sink=None, vs: Optional[int] = None) -> None:
     """``attn_decode`` with the K/V tiles fetched by TMA (head_dim 64 or 128, page sizes 8 to 64);
-    items hold at most ``attn_decode_tma_rows // (H // KV)`` tokens. ``max_rows``: the most rows
+    items hold at most ``attn_decode_tma_rows // (H // KV)`` tokens, and an item all the rows that its sequence has in the
+    step: keys before its first position are read before the kernel before this one is waited for, like work list, items
+    and block table. ``max_rows``: the most rows
     (tokens x query heads of a KV head) of any item when the caller knows it (0: unknown); at most 8
     rows run the variant with the products taken the other way round.
     ``work`` (int32 [W, 4], rows of (item, split, splits of that item, first slot of that item); item -1:
@@ -2113,7 +2115,8 @@ def moe_gemm_pairs(a, ids, w, out, by_row: bool, act: str = "none", limit: float
     [T, top] that chose expert e, row = p / top (``by_row``: ``a`` [T, K]) or p (``a`` [T * top, K]). Pairs whose id is not below
     E are left alone; a row's choices are different experts (where they are not, the expert's weights are read again for what its tile has no room for). ``out`` and ``act`` as for ``moe_gemm``.
     ``shared`` {"a" [T, K'], "w" [N', K'], "out", "form" one of ``MOE_SHARED_FORMS``, "bias", "limit", "alpha"}: a product that every row
-    takes, in the same launch, as ``gemm_skinny`` and its gated forms (rows of w in groups of 8 gates and 8 ups) give it."""
+    takes, in the same launch, as ``gemm_skinny`` and its gated forms (rows of w in groups of 8 gates and 8 ups) give it; like theirs its
+    weights are read before the kernel before this one is waited for."""
     _cuda(a, ids, w, out)
     _i32(ids, "ids")
     _need(act in MOE_ACTS, f"moe_gemm_pairs: act {act!r} is not one of {sorted(MOE_ACTS)}")
