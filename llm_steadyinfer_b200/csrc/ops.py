@@ -572,10 +572,12 @@ def split_work(tiles, budget: int, entries: int, max_splits: int = 128, min_tile
     len(tiles)`` always suffices; more entries allow finer cuts when items outnumber the budget."""
     import numpy as np
     key = (tuple(tiles), budget, entries, max_splits, min_tiles, second_round)
-    if _split_memo.get("key") == key:               # tile counts change once in 64 decode steps of a sequence
-        return _split_memo["work"]
-    _split_memo["key"], _split_memo["work"] = key, _split_work(np, tiles, budget, entries, max_splits, min_tiles, second_round)
-    return _split_memo["work"]
+    last = _split_memo.get("last")                  # (key, work) in one object: another thread sees both or neither
+    if last is not None and last[0] == key:         # tile counts change once in 64 decode steps of a sequence
+        return last[1]
+    work = _split_work(np, tiles, budget, entries, max_splits, min_tiles, second_round)
+    _split_memo["last"] = (key, work)
+    return work
 
 
 _split_memo: dict = {}
@@ -2113,7 +2115,8 @@ def moe_gemm_pairs(a, ids, w, out, by_row: bool, act: str = "none", limit: float
                    shared=None) -> None:
     """The grouped product without a plan, for few pairs: out[p, :] = act(a[row, :] @ w[e]^T) for the pair p of ``ids`` int32
     [T, top] that chose expert e, row = p / top (``by_row``: ``a`` [T, K]) or p (``a`` [T * top, K]). Pairs whose id is not below
-    E are left alone; a row's choices are different experts (where they are not, the expert's weights are read again for what its tile has no room for). ``out`` and ``act`` as for ``moe_gemm``.
+    E are left alone; a row's choices are different experts (where they are not, the expert's weights are read again for what its tile
+    has no room for). ``out`` and ``act`` as for ``moe_gemm``.
     ``shared`` {"a" [T, K'], "w" [N', K'], "out", "form" one of ``MOE_SHARED_FORMS``, "bias", "limit", "alpha"}: a product that every row
     takes, in the same launch, as ``gemm_skinny`` and its gated forms (rows of w in groups of 8 gates and 8 ups) give it; like theirs its
     weights are read before the kernel before this one is waited for."""

@@ -3,6 +3,7 @@ import random
 
 import numpy as np
 
+from llm_steadyinfer_b200.csrc import ops
 from llm_steadyinfer_b200.csrc.ops import split_work
 
 
@@ -111,3 +112,23 @@ def test_sequences_of_one_length_class_stay_in_one_round():
     for _ in range(200):
         tiles = [rng.randint(16, 32) for _ in range(61)]
         assert (split_work(tiles, 74, 111, 32, 2) == split_work(tiles, 74, 111, 32, 2, second_round=True)).all()
+
+
+def test_a_second_thread_never_gets_another_call_s_cut(monkeypatch):
+    """The last cut is kept for the next step. Another engine's call that comes in while it is being stored gets its own cut."""
+    seen = []
+
+    class Store(dict):
+        def __setitem__(self, key, value):
+            super().__setitem__(key, value)
+            if not seen:
+                seen.append(None)
+                seen.append(split_work([128, 4], 37, 40, 32, 2))
+
+    monkeypatch.setattr(ops, "_split_memo", Store())
+    seen.append(None)
+    want = split_work([128, 4], 37, 40, 32, 2).copy()
+    split_work([3, 3, 3], 37, 40, 32, 2)
+    seen.clear()
+    split_work([128, 4], 37, 40, 32, 2)
+    assert len(seen) == 2 and (seen[1] == want).all()
